@@ -14,6 +14,7 @@
 // launch ahead of it before it touches memory, so activations and caches are read with plain loads, never through
 // the read-only path (only weights are).
 #include "bpdq_common.cuh"
+#include "gqa_attention.cuh"
 #include "launch.cuh"
 #include "../../include/bpdq.h"
 
@@ -284,7 +285,8 @@ __global__ void __launch_bounds__(256) k_kv_write(void* cache, const float* src,
     }
 }
 
-// One CTA per (query token, query head).  In the reference ALL n_kv cache rows take part: rows past
+// Contexts of up to 64 keys and the shapes that gqa_attention.cu leaves (head sizes other than 64 and 128, unaligned pointers):
+// one CTA per (query token, query head), sums in the reference's order.  In the reference ALL n_kv cache rows take part: rows past
 // the query's position score -1e38 and weigh exp(-huge) = 0, so they add exact zeros to the sum and to
 // the output (the cache holds finite values); they are skipped here, which leaves every bit as it is.
 // Scores: raw dot products (multiply, then add, in index order, one thread per cache row, the row read
@@ -411,6 +413,8 @@ static int launch_attn(const float* q, const void* kc, const void* vc, float* ds
 {
     const size_t sh = (size_t)(n_kv + D) * sizeof(float);
     if (sh > 200 * 1024) return BPDQ_ERR_RANGE;      // scores live in shared memory
+    const int other = gqa_attention(GqaShape{n_q, n_kv, H, HKV, D, scale, kv_offset, f16}, q, kc, vc, dst, s);
+    if (other != 1) return other;
     static bool attr_set[2][64] = {{false}};
     int dev = 0;
     cudaGetDevice(&dev);

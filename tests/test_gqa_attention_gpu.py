@@ -1,0 +1,82 @@
+"""Attention of the Q8_0 Llama over more than a few keys, through the C ABI, against 64-bit sums.
+
+Bound: the bar of fp32 results in this suite (1e-5 of the largest output).  A score adds up to 16 truncated tensor-core sums, each
+within 2^-23 of sum |q_d k_d| scale (about 7 for these inputs): 1.3e-5 for the worst row, a tenth of it on average."""
+import numpy as np
+import pytest
+
+from tests.util import Dev
+
+
+def expected(q, k, v, off, scale, n_kv):
+    """Scores, softmax and sums in binary64; query t sees keys 0 .. off + t."""
+    T, H, D = q.shape
+    rep = H // k.shape[1]
+    q, k, v = q.astype(np.float64), k.astype(np.float64), v.astype(np.float64)
+    out = np.empty((T, H, D))
+    for h in range(H):
+        s = q[:, h] @ k[:, h // rep].T * scale
+        s[np.arange(len(k))[None] >= np.minimum(off + 1 + np.arange(T), n_kv)[:, None]] = -np.inf
+        e = np.exp(s - s.max(axis=1, keepdims=True))
+        out[:, h] = (e / e.sum(axis=1, keepdims=True)) @ v[:, h // rep]
+    return out
+
+
+def attend(lib, q, k, v, off, scale, n_kv):
+    T, H, D = q.shape
+    d = [Dev(lib, a) for a in (q, k, v)]
+    out = Dev(lib, nbytes=q.nbytes + 64, fill=0xFF)
+    assert lib.bpd_gqa_attn_cuda(d[0].ptr, d[1].ptr, d[2].ptr, out.ptr, T, n_kv, H, k.shape[1], D, scale, off, int(k.dtype == np.float16), None) == 0
+    lib.bpdq_sync()
+    assert lib.bpdq_last_status() == 0
+    raw = out.read(np.uint8)
+    assert (raw[q.nbytes:] == 0xFF).all()
+    return raw[:q.nbytes].view(np.float32).reshape(q.shape)
+
+
+def inputs(T, S, H, HKV, D, kind, seed):
+    rng = np.random.default_rng(seed)
+    return (1.5 * rng.standard_normal((T, H, D), dtype=np.float32), rng.standard_normal((S, HKV, D), dtype=np.float32).astype(kind),
+            rng.standard_normal((S, HKV, D), dtype=np.float32).astype(kind))
+
+
+# queries, keys before them, heads, key heads, head size: contexts just beyond the short ones, at and around a block of 64 keys and
+# a cluster's stretches; one query and as many as a tile needs; heads per key head from 1 to 8, groups with heads left over
+SHAPES = [(1, 64, 8, 2, 64), (1, 127, 4, 4, 128), (1, 128, 6, 2, 128), (1, 1100, 8, 1, 128), (2, 700, 10, 2, 64), (3, 64, 4, 2, 64),
+          (65, 0, 32, 8, 128), (128, 0, 32, 32, 64), (129, 63, 24, 8, 128), (200, 1, 16, 2, 64), (700, 3, 8, 4, 64), (130, 500, 10, 2, 128)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,off,H,HKV,D", SHAPES)
+@pytest.mark.parametrize("kind", [np.float16, np.float32])
+def test_attention_against_64_bits(lib, T, off, H, HKV, D, kind):
+    q, k, v = inputs(T, off + T, H, HKV, D, kind, T + off)
+    q[0] *= 40.0                       # one row with a peaked softmax, one of zeros (all weights equal)
+    q[-1, 0] = 0.0
+    scale = np.float32(D ** -0.5)
+    got, want = attend(lib, q, k, v, off, scale, off + T), expected(q, k, v, off, float(scale), off + T)
+    assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+
+
+@pytest.mark.gpu
+def test_attention_never_reads_beyond_the_keys_that_count(lib):
+    """n_kv below the last query's position caps what it sees; rows behind are poison."""
+    q, k, v = inputs(100, 200, 8, 2, 128, np.float16, 1)
+    k[150:], v[150:] = np.nan, np.nan
+    got, want = attend(lib, q, k, v, 90, 0.1, 150), expected(q, k[:150], v[:150], 90, 0.1, 150)
+    assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+
+
+@pytest.mark.gpu
+def test_values_that_are_not_finite_reach_only_the_queries_that_see_them(lib):
+    """A prompt whose token 70 has an infinite value and token 90 a NaN key: earlier queries are as before, others carry it."""
+    T = 128
+    q, k, v = inputs(T, T, 32, 8, 128, np.float16, 2)
+    want = expected(q, k, v, 0, 0.1, T)
+    v[70, 3, 5], k[90, 1, 7] = np.inf, np.nan
+    got = attend(lib, q, k, v, 0, 0.1, T)
+    clean = np.ones(got.shape, bool)
+    clean[70:, 12:16, 5] = False
+    clean[90:, 4:8] = False
+    assert np.abs(got - want)[clean].max() <= 1e-5 * np.abs(want).max()
+    assert np.isposinf(got[70:, 12:16, 5]).all() and np.isnan(got[90:, 4:8]).all()
