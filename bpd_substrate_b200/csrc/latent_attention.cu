@@ -13,6 +13,7 @@
 //   k_latent_values        joins the splits and applies W_uv
 //   k_expanded_attn_mma    bf16 prompts: 64 queries of a head per CTA against expanded keys and values
 #include "latent_attention.cuh"
+#include "cluster_device.cuh"
 #include "launch.cuh"
 #include "mma_device.cuh"
 #include "../../include/bpdq.h"
@@ -514,18 +515,27 @@ __global__ void __launch_bounds__(256) k_latent_attn_rows(LatentShape p, const A
     }
 }
 
-// grid (value columns / 32, heads, tokens): joins the splits (every CTA of a head again; the sums sit in L2), then W_uv: a
-// warp per four value columns, whose weights are requested before the launch ahead has finished.
+// Threads that share a column of a CTA's slice, each with some of the splits.
+__host__ __device__ inline int latent_phases(int slice) { return slice >= 512 ? 2 : slice >= 256 ? 4 : 8; }
+
+// grid (heads, value columns / 32, tokens): joins the splits, then W_uv: a warp has four value columns, whose weights are requested
+// before the launch ahead has finished.  The CTAs of a head are a cluster where they are at most eight: each joins the splits of its
+// slice of the latent columns and hands the sums to the others.  Bound by the latency of reading the splits: 16 heads, 148 splits of 512
+// columns, 4 CTAs per head that each joined all of them (74 rounds of two threads per column): 20 us; a slice of 128 columns with
+// eight threads per column 14 us (a decoded token at 4000 keys, two such layers, 295 -> 283 us).
 template <typename A>
 __global__ void __launch_bounds__(256) k_latent_values(LatentShape p, float* partial, int splits, const bf16* __restrict__ w_uv, A* o,
                                                        const int* pos_p, int T)
 {
-    extern __shared__ __align__(16) float lat[];      // [2][rank_pad], then [splits] weights
-    float* sw = lat + 2 * p.rank_pad;
-    const int h = blockIdx.y, t = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    extern __shared__ __align__(16) float lat[];      // [rank_pad], then [phases][slice], then [splits] weights
+    const int ranks = (int)cluster_size(), slice = (p.rank_pad / 4 + ranks - 1) / ranks * 4, phases = latent_phases(slice);
+    float* part = lat + p.rank_pad;
+    float* sw = part + phases * slice;
+    const int h = blockIdx.x, t = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long row = (long)t * p.heads + h;
     pdl_launch_dependents();
-    const int c0 = blockIdx.x * 32 + 4 * warp;
+    if (ranks > 1) cluster_arrive();        // (everybody is there before anybody's shared memory is written)
+    const int c0 = blockIdx.y * 32 + 4 * warp;
     const bf16* w = w_uv + ((size_t)h * p.value_pad + c0) * p.rank_pad;
     uint4 u[4][2];                                     // the first 512 latent columns
 #pragma unroll
@@ -561,23 +571,36 @@ __global__ void __launch_bounds__(256) k_latent_values(LatentShape p, float* par
             if (lane + 32 * i < used) sw[lane + 32 * i] = st[i].x * inv;
     }
     __syncthreads();
-    // even and odd splits by the two halves of the CTA, four columns per thread
+    // this CTA's slice, four columns per thread
     const float* sums = partial_sums(partial, row, 0, splits, p.rank_pad);
-    for (int c = 4 * (tid & 127); c < p.rank_pad; c += 512) {
+    const int first = (int)cluster_rank() * slice, n = min(slice, p.rank_pad - first), lanes = 256 / phases, phase = tid / lanes;
+    for (int c = 4 * (tid % lanes); c < n; c += 4 * lanes) {
         float4 v = make_float4(0, 0, 0, 0);
 #pragma unroll 8
-        for (int i = tid >> 7; i < used; i += 2) {
+        for (int i = phase; i < used; i += phases) {
             const float f = sw[i];
-            const float4 a = *reinterpret_cast<const float4*>(sums + (size_t)i * p.rank_pad + c);
+            const float4 a = *reinterpret_cast<const float4*>(sums + (size_t)i * p.rank_pad + first + c);
             if (f != 0.0f) {                           // a split without keys for this row holds no sums
                 v.x = fmaf(f, a.x, v.x); v.y = fmaf(f, a.y, v.y); v.z = fmaf(f, a.z, v.z); v.w = fmaf(f, a.w, v.w);
             }
         }
-        *reinterpret_cast<float4*>(lat + (tid >> 7) * p.rank_pad + c) = v;
+        *reinterpret_cast<float4*>(part + phase * slice + c) = v;
     }
     __syncthreads();
-    for (int c = tid; c < p.rank_pad; c += 256) lat[c] += lat[p.rank_pad + c];
-    __syncthreads();
+    if (ranks > 1) cluster_wait();
+    for (int c = tid; c < n; c += 256) {
+        float v = part[c];
+        for (int i = 1; i < phases; i++) v += part[i * slice + c];
+        if (ranks == 1) lat[c] = v;
+        else
+            for (int r = 0; r < ranks; r++) store_peer(lat + first + c, r, v);
+    }
+    if (ranks > 1) {
+        cluster_arrive();
+        cluster_wait();
+    } else {
+        __syncthreads();
+    }
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     auto add = [&](const uint4& q, int k, float& v) {
         const float4 a = *reinterpret_cast<const float4*>(lat + k), b = *reinterpret_cast<const float4*>(lat + k + 4);
@@ -834,8 +857,10 @@ static int attend_latents(const LatentShape& p, const void* q, const bf16* w_ukv
     }
     if (rc) return rc;
     const bf16* w_uv = w_ukv + (size_t)p.heads * p.dim_pad * p.rank_pad;
-    return launch_ordered(k_latent_values<A>, dim3((p.value_pad + 31) / 32, p.heads, T), 256, (size_t)(2 * p.rank_pad + splits) * 4, s, p,
-                          b.partial, splits, w_uv, (A*)o, pos, T);
+    const unsigned parts = (p.value_pad + 31) / 32, ranks = parts <= 8 ? parts : 1;
+    const int slice = (p.rank_pad / 4 + (int)ranks - 1) / (int)ranks * 4;
+    return launch_cluster(k_latent_values<A>, dim3(p.heads, parts, T), dim3(1, ranks, 1), 256, (size_t)(p.rank_pad + latent_phases(slice) * slice + splits) * 4, s,
+                          p, b.partial, splits, w_uv, (A*)o, pos, T);
 }
 
 int latent_attention(const LatentShape& p, void* q, const bf16* w_ukv, const void* cache, void* o, const LatentBuffers& b, const int* pos,
