@@ -62,6 +62,8 @@ struct Workspace {
 // `bytes` of scratch for `kind`: from *ws when ws is given (BPDQ_ERR_RANGE if it does not fit), else the
 // library's block for (current device, s, kind).  Returns null and sets *status on failure.
 uint8_t* scratch_take(Workspace* ws, int kind, size_t bytes, cudaStream_t s, int* status);
+// Whether scratch_take would not refuse: enough left of the workspace, or a block that holds it, or a stream that may allocate one.
+bool scratch_fits(const Workspace* ws, int kind, size_t bytes, cudaStream_t s);
 
 // gemv_batch.cu: bulk-copy GEMV for Q8_0 weights (BPDQ_ERR_RANGE when the shape needs the generic kernel)
 int gemv_q8_0_fast(const uint8_t* W, const float* x, float* out, int N, int K, cudaStream_t s);

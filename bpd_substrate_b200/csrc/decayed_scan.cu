@@ -117,25 +117,39 @@ template <int NMAX>
 struct ChunkShape {
     static constexpr int kLdN = NMAX + 8, kLdV = 72, kLdO = 68;
     static constexpr size_t kQK = (size_t)kChunk * kLdN * 2, kV = (size_t)kChunk * kLdV * 2;
-    static constexpr size_t kSmem = 2 * (2 * kQK + kV) + 2 * kV + (size_t)kChunk * kLdO * 4 + 5 * kChunk * 4;
+    static constexpr size_t kO = (size_t)kChunk * kLdO * 4;
+    // the joined outputs of a chunk take the place of its queries, which nobody reads any more, where these are as large: two CTAs per SM
+    // for heads of 65 to 128 keys
+    static constexpr bool kOverQ = kQK >= kO;
+    static constexpr size_t kSmem = 2 * (2 * kQK + kV) + 2 * kV + (kOverQ ? 0 : kO) + 5 * kChunk * 4;
+    static constexpr int kPerSm = NMAX <= 128 ? 2 : 1;
 };
 
-// One CTA: one head, 64 value columns, all tokens.  Eight warps: value rows 16 (w & 3) .. + 15 of the transposed state
-// and half (w >> 2) of its keys.
-template <int NMAX>
-__global__ void __launch_bounds__(256, 1) k_decayed_chunks(DecayedScan a, int T)
+// A prompt's portion is cut into segments that run side by side: a first launch takes every segment but the last from a state of
+// zeros to what it adds, k_decayed_fold makes the segments' starting states of that, and a second launch works the segments out.
+struct ScanSegments {
+    int chunks;             // per segment
+    float* states;          // [segments][heads][key_pad][value_pad]: the state before a segment; null: one segment, from and to a.state
+    float* log_decay;       // [segments][heads]: of a whole segment
+};
+
+// One CTA: one head, 64 value columns, a segment's tokens.  Eight warps: value rows 16 (w & 3) .. + 15 of the transposed state
+// and half (w >> 2) of its keys.  Bound by the chain of barriers from chunk to chunk, so the chip wants many short chains: 2048 tokens
+// of 8 heads of 256 x 256 as one chain per CTA (32 CTAs) 272 us, of 64 heads of 128 x 64 (64 CTAs) 192 us; in four segments about 160 and 90 us with both launches and the fold.
+// STATE: only what the segment adds to a state of zeros.
+template <int NMAX, bool STATE>
+__global__ void __launch_bounds__(256, ChunkShape<NMAX>::kPerSm) k_decayed_chunks(DecayedScan a, int tokens, ScanSegments seg)
 {
     using S = ChunkShape<NMAX>;
     constexpr int LDN = S::kLdN, LDV = S::kLdV, LDO = S::kLdO;
     constexpr int NH = NMAX / 2, NTILES = NH / 8;
     extern __shared__ __align__(128) uint8_t smem[];
-    bf16* sQ[2] = {reinterpret_cast<bf16*>(smem), reinterpret_cast<bf16*>(smem + S::kQK)};
-    bf16* sK[2] = {reinterpret_cast<bf16*>(smem + 2 * S::kQK), reinterpret_cast<bf16*>(smem + 3 * S::kQK)};
-    bf16* sV[2] = {reinterpret_cast<bf16*>(smem + 4 * S::kQK), reinterpret_cast<bf16*>(smem + 4 * S::kQK + S::kV)};
+    auto sQ = [&](int b) { return reinterpret_cast<bf16*>(smem + b * S::kQK); };
+    auto sK = [&](int b) { return reinterpret_cast<bf16*>(smem + (2 + b) * S::kQK); };
+    auto sV = [&](int b) { return reinterpret_cast<bf16*>(smem + 4 * S::kQK + b * S::kV); };
     bf16* sPh = reinterpret_cast<bf16*>(smem + 4 * S::kQK + 2 * S::kV);
     bf16* sPl = sPh + kChunk * LDV;
-    float* sO = reinterpret_cast<float*>(smem + 4 * S::kQK + 4 * S::kV);
-    float* sL = sO + kChunk * LDO;                 // [2][64] cumulative log decay of a chunk, inclusive
+    float* sL = reinterpret_cast<float*>(smem + 4 * S::kQK + 4 * S::kV + (S::kOverQ ? 0 : S::kO));      // [2][64] cumulative log decay of a chunk, inclusive
     float* sDt = sL + 2 * kChunk;                  // [2][64]
     float* sW = sDt + 2 * kChunk;                  // [64] weight of a token in the chunk's final state
 
@@ -144,9 +158,11 @@ __global__ void __launch_bounds__(256, 1) k_decayed_chunks(DecayedScan a, int T)
     const int h = blockIdx.x, grp = h / (a.heads / a.groups), p0 = blockIdx.y * 64;
     const int p_n = a.value_pad - p0 < 64 ? a.value_pad - p0 : 64;
     const int Np = a.key_pad;
-    const bf16* gq = reinterpret_cast<const bf16*>(a.q) + grp * Np;
-    const bf16* gk = reinterpret_cast<const bf16*>(a.k) + grp * Np;
-    const bf16* gv = reinterpret_cast<const bf16*>(a.v) + h * a.value_pad + p0;
+    const int first = blockIdx.z * seg.chunks * kChunk, T = tokens - first < seg.chunks * kChunk ? tokens - first : seg.chunks * kChunk;
+    const bf16* gq = reinterpret_cast<const bf16*>(a.q) + (size_t)first * a.ld_q + grp * Np;
+    const bf16* gk = reinterpret_cast<const bf16*>(a.k) + (size_t)first * a.ld_k + grp * Np;
+    const bf16* gv = reinterpret_cast<const bf16*>(a.v) + (size_t)first * a.ld_v + h * a.value_pad + p0;
+    const float* gdt = a.dt ? a.dt + (size_t)first * a.ld_dt + h : nullptr;
     pdl_launch_dependents();
     // columns beyond the head's own sizes are never loaded: zero in both buffers
     for (size_t i = tid; i < (4 * S::kQK + 2 * S::kV) / 16; i += 256) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
@@ -162,21 +178,21 @@ __global__ void __launch_bounds__(256, 1) k_decayed_chunks(DecayedScan a, int T)
         for (int i = tid; i < kChunk * un; i += 256) {
             const int r = i / un, u = i - r * un, t = t0 + r;
             const int tc = t < T ? t : T - 1;
-            cp_async16(sQ[b] + r * LDN + 8 * u, gq + (size_t)tc * a.ld_q + 8 * u, t < T);
-            cp_async16(sK[b] + r * LDN + 8 * u, gk + (size_t)tc * a.ld_k + 8 * u, t < T);
+            if constexpr (!STATE) cp_async16(sQ(b) + r * LDN + 8 * u, gq + (size_t)tc * a.ld_q + 8 * u, t < T);
+            cp_async16(sK(b) + r * LDN + 8 * u, gk + (size_t)tc * a.ld_k + 8 * u, t < T);
         }
         for (int i = tid; i < kChunk * uv; i += 256) {
             const int r = i / uv, u = i - r * uv, t = t0 + r;
             const int tc = t < T ? t : T - 1;
-            cp_async16(sV[b] + r * LDV + 8 * u, gv + (size_t)tc * a.ld_v + 8 * u, t < T);
+            cp_async16(sV(b) + r * LDV + 8 * u, gv + (size_t)tc * a.ld_v + 8 * u, t < T);
         }
         cp_async_commit();
     };
     // lane i of warp 0 holds tokens 2 i and 2 i + 1 of a chunk
     auto dt_of = [&](int c, float& d0, float& d1) {
         const int t = c * kChunk + 2 * lane;
-        d0 = t < T ? (a.dt ? a.dt[(size_t)t * a.ld_dt + h] : 1.0f) : 0.0f;
-        d1 = t + 1 < T ? (a.dt ? a.dt[(size_t)(t + 1) * a.ld_dt + h] : 1.0f) : 0.0f;
+        d0 = t < T ? (gdt ? gdt[(size_t)t * a.ld_dt] : 1.0f) : 0.0f;
+        d1 = t + 1 < T ? (gdt ? gdt[(size_t)(t + 1) * a.ld_dt] : 1.0f) : 0.0f;
     };
     auto scan_decays = [&](float d0, float d1, int b) {
         const float l0 = a.dt ? rate * d0 : fixed * d0, l1 = a.dt ? rate * d1 : fixed * d1;    // no decay beyond the last token
@@ -194,13 +210,13 @@ __global__ void __launch_bounds__(256, 1) k_decayed_chunks(DecayedScan a, int T)
 
     // the state, transposed: rows p = 16 pw + .., columns n = NH half + ..
     float st[NTILES][4];
-    float* gs = a.state + (size_t)h * Np * a.value_pad + p0;
+    float* gs = (seg.states ? seg.states + ((size_t)blockIdx.z * a.heads + h) * Np * a.value_pad : a.state + (size_t)h * Np * a.value_pad) + p0;
 #pragma unroll
     for (int j = 0; j < NTILES; j++)
 #pragma unroll
         for (int e = 0; e < 4; e++) {
             const int n = half * NH + 8 * j + 2 * t4 + (e & 1), p = 16 * pw + g4 + 8 * (e >> 1);
-            st[j][e] = (n < Np && p < p_n) ? gs[(size_t)n * a.value_pad + p] : 0.0f;
+            st[j][e] = (!STATE && n < Np && p < p_n) ? gs[(size_t)n * a.value_pad + p] : 0.0f;
         }
 
     const int chunks = (T + kChunk - 1) / kChunk;
@@ -210,8 +226,10 @@ __global__ void __launch_bounds__(256, 1) k_decayed_chunks(DecayedScan a, int T)
         dt_of(0, d0, d1);
         scan_decays(d0, d1, 0);
     }
+    float whole = 0.0f;
     for (int c = 0; c < chunks; c++) {
         const int b = c & 1;
+        float* sO = reinterpret_cast<float*>(S::kOverQ ? smem + b * S::kQK : smem + 4 * S::kQK + 4 * S::kV);
         cp_async_wait_all();
         __syncthreads();                            // this chunk is here; everybody has left the other buffer
         float d0 = 0, d1 = 0;
@@ -222,8 +240,11 @@ __global__ void __launch_bounds__(256, 1) k_decayed_chunks(DecayedScan a, int T)
         const float* L = sL + b * kChunk;
         const float* Dt = sDt + b * kChunk;
         const float total = L[kChunk - 1];
+        whole += total;
         if (tid < kChunk) sW[tid] = expf(total - L[tid]) * Dt[tid];
 
+        float o[8][4] = {};
+        if constexpr (!STATE) {
         // ---- scores of the chunk: rows i = 16 pw .., columns j = 32 half ..; decay and mask in fp32
         {
             float acc[4][4] = {};
@@ -231,10 +252,10 @@ __global__ void __launch_bounds__(256, 1) k_decayed_chunks(DecayedScan a, int T)
             for (int kk = 0; kk < NMAX / 16; kk++) {
                 if (16 * kk >= Np) break;
                 uint32_t af[4], b0[4], b1[4];
-                ldsm4(af, sQ[b] + (16 * pw + (lane & 15)) * LDN + 16 * kk + 8 * (lane >> 4));
+                ldsm4(af, sQ(b) + (16 * pw + (lane & 15)) * LDN + 16 * kk + 8 * (lane >> 4));
                 const int jr = 32 * half + (lane & 7) + 8 * (lane >> 4), jc = 16 * kk + 8 * ((lane >> 3) & 1);
-                ldsm4(b0, sK[b] + jr * LDN + jc);
-                ldsm4(b1, sK[b] + (jr + 16) * LDN + jc);
+                ldsm4(b0, sK(b) + jr * LDN + jc);
+                ldsm4(b1, sK(b) + (jr + 16) * LDN + jc);
                 mma_bf16(acc[0], af, b0[0], b0[1]);
                 mma_bf16(acc[1], af, b0[2], b0[3]);
                 mma_bf16(acc[2], af, b1[0], b1[1]);
@@ -254,7 +275,6 @@ __global__ void __launch_bounds__(256, 1) k_decayed_chunks(DecayedScan a, int T)
                 }
         }
         // ---- what the state before the chunk gives: o^T[p][i] += S^T[p][n] q[i][n], then the decay up to token i
-        float o[8][4] = {};
 #pragma unroll
         for (int kk = 0; kk < NH / 16; kk++) {
             if (half * NH + 16 * kk >= Np) break;
@@ -266,7 +286,7 @@ __global__ void __launch_bounds__(256, 1) k_decayed_chunks(DecayedScan a, int T)
 #pragma unroll
             for (int ct = 0; ct < 8; ct += 2) {
                 uint32_t bq[4];
-                ldsm4(bq, sQ[b] + (8 * ct + (lane & 7) + 8 * (lane >> 4)) * LDN + half * NH + 16 * kk + 8 * ((lane >> 3) & 1));
+                ldsm4(bq, sQ(b) + (8 * ct + (lane & 7) + 8 * (lane >> 4)) * LDN + half * NH + 16 * kk + 8 * ((lane >> 3) & 1));
                 mma_bf16(o[ct], ah, bq[0], bq[1]);
                 mma_bf16(o[ct], al, bq[0], bq[1]);
                 mma_bf16(o[ct + 1], ah, bq[2], bq[3]);
@@ -278,13 +298,15 @@ __global__ void __launch_bounds__(256, 1) k_decayed_chunks(DecayedScan a, int T)
             const float e0 = expf(L[8 * ct + 2 * t4]), e1 = expf(L[8 * ct + 2 * t4 + 1]);
             o[ct][0] *= e0; o[ct][1] *= e1; o[ct][2] *= e0; o[ct][3] *= e1;
         }
+        }
         __syncthreads();                            // scores and sW are complete
+        if constexpr (!STATE) {
         // ---- the chunk's own tokens: o^T[p][i] += v[j][p] P[i][j], j in this warp's half
 #pragma unroll
         for (int kk = 0; kk < 2; kk++) {
             const int j0 = 32 * half + 16 * kk;
             uint32_t av[4];
-            ldsm4_t(av, sV[b] + (j0 + (lane & 7) + 8 * (lane >> 4)) * LDV + 16 * pw + 8 * ((lane >> 3) & 1));
+            ldsm4_t(av, sV(b) + (j0 + (lane & 7) + 8 * (lane >> 4)) * LDV + 16 * pw + 8 * ((lane >> 3) & 1));
 #pragma unroll
             for (int ct = 0; ct < 8; ct += 2) {
                 if (j0 > 8 * ct + 15) continue;     // later tokens only
@@ -304,6 +326,7 @@ __global__ void __launch_bounds__(256, 1) k_decayed_chunks(DecayedScan a, int T)
             if ((ct >> 2) != half)
 #pragma unroll
                 for (int e = 0; e < 4; e++) sO[(8 * ct + 2 * t4 + (e & 1)) * LDO + 16 * pw + g4 + 8 * (e >> 1)] = o[ct][e];
+        }
         // ---- the state after the chunk
         const float carry = expf(total);
 #pragma unroll
@@ -314,7 +337,7 @@ __global__ void __launch_bounds__(256, 1) k_decayed_chunks(DecayedScan a, int T)
         for (int kk = 0; kk < 4; kk++) {
             const int j0 = 16 * kk;
             uint32_t av[4], ah[4], al[4];
-            ldsm4_t(av, sV[b] + (j0 + (lane & 7) + 8 * (lane >> 4)) * LDV + 16 * pw + 8 * ((lane >> 3) & 1));
+            ldsm4_t(av, sV(b) + (j0 + (lane & 7) + 8 * (lane >> 4)) * LDV + 16 * pw + 8 * ((lane >> 3) & 1));
             const float w0 = sW[j0 + 2 * t4], w1 = sW[j0 + 2 * t4 + 1], w2 = sW[j0 + 2 * t4 + 8], w3 = sW[j0 + 2 * t4 + 9];
             split_bf16(bf_lo(av[0]) * w0, bf_hi(av[0]) * w1, ah[0], al[0]);
             split_bf16(bf_lo(av[1]) * w0, bf_hi(av[1]) * w1, ah[1], al[1]);
@@ -324,7 +347,7 @@ __global__ void __launch_bounds__(256, 1) k_decayed_chunks(DecayedScan a, int T)
             for (int j = 0; j < NTILES; j += 2) {
                 if (half * NH + 8 * j >= Np) break;
                 uint32_t bk[4];
-                ldsm4_t(bk, sK[b] + (j0 + (lane & 7) + 8 * ((lane >> 3) & 1)) * LDN + half * NH + 8 * j + 8 * (lane >> 4));
+                ldsm4_t(bk, sK(b) + (j0 + (lane & 7) + 8 * ((lane >> 3) & 1)) * LDN + half * NH + 8 * j + 8 * (lane >> 4));
                 mma_bf16(st[j], ah, bk[0], bk[1]);
                 mma_bf16(st[j], al, bk[0], bk[1]);
                 mma_bf16(st[j + 1], ah, bk[2], bk[3]);
@@ -332,6 +355,7 @@ __global__ void __launch_bounds__(256, 1) k_decayed_chunks(DecayedScan a, int T)
             }
         }
         if (warp == 0 && c + 1 < chunks) scan_decays(d0, d1, b ^ 1);
+        if constexpr (!STATE) {
         __syncthreads();                            // the other half's part is in sO
 #pragma unroll
         for (int ct = 0; ct < 8; ct++)
@@ -347,15 +371,24 @@ __global__ void __launch_bounds__(256, 1) k_decayed_chunks(DecayedScan a, int T)
             if (t < T && u < p_n) {
                 float4 v = *reinterpret_cast<const float4*>(sO + r * LDO + u);
                 if (a.d_skip) {
-                    const float4 x = act_load4(sV[b] + r * LDV + u);
+                    const float4 x = act_load4(sV(b) + r * LDV + u);
                     v.x = fmaf(skip, x.x, v.x); v.y = fmaf(skip, x.y, v.y); v.z = fmaf(skip, x.z, v.z); v.w = fmaf(skip, x.w, v.w);
                 }
                 uint2 w;
                 w.x = pack_bf16(v.x, v.y);
                 w.y = pack_bf16(v.z, v.w);
-                *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(a.o) + (size_t)t * a.ld_o + h * a.value_pad + p0 + u) = w;
+                *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(a.o) + (size_t)(first + t) * a.ld_o + h * a.value_pad + p0 + u) = w;
             }
         }
+        }
+    }
+    // the state after the segment: what it adds goes to the next one's place; the last one's is the sequence's
+    if (STATE) {
+        gs += (size_t)a.heads * Np * a.value_pad;
+        if (tid == 0 && blockIdx.y == 0) seg.log_decay[blockIdx.z * a.heads + h] = whole;
+    } else if (seg.states) {
+        if (blockIdx.z + 1 < gridDim.z) return;
+        gs = a.state + (size_t)h * Np * a.value_pad + p0;
     }
 #pragma unroll
     for (int j = 0; j < NTILES; j++)
@@ -377,21 +410,79 @@ static int launch_recurrence(const DecayedScan& a, int T, cudaStream_t s)
     return latch(BPDQ_ERR_RANGE);
 }
 
-template <int NMAX>
-static int launch_chunks(const DecayedScan& a, int T, cudaStream_t s)
+// states[0] = state, states[i + 1] = states[i] decayed over segment i, plus what that segment adds (which is there at the start).
+__global__ void __launch_bounds__(256) k_decayed_fold(const float* state, ScanSegments seg, int segments, int heads, int per_head)
 {
-    int rc = allow_smem<k_decayed_chunks<NMAX>>((int)ChunkShape<NMAX>::kSmem);
-    if (rc) return rc;
-    return launch_ordered(k_decayed_chunks<NMAX>, dim3(a.heads, (a.value_pad + 63) / 64), 256, ChunkShape<NMAX>::kSmem, s, a, T);
+    pdl_launch_dependents();
+    pdl_wait();
+    const int i = blockIdx.x * 256 + threadIdx.x, n = heads * per_head / 4;
+    if (i >= n) return;
+    const int h = 4 * i / per_head;
+    float4 s = reinterpret_cast<const float4*>(state)[i];
+    float4* at = reinterpret_cast<float4*>(seg.states) + i;
+    *at = s;
+#pragma unroll 4
+    for (int j = 1; j < segments; j++) {
+        const float d = expf(seg.log_decay[(j - 1) * heads + h]);
+        const float4 add = at[(size_t)j * n];
+        s = make_float4(fmaf(s.x, d, add.x), fmaf(s.y, d, add.y), fmaf(s.z, d, add.z), fmaf(s.w, d, add.w));
+        at[(size_t)j * n] = s;
+    }
 }
 
 // From this many tokens on a bf16 prompt goes through the chunked kernel.
 constexpr int kChunkedMinTokens = 24;
+constexpr int kMaxSegments = 16;
+
+// Segments of a portion, and chunks of each.  As many as there are CTAs to run at once; a chunk of the first launch takes about
+// half of the second's, and the fold with the launches as long as two chunks, so short portions stay one segment.
+static int scan_segments(int heads, int key_pad, int value_pad, int T, int* per_segment)
+{
+    const int chunks = (T + kChunk - 1) / kChunk, chains = heads * ((value_pad + 63) / 64);
+    int segments = sm_count() * (key_pad <= 128 ? 2 : 1) / chains;
+    if (segments > kMaxSegments) segments = kMaxSegments;
+    *per_segment = chunks;
+    if (segments < 2) return 1;
+    const int per = (chunks + segments - 1) / segments;
+    if (3 * per + 4 >= 2 * chunks) return 1;
+    *per_segment = per;
+    return (chunks + per - 1) / per;
+}
+
+static bool takes_chunks(int key_pad, int T, bool act_bf16) { return act_bf16 && T >= kChunkedMinTokens && key_pad <= 256; }
+
+size_t decayed_scratch_bytes(int heads, int key_pad, int value_pad, int T, bool act_bf16)
+{
+    if (!takes_chunks(key_pad, T, act_bf16)) return 0;
+    int per;
+    const int segments = scan_segments(heads, key_pad, value_pad, T, &per);
+    return segments < 2 ? 0 : (size_t)segments * heads * ((size_t)key_pad * value_pad + 1) * sizeof(float);
+}
+
+template <int NMAX>
+static int launch_chunks(const DecayedScan& a, int T, cudaStream_t s)
+{
+    constexpr size_t smem = ChunkShape<NMAX>::kSmem;
+    int rc = allow_smem<k_decayed_chunks<NMAX, false>>((int)smem);
+    if (rc) return rc;
+    const unsigned slices = (a.value_pad + 63) / 64;
+    ScanSegments seg = {(T + kChunk - 1) / kChunk, nullptr, nullptr};
+    int segments = 1;
+    if (a.scratch && (segments = scan_segments(a.heads, a.key_pad, a.value_pad, T, &seg.chunks)) > 1) {
+        const int per_head = a.key_pad * a.value_pad;
+        seg.states = (float*)a.scratch;
+        seg.log_decay = seg.states + (size_t)segments * a.heads * per_head;
+        if ((rc = allow_smem<k_decayed_chunks<NMAX, true>>((int)smem))) return rc;
+        if ((rc = launch_ordered(k_decayed_chunks<NMAX, true>, dim3(a.heads, slices, segments - 1), 256, smem, s, a, T, seg))) return rc;
+        if ((rc = launch_ordered(k_decayed_fold, (a.heads * per_head / 4 + 255) / 256, 256, 0, s, a.state, seg, segments, a.heads, per_head))) return rc;
+    }
+    return launch_ordered(k_decayed_chunks<NMAX, false>, dim3(a.heads, slices, segments), 256, smem, s, a, T, seg);
+}
 
 int decayed_scan(const DecayedScan& a, int T, bool act_bf16, cudaStream_t s)
 {
     if (a.heads < 1 || a.groups < 1 || a.heads % a.groups || a.key_pad % 16 || a.value_pad % 16 || T < 1) return latch(BPDQ_ERR_ARG);
-    if (act_bf16 && T >= kChunkedMinTokens && !a.rot_freq && a.key_pad <= 256) {
+    if (takes_chunks(a.key_pad, T, act_bf16) && !a.rot_freq) {
         if (a.key_pad <= 64) return launch_chunks<64>(a, T, s);
         if (a.key_pad <= 128) return launch_chunks<128>(a, T, s);
         return launch_chunks<256>(a, T, s);
@@ -739,6 +830,12 @@ int bpd_decayed_scan_cuda(const void* q, int ld_q, const void* k, int ld_k, cons
     a.d_skip = d_skip;
     a.state = state;
     a.o = o; a.ld_o = ld_o;
+    // one segment where a capture cannot allocate the states of several
+    const size_t scratch = decayed_scratch_bytes(heads, key_pad, value_pad, n_tokens, act_bf16 != 0);
+    if (scratch && !((uintptr_t)state & 15) && scratch_fits(nullptr, kScratchDelta, scratch, (cudaStream_t)stream)) {
+        int rc = 0;
+        if (!(a.scratch = scratch_take(nullptr, kScratchDelta, scratch, (cudaStream_t)stream, &rc))) return rc;
+    }
     return decayed_scan(a, n_tokens, act_bf16 != 0, (cudaStream_t)stream);
 }
 

@@ -23,7 +23,9 @@ struct DecayedScan {
     float* state;
     void* o;                            // activation type, [T][ld_o]
     int ld_o;
+    void* scratch;                      // decayed_scratch_bytes(), 16-byte aligned like state, or null: a long portion is one chain per head then
 };
+size_t decayed_scratch_bytes(int heads, int key_pad, int value_pad, int T, bool act_bf16);
 int decayed_scan(const DecayedScan& a, int T, bool act_bf16, cudaStream_t s);
 
 // Rotate-half rotary positions on q and k in place (`heads` heads of `dim_pad`, token t at *pos + t), k then times

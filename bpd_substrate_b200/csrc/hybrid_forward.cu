@@ -135,6 +135,9 @@ size_t lay_out(const Plan& p, Buffers& b, uint8_t* base, int T, int context, int
         if (l.mixer == BPDQ_MIX_MAMBA2) {
             grow(xbc, t * conv_channels(l));
             grow(dt, t * l.heads);
+            grow(chunks, decayed_scratch_bytes(l.heads, l.key_pad, l.value_pad, T, p.bf16_acts));
+        } else if (l.mixer == BPDQ_MIX_RETENTION) {
+            grow(chunks, decayed_scratch_bytes(l.heads, l.key_pad, l.value_pad, T, p.bf16_acts));
         } else if (l.mixer == BPDQ_MIX_DELTA) {
             grow(xbc, t * conv_channels(l));
             grow(dt, t * l.heads);
@@ -306,6 +309,7 @@ struct Runner {
         } else if ((rc = rotate_half_qk(b.u, at(b.u, HD), N, l.heads, l.key_pad, l.rot_dims, l.rot_freq, l.scale, b.pos, T, p.bf16_acts, s))) {
             return rc;
         }
+        a.scratch = b.chunks;
         if ((rc = decayed_scan(a, T, p.bf16_acts, s))) return rc;
         if ((rc = gated_norm(b.o, HV, at(b.u, 2 * HD + HV), N, nullptr, b.y, HV, l.heads, l.value_dim, l.value_pad, l.heads, 0, p.cfg.eps, T,
                              p.bf16_acts, s)))
@@ -336,6 +340,7 @@ struct Runner {
         a.d_skip = l.d_skip;
         a.state = (float*)(state + l.state_offset);
         a.o = b.o; a.ld_o = HV;
+        a.scratch = b.chunks;
         if ((rc = decayed_scan(a, T, p.bf16_acts, s))) return rc;
         if ((rc = gated_norm(b.o, HV, b.u, ld, l.norm_w, b.y, HV, l.heads, l.value_dim, l.value_pad, l.norm_groups, 1, p.cfg.eps, T, p.bf16_acts, s)))
             return rc;

@@ -76,6 +76,21 @@ std::vector<ScratchBlock> g_scratch;     // live blocks
 std::vector<void*> g_scratch_retired;    // replaced blocks: kept allocated, earlier launches and graphs may use them
 }  // namespace
 
+bool scratch_fits(const Workspace* ws, int kind, size_t bytes, cudaStream_t s)
+{
+    if (ws) return ws->base && (ws->used + 255) / 256 * 256 + ((256 - ((uintptr_t)ws->base & 255)) & 255) + bytes <= ws->bytes;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    {
+        std::lock_guard<std::mutex> lock(g_scratch_mutex);
+        for (auto& b : g_scratch)
+            if (!b.orphan && b.dev == dev && b.kind == kind && b.stream == s && b.cap >= bytes) return true;
+    }
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) (void)cudaGetLastError();
+    return cap == cudaStreamCaptureStatusNone;
+}
+
 uint8_t* scratch_take(Workspace* ws, int kind, size_t bytes, cudaStream_t s, int* status)
 {
     *status = 0;
