@@ -193,17 +193,22 @@ __global__ void __launch_bounds__(256) k_linear_tile(Linear l, int T)
 
 // ------------------------------------------------------------------ several tokens, bf16, tensor cores
 
+// BN: the most tokens of a tile; a launch takes bn of them, a multiple of 16 above BN / 2, and as many ring stages as fit then.
 template <int BN>
 struct Tc5Linear {
-    static constexpr int kRows = 128, kDepth = 64;                     // weight rows per tile, K elements per ring stage
-    static constexpr int kABytes = kRows * kDepth * 2, kBBytes = BN * kDepth * 2;
-    static constexpr int kStageBytes = kABytes + kBBytes;              // a multiple of 1024: the swizzle's atom
-    static constexpr int kStages = BN == 256 ? 4 : BN == 128 ? 6 : 8;
     static constexpr int kEpiWarps = 8;                                // two per TMEM lane quarter, each half of the columns
     static constexpr int kThreads = 32 * (2 + kEpiWarps);
     static constexpr int kTmemCols = 2 * BN;
-    static constexpr size_t kSmem = 1024 + (size_t)kStages * kStageBytes + 8 * (2 * kStages + 4) + 16;
 };
+constexpr int kTc5Rows = 128, kTc5Depth = 64;                          // weight rows per tile, K elements per ring stage
+constexpr int kTc5ABytes = kTc5Rows * kTc5Depth * 2, kTc5MaxStages = 8;
+__host__ __device__ constexpr int tc5_stage_bytes(int bn) { return kTc5ABytes + bn * kTc5Depth * 2; }      // a multiple of 1024: the swizzle's atom
+__host__ __device__ constexpr int tc5_stages(int bn)
+{
+    const int fit = 200 * 1024 / tc5_stage_bytes(bn);
+    return fit < kTc5MaxStages ? fit : kTc5MaxStages;
+}
+constexpr int tc5_smem(int bn) { return 1024 + tc5_stages(bn) * tc5_stage_bytes(bn) + 8 * (2 * kTc5MaxStages + 4) + 16; }
 
 // K-major operand in the 128-byte swizzle: 8-row groups 1024 bytes apart.
 __device__ __forceinline__ uint64_t swizzled_desc(uint32_t saddr)
@@ -221,20 +226,20 @@ __device__ __forceinline__ void umma_bf16_ss(uint32_t d_tmem, uint64_t adesc, ui
 
 template <int BN>
 __global__ void __launch_bounds__(Tc5Linear<BN>::kThreads, 1)
-k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, Linear l, int T, int* err)
+k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, Linear l, int T, int bn, int* err)
 {
     using S = Tc5Linear<BN>;
-    constexpr int kStages = S::kStages;
+    const int stages = tc5_stages(bn), stage_bytes = tc5_stage_bytes(bn);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* ring = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t* full = reinterpret_cast<uint64_t*>(ring + (size_t)kStages * S::kStageBytes);
-    uint64_t* empty = full + kStages;
-    uint64_t* acc_full = empty + kStages;      // [2]
+    uint64_t* full = reinterpret_cast<uint64_t*>(ring + (size_t)stages * stage_bytes);
+    uint64_t* empty = full + kTc5MaxStages;
+    uint64_t* acc_full = empty + kTc5MaxStages;      // [2]
     uint64_t* acc_empty = acc_full + 2;        // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
-        for (int s = 0; s < kStages; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < stages; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         for (int s = 0; s < 2; s++) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], S::kEpiWarps); }
         mbar_init_fence();
     }
@@ -249,40 +254,51 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
     const uint32_t tmem_base = *tmem_slot;
     pdl_launch_dependents();
 
-    const int n_tiles = (l.N + S::kRows - 1) / S::kRows, t_tiles = (T + BN - 1) / BN;
+    const int n_tiles = (l.N + kTc5Rows - 1) / kTc5Rows, t_tiles = (T + bn - 1) / bn;
     // tokens vary fastest: the CTAs at work share few rows of weights, which go through HBM once
-    const int tiles = n_tiles * t_tiles, kb_n = (l.K + S::kDepth - 1) / S::kDepth;
+    const int tiles = n_tiles * t_tiles, kb_n = (l.K + kTc5Depth - 1) / kTc5Depth;
 
     if (warp == 0) {
         // ---------------- producer: the weights of the first ring round are requested before the launch ahead has finished
         if (lane == 0) {
-            const int mine = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-            const long steps = (long)mine * kb_n;
-            auto weights = [&](long i, int s) {
-                const int tile = blockIdx.x + (int)(i / kb_n) * gridDim.x, kb = (int)(i % kb_n);
-                mbar_expect_tx(&full[s], S::kStageBytes);
-                tma_rows_2d(ring + (size_t)s * S::kStageBytes, &wmap, kb * S::kDepth, (tile / t_tiles) * S::kRows, &full[s]);
+            // two walks over the same (tile, K block)s, weights ahead of tokens by a ring round; counted, not divided out of a step's
+            // number: two 64-bit divisions per request held a K block of any width at 680 cycles
+            struct Walk { int tile, kb; };
+            Walk ww = {(int)blockIdx.x, 0}, wt = ww;
+            auto step = [&](Walk& w) {
+                if (++w.kb == kb_n) {
+                    w.kb = 0;
+                    w.tile += gridDim.x;
+                }
             };
-            auto tokens = [&](long i, int s) {
-                const int tile = blockIdx.x + (int)(i / kb_n) * gridDim.x, kb = (int)(i % kb_n);
-                tma_rows_2d(ring + (size_t)s * S::kStageBytes + S::kABytes, &xmap, kb * S::kDepth, (tile % t_tiles) * BN, &full[s]);
+            int row = (ww.tile / t_tiles) * kTc5Rows, tok = (wt.tile % t_tiles) * bn;
+            auto weights = [&](int s) {
+                mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
+                tma_rows_2d(ring + (size_t)s * stage_bytes, &wmap, ww.kb * kTc5Depth, row, &full[s]);
+                step(ww);
+                if (ww.kb == 0) row = (ww.tile / t_tiles) * kTc5Rows;
             };
-            const long ahead = steps < kStages ? steps : kStages;
-            for (long i = 0; i < ahead; i++) weights(i, (int)i);
+            auto tokens = [&](int s) {
+                tma_rows_2d(ring + (size_t)s * stage_bytes + kTc5ABytes, &xmap, wt.kb * kTc5Depth, tok, &full[s]);
+                step(wt);
+                if (wt.kb == 0) tok = (wt.tile % t_tiles) * bn;
+            };
+            int ahead = 0;
+            for (; ahead < stages && ww.tile < tiles; ahead++) weights(ahead);
             pdl_wait();
-            for (long i = 0; i < ahead; i++) tokens(i, (int)i);
+            for (int i = 0; i < ahead; i++) tokens(i);
             int s = 0;
             uint32_t par = 0;
-            for (long i = ahead; i < steps; i++) {
+            while (ww.tile < tiles) {
                 if (!mbar_wait_bounded(&empty[s], par, err, 41)) break;
-                weights(i, s);
-                tokens(i, s);
-                if (++s == kStages) { s = 0; par ^= 1u; }
+                weights(s);
+                tokens(s);
+                if (++s == stages) { s = 0; par ^= 1u; }
             }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer
-        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(S::kRows >> 4) << 24);
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kTc5Rows >> 4) << 24);
         int s = 0, local = 0;
         uint32_t full_par = 0;
         bool ok = true;
@@ -293,9 +309,9 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
             for (int kb = 0; kb < kb_n; kb++) {
                 if (!mbar_wait_bounded(&full[s], full_par, err, 43)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t stage = smem_addr(ring + (size_t)s * S::kStageBytes);
-                const uint64_t ad = swizzled_desc(stage), bd = swizzled_desc(stage + S::kABytes);
-                const int left = (l.K - kb * S::kDepth) / 16, k_n = left < 4 ? left : 4;
+                const uint32_t stage = smem_addr(ring + (size_t)s * stage_bytes);
+                const uint64_t ad = swizzled_desc(stage), bd = swizzled_desc(stage + kTc5ABytes);
+                const int left = (l.K - kb * kTc5Depth) / 16, k_n = left < 4 ? left : 4;
                 if (elect_one()) {
                     for (int k = 0; k < k_n; k++)
                         umma_bf16_ss(tmem_base + (uint32_t)(a * BN), ad + 2 * k, bd + 2 * k, idesc, (kb | k) ? 1u : 0u);
@@ -303,13 +319,13 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
                     if (kb + 1 == kb_n) umma_commit(&acc_full[a]);
                 }
                 __syncwarp();
-                if (++s == kStages) { s = 0; full_par ^= 1u; }
+                if (++s == stages) { s = 0; full_par ^= 1u; }
             }
         }
     } else {
         // ---------------- epilogue: a thread owns one weight row of the tile and walks over its tokens
         const int quarter = warp & 3, half = (warp - 2) >> 2;
-        constexpr int kCols = BN / 2;
+        const int split = (bn / 16 + 1) / 2 * 16, c_begin = half ? split : 0, c_end = half ? bn : split;
         const int r = 32 * quarter + lane;
         int local = 0;
         pdl_wait();
@@ -317,10 +333,10 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
             const int a = local & 1;
             if (!mbar_wait_bounded(&acc_full[a], (uint32_t)(local >> 1) & 1u, err, 44)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int n = (tile / t_tiles) * S::kRows + r;
-            const int tb = (tile % t_tiles) * BN + half * kCols;
+            const int n = (tile / t_tiles) * kTc5Rows + r;
+            const int tb = (tile % t_tiles) * bn;
             const bool live = n < l.N;
-            const uint32_t ta = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(a * BN + half * kCols);
+            const uint32_t ta = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(a * BN);
             DynTanh post = l.post, next = l.next;
             float pw = 0, pb = 0, nw = 0, nb = 0;
             if (l.mode == kLinResidual && live) {
@@ -336,7 +352,7 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
             const int n_end = (n - lane) + 32;
             const bool plain_warp = !((l.N | l.ld_out) & 1) &&
                                     (l.mode == kLinAct || l.mode == kLinGelu || (l.mode == kLinMixerIn && n_end <= l.dt_row && !l.conv.w));
-            for (int c0 = 0; c0 < kCols; c0 += 16) {
+            for (int c0 = c_begin; c0 < c_end; c0 += 16) {
                 int v[16];
                 tmem_ld(ta + c0, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -440,17 +456,31 @@ static int bf16_map(CUtensorMap* map, const void* p, int rows, int cols, int ld,
 }
 
 template <int BN>
-static int launch_tc5(const Linear& l, int T, cudaStream_t s)
+static int launch_tc5(const Linear& l, int T, int bn, cudaStream_t s)
 {
     using S = Tc5Linear<BN>;
     CUtensorMap wmap, xmap;
     int rc;
-    if ((rc = bf16_map(&wmap, l.W, l.N, l.K, l.K, S::kRows))) return rc;
-    if ((rc = bf16_map(&xmap, l.in, T, l.K, l.ld_in, BN))) return rc;
-    if ((rc = allow_smem<k_linear_tc5<BN>>((int)S::kSmem))) return rc;
-    const long tiles = (long)((l.N + S::kRows - 1) / S::kRows) * ((T + BN - 1) / BN);
+    if ((rc = bf16_map(&wmap, l.W, l.N, l.K, l.K, kTc5Rows))) return rc;
+    if ((rc = bf16_map(&xmap, l.in, T, l.K, l.ld_in, bn))) return rc;
+    if ((rc = allow_smem<k_linear_tc5<BN>>(227 * 1024))) return rc;
+    const long tiles = (long)((l.N + kTc5Rows - 1) / kTc5Rows) * ((T + bn - 1) / bn);
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
-    return launch_ordered(k_linear_tc5<BN>, grid, S::kThreads, S::kSmem, s, wmap, xmap, l, T, device_error_flag());
+    return launch_ordered(k_linear_tc5<BN>, grid, S::kThreads, tc5_smem(bn), s, wmap, xmap, l, T, bn, device_error_flag());
+}
+
+// Tokens of a tile: the multiple of 16 with the least time, in waves of CTAs over the SMs times a tile's time.
+static int tc5_tokens(const Linear& l, int T)
+{
+    const long n_tiles = (l.N + kTc5Rows - 1) / kTc5Rows, top = (T + 15) / 16 * 16 < 256 ? (T + 15) / 16 * 16 : 256;
+    int best = 16;
+    double least = 0.0;
+    for (int bn = 16; bn <= top; bn += 16) {
+        const long tiles = n_tiles * ((T + bn - 1) / bn);
+        const double time = (double)((tiles + sm_count() - 1) / sm_count()) * (double)(400 + bn);
+        if (bn == 16 || time <= least) { best = bn; least = time; }
+    }
+    return best;
 }
 
 int linear_forward(const Linear& l, int T, bool act_bf16, cudaStream_t s)
@@ -468,11 +498,11 @@ int linear_forward(const Linear& l, int T, bool act_bf16, cudaStream_t s)
         return act_bf16 ? launch_ordered(k_linear_vec<bf16>, grid, 256, smem, s, l) : launch_ordered(k_linear_vec<float>, grid, 256, smem, s, l);
     }
     if (!act_bf16) return launch_ordered(k_linear_tile, dim3((l.N + 63) / 64, (T + 63) / 64), 256, 0, s, l, T);
-    const long n_tiles = (l.N + 127) / 128;
-    if (T > 128 && n_tiles * ((T + 255) / 256) >= sm_count()) return launch_tc5<256>(l, T, s);
-    if (T > 64) return launch_tc5<128>(l, T, s);
-    if (T > 32) return launch_tc5<64>(l, T, s);
-    return launch_tc5<32>(l, T, s);
+    const int bn = tc5_tokens(l, T);
+    if (bn > 128) return launch_tc5<256>(l, T, bn, s);
+    if (bn > 64) return launch_tc5<128>(l, T, bn, s);
+    if (bn > 32) return launch_tc5<64>(l, T, bn, s);
+    return launch_tc5<32>(l, T, bn, s);
 }
 
 }  // namespace bpdq
