@@ -20,6 +20,20 @@ __device__ __forceinline__ bool mbar_wait_sleepy(uint64_t* bar, uint32_t parity,
     return false;
 }
 
+// Whether a phase is complete, without waiting.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo)
 {
     // K-major, no swizzle: start address, leading (K-chunk) and stride (8-row group) byte offsets
