@@ -28,15 +28,11 @@
 //              (row, token, block)
 // All mbarrier waits are bounded; on a timeout the role records an error code and leaves, the others
 // time out in turn, and warp 1 frees the tensor memory before it returns.
-#include "bpdq_common.cuh"
+#include "q8_0_tiles.cuh"
 #include "tcgen05_device.cuh"
 #include "../../include/bpdq.h"
 
 namespace bpdq {
-
-constexpr int kTileRows = 128;
-constexpr int kTileQuants = kTileRows * 32;              // 4096
-constexpr int kTileUnit = kTileRows * BPDQ_Q80_BYTES;    // 4352
 
 template <int T>
 struct Q8tShape {
@@ -378,6 +374,8 @@ int gemm_q8_0_tiles(const uint8_t* tiles, const float* X, float* out, int M, int
     if (M == 0 || N == 0) return 0;
     if (!tiles || !X || !out) return latch(BPDQ_ERR_ARG);
     if (((uintptr_t)tiles & 15) || ((uintptr_t)X & 15) || ((uintptr_t)out & 3)) return latch(BPDQ_ERR_ALIGN);
+    const int wide = gemm_q8_0_wide(1, &tiles, &out, &N, X, M, K, s, ws);
+    if (wide != kWideRefused) return wide;
     const int nb = K / 32;
     // Token tile: 16, 32 or 64, whichever needs the least time by a model of waves of CTAs over the SMs
     // times the measured cost of one block at that width (1 : 1.5 : 2.95); a narrower tile re-reads the
@@ -420,11 +418,13 @@ int gemm_q8_0_tiles(const uint8_t* tiles, const float* X, float* out, int M, int
     return rc ? latch(rc) : 0;
 }
 
-// scratch bytes of gemm_q8_0_tiles: 36 bytes per 32 activations, tokens padded to the widest token tile
+// scratch bytes of gemm_q8_0_tiles: 36 bytes per 32 activations (80 on the wide kernel), tokens padded to the widest token tile
 size_t gemm_q8_0_tiles_workspace(int M, int N, int K)
 {
     (void)N;
-    return (size_t)((M + 63) / 64) * (size_t)(K / 32) * 36 * 64 + 256;
+    const size_t narrow = (size_t)((M + 63) / 64) * (size_t)(K / 32) * 36 * 64;
+    const size_t wide = (size_t)((M + 127) / 128) * (size_t)(K / 32) * 80 * 128;
+    return (M >= kWideMinTokens ? wide : narrow) + 256;
 }
 
 }  // namespace bpdq

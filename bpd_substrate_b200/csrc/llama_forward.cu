@@ -16,6 +16,7 @@
 #include "bpdq_common.cuh"
 #include "gqa_attention.cuh"
 #include "launch.cuh"
+#include "q8_0_tiles.cuh"
 #include "../../include/bpdq.h"
 
 #include <cuda_fp16.h>
@@ -471,6 +472,13 @@ static int products_shared_input(int n, const uint8_t* const* Ws, const uint8_t*
                                  const float* x, int n_tokens, int K, cudaStream_t s, Workspace* ws)
 {
     if (n_tokens == 1 && gemv_q8_0_fast_multi(n, Ws, outs, Ns, x, K, s) == 0) return 0;
+    bool all = n_tokens >= kTilesMinTokens;
+    for (int j = 0; j < n; j++) all = all && Ts[j];
+    if (all) {
+        Workspace one = ws ? *ws : Workspace{nullptr, 0, 0};
+        const int rc = gemm_q8_0_wide(n, Ts, outs, Ns, x, n_tokens, K, s, ws ? &one : nullptr);
+        if (rc != kWideRefused) return rc;
+    }
     for (int j = 0; j < n; j++) {
         int rc = product(Ws[j], Ts[j], x, outs[j], n_tokens, Ns[j], K, s, ws);
         if (rc) return rc;
