@@ -53,7 +53,7 @@ Tuning& tuning();
 // Such a block only grows, and a block that has been handed out is never freed before the process
 // ends (a larger replacement is a new allocation; launches in flight and captured graphs that hold
 // the old address stay valid).  Growing is refused while the stream is being captured.
-enum ScratchKind { kScratchGemmActs = 0, kScratchTc5Acts, kScratchTc5Reduce, kScratchTilesActs, kScratchForward,
+enum ScratchKind { kScratchGemmActs = 0, kScratchTilesActs, kScratchForward,
                    kScratchQ4ktActs, kScratchQ4ktReduce, kScratchQ80Acts, kScratchLatent, kScratchDelta, kScratchKinds };
 struct Workspace {
     uint8_t* base;
@@ -89,6 +89,7 @@ size_t gemm_q4k_q8k_mma_workspace(int tokens, int K);
 int gemm_q4k_q8k_tc5(const uint8_t* W, const float* X, float* out, int tokens, int N, int K, cudaStream_t s,
                      Workspace* ws = nullptr, int32_t* sb_ints = nullptr);
 size_t gemm_q4k_q8k_tc5_workspace(int tokens, int N, int K);
+bool gemm_q4k_q8k_tc5_faster(int tokens, int N, int K);
 // gemm_q8_0_tiles.cu: tcgen05 product on re-tiled Q8_0 weights, out[m*N + n], the scalar reference's fp32 order
 int gemm_q8_0_tiles(const uint8_t* tiles, const float* X, float* out, int M, int N, int K, cudaStream_t s,
                     Workspace* ws = nullptr);

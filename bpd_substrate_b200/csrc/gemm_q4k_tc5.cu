@@ -29,6 +29,8 @@
 // All mbarrier waits are bounded; on a timeout the role records an error code and leaves, the
 // others time out in turn, and warp 13 frees the tensor memory before it returns.
 #include "bpdq_common.cuh"
+#include "cluster_device.cuh"
+#include "launch.cuh"
 #include "tcgen05_device.cuh"
 #include "../../include/bpdq.h"
 
@@ -39,16 +41,15 @@ namespace bpdq {
 
 constexpr int kRows = 128;
 constexpr int kMaxRawStages = 6, kMaxOpStages = 4, kSideSlots = 8;
+constexpr int kMaxSplits = 8;
 constexpr int kOpCols = 64;                        // TMEM columns of one A stage: lo plane 32 (4 sub-blocks x K=32 bytes), hi plane 32
 constexpr int kMinCols = 8;                        // one K=32 step: columns 0,1 = the eight mins, rest zero
 constexpr int kRowsBytes = kRows * BPDQ_Q4K_BYTES; // 18432
 
 struct Tc5Plan {
     int N, nb, tokens, npad;      // weight rows, super-blocks per row, valid / padded tokens (16, 32 or 64)
-    int n_tiles, grid, raw_stages;
-    int splits, sb_per_unit, n_units;   // K is cut into `splits` ranges of sb_per_unit super-blocks; unit = (tile, range)
-    float* partials;              // [splits][tokens][N] fp32, used when splits > 1
-    unsigned* arrivals;           // [n_tiles][2] units of a tile (and token half) that have stored their partial
+    int n_tiles, raw_stages;
+    int splits;                   // K is cut into `splits` ranges of super-blocks: a CTA per (row tile, range), a tile's are a cluster
     int act_bytes;                // scratch bytes per super-block: 324 * npad
     int raw_bytes;                // ring slot: rows + activations
     int off_raw, off_side, off_bar;
@@ -74,16 +75,13 @@ __device__ __forceinline__ unsigned long long tc5_timer()
 //   [32*npad]  bl plane, [32*npad] bh plane (K = 32 bytes per token, bytes 0..7 = sub-blocks 0..7, rest 0)
 //   [4*npad]   fp32 block scales
 __global__ void __launch_bounds__(256) k_quant_tc5_acts(const float* __restrict__ X, uint8_t* __restrict__ scratch,
-                                                        int tokens, int npad, int K, unsigned* __restrict__ arrivals,
-                                                        int n_arrivals)
+                                                        int tokens, int npad, int K)
 {
     // Programmatic launch on both sides: the product's CTAs may start their weight loads while this
     // kernel runs, and this kernel is resident before the launch ahead of it has finished, which it
     // waits for here because that launch may produce X and may still read the scratch.
     pdl_launch_dependents();
     pdl_wait();
-    // the split-K arrival counters of the product that follows start at zero
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n_arrivals; q += gridDim.x * blockDim.x) arrivals[q] = 0u;
     const int nb = K / 256;
     const int lane = threadIdx.x & 31;
     const long warp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -209,35 +207,22 @@ k_gemm_q4k_q8k_tc5(const __grid_constant__ CUtensorMap wmap, const uint8_t* __re
     const uint32_t tmem_base = *tmem_slot;
     pdl_launch_dependents();
     // Everything up to here, the weight loads of the first ring round and their transform overlap the
-    // activation quantizer launched just before this kernel: only what that kernel wrote (the
-    // activation blocks, the split-K counters) waits for it, in the producer and the epilogue warps.
+    // activation quantizer launched just before this kernel: only its activation blocks are waited for, by the producer.
 
-    const int my_units = (p.n_units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-    const int total_sb = my_units * p.sb_per_unit;   // super-blocks this CTA walks, over all its units
+    const int tile = blockIdx.x, split = blockIdx.y;
+    const int first_sb = split * p.nb / p.splits, total_sb = (split + 1) * p.nb / p.splits - first_sb;      // this CTA's super-blocks
+    // [NPAD][128] partial sums of a range, in a ring slot that is idle when they are complete: the last super-block is in another
+    float* part_sums = reinterpret_cast<float*>(raw + (size_t)(total_sb % kRawStages) * p.raw_bytes);
 
     if (warp == kProducerWarp) {
         // ---------------- producer
         if (lane == 0) {
-            // two walks over the same sequence of (tile, super-block): weights may run ahead of the
-            // activations by the ring's depth, and do so before the quantizer has finished
-            struct Walk { int q, unit, tile, b; };
-            auto start = [&]() { Walk w; w.q = 0; w.unit = blockIdx.x; w.tile = w.unit / p.splits; w.b = (w.unit - w.tile * p.splits) * p.sb_per_unit; return w; };
-            auto step = [&](Walk& w) {
-                w.b++;
-                if (++w.q == p.sb_per_unit) {
-                    w.q = 0;
-                    w.unit += gridDim.x;
-                    w.tile = w.unit / p.splits;
-                    w.b = (w.unit - w.tile * p.splits) * p.sb_per_unit;
-                }
-            };
-            Walk ww = start(), wa = start();
+            // weights run ahead of the activations by the ring's depth, and do so before the quantizer has finished
             const int ahead = total_sb < kRawStages ? total_sb : kRawStages;
             for (int i = 0; i < ahead; i++) {
                 mbar_expect_tx(&w_full[i], (uint32_t)kRowsBytes);
-                tma_rows_2d(raw + (size_t)i * p.raw_bytes, &wmap, ww.b * (BPDQ_Q4K_BYTES / 4), ww.tile * kRows, &w_full[i]);
+                tma_rows_2d(raw + (size_t)i * p.raw_bytes, &wmap, (first_sb + i) * (BPDQ_Q4K_BYTES / 4), tile * kRows, &w_full[i]);
                 TC5_TRACE(0, i);
-                step(ww);
             }
             pdl_wait();
             int s = 0;
@@ -247,13 +232,11 @@ k_gemm_q4k_q8k_tc5(const __grid_constant__ CUtensorMap wmap, const uint8_t* __re
                 if (i >= kRawStages) {
                     if (!mbar_wait_sleepy(&raw_empty[s], par, err, 11)) break;
                     mbar_expect_tx(&w_full[s], (uint32_t)kRowsBytes);
-                    tma_rows_2d(slot, &wmap, ww.b * (BPDQ_Q4K_BYTES / 4), ww.tile * kRows, &w_full[s]);
+                    tma_rows_2d(slot, &wmap, (first_sb + i) * (BPDQ_Q4K_BYTES / 4), tile * kRows, &w_full[s]);
                     TC5_TRACE(0, i);
-                    step(ww);
                 }
                 mbar_expect_tx(&a_full[s], (uint32_t)p.act_bytes);
-                bulk_g2s(slot + kRowsBytes, acts + (size_t)wa.b * p.act_bytes, (uint32_t)p.act_bytes, &a_full[s]);
-                step(wa);
+                bulk_g2s(slot + kRowsBytes, acts + (size_t)(first_sb + i) * p.act_bytes, (uint32_t)p.act_bytes, &a_full[s]);
                 if (++s == kRawStages) { s = 0; par ^= 1u; }
             }
         }
@@ -418,104 +401,55 @@ k_gemm_q4k_q8k_tc5(const __grid_constant__ CUtensorMap wmap, const uint8_t* __re
         const int r = 32 * (e & 3) + lane, c0 = pass * kEpiCols;
         const uint32_t lane_base = tmem_base + ((uint32_t)(32 * (e & 3)) << 16);
         float facc[kEpiCols];
-        int i = 0;
-        int* last_flag = reinterpret_cast<int*>(tmem_slot + 2) + pass;
-        pdl_wait();   // the quantizer zeroed the split-K counters
-        for (int ul = 0; ul < my_units; ul++) {
 #pragma unroll
-            for (int t = 0; t < kEpiCols; t++) facc[t] = 0.0f;
-            bool gave_up = false;
-            const int unit = blockIdx.x + ul * gridDim.x;
-            const int tile = unit / p.splits, split = unit - tile * p.splits;
-            const int rowg = tile * kRows + r;
-            for (int b = 0; b < p.sb_per_unit; b++, i++) {
-                const int a = kPasses == 2 ? pass : (i & 1);
-                const int use = kPasses == 2 ? i : (i >> 1);
-                if (!mbar_wait_sleepy(&acc_full[a], (uint32_t)use & 1u, err, 17)) { gave_up = true; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const float* sd = side + (size_t)(i % kSideSlots) * kSideFloats;
-                const float2 dd = *reinterpret_cast<const float2*>(sd + 2 * r);
-                const float d = dd.x, dmin = dd.y;
-                const uint32_t col0 = lane_base + (uint32_t)(a * 4) * kAccCols;
+        for (int t = 0; t < kEpiCols; t++) facc[t] = 0.0f;
+        bool gave_up = false;
+        const int rowg = tile * kRows + r;
+        for (int i = 0; i < total_sb; i++) {
+            const int a = kPasses == 2 ? pass : (i & 1);
+            const int use = kPasses == 2 ? i : (i >> 1);
+            if (!mbar_wait_sleepy(&acc_full[a], (uint32_t)use & 1u, err, 17)) { gave_up = true; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const float* sd = side + (size_t)(i % kSideSlots) * kSideFloats;
+            const float2 dd = *reinterpret_cast<const float2*>(sd + 2 * r);
+            const float d = dd.x, dmin = dd.y;
+            const uint32_t col0 = lane_base + (uint32_t)(a * 4) * kAccCols;
 #pragma unroll
-                for (int c = 0; c < kEpiCols / 8; c++) {
-                    int lo[8], hi[8], ml[8], mh[8];
-                    tmem_ld(col0 + 8 * c, lo);
-                    tmem_ld(col0 + kAccCols + 8 * c, hi);
-                    tmem_ld(col0 + 2 * kAccCols + 8 * c, ml);
-                    tmem_ld(col0 + 3 * kAccCols + 8 * c, mh);
-                    const float4 dA0 = *reinterpret_cast<const float4*>(sd + 256 + c0 + 8 * c);
-                    const float4 dA1 = *reinterpret_cast<const float4*>(sd + 256 + c0 + 8 * c + 4);
-                    const float dA[8] = {dA0.x, dA0.y, dA0.z, dA0.w, dA1.x, dA1.y, dA1.z, dA1.w};
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            for (int c = 0; c < kEpiCols / 8; c++) {
+                int lo[8], hi[8], ml[8], mh[8];
+                tmem_ld(col0 + 8 * c, lo);
+                tmem_ld(col0 + kAccCols + 8 * c, hi);
+                tmem_ld(col0 + 2 * kAccCols + 8 * c, ml);
+                tmem_ld(col0 + 3 * kAccCols + 8 * c, mh);
+                const float4 dA0 = *reinterpret_cast<const float4*>(sd + 256 + c0 + 8 * c);
+                const float4 dA1 = *reinterpret_cast<const float4*>(sd + 256 + c0 + 8 * c + 4);
+                const float dA[8] = {dA0.x, dA0.y, dA0.z, dA0.w, dA1.x, dA1.y, dA1.z, dA1.w};
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                    for (int t = 0; t < 8; t++) {
-                        const float v = d * (float)(8 * hi[t] + lo[t]) - dmin * (float)(64 * mh[t] + ml[t]);
-                        facc[8 * c + t] = fmaf(dA[t], v, facc[8 * c + t]);
-                    }
-                    if (p.ints && rowg < p.N) {
-#pragma unroll
-                        for (int t = 0; t < 8; t++)
-                            if (c0 + 8 * c + t < p.tokens)
-                                *reinterpret_cast<int2*>(p.ints + (((size_t)(c0 + 8 * c + t) * p.N + rowg) * p.nb + (split * p.sb_per_unit + b)) * 2) =
-                                    make_int2(8 * hi[t] + lo[t], 64 * mh[t] + ml[t]);
-                    }
+                for (int t = 0; t < 8; t++) {
+                    const float v = d * (float)(8 * hi[t] + lo[t]) - dmin * (float)(64 * mh[t] + ml[t]);
+                    facc[8 * c + t] = fmaf(dA[t], v, facc[8 * c + t]);
                 }
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&acc_empty[a]);
-                if (tid == 32 * kTransformWarps) TC5_TRACE(4, i);
-            }
-            if (gave_up) break;
-            if (p.splits == 1) {
-                if (rowg < p.N) {
+                if (p.ints && rowg < p.N) {
 #pragma unroll
-                    for (int t = 0; t < kEpiCols; t++)
-                        if (c0 + t < p.tokens) out[(size_t)(c0 + t) * p.N + rowg] = facc[t];
-                }
-            } else {
-                // split K: store this range's partial sums; the unit that arrives last adds the ranges in
-                // their fixed order 0, 1, ..., so the result does not depend on which one that was
-                if (rowg < p.N) {
-#pragma unroll
-                    for (int t = 0; t < kEpiCols; t++)
-                        if (c0 + t < p.tokens) __stcg(p.partials + ((size_t)split * p.tokens + (c0 + t)) * p.N + rowg, facc[t]);
-                }
-                __threadfence();
-                named_bar_sync(1 + pass, 128);
-                if ((e & 3) == 0 && lane == 0) {
-                    const unsigned before = atomicAdd(p.arrivals + 2 * tile + pass, 1u);
-                    *last_flag = (before == (unsigned)p.splits - 1u) ? 1 : 0;
-                }
-                named_bar_sync(1 + pass, 128);
-                const bool last = *last_flag != 0;
-                named_bar_sync(1 + pass, 128);   // everybody has read the flag before the next unit rewrites it
-                if (last) {
-                    __threadfence();
-                    if (rowg < p.N) {
-                        // four tokens x up to eight ranges of loads in flight, then the sums in range order
-#pragma unroll 1
-                        for (int t0 = 0; t0 < kEpiCols && c0 + t0 < p.tokens; t0 += 4) {
-                            float v[4][8];
-#pragma unroll
-                            for (int tt = 0; tt < 4; tt++)
-#pragma unroll
-                                for (int q = 0; q < 8; q++)
-                                    v[tt][q] = (q < p.splits && c0 + t0 + tt < p.tokens)
-                                                   ? __ldcg(p.partials + ((size_t)q * p.tokens + (c0 + t0 + tt)) * p.N + rowg)
-                                                   : 0.0f;
-#pragma unroll
-                            for (int tt = 0; tt < 4; tt++) {
-                                float sum = 0.0f;
-#pragma unroll
-                                for (int q = 0; q < 8; q++)
-                                    if (q < p.splits) sum += v[tt][q];
-                                if (c0 + t0 + tt < p.tokens) out[(size_t)(c0 + t0 + tt) * p.N + rowg] = sum;
-                            }
-                        }
-                    }
+                    for (int t = 0; t < 8; t++)
+                        if (c0 + 8 * c + t < p.tokens)
+                            *reinterpret_cast<int2*>(p.ints + (((size_t)(c0 + 8 * c + t) * p.N + rowg) * p.nb + (first_sb + i)) * 2) =
+                                make_int2(8 * hi[t] + lo[t], 64 * mh[t] + ml[t]);
                 }
             }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[a]);
+            if (tid == 32 * kTransformWarps) TC5_TRACE(4, i);
+        }
+        if (p.splits > 1) {
+#pragma unroll
+            for (int t = 0; t < kEpiCols; t++) part_sums[(c0 + t) * kRows + r] = facc[t];
+        } else if (!gave_up && rowg < p.N) {
+#pragma unroll
+            for (int t = 0; t < kEpiCols; t++)
+                if (c0 + t < p.tokens) out[(size_t)(c0 + t) * p.N + rowg] = facc[t];
         }
     }
     // ---------------- teardown: everybody meets, then the allocating warp frees tensor memory
@@ -524,6 +458,32 @@ k_gemm_q4k_q8k_tc5(const __grid_constant__ CUtensorMap wmap, const uint8_t* __re
     if (warp == kMmaWarp) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+    }
+    if (p.splits > 1) {
+        // the ranges of a tile: each CTA of the cluster adds up a share of the tokens, ranges in order 0, 1, ...  (Through memory, by the
+        // range that arrived last: 12 us of 26.7 at 4096 x 4096 and 64 tokens, which take 14.9 now; 4096 x 14336: 41.3, 28.0.)
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        constexpr int kShare = Tc5Shape<NPAD>::kThreads / kRows;      // tokens at a time
+        const int rowg = tile * kRows + tid % kRows, t_end = (split + 1) * p.tokens / p.splits;
+        if (tid < kShare * kRows && rowg < p.N)
+            for (int t = split * p.tokens / p.splits + tid / kRows; t < t_end; t += kShare) {
+                float v[kMaxSplits], sum = 0.0f;
+#pragma unroll
+                for (int q = 0; q < kMaxSplits; q++) {
+                    // (every range has its own number of super-blocks, and with it its own idle slot)
+                    const int blocks = (q + 1) * p.nb / p.splits - q * p.nb / p.splits;
+                    const float* from = reinterpret_cast<const float*>(raw + (size_t)(blocks % kRawStages) * p.raw_bytes);
+                    v[q] = q < p.splits ? load_peer(from + t * kRows + tid % kRows, q) : 0.0f;
+                }
+#pragma unroll
+                for (int q = 0; q < kMaxSplits; q++)
+                    if (q < p.splits) sum += v[q];
+                out[(size_t)t * p.N + rowg] = sum;
+            }
+        cluster_arrive();       // nobody leaves while its sums are read
+        cluster_wait();
     }
 }
 
@@ -551,29 +511,73 @@ static int tc5_weight_map(CUtensorMap* map, const uint8_t* W, int N, int nb)
     return r == CUDA_SUCCESS ? 0 : latch(BPDQ_ERR_CUDA - 900 - (int)r);
 }
 
+// Clusters of `ranges` CTAs that run at once (a CTA has an SM to itself).
 template <int NPAD>
-static int launch_tc5(const CUtensorMap& wmap, const uint8_t* acts, float* out, const Tc5Plan& p, cudaStream_t s)
+static int tc5_clusters(int ranges)
 {
-    auto kern = k_gemm_q4k_q8k_tc5<NPAD>;
-    static bool attr_set[64] = {false};
+    static int known[64][kMaxSplits + 1] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        if (rc) return rc;
-        attr_set[dev] = true;
-    }
+    if (dev >= 0 && dev < 64 && known[dev][ranges]) return known[dev][ranges];
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p.grid);
+    cfg.gridDim = dim3(1, (unsigned)ranges);
     cfg.blockDim = dim3(Tc5Shape<NPAD>::kThreads);
-    cfg.dynamicSmemBytes = p.smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = tuning().pdl ? 1 : 0;
-    return check_cuda(cudaLaunchKernelEx(&cfg, kern, wmap, acts, out, p, device_error_flag()));
+    cfg.dynamicSmemBytes = 200 * 1024;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = at.val.clusterDim.z = 1;
+    at.val.clusterDim.y = (unsigned)ranges;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_gemm_q4k_q8k_tc5<NPAD>, &cfg) != cudaSuccess) (void)cudaGetLastError();
+    if (n < 1) n = sm_count() / ranges;
+    if (dev >= 0 && dev < 64) known[dev][ranges] = n;
+    return n;
+}
+
+// Split K so that every SM has work and the per-CTA chain of super-blocks is short: the number of ranges (at least two
+// super-blocks each) with the fewest super-block steps on the busiest SM, charging each CTA two steps of set-up and a cluster two
+// for its sums.
+struct Tc5Split { int ranges; long steps; };
+template <int NPAD>
+static Tc5Split tc5_split(int n_tiles, int nb)
+{
+    Tc5Split best = {1, -1};
+    for (int sp = 1; sp <= kMaxSplits && (sp == 1 || nb / sp >= 2); sp++) {
+        const int at_once = tc5_clusters<NPAD>(sp);
+        const long steps = (long)((n_tiles + at_once - 1) / at_once) * ((nb + sp - 1) / sp + 2) + (sp > 1 ? 2 : 0);
+        if (best.steps < 0 || steps < best.steps) best = {sp, steps};
+    }
+    return best;
+}
+
+// Whether this kernel is faster than gemm_q4k_mma.cu's, by estimates of both (us) fitted to 10 shapes of 500 x 14336 to 20000 x 1024 and 4 to
+// 64 tokens.  There a warp walks whole rows: its time grows with their length, and with the rows beyond about 7500.  Measured sides of the line
+// (here, there; 16 tokens): 4096x4096 9.9, 15.0; 500x14336 11.2, 41.6; 14336x4096 16.5, 18.2; 8192x2048 10.0, 9.5; 20000x1024 11.8, 10.8.
+bool gemm_q4k_q8k_tc5_faster(int tokens, int N, int K)
+{
+    if (N < kRows) return false;
+    const int T = tokens < 64 ? tokens : 64, n_tiles = (N + kRows - 1) / kRows, nb = K / 256;
+    // (the limits that the number of clusters depends on)
+    if (allow_smem<k_gemm_q4k_q8k_tc5<16>>(227 * 1024) || allow_smem<k_gemm_q4k_q8k_tc5<32>>(227 * 1024) || allow_smem<k_gemm_q4k_q8k_tc5<64>>(227 * 1024))
+        return false;
+    const long steps = (T <= 16 ? tc5_split<16>(n_tiles, nb) : T <= 32 ? tc5_split<32>(n_tiles, nb) : tc5_split<64>(n_tiles, nb)).steps;
+    const double here = 4.0 + (T <= 16 ? 0.7 : T <= 32 ? 0.88 : 1.25) * (double)steps;
+    const double there = 3.7 + (T <= 8 ? 0.3 : T <= 32 ? 0.68 : 1.19) * nb * (N > 7500 ? N / 7500.0 : 1.0);
+    return here < there;
+}
+
+template <int NPAD>
+static int launch_tc5(const CUtensorMap& wmap, uint8_t* acts, const float* X, int K, float* out, Tc5Plan& p, cudaStream_t s)
+{
+    int rc = allow_smem<k_gemm_q4k_q8k_tc5<NPAD>>(227 * 1024);
+    if (rc) return rc;
+    p.splits = tc5_split<NPAD>(p.n_tiles, p.nb).ranges;
+    const long want = ((long)p.nb * NPAD + 7) / 8, cap = (long)sm_count() * 8;
+    if ((rc = launch_ordered(k_quant_tc5_acts, (unsigned)(want < cap ? want : cap), 256, 0, s, X, acts, p.tokens, NPAD, K))) return rc;
+    return launch_cluster(k_gemm_q4k_q8k_tc5<NPAD>, dim3((unsigned)p.n_tiles, (unsigned)p.splits), dim3(1, (unsigned)p.splits, 1), Tc5Shape<NPAD>::kThreads,
+                          p.smem, s, wmap, acts, out, p, device_error_flag());
 }
 
 // out[tokens][N], X fp32 [tokens][K], C-ABI nibble order; N >= 128 rows (the TMA box), up to 64 tokens per pass.
@@ -602,23 +606,6 @@ int gemm_q4k_q8k_tc5(const uint8_t* W, const float* X, float* out, int tokens, i
         p.ints = sb_ints ? sb_ints + (size_t)t0 * N * p.nb * 2 : nullptr;
         p.npad = T <= 16 ? 16 : (T <= 32 ? 32 : 64);
         p.n_tiles = (N + kRows - 1) / kRows;
-        // Split K so that every SM has work and the per-CTA chain of super-blocks is short: pick the
-        // number of ranges (a power of two dividing the super-blocks per row, at least two per range)
-        // with the fewest super-block steps on the busiest SM, charging each unit two steps of set-up.
-        p.splits = 1;
-        {
-            long best = -1;
-            for (int sp = 1; sp <= 8; sp *= 2) {
-                if (p.nb % sp != 0 || p.nb / sp < 2) break;
-                const long units = (long)p.n_tiles * sp;
-                const long waves = (units + sm_count() - 1) / sm_count();
-                const long cost = waves * (p.nb / sp + 2);
-                if (best < 0 || cost < best) { best = cost; p.splits = sp; }
-            }
-        }
-        p.sb_per_unit = p.nb / p.splits;
-        p.n_units = p.n_tiles * p.splits;
-        p.grid = p.n_units < sm_count() ? p.n_units : sm_count();
         p.act_bytes = 324 * p.npad;
         p.raw_bytes = (kRowsBytes + p.act_bytes + 127) / 128 * 128;
         size_t off = 0;
@@ -635,44 +622,22 @@ int gemm_q4k_q8k_tc5(const uint8_t* W, const float* X, float* out, int tokens, i
         // every pass of 64 tokens uses the same scratch: the quantizer waits for the pass before it
         Workspace pass_ws = ws ? *ws : Workspace{nullptr, 0, 0};
         int src = 0;
-        uint8_t* acts = scratch_take(ws ? &pass_ws : nullptr, kScratchTc5Acts, (size_t)p.nb * p.act_bytes, s, &src);
+        uint8_t* acts = scratch_take(ws ? &pass_ws : nullptr, kScratchGemmActs, (size_t)p.nb * p.act_bytes, s, &src);
         if (!acts) return src;
-        const size_t arrivals_bytes = ((size_t)p.n_tiles * 2 * sizeof(unsigned) + 255) / 256 * 256;
-        uint8_t* red = scratch_take(ws ? &pass_ws : nullptr, kScratchTc5Reduce,
-                                    arrivals_bytes + (p.splits > 1 ? (size_t)p.splits * T * N * sizeof(float) : 0), s, &src);
-        if (!red) return src;
-        p.arrivals = reinterpret_cast<unsigned*>(red);
-        p.partials = reinterpret_cast<float*>(red + arrivals_bytes);
-        const long units = (long)p.nb * p.npad;
-        long want = (units + 7) / 8, cap = (long)sm_count() * 8;
-        {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)(want < cap ? want : cap));
-            cfg.blockDim = dim3(256);
-            cfg.stream = s;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            at[0].val.programmaticStreamSerializationAllowed = 1;
-            cfg.attrs = at;
-            cfg.numAttrs = tuning().pdl ? 1 : 0;
-            rc = check_cuda(cudaLaunchKernelEx(&cfg, k_quant_tc5_acts, (const float*)(X + (size_t)t0 * K), acts, T, p.npad, K,
-                                               p.arrivals, p.n_tiles * 2));
-            if (rc) return rc;
-        }
         float* o = out + (size_t)t0 * N;
-        rc = p.npad == 16 ? launch_tc5<16>(wmap, acts, o, p, s) : (p.npad == 32 ? launch_tc5<32>(wmap, acts, o, p, s) : launch_tc5<64>(wmap, acts, o, p, s));
+        const float* x = X + (size_t)t0 * K;
+        rc = p.npad == 16 ? launch_tc5<16>(wmap, acts, x, K, o, p, s)
+                          : (p.npad == 32 ? launch_tc5<32>(wmap, acts, x, K, o, p, s) : launch_tc5<64>(wmap, acts, x, K, o, p, s));
         if (rc) return latch(rc);
     }
     return 0;
 }
 
-// scratch bytes of gemm_q4k_q8k_tc5 (an upper bound: widest token padding, eight K ranges)
+// scratch bytes of gemm_q4k_q8k_tc5
 size_t gemm_q4k_q8k_tc5_workspace(int tokens, int N, int K)
 {
-    const int T = tokens < 64 ? tokens : 64;
-    const int n_tiles = (N + kRows - 1) / kRows;
-    return (size_t)(K / 256) * 324 * 64 + 256 + ((size_t)n_tiles * 2 * sizeof(unsigned) + 255) / 256 * 256 +
-           (size_t)8 * T * N * sizeof(float) + 512;
+    (void)N;
+    return (size_t)(K / 256) * 324 * (tokens <= 16 ? 16 : tokens <= 32 ? 32 : 64) + 256;
 }
 
 }  // namespace bpdq

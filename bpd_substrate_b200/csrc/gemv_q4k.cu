@@ -581,15 +581,12 @@ int gemm_q4k_q8k(const uint8_t* W, const void* x, float* out, int tokens, int M,
                  int32_t* dbg, cudaStream_t s, Workspace* ws)
 {
     if (M < 0) return latch(BPDQ_ERR_ARG);
-    // many tokens: the weights would be streamed once per four tokens here; the tensor-core
-    // kernels read them once per 64.  Measured on 14336x4096, 4096x14336, 4096x4096 and 1024x4096:
-    // the tcgen05 kernel (128-row tiles, split K) is ahead from 24 tokens on matrices of 2^25
-    // weights and more (from 33 when there are fewer than 8192 rows), mma.sync everywhere else.
-    const bool large = (long)M * K >= (1L << 25);
-    // 3 and 4 tokens on such matrices: 13.3 / 18.6 us here (the dp4a work grows with the tokens)
-    // against 10.8 us for the mma.sync kernel; smaller matrices stay here (4096x4096: 9.0 against 10.2)
-    if (tokens > (large ? 2 : 4) && layout == BPDQ_LAYOUT_BPD && xsrc == 0 && !dbg) {
-        if (large && (tokens >= 33 || (tokens >= 24 && M >= 8192)))
+    // many tokens: the weights would be streamed once per four tokens here; the tensor-core kernels read them once per 64.  2 tokens
+    // stay here, 3 on matrices below 2^25 weights (13.3 us here against 10.8 above that), 4 on those of up to 2^22 (1024x4096: 7.1
+    // against 7.2; 4096x4096: 9.4 against 8.9; 20000x1024: 20.0 against 8.1).
+    const long weights = (long)M * K;
+    if (tokens > (weights >= (1L << 25) ? 2 : weights > (1L << 22) ? 3 : 4) && layout == BPDQ_LAYOUT_BPD && xsrc == 0 && !dbg) {
+        if (gemm_q4k_q8k_tc5_faster(tokens, M, K) && scratch_fits(ws, kScratchGemmActs, gemm_q4k_q8k_tc5_workspace(tokens, M, K), s))
             return gemm_q4k_q8k_tc5(W, reinterpret_cast<const float*>(x), out, tokens, M, K, s, ws);
         return gemm_q4k_q8k_mma(W, reinterpret_cast<const float*>(x), out, tokens, M, K, s, ws);
     }
