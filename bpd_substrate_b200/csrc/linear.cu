@@ -347,11 +347,18 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
         pdl_wait();
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, local++) {
             const int a = local & 1;
-            if (!mbar_wait_bounded(&acc_full[a], (uint32_t)(local >> 1) & 1u, err, 44)) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int n = (tile / t_tiles) * kTc5Rows + r;
             const int tb = (tile % t_tiles) * bn;
             const bool live = n < l.N;
+            // residual rows are fetched a step of 16 tokens ahead, the first under the tile's products
+            float xv[16];
+            auto fetch_x = [&](int c0) {
+#pragma unroll
+                for (int j = 0; j < 16; j++) xv[j] = (live && tb + c0 + j < T) ? l.x[(size_t)(tb + c0 + j) * l.ld_x + n] : 0.0f;
+            };
+            if (l.mode == kLinResidual && c_begin < c_end) fetch_x(c_begin);
+            if (!mbar_wait_bounded(&acc_full[a], (uint32_t)(local >> 1) & 1u, err, 44)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t ta = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(a * BN);
             DynTanh post = l.post, next = l.next;
             float pw = 0, pb = 0, nw = 0, nb = 0;
@@ -375,12 +382,13 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
                 const int t0 = tb + c0;
                 if (t0 >= T) continue;
                 if (l.mode == kLinResidual) {
-                    float xv[16];
+                    float xr[16];
 #pragma unroll
-                    for (int j = 0; j < 16; j++) xv[j] = (live && t0 + j < T) ? l.x[(size_t)(t0 + j) * l.ld_x + n] : 0.0f;
+                    for (int j = 0; j < 16; j++) xr[j] = xv[j];
+                    if (c0 + 16 < c_end) fetch_x(c0 + 16);
 #pragma unroll
                     for (int j = 0; j < 16; j++) {
-                        const float q = xv[j] + fmaf(tanhf(post.alpha * __int_as_float(v[j])), pw, pb);
+                        const float q = xr[j] + fmaf(tanhf(post.alpha * __int_as_float(v[j])), pw, pb);
                         if (live && t0 + j < T) {
                             l.x[(size_t)(t0 + j) * l.ld_x + n] = q;
                             if (next.w)
