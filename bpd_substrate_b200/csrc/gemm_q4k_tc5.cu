@@ -511,29 +511,33 @@ static int tc5_weight_map(CUtensorMap* map, const uint8_t* W, int N, int nb)
     return r == CUDA_SUCCESS ? 0 : latch(BPDQ_ERR_CUDA - 900 - (int)r);
 }
 
-// Clusters of `ranges` CTAs that run at once (a CTA has an SM to itself).
+// Clusters of 1 .. kMaxSplits CTAs that run at once on the current device (a CTA has an SM to itself).
+struct Tc5Clusters { int of[kMaxSplits + 1]; };
 template <int NPAD>
-static int tc5_clusters(int ranges)
+static const Tc5Clusters* tc5_clusters()
 {
-    static int known[64][kMaxSplits + 1] = {};
+    static Tc5Clusters known[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && known[dev][ranges]) return known[dev][ranges];
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1, (unsigned)ranges);
-    cfg.blockDim = dim3(Tc5Shape<NPAD>::kThreads);
-    cfg.dynamicSmemBytes = 200 * 1024;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = at.val.clusterDim.z = 1;
-    at.val.clusterDim.y = (unsigned)ranges;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_gemm_q4k_q8k_tc5<NPAD>, &cfg) != cudaSuccess) (void)cudaGetLastError();
-    if (n < 1) n = sm_count() / ranges;
-    if (dev >= 0 && dev < 64) known[dev][ranges] = n;
-    return n;
+    Tc5Clusters* c = &known[dev >= 0 && dev < 64 ? dev : 0];
+    if (c->of[1]) return c;
+    if (allow_smem<k_gemm_q4k_q8k_tc5<NPAD>>(227 * 1024)) return nullptr;
+    for (int ranges = kMaxSplits; ranges >= 1; ranges--) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1, (unsigned)ranges);
+        cfg.blockDim = dim3(Tc5Shape<NPAD>::kThreads);
+        cfg.dynamicSmemBytes = 200 * 1024;
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = at.val.clusterDim.z = 1;
+        at.val.clusterDim.y = (unsigned)ranges;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, k_gemm_q4k_q8k_tc5<NPAD>, &cfg) != cudaSuccess) (void)cudaGetLastError();
+        c->of[ranges] = n > 0 ? n : sm_count() / ranges;      // (of[1] last: it says that the others are known)
+    }
+    return c;
 }
 
 // Split K so that every SM has work and the per-CTA chain of super-blocks is short: the number of ranges (at least two
@@ -543,10 +547,10 @@ struct Tc5Split { int ranges; long steps; };
 template <int NPAD>
 static Tc5Split tc5_split(int n_tiles, int nb)
 {
+    const Tc5Clusters* at_once = tc5_clusters<NPAD>();
     Tc5Split best = {1, -1};
-    for (int sp = 1; sp <= kMaxSplits && (sp == 1 || nb / sp >= 2); sp++) {
-        const int at_once = tc5_clusters<NPAD>(sp);
-        const long steps = (long)((n_tiles + at_once - 1) / at_once) * ((nb + sp - 1) / sp + 2) + (sp > 1 ? 2 : 0);
+    for (int sp = 1; at_once && sp <= kMaxSplits && (sp == 1 || nb / sp >= 2); sp++) {
+        const long steps = (long)((n_tiles + at_once->of[sp] - 1) / at_once->of[sp]) * ((nb + sp - 1) / sp + 2) + (sp > 1 ? 2 : 0);
         if (best.steps < 0 || steps < best.steps) best = {sp, steps};
     }
     return best;
@@ -559,13 +563,11 @@ bool gemm_q4k_q8k_tc5_faster(int tokens, int N, int K)
 {
     if (N < kRows) return false;
     const int T = tokens < 64 ? tokens : 64, n_tiles = (N + kRows - 1) / kRows, nb = K / 256;
-    // (the limits that the number of clusters depends on)
-    if (allow_smem<k_gemm_q4k_q8k_tc5<16>>(227 * 1024) || allow_smem<k_gemm_q4k_q8k_tc5<32>>(227 * 1024) || allow_smem<k_gemm_q4k_q8k_tc5<64>>(227 * 1024))
-        return false;
     const long steps = (T <= 16 ? tc5_split<16>(n_tiles, nb) : T <= 32 ? tc5_split<32>(n_tiles, nb) : tc5_split<64>(n_tiles, nb)).steps;
-    const double here = 4.0 + (T <= 16 ? 0.7 : T <= 32 ? 0.88 : 1.25) * (double)steps;
-    const double there = 3.7 + (T <= 8 ? 0.3 : T <= 32 ? 0.68 : 1.19) * nb * (N > 7500 ? N / 7500.0 : 1.0);
-    return here < there;
+    const double here = 4.0 + (T <= 8 ? 0.7 : T <= 16 ? 0.74 : T <= 32 ? 0.88 : 1.25) * (double)steps;
+    const double rows = N > 7500 ? N / 7500.0 : T <= 8 ? 1.0 + N / 16000.0 : 1.0;
+    const double there = 3.7 + (T <= 8 ? 0.3 : T <= 32 ? 0.68 : 1.19) * nb * rows;
+    return steps > 0 && here < there;
 }
 
 template <int NPAD>

@@ -380,12 +380,13 @@ static int launch_wide(const WideProducts& p, const float* X, int K, cudaStream_
 // time of a tile of 4096 columns (us; narrow 14, 20.5 and 40 at 16, 32 and 64 tokens, here 23, 32 and 45 at 32, 64 and 128).
 static int wide_tokens(const WideProducts& p)
 {
+    const int sms = sm_count();
     auto least = [&](long row_tiles, const int (&widths)[3], const double (&us)[3], int* width) {
         double best = 0.0;
         for (int i = 0; i < 3; i++) {
             if (i > 0 && p.M <= widths[i - 1]) break;
             const long tiles = row_tiles * ((p.M + widths[i] - 1) / widths[i]);
-            const double t = (double)((tiles + sm_count() - 1) / sm_count()) * us[i];
+            const double t = (double)((tiles + sms - 1) / sms) * us[i];
             if (i == 0 || t <= best) { best = t; *width = widths[i]; }
         }
         return best;

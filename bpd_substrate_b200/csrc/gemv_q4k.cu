@@ -581,11 +581,13 @@ int gemm_q4k_q8k(const uint8_t* W, const void* x, float* out, int tokens, int M,
                  int32_t* dbg, cudaStream_t s, Workspace* ws)
 {
     if (M < 0) return latch(BPDQ_ERR_ARG);
-    // many tokens: the weights would be streamed once per four tokens here; the tensor-core kernels read them once per 64.  2 tokens
-    // stay here, 3 on matrices below 2^25 weights (13.3 us here against 10.8 above that), 4 on those of up to 2^22 (1024x4096: 7.1
-    // against 7.2; 4096x4096: 9.4 against 8.9; 20000x1024: 20.0 against 8.1).
+    // many tokens: the weights would be streamed once per four tokens here, the tensor-core kernels read them once per 64.  The first of
+    // these many, by what a token costs here (us here, there): 2 tokens on many short rows (20000x1024: 11.2, 8.1; 14336x4096: 11.3, 12.5),
+    // 3 on 2^25 weights or 8192 rows (14336x4096: 13.3, 10.8; 8192x2048: 7.6, 6.6), 4 beyond 2^22 weights (4096x4096: 9.4, 8.9), else 5
+    // (1024x4096, 4 tokens: 7.1, 7.2).
     const long weights = (long)M * K;
-    if (tokens > (weights >= (1L << 25) ? 2 : weights > (1L << 22) ? 3 : 4) && layout == BPDQ_LAYOUT_BPD && xsrc == 0 && !dbg) {
+    const int many = M >= 14336 && K <= 2048 ? 2 : weights >= (1L << 25) || M >= 8192 ? 3 : weights > (1L << 22) ? 4 : 5;
+    if (tokens >= many && layout == BPDQ_LAYOUT_BPD && xsrc == 0 && !dbg) {
         if (gemm_q4k_q8k_tc5_faster(tokens, M, K) && scratch_fits(ws, kScratchGemmActs, gemm_q4k_q8k_tc5_workspace(tokens, M, K), s))
             return gemm_q4k_q8k_tc5(W, reinterpret_cast<const float*>(x), out, tokens, M, K, s, ws);
         return gemm_q4k_q8k_mma(W, reinterpret_cast<const float*>(x), out, tokens, M, K, s, ws);

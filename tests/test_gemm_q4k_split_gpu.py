@@ -21,7 +21,7 @@ def test_uneven_ranges(lib, oracle, T, N, K):
 
 
 # both sides of the dispatcher's lines: 2 to 4 tokens, short and long rows, few and many of them
-@pytest.mark.parametrize("T,N,K", [(3, 1024, 4352), (4, 1024, 4096), (4, 1024, 4352), (9, 512, 8192), (16, 8192, 512), (33, 260, 2048), (70, 300, 1024)])
+@pytest.mark.parametrize("T,N,K", [(3, 1024, 4352), (4, 1024, 4096), (4, 1024, 4352), (2, 14336, 512), (9, 512, 8192), (16, 8192, 512), (33, 260, 2048), (70, 300, 1024)])
 def test_dispatcher(lib, oracle, T, N, K):
     rng = np.random.default_rng(T * N + K)
     W, X = synth.q4k_matrix(N, K, rng), synth.activations(K, rng, rows=T)
