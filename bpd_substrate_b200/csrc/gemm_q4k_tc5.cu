@@ -41,7 +41,7 @@ namespace bpdq {
 
 constexpr int kRows = 128;
 constexpr int kMaxRawStages = 6, kMaxOpStages = 4, kSideSlots = 8;
-constexpr int kMaxSplits = 8;
+constexpr int kMaxSplits = 8;                      // CTAs of a portable cluster
 constexpr int kOpCols = 64;                        // TMEM columns of one A stage: lo plane 32 (4 sub-blocks x K=32 bytes), hi plane 32
 constexpr int kMinCols = 8;                        // one K=32 step: columns 0,1 = the eight mins, rest zero
 constexpr int kRowsBytes = kRows * BPDQ_Q4K_BYTES; // 18432
@@ -511,35 +511,6 @@ static int tc5_weight_map(CUtensorMap* map, const uint8_t* W, int N, int nb)
     return r == CUDA_SUCCESS ? 0 : latch(BPDQ_ERR_CUDA - 900 - (int)r);
 }
 
-// Clusters of 1 .. kMaxSplits CTAs that run at once on the current device (a CTA has an SM to itself).
-struct Tc5Clusters { int of[kMaxSplits + 1]; };
-template <int NPAD>
-static const Tc5Clusters* tc5_clusters()
-{
-    static Tc5Clusters known[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    Tc5Clusters* c = &known[dev >= 0 && dev < 64 ? dev : 0];
-    if (c->of[1]) return c;
-    if (allow_smem<k_gemm_q4k_q8k_tc5<NPAD>>(227 * 1024)) return nullptr;
-    for (int ranges = kMaxSplits; ranges >= 1; ranges--) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(1, (unsigned)ranges);
-        cfg.blockDim = dim3(Tc5Shape<NPAD>::kThreads);
-        cfg.dynamicSmemBytes = 200 * 1024;
-        cudaLaunchAttribute at;
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = at.val.clusterDim.z = 1;
-        at.val.clusterDim.y = (unsigned)ranges;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, k_gemm_q4k_q8k_tc5<NPAD>, &cfg) != cudaSuccess) (void)cudaGetLastError();
-        c->of[ranges] = n > 0 ? n : sm_count() / ranges;      // (of[1] last: it says that the others are known)
-    }
-    return c;
-}
-
 // Split K so that every SM has work and the per-CTA chain of super-blocks is short: the number of ranges (at least two
 // super-blocks each) with the fewest super-block steps on the busiest SM, charging each CTA two steps of set-up and a cluster two
 // for its sums.
@@ -547,10 +518,10 @@ struct Tc5Split { int ranges; long steps; };
 template <int NPAD>
 static Tc5Split tc5_split(int n_tiles, int nb)
 {
-    const Tc5Clusters* at_once = tc5_clusters<NPAD>();
+    const int* at_once = active_clusters<k_gemm_q4k_q8k_tc5<NPAD>>(Tc5Shape<NPAD>::kThreads, 200 * 1024);      // (a CTA has an SM to itself)
     Tc5Split best = {1, -1};
     for (int sp = 1; at_once && sp <= kMaxSplits && (sp == 1 || nb / sp >= 2); sp++) {
-        const long steps = (long)((n_tiles + at_once->of[sp] - 1) / at_once->of[sp]) * ((nb + sp - 1) / sp + 2) + (sp > 1 ? 2 : 0);
+        const long steps = (long)((n_tiles + at_once[sp] - 1) / at_once[sp]) * ((nb + sp - 1) / sp + 2) + (sp > 1 ? 2 : 0);
         if (best.steps < 0 || steps < best.steps) best = {sp, steps};
     }
     return best;

@@ -10,6 +10,7 @@
 //                  (TMEM columns) per tile, persistent CTAs, operands by tiled TMA into a 128-byte-swizzled ring, two
 //                  accumulators so that a tile's epilogue runs under the next tile's products
 //   k_linear_tile  several tokens, fp32: plain fp32 multiply-adds on 64 x 64 tiles
+#include "cluster_device.cuh"
 #include "decoder_device.cuh"
 #include "launch.cuh"
 #include "tcgen05_device.cuh"
@@ -256,7 +257,110 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
 
     const int n_tiles = (l.N + kTc5Rows - 1) / kTc5Rows, t_tiles = (T + bn - 1) / bn;
     // tokens vary fastest: the CTAs at work share few rows of weights, which go through HBM once
-    const int tiles = n_tiles * t_tiles, kb_n = (l.K + kTc5Depth - 1) / kTc5Depth;
+    const int tiles = n_tiles * t_tiles, kb_all = (l.K + kTc5Depth - 1) / kTc5Depth;
+    // few tiles: the CTAs of a cluster take a range of K each and join their sums through shared memory (one tile per cluster then)
+    const int ranges = gridDim.y, range = blockIdx.y, kb0 = range * kb_all / ranges, kb_n = (range + 1) * kb_all / ranges - kb0;
+    float* part_sums = reinterpret_cast<float*>(ring);      // [bn][128], once all products are done
+
+    // What follows the sums of a tile: a thread owns one weight row and walks over its tokens, 16 at a time.  sums(c0, v) gives tokens c0 ..
+    // of the row, next_of(c0) the step that this thread takes after c0 (bn and beyond: none); the first residual rows are fetched before ready().
+    const int quarter = warp & 3, r = 32 * quarter + lane;
+    auto finish = [&](int tile, int c_first, auto ready, auto sums, auto next_of) {
+        const int n = (tile / t_tiles) * kTc5Rows + r;
+        const int tb = (tile % t_tiles) * bn;
+        const bool live = n < l.N;
+        // residual rows are fetched a step of 16 tokens ahead, the first under the tile's products
+        float xv[16];
+        auto fetch_x = [&](int c0) {
+#pragma unroll
+            for (int j = 0; j < 16; j++) xv[j] = (live && tb + c0 + j < T) ? l.x[(size_t)(tb + c0 + j) * l.ld_x + n] : 0.0f;
+        };
+        if (l.mode == kLinResidual && c_first < bn) fetch_x(c_first);
+        if (!ready()) return false;
+        DynTanh post = l.post, next = l.next;
+        float pw = 0, pb = 0, nw = 0, nb = 0;
+        if (l.mode == kLinResidual && live) {
+            pw = post.w[n]; pb = post.b[n];
+            if (next.w) { nw = next.w[n]; nb = next.b[n]; }
+        } else if (l.mode == kLinLogDecay && live) {
+            pw = l.neg_exp_a[n]; pb = l.dt_bias[n];
+        }
+        const bool is_step = l.mode == kLinMixerIn && live && n >= l.dt_row;      // (lanes of one warp may differ)
+        if (is_step && l.dt_bias) pb = l.dt_bias[n - l.dt_row];
+        const bool plain_f32 = l.mode == kLinF32 && l.cap == 0.0f;
+        // rows of this warp that are only rounded and stored (after a GELU)
+        const int n_end = (n - lane) + 32;
+        const bool plain_warp = !((l.N | l.ld_out) & 1) &&
+                                (l.mode == kLinAct || l.mode == kLinGelu || (l.mode == kLinMixerIn && n_end <= l.dt_row && !l.conv.w));
+        auto step = [&](int c0, int c_next, int (&v)[16]) {
+            const int t0 = tb + c0;
+            if (t0 >= T) return;
+            if (l.mode == kLinResidual) {
+                float xr[16];
+#pragma unroll
+                for (int j = 0; j < 16; j++) xr[j] = xv[j];
+                if (c_next < bn) fetch_x(c_next);
+#pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    const float q = xr[j] + fmaf(tanhf(post.alpha * __int_as_float(v[j])), pw, pb);
+                    if (live && t0 + j < T) {
+                        l.x[(size_t)(t0 + j) * l.ld_x + n] = q;
+                        if (next.w)
+                            reinterpret_cast<bf16*>(l.out)[(size_t)(t0 + j) * l.ld_out + n] =
+                                act_from<bf16>(fmaf(tanhf(next.alpha * q), nw, nb));
+                    }
+                }
+            } else if (l.mode == kLinSwiglu) {
+                // lane pairs hold gate (even) and up (odd): the even lane finishes even tokens, the odd lane odd ones
+#pragma unroll
+                for (int j = 0; j < 16; j += 2) {
+                    const float keep = __int_as_float((lane & 1) ? v[j + 1] : v[j]);
+                    const float other = __shfl_xor_sync(0xFFFFFFFFu, __int_as_float((lane & 1) ? v[j] : v[j + 1]), 1);
+                    const float g = (lane & 1) ? other : keep, u = (lane & 1) ? keep : other;
+                    const int t = t0 + j + (lane & 1);
+                    if (live && t < T) reinterpret_cast<bf16*>(l.out)[(size_t)t * l.ld_out + n / 2] = act_from<bf16>(silu_act<bf16>(g) * u);
+                }
+            } else if (plain_warp) {
+                if (l.mode == kLinGelu)
+#pragma unroll
+                    for (int j = 0; j < 16; j++) v[j] = __float_as_int(gelu_act<bf16>(__int_as_float(v[j])));
+                // two neighbouring rows per store: the even lane finishes even tokens, the odd lane odd ones
+#pragma unroll
+                for (int j = 0; j < 16; j += 2) {
+                    const float keep = __int_as_float((lane & 1) ? v[j + 1] : v[j]);
+                    const float other = __shfl_xor_sync(0xFFFFFFFFu, __int_as_float((lane & 1) ? v[j] : v[j + 1]), 1);
+                    const __nv_bfloat162 two = __floats2bfloat162_rn((lane & 1) ? other : keep, (lane & 1) ? keep : other);
+                    const int t = t0 + j + (lane & 1);
+                    if (live && t < T) *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<bf16*>(l.out) + (size_t)t * l.ld_out + (n & ~1)) = two;
+                }
+            } else if (plain_f32) {
+#pragma unroll
+                for (int j = 0; j < 16; j++)
+                    if (live && t0 + j < T) reinterpret_cast<float*>(l.out)[(size_t)(t0 + j) * l.ld_out + n] = __int_as_float(v[j]);
+            } else if (l.mode == kLinLogDecay) {
+#pragma unroll
+                for (int j = 0; j < 16; j++)
+                    if (live && t0 + j < T) l.dt[(size_t)(t0 + j) * l.ld_dt + n] = pw * softplus_act<bf16>(__int_as_float(v[j]) + pb);
+            } else if (is_step) {
+                float q[16];
+#pragma unroll
+                for (int j = 0; j < 16; j++) q[j] = l.dt_bias ? softplus_act<bf16>(__int_as_float(v[j]) + pb) : sigmoid_act<bf16>(__int_as_float(v[j]));
+#pragma unroll
+                for (int j = 0; j < 16; j++)
+                    if (t0 + j < T) l.dt[(size_t)(t0 + j) * l.ld_dt + n - l.dt_row] = q[j];
+            } else if (live) {
+#pragma unroll
+                for (int j = 0; j < 16; j++)
+                    if (t0 + j < T) linear_store<bf16>(l, t0 + j, n, __int_as_float(v[j]));
+            }
+        };
+        for (int c0 = c_first; c0 < bn; c0 = next_of(c0)) {
+            int v[16];
+            sums(c0, v);
+            step(c0, next_of(c0), v);
+        }
+        return true;
+    };
 
     if (warp == 0) {
         // ---------------- producer: the weights of the first ring round are requested before the launch ahead has finished
@@ -274,12 +378,12 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
             int row = (ww.tile / t_tiles) * kTc5Rows, tok = (wt.tile % t_tiles) * bn;
             auto weights = [&](int s) {
                 mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
-                tma_rows_2d(ring + (size_t)s * stage_bytes, &wmap, ww.kb * kTc5Depth, row, &full[s]);
+                tma_rows_2d(ring + (size_t)s * stage_bytes, &wmap, (kb0 + ww.kb) * kTc5Depth, row, &full[s]);
                 step(ww);
                 if (ww.kb == 0) row = (ww.tile / t_tiles) * kTc5Rows;
             };
             auto tokens = [&](int s) {
-                tma_rows_2d(ring + (size_t)s * stage_bytes + kTc5ABytes, &xmap, wt.kb * kTc5Depth, tok, &full[s]);
+                tma_rows_2d(ring + (size_t)s * stage_bytes + kTc5ABytes, &xmap, (kb0 + wt.kb) * kTc5Depth, tok, &full[s]);
                 step(wt);
                 if (wt.kb == 0) tok = (wt.tile % t_tiles) * bn;
             };
@@ -322,7 +426,7 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t stage = smem_addr(ring + (size_t)s * stage_bytes);
                     const uint64_t ad = swizzled_desc(stage), bd = swizzled_desc(stage + kTc5ABytes);
-                    const int left = (l.K - kb * kTc5Depth) / 16;
+                    const int left = (l.K - (kb0 + kb) * kTc5Depth) / 16;
                     umma_bf16_ss(d, ad, bd, idesc, kb ? 1u : 0u);
                     if (left >= 4) {
 #pragma unroll
@@ -339,106 +443,33 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
         }
         __syncwarp();
     } else {
-        // ---------------- epilogue: a thread owns one weight row of the tile and walks over its tokens
-        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        // ---------------- epilogue
+        const int half = (warp - 2) >> 2;
         const int split = (bn / 16 + 1) / 2 * 16, c_begin = half ? split : 0, c_end = half ? bn : split;
-        const int r = 32 * quarter + lane;
         int local = 0;
         pdl_wait();
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, local++) {
             const int a = local & 1;
-            const int n = (tile / t_tiles) * kTc5Rows + r;
-            const int tb = (tile % t_tiles) * bn;
-            const bool live = n < l.N;
-            // residual rows are fetched a step of 16 tokens ahead, the first under the tile's products
-            float xv[16];
-            auto fetch_x = [&](int c0) {
-#pragma unroll
-                for (int j = 0; j < 16; j++) xv[j] = (live && tb + c0 + j < T) ? l.x[(size_t)(tb + c0 + j) * l.ld_x + n] : 0.0f;
-            };
-            if (l.mode == kLinResidual && c_begin < c_end) fetch_x(c_begin);
-            if (!mbar_wait_bounded(&acc_full[a], (uint32_t)(local >> 1) & 1u, err, 44)) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t ta = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(a * BN);
-            DynTanh post = l.post, next = l.next;
-            float pw = 0, pb = 0, nw = 0, nb = 0;
-            if (l.mode == kLinResidual && live) {
-                pw = post.w[n]; pb = post.b[n];
-                if (next.w) { nw = next.w[n]; nb = next.b[n]; }
-            } else if (l.mode == kLinLogDecay && live) {
-                pw = l.neg_exp_a[n]; pb = l.dt_bias[n];
-            }
-            const bool is_step = l.mode == kLinMixerIn && live && n >= l.dt_row;      // (lanes of one warp may differ)
-            if (is_step && l.dt_bias) pb = l.dt_bias[n - l.dt_row];
-            const bool plain_f32 = l.mode == kLinF32 && l.cap == 0.0f;
-            // rows of this warp that are only rounded and stored (after a GELU)
-            const int n_end = (n - lane) + 32;
-            const bool plain_warp = !((l.N | l.ld_out) & 1) &&
-                                    (l.mode == kLinAct || l.mode == kLinGelu || (l.mode == kLinMixerIn && n_end <= l.dt_row && !l.conv.w));
-            for (int c0 = c_begin; c0 < c_end; c0 += 16) {
-                int v[16];
+            auto ready = [&]() {
+                if (!mbar_wait_bounded(&acc_full[a], (uint32_t)(local >> 1) & 1u, err, 44)) return false;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                return true;
+            };
+            auto sums = [&](int c0, int (&v)[16]) {
                 tmem_ld(ta + c0, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                const int t0 = tb + c0;
-                if (t0 >= T) continue;
-                if (l.mode == kLinResidual) {
-                    float xr[16];
+            };
+            if (ranges > 1) {
+                if (!ready()) break;
+                for (int c0 = c_begin; c0 < c_end; c0 += 16) {
+                    int v[16];
+                    sums(c0, v);
 #pragma unroll
-                    for (int j = 0; j < 16; j++) xr[j] = xv[j];
-                    if (c0 + 16 < c_end) fetch_x(c0 + 16);
-#pragma unroll
-                    for (int j = 0; j < 16; j++) {
-                        const float q = xr[j] + fmaf(tanhf(post.alpha * __int_as_float(v[j])), pw, pb);
-                        if (live && t0 + j < T) {
-                            l.x[(size_t)(t0 + j) * l.ld_x + n] = q;
-                            if (next.w)
-                                reinterpret_cast<bf16*>(l.out)[(size_t)(t0 + j) * l.ld_out + n] =
-                                    act_from<bf16>(fmaf(tanhf(next.alpha * q), nw, nb));
-                        }
-                    }
-                } else if (l.mode == kLinSwiglu) {
-                    // lane pairs hold gate (even) and up (odd): the even lane finishes even tokens, the odd lane odd ones
-#pragma unroll
-                    for (int j = 0; j < 16; j += 2) {
-                        const float keep = __int_as_float((lane & 1) ? v[j + 1] : v[j]);
-                        const float other = __shfl_xor_sync(0xFFFFFFFFu, __int_as_float((lane & 1) ? v[j] : v[j + 1]), 1);
-                        const float g = (lane & 1) ? other : keep, u = (lane & 1) ? keep : other;
-                        const int t = t0 + j + (lane & 1);
-                        if (live && t < T) reinterpret_cast<bf16*>(l.out)[(size_t)t * l.ld_out + n / 2] = act_from<bf16>(silu_act<bf16>(g) * u);
-                    }
-                } else if (plain_warp) {
-                    if (l.mode == kLinGelu)
-#pragma unroll
-                        for (int j = 0; j < 16; j++) v[j] = __float_as_int(gelu_act<bf16>(__int_as_float(v[j])));
-                    // two neighbouring rows per store: the even lane finishes even tokens, the odd lane odd ones
-#pragma unroll
-                    for (int j = 0; j < 16; j += 2) {
-                        const float keep = __int_as_float((lane & 1) ? v[j + 1] : v[j]);
-                        const float other = __shfl_xor_sync(0xFFFFFFFFu, __int_as_float((lane & 1) ? v[j] : v[j + 1]), 1);
-                        const __nv_bfloat162 two = __floats2bfloat162_rn((lane & 1) ? other : keep, (lane & 1) ? keep : other);
-                        const int t = t0 + j + (lane & 1);
-                        if (live && t < T) *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<bf16*>(l.out) + (size_t)t * l.ld_out + (n & ~1)) = two;
-                    }
-                } else if (plain_f32) {
-#pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        if (live && t0 + j < T) reinterpret_cast<float*>(l.out)[(size_t)(t0 + j) * l.ld_out + n] = __int_as_float(v[j]);
-                } else if (l.mode == kLinLogDecay) {
-#pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        if (live && t0 + j < T) l.dt[(size_t)(t0 + j) * l.ld_dt + n] = pw * softplus_act<bf16>(__int_as_float(v[j]) + pb);
-                } else if (is_step) {
-                    float q[16];
-#pragma unroll
-                    for (int j = 0; j < 16; j++) q[j] = l.dt_bias ? softplus_act<bf16>(__int_as_float(v[j]) + pb) : sigmoid_act<bf16>(__int_as_float(v[j]));
-#pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        if (t0 + j < T) l.dt[(size_t)(t0 + j) * l.ld_dt + n - l.dt_row] = q[j];
-                } else if (live) {
-#pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        if (t0 + j < T) linear_store<bf16>(l, t0 + j, n, __int_as_float(v[j]));
+                    for (int j = 0; j < 16; j++) part_sums[(c0 + j) * kTc5Rows + r] = __int_as_float(v[j]);
                 }
+            } else if (!finish(tile, c_begin < c_end ? c_begin : bn, ready, sums, [&](int c0) { return c0 + 16 < c_end ? c0 + 16 : bn; })) {
+                break;
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -450,6 +481,34 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(S::kTmemCols) : "memory");
+    }
+    if (ranges > 1) {
+        // every CTA finishes some of the tile's steps of 16 tokens, its epilogue warps' halves taking turns; ranges are added in their order
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        if (warp >= 2) {
+            const int turn = 32 * ranges;
+            finish(blockIdx.x, 16 * (2 * range + ((warp - 2) >> 2)), []() { return true; },
+                   [&](int c0, int (&v)[16]) {
+                       float t[16];
+#pragma unroll
+                       for (int j = 0; j < 16; j++) t[j] = load_peer(part_sums + (c0 + j) * kTc5Rows + r, 0);
+                       for (int q = 1; q < ranges; q++) {
+                           float u[16];
+#pragma unroll
+                           for (int j = 0; j < 16; j++) u[j] = load_peer(part_sums + (c0 + j) * kTc5Rows + r, q);
+#pragma unroll
+                           for (int j = 0; j < 16; j++) t[j] += u[j];
+                       }
+#pragma unroll
+                       for (int j = 0; j < 16; j++) v[j] = __float_as_int(t[j]);
+                   },
+                   [&](int c0) { return c0 + turn; });
+        }
+        __syncwarp();
+        cluster_arrive();       // nobody leaves while its sums are read
+        cluster_wait();
     }
 }
 
@@ -479,30 +538,41 @@ static int bf16_map(CUtensorMap* map, const void* p, int rows, int cols, int ld,
     return r == CUDA_SUCCESS ? 0 : latch(BPDQ_ERR_CUDA - 900 - (int)r);
 }
 
+struct Tc5Tiles { int tokens, ranges; };      // of a tile; of K
+
 template <int BN>
-static int launch_tc5(const Linear& l, int T, int bn, cudaStream_t s)
+static int launch_tc5(const Linear& l, int T, Tc5Tiles t, cudaStream_t s)
 {
     using S = Tc5Linear<BN>;
     CUtensorMap wmap, xmap;
     int rc;
     if ((rc = bf16_map(&wmap, l.W, l.N, l.K, l.K, kTc5Rows))) return rc;
-    if ((rc = bf16_map(&xmap, l.in, T, l.K, l.ld_in, bn))) return rc;
+    if ((rc = bf16_map(&xmap, l.in, T, l.K, l.ld_in, t.tokens))) return rc;
     if ((rc = allow_smem<k_linear_tc5<BN>>(227 * 1024))) return rc;
-    const long tiles = (long)((l.N + kTc5Rows - 1) / kTc5Rows) * ((T + bn - 1) / bn);
-    const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
-    return launch_ordered(k_linear_tc5<BN>, grid, S::kThreads, tc5_smem(bn), s, wmap, xmap, l, T, bn, device_error_flag());
+    const long tiles = (long)((l.N + kTc5Rows - 1) / kTc5Rows) * ((T + t.tokens - 1) / t.tokens);
+    const unsigned grid = (unsigned)(t.ranges > 1 || tiles < sm_count() ? tiles : sm_count());
+    return launch_cluster(k_linear_tc5<BN>, dim3(grid, (unsigned)t.ranges), dim3(1, (unsigned)t.ranges, 1), S::kThreads, tc5_smem(t.tokens), s, wmap, xmap, l, T,
+                          t.tokens, device_error_flag());
 }
 
-// Tokens of a tile: the multiple of 16 with the least time, in waves of CTAs over the SMs times a tile's time.
-static int tc5_tokens(const Linear& l, int T)
+// Tokens of a tile (a multiple of 16) and ranges of K with the least time in cycles: waves of CTAs over the SMs times a tile's K blocks, each
+// 310 + 1.3 per token (measured: 325 at 16 tokens, 650 at 256); K is cut, into ranges of at least four blocks, where all its tiles' clusters
+// run at once, and joining r ranges costs 3000 + 800 r + 25 per token.  2048 rows of 10752 (us, one range, several): 48 tokens 33.5, 14.2 at
+// six; 200 tokens 33.9, 19.0 at four; of 2048: 16 tokens 8.8, 7.3 at four; 200 tokens 9.2, 9.3.
+static Tc5Tiles tc5_tiles(const Linear& l, int T)
 {
-    const long n_tiles = (l.N + kTc5Rows - 1) / kTc5Rows, top = (T + 15) / 16 * 16 < 256 ? (T + 15) / 16 * 16 : 256;
-    int best = 16;
+    const int n_tiles = (l.N + kTc5Rows - 1) / kTc5Rows, top = (T + 15) / 16 * 16 < 256 ? (T + 15) / 16 * 16 : 256;
+    const int kb = (l.K + kTc5Depth - 1) / kTc5Depth, sms = sm_count();
+    const int* clusters = active_clusters<k_linear_tc5<256>>(Tc5Linear<256>::kThreads, 200 * 1024);      // (a CTA has an SM to itself)
+    Tc5Tiles best = {16, 1};
     double least = 0.0;
     for (int bn = 16; bn <= top; bn += 16) {
-        const long tiles = n_tiles * ((T + bn - 1) / bn);
-        const double time = (double)((tiles + sm_count() - 1) / sm_count()) * (double)(400 + bn);
-        if (bn == 16 || time <= least) { best = bn; least = time; }
+        const long tiles = (long)n_tiles * ((T + bn - 1) / bn);
+        for (int ranges = 1; ranges <= 8 && (ranges == 1 || (clusters && tiles <= clusters[ranges] && kb / ranges >= 4)); ranges++) {
+            const long waves = ranges > 1 ? 1 : (tiles + sms - 1) / sms;
+            const double time = (double)waves * ((kb + ranges - 1) / ranges) * (310.0 + 1.3 * bn) + (ranges > 1 ? 3000.0 + 800.0 * ranges + 25.0 * bn : 0.0);
+            if ((bn == 16 && ranges == 1) || time <= least) { best = {bn, ranges}; least = time; }
+        }
     }
     return best;
 }
@@ -522,11 +592,11 @@ int linear_forward(const Linear& l, int T, bool act_bf16, cudaStream_t s)
         return act_bf16 ? launch_ordered(k_linear_vec<bf16>, grid, 256, smem, s, l) : launch_ordered(k_linear_vec<float>, grid, 256, smem, s, l);
     }
     if (!act_bf16) return launch_ordered(k_linear_tile, dim3((l.N + 63) / 64, (T + 63) / 64), 256, 0, s, l, T);
-    const int bn = tc5_tokens(l, T);
-    if (bn > 128) return launch_tc5<256>(l, T, bn, s);
-    if (bn > 64) return launch_tc5<128>(l, T, bn, s);
-    if (bn > 32) return launch_tc5<64>(l, T, bn, s);
-    return launch_tc5<32>(l, T, bn, s);
+    const Tc5Tiles t = tc5_tiles(l, T);
+    if (t.tokens > 128) return launch_tc5<256>(l, T, t, s);
+    if (t.tokens > 64) return launch_tc5<128>(l, T, t, s);
+    if (t.tokens > 32) return launch_tc5<64>(l, T, t, s);
+    return launch_tc5<32>(l, T, t, s);
 }
 
 }  // namespace bpdq
