@@ -20,30 +20,32 @@ namespace bpdq {
 
 // ------------------------------------------------------------------ one token
 
-template <typename A>
+// R rows of a warp at a time: two, or one where there are not enough rows to give every warp two (16 loads in flight either way).
+// What bounds it: HBM behind the latency of a group of rows. 2048 rows of 7168 with two rows each gave 1024 of 2368 warps work.  A decoded token of
+// the hybrid decoder at 4000 keys: 281 us with pairs only, 272 with single rows where they fit.
+template <typename A, int R>
 __global__ void __launch_bounds__(256, 2) k_linear_vec(Linear l)
 {
     extern __shared__ float4 xs[];      // [2][K / 8]: first and second four of every eight activations (split: twice)
     __shared__ float s_sum[8];
-    constexpr int kBatch = 8;           // 16-byte loads in flight per row and lane
-    const int units = l.K / 8, pairs = (l.N + 1) / 2;
+    constexpr int kBatch = 16 / R;      // 16-byte loads in flight per row and lane
+    const int units = l.K / 8, groups = (l.N + R - 1) / R;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int stride = gridDim.x * 8;
-    int p = blockIdx.x + gridDim.x * warp;      // row pairs are dealt over the CTAs first: every SM gets its share
+    int p = blockIdx.x + gridDim.x * warp;      // groups of rows are dealt over the CTAs first: every SM gets its share
     pdl_launch_dependents();
-    uint4 w[2][kBatch];
+    uint4 w[R][kBatch];
     auto fetch = [&](int base) {
-        const int r1 = 2 * p + 1 < l.N ? 2 * p + 1 : 2 * p;
-        const uint4* a = reinterpret_cast<const uint4*>(l.W + (size_t)(2 * p) * l.K);
-        const uint4* b = reinterpret_cast<const uint4*>(l.W + (size_t)r1 * l.K);
+        const uint4* a = reinterpret_cast<const uint4*>(l.W + (size_t)(R * p) * l.K);
+        const uint4* b = reinterpret_cast<const uint4*>(l.W + (size_t)(R * p + R - 1 < l.N ? R * p + R - 1 : R * p) * l.K);
 #pragma unroll
         for (int i = 0; i < kBatch; i++) {
             const int u = base + lane + 32 * i;
             w[0][i] = u < units ? __ldg(a + u) : make_uint4(0, 0, 0, 0);
-            w[1][i] = u < units ? __ldg(b + u) : make_uint4(0, 0, 0, 0);
+            if (R > 1) w[R - 1][i] = u < units ? __ldg(b + u) : make_uint4(0, 0, 0, 0);
         }
     };
-    if (p < pairs) fetch(0);
+    if (p < groups) fetch(0);
     pdl_wait();
     float rnorm = 1.0f;
     if (l.norm_w) {
@@ -70,24 +72,24 @@ __global__ void __launch_bounds__(256, 2) k_linear_vec(Linear l)
         __syncthreads();
     }
     bool have = true;
-    for (; p < pairs; p += stride) {
-        const int row = 2 * p + lane;
-        const float4* x = l.split && 2 * p >= l.split ? xs + 2 * units : xs;
-        const bool residual = l.mode == kLinResidual && lane < 2 && row < l.N;
-        const bool streams = l.mode == kLinStreams && lane < 2 && row < l.N;
+    for (; p < groups; p += stride) {
+        const int row = R * p + lane;
+        const float4* x = l.split && R * p >= l.split ? xs + 2 * units : xs;
+        const bool residual = l.mode == kLinResidual && lane < R && row < l.N;
+        const bool streams = l.mode == kLinStreams && lane < R && row < l.N;
         float xo[kMaxStreams];
         if (streams) {
 #pragma unroll
             for (int i = 0; i < kMaxStreams; i++) xo[i] = i < l.streams.n ? l.x[(size_t)i * l.ld_x + row] : 0.0f;
         }
-        float xr = 0, pw = 0, pb = 0, nw = 0, nb = 0;       // what the residual epilogue of row 2 p + lane needs, ahead of its use
+        float xr = 0, pw = 0, pb = 0, nw = 0, nb = 0;       // what the residual epilogue of row R p + lane needs, ahead of its use
         if (residual) {
             xr = l.x[row];
             pw = l.post.w[row];
             pb = l.post.b[row];
             if (l.next.w) { nw = l.next.w[row]; nb = l.next.b[row]; }
         }
-        float acc[2] = {0.0f, 0.0f};
+        float acc[R] = {};
         for (int base = 0; base < units; base += 32 * kBatch) {
             if (!have) fetch(base);
             have = false;
@@ -97,7 +99,7 @@ __global__ void __launch_bounds__(256, 2) k_linear_vec(Linear l)
                 if (u >= units) break;
                 const float4 x0 = x[u], x1 = x[units + u];
 #pragma unroll
-                for (int r = 0; r < 2; r++) {
+                for (int r = 0; r < R; r++) {
                     const uint4 q = w[r][i];
                     acc[r] = fmaf(__uint_as_float(q.x << 16), x0.x, acc[r]);
                     acc[r] = fmaf(__uint_as_float(q.x & 0xFFFF0000u), x0.y, acc[r]);
@@ -110,11 +112,11 @@ __global__ void __launch_bounds__(256, 2) k_linear_vec(Linear l)
                 }
             }
         }
-        acc[0] = warp_sum(acc[0]);
-        acc[1] = warp_sum(acc[1]);
-        const float v = (lane ? acc[1] : acc[0]) * rnorm;
+#pragma unroll
+        for (int r = 0; r < R; r++) acc[r] = warp_sum(acc[r]);
+        const float v = (lane ? acc[R - 1] : acc[0]) * rnorm;
         if (l.mode == kLinSwiglu) {
-            if (lane == 0) reinterpret_cast<A*>(l.out)[p] = act_from<A>(silu_act<A>(acc[0] * rnorm) * (acc[1] * rnorm));
+            if (lane == 0) reinterpret_cast<A*>(l.out)[p] = act_from<A>(silu_act<A>(acc[0] * rnorm) * (acc[R - 1] * rnorm));
         } else if (streams) {
             float u = 0.0f;
 #pragma unroll
@@ -132,7 +134,7 @@ __global__ void __launch_bounds__(256, 2) k_linear_vec(Linear l)
             const float r = xr + fmaf(tanhf(l.post.alpha * v), pw, pb);
             l.x[row] = r;
             if (l.next.w) reinterpret_cast<A*>(l.out)[row] = act_from<A>(fmaf(tanhf(l.next.alpha * r), nw, nb));
-        } else if (l.mode != kLinResidual && l.mode != kLinStreams && lane < 2 && row < l.N) {
+        } else if (l.mode != kLinResidual && l.mode != kLinStreams && lane < R && row < l.N) {
             linear_store<A>(l, 0, row, v);
         }
     }
@@ -577,6 +579,15 @@ static Tc5Tiles tc5_tiles(const Linear& l, int T)
     return best;
 }
 
+template <typename A, int R>
+static int launch_vec(const Linear& l, size_t smem, cudaStream_t s)
+{
+    int rc = allow_smem<k_linear_vec<A, R>>(200 * 1024);
+    if (rc) return rc;
+    const int want = (l.N + R - 1) / R, cap = 2 * sm_count();
+    return launch_ordered(k_linear_vec<A, R>, want < cap ? want : cap, 256, smem, s, l);
+}
+
 int linear_forward(const Linear& l, int T, bool act_bf16, cudaStream_t s)
 {
     if (l.K % 16 || l.K < 16 || l.N < 1 || T < 1 || l.ld_in % 8) return latch(BPDQ_ERR_ARG);
@@ -585,11 +596,11 @@ int linear_forward(const Linear& l, int T, bool act_bf16, cudaStream_t s)
     if (T == 1) {
         const size_t smem = (size_t)l.K * (l.split ? 8 : 4);
         if (smem > 200 * 1024) return latch(BPDQ_ERR_RANGE);
-        int rc = act_bf16 ? allow_smem<k_linear_vec<bf16>>(200 * 1024) : allow_smem<k_linear_vec<float>>(200 * 1024);
-        if (rc) return rc;
-        const int want = (l.N + 1) / 2, cap = 2 * sm_count();
-        const int grid = want < cap ? want : cap;
-        return act_bf16 ? launch_ordered(k_linear_vec<bf16>, grid, 256, smem, s, l) : launch_ordered(k_linear_vec<float>, grid, 256, smem, s, l);
+        // one row per warp and step as long as two would leave warps without any (a gate and its up are always two)
+        const int warps = 2 * sm_count() * 8;
+        const bool one = l.mode != kLinSwiglu && l.N <= warps;
+        return act_bf16 ? (one ? launch_vec<bf16, 1>(l, smem, s) : launch_vec<bf16, 2>(l, smem, s))
+                        : (one ? launch_vec<float, 1>(l, smem, s) : launch_vec<float, 2>(l, smem, s));
     }
     if (!act_bf16) return launch_ordered(k_linear_tile, dim3((l.N + 63) / 64, (T + 63) / 64), 256, 0, s, l, T);
     const Tc5Tiles t = tc5_tiles(l, T);
