@@ -84,7 +84,7 @@ __device__ __forceinline__ void unpack16(const uint4& w, float (&f)[F16 ? 8 : 4]
     }
 }
 
-constexpr int kSplitThreads = 256, kSplitWarps = kSplitThreads / 32;
+constexpr int kSplitThreads = 256, kSplitWarps = kSplitThreads / 32, kMaxCluster = 16;
 
 // What bounds it: the read of the cache rows (4001 keys of 8 heads of 128: 16.4 MB, 2.5 us), and below about 1000 keys the launch.
 // One CTA per (token, head) took 202 us there, most of it in the sums that one thread added in order; 12 us now (65 keys: 9.2,
@@ -155,6 +155,12 @@ __global__ void __launch_bounds__(kSplitThreads) k_gqa_split(GqaShape p, const f
             }
         }
     }
+    // the warp's first values are requested ahead of the softmax
+    uint4 vw[8];
+    if (warp * 8 * P < n) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) vw[j] = __ldcg(reinterpret_cast<const uint4*>(vbase + (size_t)min(warp * 8 * P + j * P + lane / L, n - 1) * row));
+    }
     __syncthreads();
     // thread t: head t % R
     float m = kLowest;
@@ -194,7 +200,12 @@ __global__ void __launch_bounds__(kSplitThreads) k_gqa_split(GqaShape p, const f
         for (int b = warp * 8 * P; b < n; b += kSplitWarps * 8 * P) {
             uint4 w[8];
 #pragma unroll
-            for (int j = 0; j < 8; j++) w[j] = __ldcg(reinterpret_cast<const uint4*>(vbase + (size_t)min(b + j * P + lane / L, n - 1) * row));
+            for (int j = 0; j < 8; j++) w[j] = vw[j];
+            const int next = b + kSplitWarps * 8 * P;
+            if (next < n) {
+#pragma unroll
+                for (int j = 0; j < 8; j++) vw[j] = __ldcg(reinterpret_cast<const uint4*>(vbase + (size_t)min(next + j * P + lane / L, n - 1) * row));
+            }
 #pragma unroll
             for (int j = 0; j < 8; j++) {
                 const int key = b + j * P + lane / L;
@@ -238,14 +249,26 @@ __global__ void __launch_bounds__(kSplitThreads) k_gqa_split(GqaShape p, const f
     const int slice = (R * D + ranks - 1) / ranks;
     for (int i = rank * slice + tid; i < min(R * D, (rank + 1) * slice); i += kSplitThreads) {
         const int r = i / D;
-        float top = kLowest;
-        for (int c = 0; c < ranks; c++) top = fmaxf(top, load_peer(&s_m[r], c));
-        float sum = 0.0f, out = 0.0f;
-        for (int c = 0; c < ranks; c++) {
-            const float f = exp_below(load_peer(&s_m[r], c) - top);
-            sum = fmaf(f, load_peer(&s_l[r], c), sum);
-            out = fmaf(f, load_peer(&s_out[i], c), out);
+        // all CTAs' loads in flight before the first is used (one after the other: 3 us of 12 with 16 CTAs)
+        float pm[kMaxCluster], pl[kMaxCluster], po[kMaxCluster], top = kLowest;
+#pragma unroll
+        for (int c = 0; c < kMaxCluster; c++) {
+            const int from = c < ranks ? c : 0;
+            pm[c] = load_peer(&s_m[r], from);
+            pl[c] = load_peer(&s_l[r], from);
+            po[c] = load_peer(&s_out[i], from);
         }
+#pragma unroll
+        for (int c = 0; c < kMaxCluster; c++)
+            if (c < ranks) top = fmaxf(top, pm[c]);
+        float sum = 0.0f, out = 0.0f;
+#pragma unroll
+        for (int c = 0; c < kMaxCluster; c++)
+            if (c < ranks) {
+                const float f = exp_below(pm[c] - top);
+                sum = fmaf(f, pl[c], sum);
+                out = fmaf(f, po[c], out);
+            }
         if (h0 + r < rep) dst[((size_t)qt * p.heads + head(r)) * D + i % D] = out * (sum == 0.0f ? 0.0f : __fdiv_rn(1.0f, sum));
     }
     cluster_arrive();       // nobody leaves while its shared memory is read
@@ -519,7 +542,6 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_gqa_tile(GqaShape p, const 
 template <int F16, int D, int R>
 static int launch_split(const GqaShape& p, const float* q, const void* k, const void* v, float* dst, cudaStream_t s)
 {
-    constexpr int kMaxCluster = 16;
     constexpr int kMaxSmem = 96 * 1024;
     auto kern = k_gqa_split<F16, D, R>;
     static int ready[64] = {0};       // the largest cluster of the kernel on a device
