@@ -55,8 +55,10 @@ struct WideProducts {
 
 // X fp32 [M][K] -> per (token tile, block) a unit of 80 T bytes: element (t, k) as fp16 at (k/8)*16*T + 16 t + 2 (k%8), then per token
 // the fp16 scale and seven zeros.  The numbers are those of k_quant_q8_0_tiles (eight lanes per block); tokens beyond M quantize zeros.
+// With `up` the numbers are silu(X) * up: 1000 tokens of 14336 a step of its own ahead of the quantizer made a prompt of 1000 tokens (four
+// layers of an 8B Llama) 5.97 ms, with the step in here 5.86.
 template <int T>
-__global__ void __launch_bounds__(256) k_quant_q8_0_wide(const float* X, uint8_t* acts, int M, int K, long n_items)
+__global__ void __launch_bounds__(256) k_quant_q8_0_wide(const float* X, const float* up, uint8_t* acts, int M, int K, long n_items)
 {
     pdl_launch_dependents();
     pdl_wait();
@@ -71,6 +73,10 @@ __global__ void __launch_bounds__(256) k_quant_q8_0_wide(const float* X, uint8_t
         const long tok = tile * T + t;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (tok < M) v = *(reinterpret_cast<const float4*>(X + (size_t)tok * K + (size_t)b * 32) + l);
+        if (tok < M && up) {
+            const float4 u = *(reinterpret_cast<const float4*>(up + (size_t)tok * K + (size_t)b * 32) + l);
+            v = make_float4(swiglu_rounded(v.x, u.x), swiglu_rounded(v.y, u.y), swiglu_rounded(v.z, u.z), swiglu_rounded(v.w, u.w));
+        }
         float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
@@ -359,7 +365,7 @@ k_gemm_q8_0_wide(const __grid_constant__ WideProducts p, const uint8_t* acts, fl
 // ------------------------------------------------------------------ host side
 
 template <int T>
-static int launch_wide(const WideProducts& p, const float* X, int K, cudaStream_t s, Workspace* ws)
+static int launch_wide(const WideProducts& p, const float* X, const float* up, int K, cudaStream_t s, Workspace* ws)
 {
     using S = WideShape<T>;
     const long t_tiles = (p.M + T - 1) / T, tiles = t_tiles * p.row_tile[p.n];
@@ -370,7 +376,7 @@ static int launch_wide(const WideProducts& p, const float* X, int K, cudaStream_
     uint8_t* acts = scratch_take(ws, kScratchTilesActs, bytes, s, &rc);
     if (!acts) return rc;
     const long items = t_tiles * p.nb * T * 8;
-    if ((rc = launch_ordered(k_quant_q8_0_wide<T>, grid_1d(items), 256, 0, s, X, acts, p.M, K, items))) return latch(rc);
+    if ((rc = launch_ordered(k_quant_q8_0_wide<T>, grid_1d(items), 256, 0, s, X, up, acts, p.M, K, items))) return latch(rc);
     rc = launch_ordered(k_gemm_q8_0_wide<T>, (unsigned)(tiles < sm_count() ? tiles : sm_count()), S::kThreads, S::kSmem, s, p, acts, -0.0f,
                         device_error_flag());
     return rc ? latch(rc) : 0;
@@ -398,7 +404,7 @@ static int wide_tokens(const WideProducts& p)
 }
 
 int gemm_q8_0_wide(int n, const uint8_t* const* tiles, float* const* outs, const int* Ns, const float* X, int M, int K, cudaStream_t s,
-                   Workspace* ws)
+                   Workspace* ws, const float* up)
 {
     if (n < 1 || n > kWideMatrices || M < kWideMinTokens || K < 32 || K % 32) return kWideRefused;
     WideProducts p = {};
@@ -412,9 +418,9 @@ int gemm_q8_0_wide(int n, const uint8_t* const* tiles, float* const* outs, const
         p.N[i] = Ns[i];
         p.row_tile[i + 1] = p.row_tile[i] + (Ns[i] + kTileRows - 1) / kTileRows;
     }
-    if (!X || ((uintptr_t)X & 15)) return kWideRefused;
+    if (!X || (((uintptr_t)X | (uintptr_t)up) & 15)) return kWideRefused;
     const int T = wide_tokens(p);
-    return T == 128 ? launch_wide<128>(p, X, K, s, ws) : T == 64 ? launch_wide<64>(p, X, K, s, ws) : T == 32 ? launch_wide<32>(p, X, K, s, ws) : kWideRefused;
+    return T == 128 ? launch_wide<128>(p, X, up, K, s, ws) : T == 64 ? launch_wide<64>(p, X, up, K, s, ws) : T == 32 ? launch_wide<32>(p, X, up, K, s, ws) : kWideRefused;
 }
 
 }  // namespace bpdq

@@ -167,15 +167,6 @@ __global__ void __launch_bounds__(256) k_add_rmsnorm_llama(float* x_io, const fl
     cta_rmsnorm_row(x, w, out + (size_t)blockIdx.x * cols, cols, eps, t);
 }
 
-// The reference's libm returns the correctly rounded fp32 value of expf / cosf / sinf for all but
-// a fraction of a percent of arguments; the device's fp32 versions are 1-2 ulp off for about half of
-// them.  Such last-bit differences are harmless by themselves, but every product that follows
-// re-quantizes its input to int8, where a last-bit difference now and then flips a rounding and
-// becomes a 1e-3 difference.  So these small kernels evaluate in binary64 and round once.
-__device__ __forceinline__ float exp_rounded(float x) { return (float)exp((double)x); }
-__device__ __forceinline__ float cos_rounded(float x) { return (float)cos((double)x); }
-__device__ __forceinline__ float sin_rounded(float x) { return (float)sin((double)x); }
-
 // In place or out of place.  Thread = (token, head, pair).  theta is reached as the reference reaches
 // it, by repeated multiplication from (float)pos, so that the angle has the same bits.
 __device__ __forceinline__ void rope_angle(int pair, int pos, const float* __restrict__ freq_factors, float theta_scale, float& c, float& s)
@@ -401,8 +392,7 @@ __global__ void __launch_bounds__(256) k_swiglu_f32(const float* gate, const flo
     pdl_launch_dependents();
     pdl_wait();
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const float g = gate[i];
-        dst[i] = __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, exp_rounded(-g))), up[i]);
+        dst[i] = swiglu_rounded(gate[i], up[i]);
     }
 }
 __global__ void __launch_bounds__(256) k_add_f32(const float* a, const float* b, float* dst, long n)
@@ -562,8 +552,17 @@ static int block_forward(float* x, const bpd_llama_layer_weights* lw, const bpd_
         const int Ns[2] = {F, F};
         if ((rc = products_shared_input(2, Ws, Ts, outs, Ns, s1, n_tokens, E, s, ws))) return rc;
     }
-    launch_ordered(k_swiglu_f32, grid_1d((long)n_tokens * F), 256, 0, s, s2, s3, s2, (long)n_tokens * F);
-    if ((rc = product(lw->w_down, lt ? lt->w_down : nullptr, s2, s1, n_tokens, E, F, s, ws))) return rc;
+    // where the product of many tokens takes the matrix it forms silu(gate) * up as it quantizes
+    rc = kWideRefused;
+    if (lt && lt->w_down) {
+        Workspace one = ws ? *ws : Workspace{nullptr, 0, 0};
+        rc = gemm_q8_0_wide(1, &lt->w_down, &s1, &E, s2, n_tokens, F, s, ws ? &one : nullptr, s3);
+    }
+    if (rc == kWideRefused) {
+        launch_ordered(k_swiglu_f32, grid_1d((long)n_tokens * F), 256, 0, s, s2, s3, s2, (long)n_tokens * F);
+        rc = product(lw->w_down, lt ? lt->w_down : nullptr, s2, s1, n_tokens, E, F, s, ws);
+    }
+    if (rc) return rc;
     if (fuse_next) launch_ordered(k_add_rmsnorm_llama, n_tokens, 256, 0, s, x, s1, next_norm_w, s1, E, cfg->rms_eps);
     else launch_ordered(k_add_f32, grid_1d((long)n_tokens * E), 256, 0, s, x, s1, x, (long)n_tokens * E);
     return check_cuda(cudaGetLastError());

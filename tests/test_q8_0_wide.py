@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 # sizes that take the wide kernel: rows that fill the narrow one's waves badly (N * M), at tokens around the edges of its tiles, rows below
 # and beyond a row tile, K of one block and of a number of blocks that leaves a stage, and a set of accumulators, partly filled
-SHAPES = [(64, 14400, 32), (40, 14336, 96), (129, 9600, 64), (257, 9580, 32), (300, 6000, 96), (640, 3300, 160), (1000, 2500, 96), (1000, 2430, 32)]
+SHAPES = [(64, 14400, 32), (40, 14336, 96), (129, 9600, 64), (257, 9580, 32), (300, 6000, 96), (640, 3300, 160), (1000, 2500, 96), (1000, 4096, 64), (333, 6100, 32),
+          (480, 4600, 32)]
 
 
 @pytest.mark.parametrize("M,N,K", SHAPES)
