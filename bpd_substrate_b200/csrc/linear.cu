@@ -9,7 +9,7 @@
 //   k_linear_tc5   several tokens, bf16: tcgen05.mma kind::f16, 128 weight rows (TMEM lanes) x up to 256 tokens
 //                  (TMEM columns) per tile, persistent CTAs, operands by tiled TMA into a 128-byte-swizzled ring, two
 //                  accumulators so that a tile's epilogue runs under the next tile's products
-//   k_linear_tile  several tokens, fp32: plain fp32 multiply-adds on 64 x 64 tiles
+//   k_linear_tile  several tokens, fp32: plain fp32 multiply-adds on tiles of 64 rows x 16 or 64 tokens
 #include "cluster_device.cuh"
 #include "decoder_device.cuh"
 #include "launch.cuh"
@@ -142,43 +142,52 @@ __global__ void __launch_bounds__(256, 2) k_linear_vec(Linear l)
 
 // ------------------------------------------------------------------ several tokens, fp32
 
+// 64 rows x 16 J tokens per CTA (J: 1 or 4), four rows and J tokens per thread.  Bound by the chain of slabs of 16 columns where there are few
+// tiles (12 tokens of 2048 x 2048: 104 us at J = 4, 82 at J = 1), else by the multiply-adds and the loads of their operands.
+template <int J>
 __global__ void __launch_bounds__(256) k_linear_tile(Linear l, int T)
 {
-    __shared__ float sw[16][68], sx[16][68];
-    const int tid = threadIdx.x, tr = tid & 15, tt = tid >> 4;      // rows 4 tr .., tokens 4 tt ..
-    const int n0 = blockIdx.x * 64, t0 = blockIdx.y * 64;
+    __shared__ __align__(16) float sw[16][68], sx[16][16 * J + 4];
+    const int tid = threadIdx.x, tr = tid & 15, tt = tid >> 4;      // rows 4 tr .., tokens J tt ..
+    const int n0 = blockIdx.x * 64, t0 = blockIdx.y * 16 * J;
     pdl_launch_dependents();
     pdl_wait();
     const float* in = reinterpret_cast<const float*>(l.in);
-    float acc[4][4] = {};
+    float acc[J][4] = {};
     const int row = tid >> 2, kq = (tid & 3) * 4;
     for (int k0 = 0; k0 < l.K; k0 += 16) {
         float4 a = make_float4(0, 0, 0, 0), b = a;
         if (n0 + row < l.N) a = act_load4(l.W + (size_t)(n0 + row) * l.K + k0 + kq);
-        if (t0 + row < T) b = act_load4(in + (size_t)(t0 + row) * l.ld_in + k0 + kq);
+        if (row < 16 * J && t0 + row < T) b = act_load4(in + (size_t)(t0 + row) * l.ld_in + k0 + kq);
         sw[kq][row] = a.x; sw[kq + 1][row] = a.y; sw[kq + 2][row] = a.z; sw[kq + 3][row] = a.w;
-        sx[kq][row] = b.x; sx[kq + 1][row] = b.y; sx[kq + 2][row] = b.z; sx[kq + 3][row] = b.w;
+        if (row < 16 * J) { sx[kq][row] = b.x; sx[kq + 1][row] = b.y; sx[kq + 2][row] = b.z; sx[kq + 3][row] = b.w; }
         __syncthreads();
-        float part[4][4] = {};      // a block's sum on its own: long sums then lose less
+        float part[J][4] = {};      // a block's sum on its own: long sums then lose less
 #pragma unroll
         for (int k = 0; k < 16; k++) {
             const float4 wv = *reinterpret_cast<const float4*>(&sw[k][4 * tr]);
-            const float4 xv = *reinterpret_cast<const float4*>(&sx[k][4 * tt]);
-            const float wr[4] = {wv.x, wv.y, wv.z, wv.w}, xr[4] = {xv.x, xv.y, xv.z, xv.w};
+            const float wr[4] = {wv.x, wv.y, wv.z, wv.w};
+            float xr[J];
+            if constexpr (J == 4) {
+                const float4 xv = *reinterpret_cast<const float4*>(&sx[k][4 * tt]);
+                xr[0] = xv.x; xr[1] = xv.y; xr[2] = xv.z; xr[3] = xv.w;
+            } else {
+                xr[0] = sx[k][tt];
+            }
 #pragma unroll
-            for (int j = 0; j < 4; j++)
+            for (int j = 0; j < J; j++)
 #pragma unroll
                 for (int i = 0; i < 4; i++) part[j][i] = fmaf(wr[i], xr[j], part[j][i]);
         }
 #pragma unroll
-        for (int j = 0; j < 4; j++)
+        for (int j = 0; j < J; j++)
 #pragma unroll
             for (int i = 0; i < 4; i++) acc[j][i] += part[j][i];
         __syncthreads();
     }
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const int t = t0 + 4 * tt + j;
+    for (int j = 0; j < J; j++) {
+        const int t = t0 + J * tt + j;
         if (t >= T) break;
         if (l.mode == kLinSwiglu) {
 #pragma unroll
@@ -602,7 +611,13 @@ int linear_forward(const Linear& l, int T, bool act_bf16, cudaStream_t s)
         return act_bf16 ? (one ? launch_vec<bf16, 1>(l, smem, s) : launch_vec<bf16, 2>(l, smem, s))
                         : (one ? launch_vec<float, 1>(l, smem, s) : launch_vec<float, 2>(l, smem, s));
     }
-    if (!act_bf16) return launch_ordered(k_linear_tile, dim3((l.N + 63) / 64, (T + 63) / 64), 256, 0, s, l, T);
+    if (!act_bf16) {
+        // narrow tiles while every SM has one at most (64 tokens of 2048 x 2048: 107 us wide, 83 narrow; 100 tokens: 107, 127), or where
+        // there is only one of either (12 tokens of 14336 x 2048: 197, 127)
+        const int n_tiles = (l.N + 63) / 64, narrow = (T + 15) / 16;
+        if (narrow == 1 || (long)n_tiles * narrow <= sm_count()) return launch_ordered(k_linear_tile<1>, dim3(n_tiles, narrow), 256, 0, s, l, T);
+        return launch_ordered(k_linear_tile<4>, dim3(n_tiles, (T + 63) / 64), 256, 0, s, l, T);
+    }
     const Tc5Tiles t = tc5_tiles(l, T);
     if (t.tokens > 128) return launch_tc5<256>(l, T, t, s);
     if (t.tokens > 64) return launch_tc5<128>(l, T, t, s);
