@@ -172,6 +172,7 @@ SIGNATURES = {
     "bpd_linear_bf16_cuda": (i32, [vp, vp, vp, i32, i32, i32, i32, vp]),
     "bpd_linear_map_cuda": (i32, [vp, vp, vp, i32, i32, i32, i32, vp, vp, f32, i32, vp]),
     "bpd_decayed_scan_cuda": (i32, [vp, i32, vp, i32, vp, i32, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp]),
+    "bpdq_decayed_scan_segments": (i32, [vp, i32, i32, i32, i32, i32]),
     "bpd_rotate_half_qk_cuda": (i32, [vp, vp, i32, i32, i32, i32, i32, vp, f32, vp, i32, vp]),
     "bpd_causal_conv_silu_cuda": (i32, [vp, i32, vp, i32, i32, i32, vp, vp, vp, i32, vp]),
     "bpd_gated_norm_cuda": (i32, [vp, i32, vp, i32, vp, vp, i32, i32, i32, i32, i32, i32, i32, f32, i32, vp]),

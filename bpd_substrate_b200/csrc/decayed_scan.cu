@@ -449,6 +449,9 @@ static int scan_segments(int heads, int key_pad, int value_pad, int T, int* per_
     return (chunks + per - 1) / per;
 }
 
+// The fold reads and writes 16 bytes of a state at a time: a state at any other address stays one chain, which does not.
+static bool folds(const void* state, const void* scratch) { return scratch && !(((uintptr_t)state | (uintptr_t)scratch) & 15); }
+
 static bool takes_chunks(int key_pad, int T, bool act_bf16) { return act_bf16 && T >= kChunkedMinTokens && key_pad <= 256; }
 
 size_t decayed_scratch_bytes(int heads, int key_pad, int value_pad, int T, bool act_bf16)
@@ -468,7 +471,7 @@ static int launch_chunks(const DecayedScan& a, int T, cudaStream_t s)
     const unsigned slices = (a.value_pad + 63) / 64;
     ScanSegments seg = {(T + kChunk - 1) / kChunk, nullptr, nullptr};
     int segments = 1;
-    if (a.scratch && (segments = scan_segments(a.heads, a.key_pad, a.value_pad, T, &seg.chunks)) > 1) {
+    if (folds(a.state, a.scratch) && (segments = scan_segments(a.heads, a.key_pad, a.value_pad, T, &seg.chunks)) > 1) {
         const int per_head = a.key_pad * a.value_pad;
         seg.states = (float*)a.scratch;
         seg.log_decay = seg.states + (size_t)segments * a.heads * per_head;
@@ -813,6 +816,13 @@ using namespace bpdq;
 
 extern "C" {
 
+int bpdq_decayed_scan_segments(const float* state, int n_tokens, int heads, int key_pad, int value_pad, int act_bf16)
+{
+    if (n_tokens < 1 || heads < 1 || key_pad < 16 || value_pad < 16) return 0;
+    int per;
+    return folds(state, state) && takes_chunks(key_pad, n_tokens, act_bf16 != 0) ? scan_segments(heads, key_pad, value_pad, n_tokens, &per) : 1;
+}
+
 int bpd_decayed_scan_cuda(const void* q, int ld_q, const void* k, int ld_k, const void* v, int ld_v, const float* decay, const float* log_decay,
                           const float* dt, const float* neg_exp_a, const float* d_skip, float* state, void* o, int ld_o, int n_tokens, int heads,
                           int groups, int key_pad, int value_pad, int act_bf16, void* stream)
@@ -832,7 +842,7 @@ int bpd_decayed_scan_cuda(const void* q, int ld_q, const void* k, int ld_k, cons
     a.o = o; a.ld_o = ld_o;
     // one segment where a capture cannot allocate the states of several
     const size_t scratch = decayed_scratch_bytes(heads, key_pad, value_pad, n_tokens, act_bf16 != 0);
-    if (scratch && !((uintptr_t)state & 15) && scratch_fits(nullptr, kScratchDelta, scratch, (cudaStream_t)stream)) {
+    if (scratch && folds(state, state) && scratch_fits(nullptr, kScratchDelta, scratch, (cudaStream_t)stream)) {
         int rc = 0;
         if (!(a.scratch = scratch_take(nullptr, kScratchDelta, scratch, (cudaStream_t)stream, &rc))) return rc;
     }

@@ -461,6 +461,9 @@ int bpd_linear_map_cuda(const uint16_t* W, const void* x, void* out, int n_token
 int bpd_decayed_scan_cuda(const void* q, int ld_q, const void* k, int ld_k, const void* v, int ld_v, const float* decay, const float* log_decay,
                           const float* dt, const float* neg_exp_a, const float* d_skip, float* state, void* o, int ld_o, int n_tokens, int heads,
                           int groups, int key_pad, int value_pad, int act_bf16, void* stream);
+/* Segments of a portion that run side by side, given scratch for their states: 1 (one chain per head) for short portions, for fp32
+ * activations and for a state that is not 16-byte aligned; 0 for sizes that are none.  `state` is not read. */
+int bpdq_decayed_scan_segments(const float* state, int n_tokens, int heads, int key_pad, int value_pad, int act_bf16);
 /* pairs (i, i + rot_dims / 2) of q and k turn by (pos + t) rot_freq[i], in place; then k *= k_scale */
 int bpd_rotate_half_qk_cuda(void* q, void* k, int ld, int n_tokens, int heads, int dim_pad, int rot_dims, const float* rot_freq, float k_scale,
                             const int32_t* pos, int act_bf16, void* stream);
