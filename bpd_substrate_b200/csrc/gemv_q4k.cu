@@ -590,7 +590,10 @@ int gemm_q4k_q8k(const uint8_t* W, const void* x, float* out, int tokens, int M,
     if (tokens >= many && layout == BPDQ_LAYOUT_BPD && xsrc == 0 && !dbg) {
         if (gemm_q4k_q8k_tc5_faster(tokens, M, K) && scratch_fits(ws, kScratchGemmActs, gemm_q4k_q8k_tc5_workspace(tokens, M, K), s))
             return gemm_q4k_q8k_tc5(W, reinterpret_cast<const float*>(x), out, tokens, M, K, s, ws);
-        return gemm_q4k_q8k_mma(W, reinterpret_cast<const float*>(x), out, tokens, M, K, s, ws);
+        // (a call of so few tokens needs no scratch, wherever its rows would be faster: without any it runs here)
+        const int always = weights >= (1L << 25) ? 2 : kMaxTokens;
+        if (tokens > always || scratch_fits(ws, kScratchGemmActs, gemm_q4k_q8k_mma_workspace(tokens, K), s))
+            return gemm_q4k_q8k_mma(W, reinterpret_cast<const float*>(x), out, tokens, M, K, s, ws);
     }
     return gemm_q4k_q8k_multi(1, &W, &out, &M, x, tokens, K, layout, xsrc, dbg, s);
 }

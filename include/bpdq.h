@@ -64,7 +64,8 @@ int bpdq_sm_count(void);
  *     was handed out is never freed before the process ends, so launches in flight and captured graphs that
  *     hold its address stay valid.  While a stream is being captured a block cannot grow: the call returns
  *     BPDQ_STATUS_ERR_CAPTURE and launches nothing -- make one call of that size on the stream before the
- *     capture (a warm-up run), or use the *_ws_cuda form. */
+ *     capture (a warm-up run), or use the *_ws_cuda form.  Up to 4 tokens of bpd_qmm_q4k_q8k_cuda and gpu_matmul_q4k (up to 2
+ *     where M * K >= 2^25) run without scratch where there is none, in either form. */
 
 /* ---- device memory helpers (additive, size_t) ------------------------------------------ */
 void* bpdq_alloc(size_t bytes);

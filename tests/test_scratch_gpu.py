@@ -5,7 +5,8 @@ import numpy as np
 import pytest
 
 from bpd_substrate_b200 import synth
-from tests.util import Dev
+from tests.test_gemm_q4k_gpu import TOL
+from tests.util import Dev, normwise
 
 pytestmark = pytest.mark.gpu
 
@@ -56,6 +57,32 @@ def test_two_streams_interleaved_equal_serial_results(lib):
     finally:
         lib.bpdq_stream_destroy(s1)
         lib.bpdq_stream_destroy(s2)
+
+
+# 2 to 4 tokens of shapes that are faster with scratch: many short rows, 8192 rows, beyond 2^22 weights, beyond 2^25
+@pytest.mark.parametrize("tokens,N,K", [(2, 14336, 512), (3, 8192, 256), (4, 8192, 256), (4, 1100, 4096), (2, 16384, 2048)])
+def test_a_few_tokens_need_no_scratch(lib, oracle, tokens, N, K):
+    """On a stream that is captured before its first call, and in a workspace that holds nothing, such calls run all the same."""
+    rng = np.random.default_rng(tokens * N)
+    W, X = synth.q4k_matrix(N, K, rng), synth.activations(K, rng, rows=tokens)
+    want = oracle.qmm_q4k_q8k(W, X, tokens, N, K)[1]
+    dW, dX, ws = Dev(lib, W), Dev(lib, X), Dev(lib, nbytes=256)
+    cold, small = Dev(lib, nbytes=4 * tokens * N, fill=0xFF), Dev(lib, nbytes=4 * tokens * N, fill=0xFF)
+    assert lib.bpd_qmm_q4k_q8k_ws_cuda(dW.ptr, dX.ptr, small.ptr, tokens, N, K, 0, 0, None, ws.ptr, 256, None) == 0
+    s = lib.bpdq_stream_create()
+    try:
+        assert lib.bpdq_graph_begin(s) == 0
+        rc = lib.bpd_qmm_q4k_q8k_cuda(dW.ptr, dX.ptr, cold.ptr, tokens, N, K, 0, 0, None, s)
+        graph = lib.bpdq_graph_end(s)
+        assert rc == 0 and graph
+        assert lib.bpdq_graph_launch(graph, s) == 0
+        lib.bpdq_sync()
+        lib.bpdq_graph_destroy(graph)
+    finally:
+        lib.bpdq_stream_destroy(s)
+    assert lib.bpdq_last_status() == 0
+    for out in (cold, small):
+        assert normwise(out.read(np.float32).reshape(tokens, N), want) <= TOL
 
 
 def test_workspace_too_small_is_refused(lib):
