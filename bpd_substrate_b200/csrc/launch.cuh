@@ -1,6 +1,7 @@
 // Launch helpers of the forward passes.
 #pragma once
 #include "bpdq_common.cuh"
+#include "per_device.h"
 
 namespace bpdq {
 
@@ -56,31 +57,33 @@ static int allow_smem(int bytes)
 }
 
 // Clusters of 1 .. 8 CTAs of a kernel that run at once on the current device, asked for once per device; null after a CUDA error.
+struct ClusterCounts { int at_once[9] = {0}; };      // [CTAs of a cluster]
 template <auto Kern>
 static const int* active_clusters(int block, int smem)
 {
-    static int known[64][9] = {{0}};
+    static PerDevice<ClusterCounts> known;
     int dev = 0;
-    cudaGetDevice(&dev);
-    int* n = known[dev >= 0 && dev < 64 ? dev : 0];
-    if (n[1]) return n;
-    if (allow_smem<Kern>(227 * 1024)) return nullptr;
-    for (int ctas = 8; ctas >= 1; ctas--) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(1, (unsigned)ctas);
-        cfg.blockDim = dim3((unsigned)block);
-        cfg.dynamicSmemBytes = (size_t)smem;
-        cudaLaunchAttribute at;
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = at.val.clusterDim.z = 1;
-        at.val.clusterDim.y = (unsigned)ctas;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        int fit = 0;
-        if (cudaOccupancyMaxActiveClusters(&fit, Kern, &cfg) != cudaSuccess) (void)cudaGetLastError();
-        n[ctas] = fit > 0 ? fit : sm_count() / ctas;      // (n[1] last: it says that the others are known)
-    }
-    return n;
+    if (check_cuda(cudaGetDevice(&dev))) return nullptr;
+    const ClusterCounts* counts = known.get(dev, [&](ClusterCounts& c) {
+        if (allow_smem<Kern>(227 * 1024)) return false;
+        for (int ctas = 1; ctas <= 8; ctas++) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(1, (unsigned)ctas);
+            cfg.blockDim = dim3((unsigned)block);
+            cfg.dynamicSmemBytes = (size_t)smem;
+            cudaLaunchAttribute at;
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = at.val.clusterDim.z = 1;
+            at.val.clusterDim.y = (unsigned)ctas;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            int fit = 0;
+            if (cudaOccupancyMaxActiveClusters(&fit, Kern, &cfg) != cudaSuccess) (void)cudaGetLastError();
+            c.at_once[ctas] = fit > 0 ? fit : sm_count() / ctas;
+        }
+        return true;
+    });
+    return counts ? counts->at_once : nullptr;
 }
 
 }  // namespace bpdq

@@ -1,0 +1,64 @@
+"""The table of values per device (csrc/per_device.h) under threads that ask for the first time at once, in a host program."""
+import os
+import subprocess
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "bpd_substrate_b200", "csrc")
+
+PROGRAM = r"""
+#include "per_device.h"
+#include <cstdio>
+#include <thread>
+#include <vector>
+struct Counts { int n[9] = {0}; };
+static bpdq::PerDevice<Counts> table;
+static std::atomic<int> fills{0}, wrong{0};
+static const Counts* ask(int dev, bool works = true)
+{
+    return table.get(dev, [&](Counts& c) {
+        fills++;
+        for (int i = 1; i < 9; i++) {
+            c.n[i] = works ? 100 * dev + i : 0;
+            std::this_thread::yield();
+        }
+        return works;
+    });
+}
+int main()
+{
+    if (ask(3, false) || fills != 1) return 1;                                     // a failure is not kept
+    std::vector<std::thread> threads;
+    for (int t = 0; t < 16; t++)
+        threads.emplace_back([] {
+            for (int k = 0; k < 64; k++)
+                for (int dev : {3, 0, 63}) {
+                    const Counts* c = ask(dev);
+                    for (int i = 1; i < 9; i++) wrong += !c || c->n[i] != 100 * dev + i;
+                }
+        });
+    for (auto& t : threads) t.join();
+    if (wrong || fills != 1 + 3) return 2;                                         // worked out once per device, never seen half filled
+    for (int dev : {64, 70, -1, 0}) {                                              // a device beyond the table has its own answer
+        const Counts* c = ask(dev);
+        if (!c || c->n[8] != 100 * dev + 8) return 3;
+    }
+    std::puts("ok");
+    return 0;
+}
+"""
+
+
+def build_and_run(tmp_path, *flags):
+    src, exe = tmp_path / "main.cpp", tmp_path / "main"
+    src.write_text(PROGRAM)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", *flags, "-I", CSRC, str(src), "-o", str(exe)], check=True, capture_output=True)
+    return subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+
+
+def test_first_calls_at_once(tmp_path):
+    r = build_and_run(tmp_path)
+    assert r.returncode == 0 and r.stdout == "ok\n", (r.returncode, r.stderr)
+
+
+def test_no_data_race(tmp_path):
+    r = build_and_run(tmp_path, "-fsanitize=thread", "-g")
+    assert r.returncode == 0 and "data race" not in r.stderr, r.stderr[-2000:]
