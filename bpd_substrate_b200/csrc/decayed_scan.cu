@@ -113,34 +113,39 @@ __global__ void __launch_bounds__(256) k_decayed_recurrence(DecayedScan a, int T
 
 constexpr int kChunk = 64;
 
-template <int NMAX>
+// A portion's only segment; one of several: what it adds to a state of zeros; its outputs from the state before it.
+enum ChunkTask { kWholePortion, kSegmentState, kSegmentOutputs };
+
+template <int NMAX, int TASK>
 struct ChunkShape {
     static constexpr int kLdN = NMAX + 8, kLdV = 72, kLdO = 68;
     static constexpr size_t kQK = (size_t)kChunk * kLdN * 2, kV = (size_t)kChunk * kLdV * 2;
     static constexpr size_t kO = (size_t)kChunk * kLdO * 4;
     // the joined outputs of a chunk take the place of its queries, which nobody reads any more, where these are as large: two CTAs per SM
     // for heads of 65 to 128 keys
-    static constexpr bool kOverQ = kQK >= kO;
+    static constexpr bool kOverQ = TASK != kWholePortion && kQK >= kO;
     static constexpr size_t kSmem = 2 * (2 * kQK + kV) + 2 * kV + (kOverQ ? 0 : kO) + 5 * kChunk * 4;
-    static constexpr int kPerSm = NMAX <= 128 ? 2 : 1;
+    static constexpr int kPerSm = TASK != kWholePortion && NMAX <= 128 ? 2 : 1;
 };
 
 // A prompt's portion is cut into segments that run side by side: a first launch takes every segment but the last from a state of
 // zeros to what it adds, k_decayed_fold makes the segments' starting states of that, and a second launch works the segments out.
 struct ScanSegments {
     int chunks;             // per segment
-    float* states;          // [segments][heads][key_pad][value_pad]: the state before a segment; null: one segment, from and to a.state
+    float* states;          // [segments][heads][key_pad][value_pad]: the state before a segment
     float* log_decay;       // [segments][heads]: of a whole segment
 };
 
 // One CTA: one head, 64 value columns, a segment's tokens.  Eight warps: value rows 16 (w & 3) .. + 15 of the transposed state
 // and half (w >> 2) of its keys.  Bound by the chain of barriers from chunk to chunk, so the chip wants many short chains: 2048 tokens
 // of 8 heads of 256 x 256 as one chain per CTA (32 CTAs) 272 us, of 64 heads of 128 x 64 (64 CTAs) 192 us; in four segments about 160 and 90 us with both launches and the fold.
-// STATE: only what the segment adds to a state of zeros.
-template <int NMAX, bool STATE>
-__global__ void __launch_bounds__(256, ChunkShape<NMAX>::kPerSm) k_decayed_chunks(DecayedScan a, int tokens, ScanSegments seg)
+// A short portion is bound by the fetch of instructions that run once or twice, so it has an instantiation that knows of no segments (a state's
+// place chosen at run time was a fifth more code: 64 tokens of 8 heads of 256 x 256 14.1 us, 11.8 without; of 64 heads of 128 x 64 10.4, 8.0).
+template <int NMAX, int TASK>
+__global__ void __launch_bounds__(256, ChunkShape<NMAX, TASK>::kPerSm) k_decayed_chunks(DecayedScan a, int tokens, ScanSegments seg)
 {
-    using S = ChunkShape<NMAX>;
+    using S = ChunkShape<NMAX, TASK>;
+    constexpr bool STATE = TASK == kSegmentState, WHOLE = TASK == kWholePortion;
     constexpr int LDN = S::kLdN, LDV = S::kLdV, LDO = S::kLdO;
     constexpr int NH = NMAX / 2, NTILES = NH / 8;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -158,7 +163,7 @@ __global__ void __launch_bounds__(256, ChunkShape<NMAX>::kPerSm) k_decayed_chunk
     const int h = blockIdx.x, grp = h / (a.heads / a.groups), p0 = blockIdx.y * 64;
     const int p_n = a.value_pad - p0 < 64 ? a.value_pad - p0 : 64;
     const int Np = a.key_pad;
-    const int first = blockIdx.z * seg.chunks * kChunk, T = tokens - first < seg.chunks * kChunk ? tokens - first : seg.chunks * kChunk;
+    const int first = WHOLE ? 0 : blockIdx.z * seg.chunks * kChunk, T = WHOLE || tokens - first < seg.chunks * kChunk ? tokens - first : seg.chunks * kChunk;
     const bf16* gq = reinterpret_cast<const bf16*>(a.q) + (size_t)first * a.ld_q + grp * Np;
     const bf16* gk = reinterpret_cast<const bf16*>(a.k) + (size_t)first * a.ld_k + grp * Np;
     const bf16* gv = reinterpret_cast<const bf16*>(a.v) + (size_t)first * a.ld_v + h * a.value_pad + p0;
@@ -210,7 +215,7 @@ __global__ void __launch_bounds__(256, ChunkShape<NMAX>::kPerSm) k_decayed_chunk
 
     // the state, transposed: rows p = 16 pw + .., columns n = NH half + ..
     float st[NTILES][4];
-    float* gs = (seg.states ? seg.states + ((size_t)blockIdx.z * a.heads + h) * Np * a.value_pad : a.state + (size_t)h * Np * a.value_pad) + p0;
+    float* gs = (WHOLE ? a.state + (size_t)h * Np * a.value_pad : seg.states + ((size_t)blockIdx.z * a.heads + h) * Np * a.value_pad) + p0;
 #pragma unroll
     for (int j = 0; j < NTILES; j++)
 #pragma unroll
@@ -386,7 +391,7 @@ __global__ void __launch_bounds__(256, ChunkShape<NMAX>::kPerSm) k_decayed_chunk
     if (STATE) {
         gs += (size_t)a.heads * Np * a.value_pad;
         if (tid == 0 && blockIdx.y == 0) seg.log_decay[blockIdx.z * a.heads + h] = whole;
-    } else if (seg.states) {
+    } else if (!WHOLE) {
         if (blockIdx.z + 1 < gridDim.z) return;
         gs = a.state + (size_t)h * Np * a.value_pad + p0;
     }
@@ -462,24 +467,28 @@ size_t decayed_scratch_bytes(int heads, int key_pad, int value_pad, int T, bool 
     return segments < 2 ? 0 : (size_t)segments * heads * ((size_t)key_pad * value_pad + 1) * sizeof(float);
 }
 
+template <int NMAX, int TASK>
+static int launch_task(const DecayedScan& a, int T, int segments, const ScanSegments& seg, cudaStream_t s)
+{
+    constexpr size_t smem = ChunkShape<NMAX, TASK>::kSmem;
+    const int rc = allow_smem<k_decayed_chunks<NMAX, TASK>>((int)smem);
+    if (rc) return rc;
+    return launch_ordered(k_decayed_chunks<NMAX, TASK>, dim3(a.heads, (a.value_pad + 63) / 64, segments), 256, smem, s, a, T, seg);
+}
+
 template <int NMAX>
 static int launch_chunks(const DecayedScan& a, int T, cudaStream_t s)
 {
-    constexpr size_t smem = ChunkShape<NMAX>::kSmem;
-    int rc = allow_smem<k_decayed_chunks<NMAX, false>>((int)smem);
-    if (rc) return rc;
-    const unsigned slices = (a.value_pad + 63) / 64;
-    ScanSegments seg = {(T + kChunk - 1) / kChunk, nullptr, nullptr};
-    int segments = 1;
-    if (folds(a.state, a.scratch) && (segments = scan_segments(a.heads, a.key_pad, a.value_pad, T, &seg.chunks)) > 1) {
-        const int per_head = a.key_pad * a.value_pad;
-        seg.states = (float*)a.scratch;
-        seg.log_decay = seg.states + (size_t)segments * a.heads * per_head;
-        if ((rc = allow_smem<k_decayed_chunks<NMAX, true>>((int)smem))) return rc;
-        if ((rc = launch_ordered(k_decayed_chunks<NMAX, true>, dim3(a.heads, slices, segments - 1), 256, smem, s, a, T, seg))) return rc;
-        if ((rc = launch_ordered(k_decayed_fold, (a.heads * per_head / 4 + 255) / 256, 256, 0, s, a.state, seg, segments, a.heads, per_head))) return rc;
-    }
-    return launch_ordered(k_decayed_chunks<NMAX, false>, dim3(a.heads, slices, segments), 256, smem, s, a, T, seg);
+    ScanSegments seg = {0, nullptr, nullptr};
+    const int segments = folds(a.state, a.scratch) ? scan_segments(a.heads, a.key_pad, a.value_pad, T, &seg.chunks) : 1;
+    if (segments < 2) return launch_task<NMAX, kWholePortion>(a, T, 1, seg, s);
+    const int per_head = a.key_pad * a.value_pad;
+    seg.states = (float*)a.scratch;
+    seg.log_decay = seg.states + (size_t)segments * a.heads * per_head;
+    int rc;
+    if ((rc = launch_task<NMAX, kSegmentState>(a, T, segments - 1, seg, s))) return rc;
+    if ((rc = launch_ordered(k_decayed_fold, (a.heads * per_head / 4 + 255) / 256, 256, 0, s, a.state, seg, segments, a.heads, per_head))) return rc;
+    return launch_task<NMAX, kSegmentOutputs>(a, T, segments, seg, s);
 }
 
 int decayed_scan(const DecayedScan& a, int T, bool act_bf16, cudaStream_t s)
