@@ -518,24 +518,25 @@ __global__ void __launch_bounds__(256) k_latent_attn_rows(LatentShape p, const A
 // Threads that share a column of a CTA's slice, each with some of the splits.
 __host__ __device__ inline int latent_phases(int slice) { return slice >= 512 ? 2 : slice >= 256 ? 4 : 8; }
 
-// grid (heads, value columns / 32, tokens): joins the splits, then W_uv: a warp has four value columns, whose weights are requested
-// before the launch ahead has finished.  The CTAs of a head are a cluster where they are at most eight: each joins the splits of its
-// slice of the latent columns and hands the sums to the others.  Bound by the latency of reading the splits: 16 heads, 148 splits of 512
-// columns, 4 CTAs per head that each joined all of them (74 rounds of two threads per column): 20 us; a slice of 128 columns with
-// eight threads per column 14 us (a decoded token at 4000 keys, two such layers, 295 -> 283 us).
-template <typename A>
+// Joins the splits, then W_uv: a warp has four value columns, whose weights are requested before the launch ahead has finished.
+// SHARED, grid (heads, value columns / 32, tokens): the CTAs of a head are a cluster; each joins the splits of its slice of the latent
+// columns and hands the sums to the others.  Else, grid (value columns / 32, heads, tokens): each joins all of them.
+// Bound by the latency of reading the splits: 16 heads, 148 splits of 512 columns, 4 CTAs per head that each joined all of them (74 rounds of
+// two threads per column): 20 us; a slice of 128 columns with eight threads per column 14 us (a decoded token at 4000 keys, two such
+// layers, 295 -> 283 us).
+template <typename A, bool SHARED>
 __global__ void __launch_bounds__(256) k_latent_values(LatentShape p, float* partial, int splits, const bf16* __restrict__ w_uv, A* o,
                                                        const int* pos_p, int T)
 {
     extern __shared__ __align__(16) float lat[];      // [rank_pad], then [phases][slice], then [splits] weights
-    const int ranks = (int)cluster_size(), slice = (p.rank_pad / 4 + ranks - 1) / ranks * 4, phases = latent_phases(slice);
+    const int ranks = SHARED ? (int)cluster_size() : 1, slice = (p.rank_pad / 4 + ranks - 1) / ranks * 4, phases = latent_phases(slice);
     float* part = lat + p.rank_pad;
     float* sw = part + phases * slice;
-    const int h = blockIdx.x, t = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int h = SHARED ? blockIdx.x : blockIdx.y, t = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long row = (long)t * p.heads + h;
     pdl_launch_dependents();
-    if (ranks > 1) cluster_arrive();        // (everybody is there before anybody's shared memory is written)
-    const int c0 = blockIdx.y * 32 + 4 * warp;
+    if (SHARED) cluster_arrive();        // (everybody is there before anybody's shared memory is written)
+    const int c0 = (SHARED ? blockIdx.y : blockIdx.x) * 32 + 4 * warp;
     const bf16* w = w_uv + ((size_t)h * p.value_pad + c0) * p.rank_pad;
     uint4 u[4][2];                                     // the first 512 latent columns
 #pragma unroll
@@ -573,7 +574,7 @@ __global__ void __launch_bounds__(256) k_latent_values(LatentShape p, float* par
     __syncthreads();
     // this CTA's slice, four columns per thread
     const float* sums = partial_sums(partial, row, 0, splits, p.rank_pad);
-    const int first = (int)cluster_rank() * slice, n = min(slice, p.rank_pad - first), lanes = 256 / phases, phase = tid / lanes;
+    const int first = SHARED ? (int)cluster_rank() * slice : 0, n = min(slice, p.rank_pad - first), lanes = 256 / phases, phase = tid / lanes;
     for (int c = 4 * (tid % lanes); c < n; c += 4 * lanes) {
         float4 v = make_float4(0, 0, 0, 0);
 #pragma unroll 8
@@ -587,15 +588,15 @@ __global__ void __launch_bounds__(256) k_latent_values(LatentShape p, float* par
         *reinterpret_cast<float4*>(part + phase * slice + c) = v;
     }
     __syncthreads();
-    if (ranks > 1) cluster_wait();
+    if (SHARED) cluster_wait();
     for (int c = tid; c < n; c += 256) {
         float v = part[c];
         for (int i = 1; i < phases; i++) v += part[i * slice + c];
-        if (ranks == 1) lat[c] = v;
+        if (!SHARED) lat[c] = v;
         else
             for (int r = 0; r < ranks; r++) store_peer(lat + first + c, r, v);
     }
-    if (ranks > 1) {
+    if (SHARED) {
         cluster_arrive();
         cluster_wait();
     } else {
@@ -830,7 +831,7 @@ static int launch_latent_mma(const LatentShape& p, const bf16* q, const bf16* ca
 
 template <typename A>
 static int attend_latents(const LatentShape& p, const void* q, const bf16* w_ukv, const void* cache, void* o, const LatentBuffers& b,
-                          const int* pos, int T, cudaStream_t s)
+                          const int* pos, int T, int context, cudaStream_t s)
 {
     constexpr bool kBf16 = sizeof(A) == 2;
     int rc = T == 1 ? launch_latent_queries<A, 1>(p, q, w_ukv, b.q_latent, pos, T, s) : launch_latent_queries<A, 4>(p, q, w_ukv, b.q_latent, pos, T, s);
@@ -857,17 +858,24 @@ static int attend_latents(const LatentShape& p, const void* q, const bf16* w_ukv
     }
     if (rc) return rc;
     const bf16* w_uv = w_ukv + (size_t)p.heads * p.dim_pad * p.rank_pad;
-    const unsigned parts = (p.value_pad + 31) / 32, ranks = parts <= 8 ? parts : 1;
+    // A cluster costs about 1 us and a step of two splits 0.1 us, less where many CTAs hide it: one token always shares (its launch may be
+    // recorded and replayed at any context), several from these splits with keys on.  Alone, shared (us; 16 heads, ranks of 512, values of 128): 4 tokens of
+    // 100 keys (2 splits) 16.3, 17.2; of 4000 (63) 27.9, 21.6; 16 tokens of 100 23.4, 26.5; of 4000 (16) 44.4, 43.7.
+    const unsigned parts = (p.value_pad + 31) / 32;
+    const int blocks = (context + kKeyBlock - 1) / kKeyBlock, per = (blocks + splits - 1) / splits, used = (blocks + per - 1) / per;
+    const unsigned ranks = parts > 1 && parts <= 8 && (T == 1 || used > 8 + T / 2) ? parts : 1;
     const int slice = (p.rank_pad / 4 + (int)ranks - 1) / (int)ranks * 4;
-    return launch_cluster(k_latent_values<A>, dim3(p.heads, parts, T), dim3(1, ranks, 1), 256, (size_t)(p.rank_pad + latent_phases(slice) * slice + splits) * 4, s,
-                          p, b.partial, splits, w_uv, (A*)o, pos, T);
+    const size_t smem = (size_t)(p.rank_pad + latent_phases(slice) * slice + splits) * 4;
+    if (ranks > 1)
+        return launch_cluster(k_latent_values<A, true>, dim3(p.heads, parts, T), dim3(1, ranks, 1), 256, smem, s, p, b.partial, splits, w_uv, (A*)o, pos, T);
+    return launch_ordered(k_latent_values<A, false>, dim3(parts, p.heads, T), 256, smem, s, p, b.partial, splits, w_uv, (A*)o, pos, T);
 }
 
 int latent_attention(const LatentShape& p, void* q, const bf16* w_ukv, const void* cache, void* o, const LatentBuffers& b, const int* pos,
                      int T, int context, bool act_bf16, cudaStream_t s)
 {
     if (!latent_expands(p, T, act_bf16))
-        return act_bf16 ? attend_latents<bf16>(p, q, w_ukv, cache, o, b, pos, T, s) : attend_latents<float>(p, q, w_ukv, cache, o, b, pos, T, s);
+        return act_bf16 ? attend_latents<bf16>(p, q, w_ukv, cache, o, b, pos, T, context, s) : attend_latents<float>(p, q, w_ukv, cache, o, b, pos, T, context, s);
     Linear l = {};
     l.W = w_ukv;
     l.in = cache;
