@@ -612,10 +612,10 @@ int linear_forward(const Linear& l, int T, bool act_bf16, cudaStream_t s)
                         : (one ? launch_vec<float, 1>(l, smem, s) : launch_vec<float, 2>(l, smem, s));
     }
     if (!act_bf16) {
-        // narrow tiles while every SM has one at most (64 tokens of 2048 x 2048: 107 us wide, 83 narrow; 100 tokens: 107, 127), or where
-        // there is only one of either (12 tokens of 14336 x 2048: 197, 127)
+        // narrow tiles while every SM has one at most (64 tokens of 2048 x 2048: 107 us wide, 83 narrow; 100 tokens: 107, 127), or two where 16
+        // tokens are all there are (12 tokens of 14336 x 2048: 264, 214; of 22000 x 2048: 281, 324)
         const int n_tiles = (l.N + 63) / 64, narrow = (T + 15) / 16;
-        if (narrow == 1 || (long)n_tiles * narrow <= sm_count()) return launch_ordered(k_linear_tile<1>, dim3(n_tiles, narrow), 256, 0, s, l, T);
+        if ((long)n_tiles * narrow <= (narrow == 1 ? 2 : 1) * sm_count()) return launch_ordered(k_linear_tile<1>, dim3(n_tiles, narrow), 256, 0, s, l, T);
         return launch_ordered(k_linear_tile<4>, dim3(n_tiles, (T + 63) / 64), 256, 0, s, l, T);
     }
     const Tc5Tiles t = tc5_tiles(l, T);
