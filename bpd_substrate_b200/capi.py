@@ -91,6 +91,7 @@ SIGNATURES = {
     "bpd_kv_cache_write_f16_cuda": (i32, [vp, vp, vp, i32, i32, i32, i32, vp]),
     "bpd_kv_cache_write_cuda": (i32, [vp, vp, vp, i32, i32, i32, i32, vp]),
     "bpd_gqa_attn_cuda": (i32, [vp, vp, vp, vp, i32, i32, i32, i32, i32, f32, i32, i32, vp]),
+    "bpdq_gqa_attn_kernel": (i32, [i32] * 7),
     "bpd_swiglu_fuse_cuda": (i32, [vp, vp, vp, i32, vp]),
     "bpd_argmax_dim_cuda": (i32, [vp, vp, i32, i32, i32, vp]),
     "bpd_llama_block_cuda": (i32, [vp, vp, vp, vp, i32, i32, vp, vp, vp, vp, vp, vp, vp]),

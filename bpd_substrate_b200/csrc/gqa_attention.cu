@@ -11,6 +11,7 @@
 #include "cluster_device.cuh"
 #include "launch.cuh"
 #include "mma_device.cuh"
+#include "../../include/bpdq.h"
 
 #include <cuda_fp16.h>
 
@@ -604,13 +605,13 @@ static int launch_tile(const GqaShape& p, const float* q, const void* k, const v
                           reinterpret_cast<const __half*>(k), reinterpret_cast<const __half*>(v), dst);
 }
 
-int gqa_attention(const GqaShape& p, const float* q, const void* k, const void* v, float* dst, cudaStream_t s)
+enum { kGeneral, kSplit, kTile };      // k_gqa_attn, k_gqa_split, k_gqa_tile
+static int gqa_kernel(const GqaShape& p)
 {
-    if (p.kv_offset < 0 || (p.dim != 64 && p.dim != 128)) return 1;
-    if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)dst) & 15) return 1;
+    if (p.kv_offset < 0 || (p.dim != 64 && p.dim != 128)) return kGeneral;
     const long sees = (long)p.kv_offset + p.n_q < p.n_kv ? (long)p.kv_offset + p.n_q : p.n_kv;
     const long rep = p.heads / p.kv_heads, rows = (long)p.n_q * rep, blocks = (rows + kTileRowsQ - 1) / kTileRowsQ;
-    if (sees <= kShortKeys || blocks > 65535 || p.n_q > 65535) return 1;
+    if (sees <= kShortKeys || blocks > 65535 || p.n_q > 65535) return kGeneral;
     // Time per 64 keys, fitted to 20 shapes of 1 to 2048 queries and 65 to 16001 keys: a tile CTA 0.5 + 0.014 dim us, two per SM at
     // a time, whatever few rows it has; the split kernel 0.64 + 0.011 (heads of a group) dim ns for every query and group.
     // Measured sides of the line (tile, split; us): 32/8 heads of 128, 532 keys, 32 queries 25, 18; 2128 keys, 128 queries
@@ -618,10 +619,36 @@ int gqa_attention(const GqaShape& p, const float* q, const void* k, const void* 
     const long group = rep > 2 ? 4 : rep, groups = (rep + group - 1) / group;
     const double tile_us = (double)((p.kv_heads * blocks + 2 * sm_count() - 1) / (2 * sm_count())) * (0.5 + 0.014 * p.dim);
     const double split_us = 1e-3 * (double)p.n_q * (double)(p.kv_heads * groups) * (0.64 + 0.011 * (double)group * p.dim);
-    const bool tile = p.f16 && tile_us < split_us;
-    if (tile) return p.dim == 64 ? launch_tile<64>(p, q, k, v, dst, s) : launch_tile<128>(p, q, k, v, dst, s);
+    if (p.f16 && tile_us < split_us) return kTile;
+    // fp32 heads of 64 that share nothing, short prompts: a CTA here costs 11 ns of the chip's time whatever few keys its query sees, there 0.1 ns
+    // a key and 5 to 9 ns.  100 tokens of 32 heads: 29.9 us there, 35.2 here; 200: 78.7, 78.6; 65 of 16 heads: 11.4, 12.6; 10 keys further on 13.8, 12.9.
+    if (!p.f16 && rep == 1 && p.dim == 64) {
+        const double waves = (double)p.n_q * p.heads / (8.0 * sm_count()), line = 28.0 + 17.0 * waves;
+        if (p.kv_offset + 0.5 * (p.n_q + 1) <= (line < 102.0 ? line : 102.0)) return kGeneral;
+    }
+    return kSplit;
+}
+
+int gqa_attention(const GqaShape& p, const float* q, const void* k, const void* v, float* dst, cudaStream_t s)
+{
+    if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)dst) & 15) return 1;
+    const int kernel = gqa_kernel(p);
+    if (kernel == kGeneral) return 1;
+    if (kernel == kTile) return p.dim == 64 ? launch_tile<64>(p, q, k, v, dst, s) : launch_tile<128>(p, q, k, v, dst, s);
     if (p.f16) return p.dim == 64 ? launch_split<1, 64>(p, q, k, v, dst, s) : launch_split<1, 128>(p, q, k, v, dst, s);
     return p.dim == 64 ? launch_split<0, 64>(p, q, k, v, dst, s) : launch_split<0, 128>(p, q, k, v, dst, s);
 }
 
 }  // namespace bpdq
+
+using namespace bpdq;
+
+extern "C" {
+
+int bpdq_gqa_attn_kernel(int n_q_tokens, int n_kv, int n_q_heads, int n_kv_heads, int head_dim, int kv_offset, int kv_is_f16)
+{
+    if (n_q_tokens < 1 || n_kv < 1 || n_q_heads < 1 || n_kv_heads < 1 || n_q_heads % n_kv_heads) return -1;
+    return gqa_kernel(GqaShape{n_q_tokens, n_kv, n_q_heads, n_kv_heads, head_dim, 1.0f, kv_offset, kv_is_f16});
+}
+
+}  // extern "C"

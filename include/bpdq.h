@@ -419,6 +419,8 @@ int bpd_kv_cache_write_cuda(float* cache, const float* src, const int32_t* pos_i
                             int max_seq_len, void* stream);
 int bpd_gqa_attn_cuda(const float* q, const void* k, const void* v, float* dst, int n_q_tokens, int n_kv, int n_q_heads,
                       int n_kv_heads, int head_dim, float scale, int kv_offset, int kv_is_f16, void* stream);
+/* which kernel that takes: 0 a CTA per query and head (sums in the reference's order), 1 keys over a cluster, 2 tiles of 64 x 64; -1 bad sizes */
+int bpdq_gqa_attn_kernel(int n_q_tokens, int n_kv, int n_q_heads, int n_kv_heads, int head_dim, int kv_offset, int kv_is_f16);
 int bpd_swiglu_fuse_cuda(const float* gate, const float* up, float* dst, int n, void* stream);
 int bpd_argmax_dim_cuda(const float* x, long long* out, int outer, int dim_size, int inner, void* stream);
 int bpd_llama_block_cuda(float* x, const bpd_llama_layer_weights* lw, const bpd_llama_config* cfg, const int32_t* pos_ids,

@@ -80,3 +80,24 @@ def test_values_that_are_not_finite_reach_only_the_queries_that_see_them(lib):
     clean[90:, 4:8] = False
     assert np.abs(got - want)[clean].max() <= 1e-5 * np.abs(want).max()
     assert np.isposinf(got[70:, 12:16, 5]).all() and np.isnan(got[90:, 4:8]).all()
+
+
+# queries, keys before them, heads, key heads, head size, fp16: kernel (0 a CTA per query and head, 1 keys over a cluster, 2 tiles)
+@pytest.mark.parametrize("T,off,H,HKV,D,f16,kernel", [
+    (1, 63, 32, 8, 128, 1, 0), (1, 64, 32, 8, 128, 1, 1), (300, 0, 32, 8, 128, 1, 2), (300, 0, 32, 8, 128, 0, 1), (300, 0, 32, 8, 96, 1, 0),
+    # fp32 heads of 64 that share nothing: short prompts, those a few keys further on, long ones
+    (65, 0, 16, 16, 64, 0, 0), (65, 10, 16, 16, 64, 0, 1), (100, 0, 32, 32, 64, 0, 0), (65, 30, 32, 32, 64, 0, 1), (210, 0, 32, 32, 64, 0, 1),
+    (128, 0, 32, 16, 64, 0, 1)])
+def test_kernel_of_a_call(T, off, H, HKV, D, f16, kernel):
+    """On 148 SMs, which are assumed where there is no device."""
+    from bpd_substrate_b200 import capi
+    assert capi.load().bpdq_gqa_attn_kernel(T, off + T, H, HKV, D, off, f16) == kernel
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,off", [(65, 0), (65, 10), (100, 0)])
+def test_short_prompts_of_unshared_fp32_heads(lib, T, off):
+    """Both kernels that such prompts take."""
+    q, k, v = inputs(T, off + T, 16, 16, 64, np.float32, T)
+    got, want = attend(lib, q, k, v, off, np.float32(0.125), off + T), expected(q, k, v, off, 0.125, off + T)
+    assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
