@@ -119,6 +119,7 @@ SIGNATURES = {
     "bpd_qmatmul_q4k_q8k_batch_static_cuda": (i32, [i32, vp, vp]),
     "bpdq_batch_static_capacity": (sz, []),
     "bpd_qmm_q4k_q8k_cuda": (i32, [vp, vp, vp, i32, i32, i32, i32, i32, vp, vp]),
+    "bpdq_qmm_q4k_q8k_kernel": (i32, [i32] * 3),
     "bpdq_qmm_q4k_q8k_workspace_bytes": (sz, [i32, i32, i32]),
     "bpd_qmm_q4k_q8k_ws_cuda": (i32, [vp, vp, vp, i32, i32, i32, i32, i32, vp, vp, sz, vp]),
     "bpd_qmm_q4k_q8k_mma_ints_cuda": (i32, [vp, vp, vp, vp, i32, i32, i32, vp]),

@@ -86,10 +86,11 @@ bool peer_targets_for(const void* lo, const void* hi, PeerTargets& t);
 int gemm_q4k_q8k_mma(const uint8_t* W, const float* X, float* out, int tokens, int N, int K, cudaStream_t s,
                      Workspace* ws = nullptr, int32_t* sb_ints = nullptr);
 size_t gemm_q4k_q8k_mma_workspace(int tokens, int K);
+double gemm_q4k_q8k_mma_us(int tokens, int N, int K);      // expected time
 int gemm_q4k_q8k_tc5(const uint8_t* W, const float* X, float* out, int tokens, int N, int K, cudaStream_t s,
                      Workspace* ws = nullptr, int32_t* sb_ints = nullptr);
 size_t gemm_q4k_q8k_tc5_workspace(int tokens, int N, int K);
-bool gemm_q4k_q8k_tc5_faster(int tokens, int N, int K);
+double gemm_q4k_q8k_tc5_us(int tokens, int N, int K);      // expected time; negative: not for this kernel
 // gemm_q8_0_tiles.cu: tcgen05 product on re-tiled Q8_0 weights, out[m*N + n], the scalar reference's fp32 order
 int gemm_q8_0_tiles(const uint8_t* tiles, const float* X, float* out, int M, int N, int K, cudaStream_t s,
                     Workspace* ws = nullptr);

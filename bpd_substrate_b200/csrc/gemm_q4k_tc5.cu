@@ -512,33 +512,40 @@ static int tc5_weight_map(CUtensorMap* map, const uint8_t* W, int N, int nb)
 }
 
 // Split K so that every SM has work and the per-CTA chain of super-blocks is short: the number of ranges (at least two
-// super-blocks each) with the fewest super-block steps on the busiest SM, charging each CTA two steps of set-up and a cluster two
-// for its sums.
-struct Tc5Split { int ranges; long steps; };
+// super-blocks each, all tiles' clusters at once: 157 tiles of 10 super-blocks in two ranges were three waves of 74 clusters and took 28 us,
+// one range takes 20) with the fewest super-block steps on the busiest SM, charging each CTA two steps of set-up and a cluster
+// two for its sums.
+struct Tc5Split { int ranges; long waves, chain; };      // chain: super-blocks of a CTA
 template <int NPAD>
 static Tc5Split tc5_split(int n_tiles, int nb)
 {
     const int* at_once = active_clusters<k_gemm_q4k_q8k_tc5<NPAD>>(Tc5Shape<NPAD>::kThreads, 200 * 1024);      // (a CTA has an SM to itself)
-    Tc5Split best = {1, -1};
-    for (int sp = 1; at_once && sp <= kMaxSplits && (sp == 1 || nb / sp >= 2); sp++) {
-        const long steps = (long)((n_tiles + at_once[sp] - 1) / at_once[sp]) * ((nb + sp - 1) / sp + 2) + (sp > 1 ? 2 : 0);
-        if (best.steps < 0 || steps < best.steps) best = {sp, steps};
+    Tc5Split best = {1, 0, 0};
+    long least = -1;
+    for (int sp = 1; at_once && sp <= kMaxSplits && (sp == 1 || (nb / sp >= 2 && n_tiles <= at_once[sp])); sp++) {
+        const long waves = (n_tiles + at_once[sp] - 1) / at_once[sp], chain = (nb + sp - 1) / sp, steps = waves * (chain + 2) + (sp > 1 ? 2 : 0);
+        if (least < 0 || steps < least) {
+            best = {sp, waves, chain};
+            least = steps;
+        }
     }
     return best;
 }
 
-// Whether this kernel is faster than gemm_q4k_mma.cu's, by estimates of both (us) fitted to 10 shapes of 500 x 14336 to 20000 x 1024 and 4 to
-// 64 tokens.  There a warp walks whole rows: its time grows with their length, and with the rows beyond about 7500.  Measured sides of the line
-// (here, there; 16 tokens): 4096x4096 9.9, 15.0; 500x14336 11.2, 41.6; 14336x4096 16.5, 18.2; 8192x2048 10.0, 9.5; 20000x1024 11.8, 10.8.
-bool gemm_q4k_q8k_tc5_faster(int tokens, int N, int K)
+// Expected time in us, or a negative number where this kernel does not run: fitted to 33 shapes of 128 x 1024 to 57344 x 1024 and 500 x 14336,
+// 2 to 64 tokens (standard deviation 5 %).
+double gemm_q4k_q8k_tc5_us(int tokens, int N, int K)
 {
-    if (N < kRows) return false;
-    const int T = tokens < 64 ? tokens : 64, n_tiles = (N + kRows - 1) / kRows, nb = K / 256;
-    const long steps = (T <= 16 ? tc5_split<16>(n_tiles, nb) : T <= 32 ? tc5_split<32>(n_tiles, nb) : tc5_split<64>(n_tiles, nb)).steps;
-    const double here = 4.0 + (T <= 8 ? 0.7 : T <= 16 ? 0.74 : T <= 32 ? 0.88 : 1.25) * (double)steps;
-    const double rows = N > 7500 ? N / 7500.0 : T <= 8 ? 1.0 + N / 16000.0 : 1.0;
-    const double there = 3.7 + (T <= 8 ? 0.3 : T <= 32 ? 0.68 : 1.19) * nb * rows;
-    return steps > 0 && here < there;
+    if (N < kRows) return -1.0;
+    if (tokens > 64) return (double)(tokens / 64) * gemm_q4k_q8k_tc5_us(64, N, K) + (tokens % 64 ? gemm_q4k_q8k_tc5_us(tokens % 64, N, K) : 0.0);
+    const int n_tiles = (N + kRows - 1) / kRows, nb = K / 256;
+    const Tc5Split p = tokens <= 16 ? tc5_split<16>(n_tiles, nb) : tokens <= 32 ? tc5_split<32>(n_tiles, nb) : tc5_split<64>(n_tiles, nb);
+    if (!p.waves) return -1.0;
+    // launch, a wave of CTAs, a super-block of a chain, the sums of several ranges, a million weights
+    struct Cost { double launch, wave, block, join, weights; };
+    const Cost c = tokens <= 8 ? Cost{1.1, 2.2, 0.59, 1.9, 0.053} : tokens <= 16 ? Cost{1.2, 2.3, 0.57, 2.4, 0.057}
+                 : tokens <= 32 ? Cost{1.7, 2.3, 0.66, 3.1, 0.075} : Cost{2.2, 2.0, 1.0, 4.0, 0.089};
+    return c.launch + (double)p.waves * (c.wave + c.block * (double)p.chain) + (p.ranges > 1 ? c.join : 0.0) + c.weights * 1e-6 * N * K;
 }
 
 template <int NPAD>

@@ -577,22 +577,45 @@ int gemm_q4k_q8k_multi(int n, const uint8_t* const* Ws, float* const* outs, cons
     return 0;
 }
 
+// Expected time here in us of 2 to 4 tokens: launch, what a group of warps walks (tiles of `rt` rows; super-blocks of those per warp), and the
+// quantization of the tokens; fitted to 41 shapes of 100 x 4096 to 32000 x 1024 and 500 x 14336 (standard deviation 7 %; of two tokens 10 %,
+// 62 shapes).  Negative: refused.
+static double vec_us(int tokens, int M, int K)
+{
+    GemvPlan p;
+    if (make_plan(&M, 1, K, tokens, p)) return -1.0;
+    struct Cost { double launch, block, row, quant; };
+    const Cost c = tokens == 2 ? Cost{0.6, 0.034, 0.70, 0.10} : tokens == 3 ? Cost{1.1, 0.0074, 0.52, 0.19} : Cost{1.5, 0.0085, 0.855, 0.23};
+    const long groups = (long)sm_count() * p.ng, rows = (p.n_tiles + groups - 1) / groups * p.rt;
+    return c.launch + (double)rows * (c.row + c.block * ((p.nb + p.kc - 1) / p.kc)) + c.quant * p.nb;
+}
+
+// The kernel of a call: here (weights streamed once per pass of 4 tokens, no scratch), or one of the two tensor-core kernels that read them once
+// per 64.  Several tokens go where the estimate is least; away from here it has to be 7 % less, as much as this estimate is off by.
+// Measured sides of the lines (us; here, mma.sync, tcgen05): 2 tokens of 14336 x 4096 10.9, 11.8, 15.1; of 14336 x 1024 8.4, 6.1, 6.3; 4 of
+// 1024 x 4096 6.6, 7.8, 6.2; of 4096 x 2048 7.4, 6.2, 6.4; 16 of 4096 x 4096 -, 16.1, 9.3; of 57344 x 1024 -, 18.4, 23.0; 64 of that -, 41.5, 32.2.
+// From 3 tokens and 2^25 weights on the passes here are no candidate (14336 x 4096: 13.3, 11.7 with 3 tokens); a call of fewer runs here, too,
+// where there is no scratch for a faster kernel.
+enum Q4Kernel { kQ4Vec, kQ4Mma, kQ4Tc5 };
+static bool q4_few(int tokens, int M, int K) { return tokens <= ((long)M * K >= (1L << 25) ? 2 : kMaxTokens); }
+static Q4Kernel q4_kernel(int tokens, int M, int K, bool vec_at_all)
+{
+    const double mma = gemm_q4k_q8k_mma_us(tokens, M, K), tc5 = gemm_q4k_q8k_tc5_us(tokens, M, K), vec = vec_at_all ? vec_us(tokens, M, K) : -1.0;
+    const bool tc5_first = tc5 >= 0.0 && tc5 < mma;
+    if (vec >= 0.0 && 0.93 * vec <= (tc5_first ? tc5 : mma)) return kQ4Vec;
+    return tc5_first ? kQ4Tc5 : kQ4Mma;
+}
+
 int gemm_q4k_q8k(const uint8_t* W, const void* x, float* out, int tokens, int M, int K, int layout, int xsrc,
                  int32_t* dbg, cudaStream_t s, Workspace* ws)
 {
     if (M < 0) return latch(BPDQ_ERR_ARG);
-    // many tokens: the weights would be streamed once per four tokens here, the tensor-core kernels read them once per 64.  The first of
-    // these many, by what a token costs here (us here, there): 2 tokens on many short rows (20000x1024: 11.2, 8.1; 14336x4096: 11.3, 12.5),
-    // 3 on 2^25 weights or 8192 rows (14336x4096: 13.3, 10.8; 8192x2048: 7.6, 6.6), 4 beyond 2^22 weights (4096x4096: 9.4, 8.9), else 5
-    // (1024x4096, 4 tokens: 7.1, 7.2).
-    const long weights = (long)M * K;
-    const int many = M >= 14336 && K <= 2048 ? 2 : weights >= (1L << 25) || M >= 8192 ? 3 : weights > (1L << 22) ? 4 : 5;
-    if (tokens >= many && layout == BPDQ_LAYOUT_BPD && xsrc == 0 && !dbg) {
-        if (gemm_q4k_q8k_tc5_faster(tokens, M, K) && scratch_fits(ws, kScratchGemmActs, gemm_q4k_q8k_tc5_workspace(tokens, M, K), s))
+    if (tokens > 1 && M > 0 && K >= 256 && layout == BPDQ_LAYOUT_BPD && xsrc == 0 && !dbg) {
+        const bool few = q4_few(tokens, M, K);
+        const Q4Kernel k = q4_kernel(tokens, M, K, few);
+        if (k == kQ4Tc5 && scratch_fits(ws, kScratchGemmActs, gemm_q4k_q8k_tc5_workspace(tokens, M, K), s))
             return gemm_q4k_q8k_tc5(W, reinterpret_cast<const float*>(x), out, tokens, M, K, s, ws);
-        // (a call of so few tokens needs no scratch, wherever its rows would be faster: without any it runs here)
-        const int always = weights >= (1L << 25) ? 2 : kMaxTokens;
-        if (tokens > always || scratch_fits(ws, kScratchGemmActs, gemm_q4k_q8k_mma_workspace(tokens, K), s))
+        if (k != kQ4Vec && (!few || scratch_fits(ws, kScratchGemmActs, gemm_q4k_q8k_mma_workspace(tokens, K), s)))
             return gemm_q4k_q8k_mma(W, reinterpret_cast<const float*>(x), out, tokens, M, K, s, ws);
     }
     return gemm_q4k_q8k_multi(1, &W, &out, &M, x, tokens, K, layout, xsrc, dbg, s);
@@ -647,6 +670,12 @@ int bpd_qmm_q4k_q8k_cuda(const uint8_t* qweight, const void* x, float* out, int 
 {
     if ((layout != 0 && layout != 1) || (xsrc != 0 && xsrc != 1)) return latch(BPDQ_ERR_ARG);
     return gemm_q4k_q8k(qweight, x, out, tokens, M, K, layout, xsrc, subdots, (cudaStream_t)stream);
+}
+
+int bpdq_qmm_q4k_q8k_kernel(int tokens, int M, int K)
+{
+    if (tokens < 1 || M < 1 || K < 256 || K % 256) return -1;
+    return tokens > 1 ? q4_kernel(tokens, M, K, q4_few(tokens, M, K)) : kQ4Vec;
 }
 
 // The same with caller-owned scratch: nothing is allocated and no state is shared with other calls, so

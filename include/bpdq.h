@@ -259,6 +259,9 @@ void bpdq_chain_destroy(void* chain);
  * [tokens][K/256]; subdots (may be NULL): int32 [M][K/256][8], token 0's exact sub-block dots */
 int bpd_qmm_q4k_q8k_cuda(const uint8_t* qweight, const void* x, float* out, int tokens, int M, int K, int layout,
                          int xsrc, int32_t* subdots, void* stream);
+/* which kernel that takes with layout and xsrc 0, subdots NULL and scratch at hand: 0 passes of four tokens over the weights,
+ * 1 mma.sync, 2 tcgen05; -1 bad sizes */
+int bpdq_qmm_q4k_q8k_kernel(int tokens, int M, int K);
 /* the same with caller-owned scratch (see "scratch memory" above) */
 size_t bpdq_qmm_q4k_q8k_workspace_bytes(int tokens, int M, int K);
 int bpd_qmm_q4k_q8k_ws_cuda(const uint8_t* qweight, const void* x, float* out, int tokens, int M, int K, int layout,
