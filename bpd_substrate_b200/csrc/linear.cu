@@ -647,6 +647,17 @@ int bpd_linear_bf16_cuda(const uint16_t* W, const void* x, float* out, int n_tok
     return linear_forward(l, n_tokens, act_bf16 != 0, (cudaStream_t)stream);
 }
 
+int bpdq_linear_bf16_tiles(int n_tokens, int N, int K, int* tokens, int* ranges)
+{
+    if (n_tokens < 2 || N < 1 || K < 16 || K % 16 || !tokens || !ranges) return BPDQ_ERR_ARG;
+    Linear l = {};
+    l.N = N; l.K = K;
+    const Tc5Tiles t = tc5_tiles(l, n_tokens);
+    *tokens = t.tokens;
+    *ranges = t.ranges;
+    return 0;
+}
+
 // The same product followed by what a decoder's epilogues do to its sums (BPDQ_MAP_*).
 int bpd_linear_map_cuda(const uint16_t* W, const void* x, void* out, int n_tokens, int N, int K, int map, const float* bias, const float* rate, float cap,
                         int act_bf16, void* stream)
