@@ -161,6 +161,7 @@ SIGNATURES = {
     "bpd_qmatmul_q8_0_llamafile_cuda": (i32, [vp, vp, vp, i32, i32, i32, vp]),
     "bpd_qmatmul_q8_0_dispatch_cuda": (i32, [vp, vp, vp, i32, i32, i32, vp]),
     **{f"bpd_gemm_q8_0_{rm}_{rn}_cuda": (i32, [vp, vp, i32, i32, i32, vp, i32, vp]) for rm in (1, 2, 4) for rn in (1, 2, 4)},
+    "bpdq_qmatmul_q8_0_tiles_width": (i32, [i32] * 3),
     "bpdq_qmatmul_q8_0_tiles_workspace_bytes": (sz, [i32, i32, i32]),
     "bpd_qmatmul_q8_0_tiles_ws_cuda": (i32, [vp, vp, vp, i32, i32, i32, vp, sz, vp]),
     "bpdq_llama_forward_workspace_bytes": (sz, [vp, i32]),

@@ -20,6 +20,7 @@
 #include "launch.cuh"
 #include "q8_0_tiles.cuh"
 #include "tcgen05_device.cuh"
+#include "../../include/bpdq.h"
 
 #include <cuda_fp16.h>
 
@@ -423,3 +424,19 @@ int gemm_q8_0_wide(int n, const uint8_t* const* tiles, float* const* outs, const
 }
 
 }  // namespace bpdq
+
+using namespace bpdq;
+
+extern "C" {
+
+int bpdq_qmatmul_q8_0_tiles_width(int M, int N, int K)
+{
+    if (M < kWideMinTokens || N < 1 || K < 32 || K % 32) return 0;
+    WideProducts p = {};
+    p.n = 1;
+    p.M = M;
+    p.row_tile[1] = (N + kTileRows - 1) / kTileRows;
+    return wide_tokens(p);
+}
+
+}  // extern "C"

@@ -362,6 +362,8 @@ int bpd_unrepack_q8_0_tiles_cuda(const uint8_t* tiles, uint8_t* raw, int N, int 
 /* bench/bpd_cpu.c:4295-4315  bpd_qmatmul_q8_0_cpu on re-tiled weights, any number of tokens M, on the
  * tcgen05 tensor cores; the fp32 operations per block are the scalar reference's, in its order */
 int bpd_qmatmul_q8_0_tiles_cuda(const uint8_t* tiles, const float* X, float* out, int M, int N, int K, void* stream);
+/* tokens of a tile where that takes the kernel of many tokens (fp16 operands), given scratch for it; 0 where it takes the other */
+int bpdq_qmatmul_q8_0_tiles_width(int M, int N, int K);
 size_t bpdq_qmatmul_q8_0_tiles_workspace_bytes(int M, int N, int K);
 int bpd_qmatmul_q8_0_tiles_ws_cuda(const uint8_t* tiles, const float* X, float* out, int M, int N, int K, void* workspace,
                                    size_t workspace_bytes, void* stream);
