@@ -1,7 +1,8 @@
 """Attention of the Q8_0 Llama over more than a few keys, through the C ABI, against 64-bit sums.
 
-Bound: the bar of fp32 results in this suite (1e-5 of the largest output).  A score adds up to 16 truncated tensor-core sums, each
-within 2^-23 of sum |q_d k_d| scale (about 7 for these inputs): 1.3e-5 for the worst row, a tenth of it on average."""
+Bound: 1e-5 of the largest output.  A score adds up to 16 truncated tensor-core sums, each within 2^-23 of sum |q_d k_d| scale (about 7 for
+these inputs): the worst score is off by 1.3e-5, and with it its key's weight.  A row's output is off by that times sum w |v - out|, which is
+at most 0.8 for values of unit variance (one key that holds all the weight has none of it), against a largest output of 3 to 4: below 4e-6 of it."""
 import numpy as np
 import pytest
 
@@ -80,6 +81,32 @@ def test_values_that_are_not_finite_reach_only_the_queries_that_see_them(lib):
     clean[90:, 4:8] = False
     assert np.abs(got - want)[clean].max() <= 1e-5 * np.abs(want).max()
     assert np.isposinf(got[70:, 12:16, 5]).all() and np.isnan(got[90:, 4:8]).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,T", [(np.float32, 1), (np.float16, 128)])
+def test_softmax_weights(lib, kind, T):
+    """Weights one by one, against binary64: scores 0, -1, -2, ... and fractions between them down to where a weight is no normal number any more;
+    key i's value is one in column i and zero elsewhere, so that output i is its weight.  A weight is a rounded argument reduction (the score's last
+    bits), a polynomial (5e-9), a sum of 127 weights and a division, each a few 2^-24: 5e-7 of it.  The tiles hold a weight times 2^10 as two fp16
+    numbers, the low one a multiple of 2^-24: off by up to 2^-35 = 3e-11."""
+    D, keys, H, HKV = 128, 128, 32, 8
+    rng = np.random.default_rng(3)
+    want_s = -np.concatenate([[0.0], np.linspace(0.5, 100.0, 67), rng.uniform(0.0, 12.0, 60)])
+    k = np.zeros((keys, HKV, D), kind)
+    k[:, :, 0] = want_s[:, None]                                    # (fp16: the nearest number is the score)
+    scores = k[:, 0, 0].astype(np.float64)
+    v = np.repeat(np.eye(keys, D, dtype=kind)[:, None], HKV, 1)
+    q = np.zeros((T, H, D), np.float32)
+    q[:, :, 0] = 1.0
+    off = keys - T
+    assert lib.bpdq_gqa_attn_kernel(T, keys, H, HKV, D, off, int(kind == np.float16)) == (2 if T > 1 else 1)
+    got = attend(lib, q, k, v, off, np.float32(1.0), keys)[-1]      # the last query sees every key
+    e = np.exp(scores)
+    want = e / e.sum()
+    assert np.array_equal(got, np.broadcast_to(got[0], got.shape))
+    small = 3e-11 if T > 1 else 1e-37
+    assert np.all(np.abs(got[0].astype(np.float64) - want) <= 5e-7 * want + small)
 
 
 # queries, keys before them, heads, key heads, head size, fp16: kernel (0 a CTA per query and head, 1 keys over a cluster, 2 tiles)
