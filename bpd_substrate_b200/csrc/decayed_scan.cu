@@ -140,7 +140,7 @@ struct ScanSegments {
 // and half (w >> 2) of its keys.  Bound by the chain of barriers from chunk to chunk, so the chip wants many short chains: 2048 tokens
 // of 8 heads of 256 x 256 as one chain per CTA (32 CTAs) 272 us, of 64 heads of 128 x 64 (64 CTAs) 192 us; in four segments about 160 and 90 us with both launches and the fold.
 // A short portion is bound by the fetch of instructions that run once or twice, so it has an instantiation that knows of no segments (a state's
-// place chosen at run time was a fifth more code: 64 tokens of 8 heads of 256 x 256 14.1 us, 11.8 without; of 64 heads of 128 x 64 10.4, 8.0).
+// place chosen at run time was a fifth more code: 64 tokens of 8 heads of 256 x 256 14.1 us, 11.4 without; of 64 heads of 128 x 64 10.4, 8.0).
 template <int NMAX, int TASK>
 __global__ void __launch_bounds__(256, ChunkShape<NMAX, TASK>::kPerSm) k_decayed_chunks(DecayedScan a, int tokens, ScanSegments seg)
 {

@@ -12,9 +12,11 @@
 //   warp 2        bulk copies of activation units (fp16 whole numbers and scales, written by k_quant_q8_0_wide)
 //   warps 3-6     int8 weights to fp16 operands in the canonical K-major order
 //   warps 7-22    epilogue: thread = row, T / 4 tokens per warp
-// What bounds it: tensor memory, which the MMAs write and the epilogue reads, with the packed fp32 instructions behind it (about 700 cycles
-// per block of 128 x 128, of which the products take 192).  14336 x 4096, 1000 tokens: 514 us in the narrow kernel, 320 here (367 TFLOP/s);
-// 4096 x 14336: 484, 329.
+// What bounds it: the handovers between the roles, about 530 of 680 cycles per block of 128 x 128 (MMA commit, sixteen warps that wait for it, their
+// arrivals, the issuer's wait, for one block at a time and two sets of accumulators).  14336 x 4096, 1000 tokens, 319 us: with neither conversion
+// nor anything in the epilogue but its barriers 252 are left; the conversion to fp16 alone adds 28, the epilogue's loads and sums 40 (its sums 15 of
+// them); with one MMA per block instead of three it is 322.  Tensor pipe active 30 % of the time, issue 67 %.  In the narrow kernel 514 us
+// (367 TFLOP/s here); 4096 x 14336: 484, 329.
 // All waits are bounded; a role that gives up records a code and leaves, the others time out in turn, and warp 1 frees the tensor memory.
 #include "bpdq_common.cuh"
 #include "launch.cuh"

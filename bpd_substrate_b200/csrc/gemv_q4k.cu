@@ -695,7 +695,7 @@ int bpd_qmm_q4k_q8k_ws_cuda(const uint8_t* qweight, const void* x, float* out, i
     return gemm_q4k_q8k(qweight, x, out, tokens, M, K, layout, xsrc, subdots, (cudaStream_t)stream, &ws);
 }
 
-// The tensor-core kernel at any token count (the dispatcher above picks it for more than 8).
+// The mma.sync kernel at any token count (q4_kernel above picks it by its estimate).
 int bpd_qmm_q4k_q8k_mma_cuda(const uint8_t* qweight, const float* X, float* out, int tokens, int M, int K, void* stream)
 {
     return gemm_q4k_q8k_mma(qweight, X, out, tokens, M, K, (cudaStream_t)stream);

@@ -1,5 +1,5 @@
 // Grouped-query attention of the Q8_0 Llama (bench/bpd_cpu.c:5370-5433 of the reference) for contexts of more than kShortKeys
-// keys; shorter ones stay on k_gqa_attn (llama_forward.cu), which adds in the reference's order.
+// keys; shorter ones, and short prompts of unshared fp32 heads, stay on k_gqa_attn (llama_forward.cu), which adds in the reference's order.
 //
 //   k_gqa_split   a few queries: keys dealt to the CTAs of a cluster, fp32 multiply-adds, parts joined through distributed
 //                 shared memory (no scratch memory, so a call can be captured without a warm-up)

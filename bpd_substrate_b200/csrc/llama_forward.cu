@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(256) k_kv_write(void* cache, const float* src,
     }
 }
 
-// Contexts of up to 64 keys and the shapes that gqa_attention.cu leaves (head sizes other than 64 and 128, unaligned pointers):
+// Contexts of up to 64 keys and the calls that gqa_attention.cu leaves (head sizes other than 64 and 128, unaligned pointers, short fp32 prompts):
 // one CTA per (query token, query head), sums in the reference's order.  In the reference ALL n_kv cache rows take part: rows past
 // the query's position score -1e38 and weigh exp(-huge) = 0, so they add exact zeros to the sum and to
 // the output (the cache holds finite values); they are skipped here, which leaves every bit as it is.

@@ -51,10 +51,12 @@ void bpdq_set_dequant_tuning(int variant, int ctas_per_sm);
 int bpdq_sm_count(void);
 
 /* ---- scratch memory of the compute entries -------------------------------------------------
- * Three kinds of entry need device scratch beyond their inputs and outputs (quantized activations,
- * split-K partial sums, the forward pass's vectors): the many-token products bpd_qmm_q4k_q8k_cuda /
- * _mma_cuda / _tc5_cuda / gpu_matmul_q4k, bpd_qmatmul_q8_0_tiles_cuda and bpd_qmatmul_q8_0_llamafile_cuda,
- * and bpd_llama_forward*_cuda.  Each has two forms:
+ * Some entries need device scratch beyond their inputs and outputs (quantized activations, states and
+ * partial sums, the forward pass's vectors): the many-token products bpd_qmm_q4k_q8k_cuda (from 2 tokens
+ * on) / _mma_cuda / _tc5_cuda / gpu_matmul_q4k, bpd_qmatmul_q8_0_tiles_cuda and bpd_qmatmul_q8_0_llamafile_cuda,
+ * bpd_llama_forward*_cuda, and of the decoders' single mechanisms bpd_decayed_scan_cuda (long bf16 portions),
+ * bpd_latent_attention_cuda and bpd_delta_rule_cuda.  The products and the forward have two forms, the
+ * mechanisms the second alone:
  *   *_ws_cuda(..., workspace, workspace_bytes, stream): the caller owns the scratch (16-byte aligned, at
  *     least the matching *_workspace_bytes()).  Nothing is allocated and no state is shared between calls:
  *     calls on different streams may overlap if their workspaces differ; BPDQ_STATUS_ERR_RANGE if too small.
@@ -65,7 +67,10 @@ int bpdq_sm_count(void);
  *     hold its address stay valid.  While a stream is being captured a block cannot grow: the call returns
  *     BPDQ_STATUS_ERR_CAPTURE and launches nothing -- make one call of that size on the stream before the
  *     capture (a warm-up run), or use the *_ws_cuda form.  Up to 4 tokens of bpd_qmm_q4k_q8k_cuda and gpu_matmul_q4k (up to 2
- *     where M * K >= 2^25) run without scratch where there is none, in either form. */
+ *     where M * K >= 2^25) run without scratch where there is none, in either form, and bpd_decayed_scan_cuda does at any length.
+ * Where the scratch of the faster kernel is not to be had but a call runs all the same, fp32 sums are added in another order: a Q4_K product
+ * of several tokens, or a decaying state, may then differ in its last bits from the same call with scratch (a capture without a warm-up, a
+ * workspace below *_workspace_bytes()).  Q8_0 products give the same bits either way. */
 
 /* ---- device memory helpers (additive, size_t) ------------------------------------------ */
 void* bpdq_alloc(size_t bytes);
@@ -266,7 +271,7 @@ int bpdq_qmm_q4k_q8k_kernel(int tokens, int M, int K);
 size_t bpdq_qmm_q4k_q8k_workspace_bytes(int tokens, int M, int K);
 int bpd_qmm_q4k_q8k_ws_cuda(const uint8_t* qweight, const void* x, float* out, int tokens, int M, int K, int layout,
                             int xsrc, int32_t* subdots, void* workspace, size_t workspace_bytes, void* stream);
-/* the int8 tensor-core kernel behind bpd_qmm_q4k_q8k_cuda for more than 8 tokens, callable at any
+/* the int8 mma.sync kernel behind bpd_qmm_q4k_q8k_cuda for several tokens (from 2 on, by an estimate of sizes), callable at any
  * token count: out[tokens][M], X float [tokens][K], nibble order of bench/bpd_quant.c:68-72 */
 int bpd_qmm_q4k_q8k_mma_cuda(const uint8_t* qweight, const float* X, float* out, int tokens, int M, int K, void* stream);
 /* the same product on tcgen05 tensor cores with TMEM accumulators (M >= 128 weight rows) */
@@ -424,7 +429,8 @@ int bpd_kv_cache_write_cuda(float* cache, const float* src, const int32_t* pos_i
                             int max_seq_len, void* stream);
 int bpd_gqa_attn_cuda(const float* q, const void* k, const void* v, float* dst, int n_q_tokens, int n_kv, int n_q_heads,
                       int n_kv_heads, int head_dim, float scale, int kv_offset, int kv_is_f16, void* stream);
-/* which kernel that takes: 0 a CTA per query and head (sums in the reference's order), 1 keys over a cluster, 2 tiles of 64 x 64; -1 bad sizes */
+/* (Beyond 64 keys a query's sums are split over keys by a rule on the call's sizes: the same query alone and within a prompt may differ in
+ * its last bits.)  Which kernel that takes: 0 a CTA per query and head (sums in the reference's order), 1 keys over a cluster, 2 tiles of 64 x 64; -1 bad sizes */
 int bpdq_gqa_attn_kernel(int n_q_tokens, int n_kv, int n_q_heads, int n_kv_heads, int head_dim, int kv_offset, int kv_is_f16);
 int bpd_swiglu_fuse_cuda(const float* gate, const float* up, float* dst, int n, void* stream);
 int bpd_argmax_dim_cuda(const float* x, long long* out, int outer, int dim_size, int inner, void* stream);
