@@ -143,14 +143,15 @@ __global__ void __launch_bounds__(256, 2) k_linear_vec(Linear l)
 // ------------------------------------------------------------------ several tokens, fp32
 
 // 64 rows x 16 J tokens per CTA (J: 1 or 4), four rows and J tokens per thread.  Bound by the chain of slabs of 16 columns where there are few
-// tiles (12 tokens of 2048 x 2048: 104 us at J = 4, 82 at J = 1), else by the multiply-adds and the loads of their operands.
+// tiles (12 tokens of 2048 x 2048: 104 us at J = 4, 82 at J = 1), else by the multiply-adds and the loads of their operands.  The next launches
+// may start only when a CTA's sums are done: waiting CTAs of several launches pile up on the SMs otherwise, and a later launch of fewer CTAs than
+// SMs finds itself on some of them (64 tokens through three layers of the hybrid decoder, width 1536: 3862 us, 2467 so).
 template <int J>
 __global__ void __launch_bounds__(256) k_linear_tile(Linear l, int T)
 {
     __shared__ __align__(16) float sw[16][68], sx[16][16 * J + 4];
     const int tid = threadIdx.x, tr = tid & 15, tt = tid >> 4;      // rows 4 tr .., tokens J tt ..
     const int n0 = blockIdx.x * 64, t0 = blockIdx.y * 16 * J;
-    pdl_launch_dependents();
     pdl_wait();
     const float* in = reinterpret_cast<const float*>(l.in);
     float acc[J][4] = {};
@@ -185,6 +186,7 @@ __global__ void __launch_bounds__(256) k_linear_tile(Linear l, int T)
             for (int i = 0; i < 4; i++) acc[j][i] += part[j][i];
         __syncthreads();
     }
+    pdl_launch_dependents();
 #pragma unroll
     for (int j = 0; j < J; j++) {
         const int t = t0 + J * tt + j;
