@@ -615,7 +615,8 @@ int linear_forward(const Linear& l, int T, bool act_bf16, cudaStream_t s)
     }
     if (!act_bf16) {
         // narrow tiles while every SM has one at most (64 tokens of 2048 x 2048: 107 us wide, 83 narrow; 100 tokens: 107, 127), or two where 16
-        // tokens are all there are (12 tokens of 14336 x 2048: 264, 214; of 22000 x 2048: 281, 324)
+        // tokens are all there are (12 tokens of 14336 x 2048: 264, 214; of 22000 x 2048: 281, 324).  Both sides were measured with the next launches
+        // started early; since then 12 tokens, back to back: narrow 14336 x 2048 144, 18944 x 2048 167; wide 19008 x 2048 221, 22000 x 2048 225
         const int n_tiles = (l.N + 63) / 64, narrow = (T + 15) / 16;
         if ((long)n_tiles * narrow <= (narrow == 1 ? 2 : 1) * sm_count()) return launch_ordered(k_linear_tile<1>, dim3(n_tiles, narrow), 256, 0, s, l, T);
         return launch_ordered(k_linear_tile<4>, dim3(n_tiles, (T + 63) / 64), 256, 0, s, l, T);
