@@ -188,6 +188,7 @@ SIGNATURES = {
     "bpdq_hybrid_create": (vp, [vp, vp]),
     "bpdq_hybrid_destroy": (None, [vp]),
     "bpdq_hybrid_forward": (i32, [vp, vp, i32, i32, vp, vp, i32, vp, i32, vp]),
+    "bpdq_hybrid_step": (i32, [vp, vp, i32, i32, vp, vp, i32, vp, vp, i32, vp]),
     "bpdq_hybrid_logits": (vp, [vp]),
     "bpdq_hybrid_picked": (vp, [vp]),
     "bpdq_hybrid_scratch_bytes": (sz, [vp]),

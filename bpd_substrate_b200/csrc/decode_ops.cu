@@ -3,6 +3,7 @@
 // library (lib/kernel_templates_llama.pl: k_vecmat :107-158, k_rms_norm :529-593, elementwise
 // :600-830, k_matmul :1104-1290).  They sit either side of the quantized GEMVs in a decode
 // step; all are memory bound and small.
+#include "argmax_device.cuh"
 #include "bpdq_common.cuh"
 #include "launch.cuh"
 #include "../../include/bpdq.h"
@@ -96,45 +97,13 @@ __global__ void __launch_bounds__(1024) k_matmul_f32(const float* __restrict__ A
     if (row < M && col < N) C[(size_t)row * N + col] = acc;
 }
 
-// One CTA per row; the largest value wins, the lowest index among equals (v > best in index order).
+// One CTA per row.
 __global__ void __launch_bounds__(1024) k_argmax_rows(const float* x, long long* out, int n)
 {
     pdl_launch_dependents();
     pdl_wait();
-    __shared__ float s_v[32];
-    __shared__ int s_i[32];
-    const float* row = x + (size_t)blockIdx.x * n;
-    float best = row[0];
-    int bi = 0;
-    auto better = [](float v, int k, float& bv, int& bk) {
-        if (v > bv || (v == bv && k < bk)) { bv = v; bk = k; }
-    };
-    for (int k0 = threadIdx.x; k0 < n; k0 += 8 * 1024) {
-        float v[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) v[j] = k0 + 1024 * j < n ? row[k0 + 1024 * j] : row[0];
-#pragma unroll
-        for (int j = 0; j < 8; j++) better(v[j], k0 + 1024 * j < n ? k0 + 1024 * j : 0, best, bi);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float v = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-        const int i = __shfl_xor_sync(0xFFFFFFFFu, bi, o);
-        better(v, i, best, bi);
-    }
-    if ((threadIdx.x & 31) == 0) { s_v[threadIdx.x >> 5] = best; s_i[threadIdx.x >> 5] = bi; }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        best = s_v[threadIdx.x];
-        bi = s_i[threadIdx.x];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float v = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-            const int i = __shfl_xor_sync(0xFFFFFFFFu, bi, o);
-            better(v, i, best, bi);
-        }
-        if (threadIdx.x == 0) out[blockIdx.x] = bi;
-    }
+    const int best = argmax_of_row(x + (size_t)blockIdx.x * n, n);
+    if (threadIdx.x == 0) out[blockIdx.x] = best;
 }
 
 static int ew_grid(long n)

@@ -13,6 +13,7 @@
 // sizes, recurrence, gate + norm, out), 4 (delta rule: in with convolutions and write shares, decays + gates, recurrence with gate
 // and norm, out), 7 (latent attention), 4 (grouped attention: in, norms + cache, attention, out), 2 (feed-forward).  One-token steps
 // are recorded as a CUDA graph per sequence slot and replayed; token and position are read from device memory.
+#include "argmax_device.cuh"
 #include "decayed_scan.cuh"
 #include "delta_rule.cuh"
 #include "grouped_attention.cuh"
@@ -21,8 +22,10 @@
 #include "residual_streams.cuh"
 #include "../../include/bpdq.h"
 
+#include <cstring>
 #include <map>
 #include <new>
+#include <utility>
 #include <vector>
 
 namespace bpdq {
@@ -56,7 +59,52 @@ __global__ void __launch_bounds__(256) k_gather_rows(const A* h, const int32_t* 
     }
 }
 
+// What a step needs from the host, as launch arguments: no copy engine, and nothing on the host that has to outlive the call.  Three copies from
+// pageable memory ahead of a prompt's first kernel, and two of pageable memory behind its last, left the device idle for about 90 us of a step.
+template <int N>
+struct StepInputs {
+    int32_t v[N];       // the position, the tokens, the wanted places
+};
+template <int N>
+__global__ void __launch_bounds__(256) k_step_inputs(const __grid_constant__ StepInputs<N> in, int32_t* ids, int* pos, int32_t* want, int T, int n_want)
+{
+    for (int i = threadIdx.x; i < 1 + T + n_want; i += 256) {
+        if (i == 0) *pos = in.v[0];
+        else if (i <= T) ids[i - 1] = in.v[i];
+        else want[i - 1 - T] = in.v[i];
+    }
+}
+constexpr int kFewInputs = 4, kManyInputs = 4096;       // (16 KB of arguments; 32 KB are the limit)
+
+// grid (1 + slices, rows): the first CTA of a row finds its largest logit (the lowest index of equal ones), the others bring the row to the host.
+constexpr int kEmitThreads = 1024, kEmitSlice = 4 * kEmitThreads;
+__global__ void __launch_bounds__(kEmitThreads) k_emit_rows(const float* logits, long long* picked, float* host_logits, long long* host_picked, int vocab)
+{
+    pdl_launch_dependents();
+    pdl_wait();
+    const float* row = logits + (size_t)blockIdx.y * vocab;
+    if (blockIdx.x == 0) {
+        const int best = argmax_of_row(row, vocab);
+        if (threadIdx.x == 0) picked[blockIdx.y] = host_picked[blockIdx.y] = best;
+        return;
+    }
+    const int at = (blockIdx.x - 1) * kEmitSlice + 4 * threadIdx.x;
+    float* to = host_logits + (size_t)blockIdx.y * vocab;
+    if (!(vocab & 3)) {
+        if (at < vocab) *reinterpret_cast<float4*>(to + at) = *reinterpret_cast<const float4*>(row + at);
+    } else {
+        for (int i = at; i < at + 4 && i < vocab; i++) to[i] = row[i];
+    }
+}
+
 namespace {
+
+// Pinned memory that a step's results pass through, at most kMaxStaging bytes per plan.
+constexpr size_t kMaxStaging = 8u << 20;
+struct Staging {
+    uint8_t* base = nullptr;
+    size_t bytes = 0;
+};
 
 struct Buffers {
     uint8_t* base = nullptr;
@@ -75,8 +123,16 @@ struct Plan {
     bool bf16_acts;
     Buffers one, many;                              // one-token steps (fixed, recorded in graphs), everything else
     Buffers* last = nullptr;                        // holds the results of the last call
-    std::map<void*, cudaGraphExec_t> graphs;        // by state base
+    struct Recorded {
+        cudaGraphExec_t exec;
+        cudaGraph_t graph;                          // (what `inputs` belongs to)
+        cudaGraphNode_t inputs;                     // its k_step_inputs
+    };
+    std::map<std::pair<void*, int>, Recorded> graphs;        // by state base and where the results go
+    Staging staging;
 };
+// Where the results of a step go besides the device: nowhere, or through `staging` (logits too, or the choices alone).
+enum { kEmitNone, kEmitPicked, kEmitAll };
 
 DynTanh norm_of(const bpdq_dyn_tanh& n) { return DynTanh{n.w, n.b, n.alpha}; }
 
@@ -189,6 +245,37 @@ size_t lay_out(const Plan& p, Buffers& b, uint8_t* base, int T, int context, int
     return at;
 }
 
+size_t staged_bytes(int n_want, int vocab, bool logits) { return ((size_t)n_want * 8 + 15) / 16 * 16 + (logits ? (size_t)n_want * vocab * 4 : 0); }
+float* staged_logits(const Staging& g, int n_want) { return reinterpret_cast<float*>(g.base + ((size_t)n_want * 8 + 15) / 16 * 16); }
+
+void forget(const Plan::Recorded& r)
+{
+    check_cuda(cudaGraphExecDestroy(r.exec));
+    check_cuda(cudaGraphDestroy(r.graph));
+}
+
+// (a step that stages has waited for its results, so nothing writes here between steps; recorded steps know the address)
+int make_staging(Plan& p, size_t need)
+{
+    if (need <= p.staging.bytes) return 0;
+    int rc;
+    if (p.staging.base) {
+        for (auto it = p.graphs.begin(); it != p.graphs.end();) {
+            if (it->first.second == kEmitNone) { ++it; continue; }
+            forget(it->second);
+            it = p.graphs.erase(it);
+        }
+        rc = check_cuda(cudaFreeHost(p.staging.base));
+        p.staging = Staging{};
+        if (rc) return rc;
+    }
+    void* m = nullptr;
+    if ((rc = check_cuda(cudaHostAlloc(&m, need, cudaHostAllocDefault)))) return rc;
+    p.staging.base = (uint8_t*)m;
+    p.staging.bytes = need;
+    return 0;
+}
+
 // Makes room for a call.  Buffers are laid out anew for every call's sizes (what depends on the number of tokens, like
 // the number of key splits, is then as that call needs it) and the memory only grows.
 int make_room(Plan& p, Buffers& b, int T, int context, int wanted, cudaStream_t s)
@@ -218,6 +305,7 @@ struct Runner {
     int T, context;
     uint8_t* state;
     cudaStream_t s;
+    int emit;
 
     void* at(void* base, size_t elements) const { return (uint8_t*)base + elements * (p.bf16_acts ? 2 : 4); }
 
@@ -514,9 +602,23 @@ struct Runner {
             head.cap = p.cfg.logit_cap;
             if ((rc = linear_forward(head, vec ? 1 : n_want, p.bf16_acts, s))) return rc;
         }
-        return bpd_argmax_dim_cuda(b.logits, b.picked, n_want, p.cfg.vocab, 1, s);
+        if (emit == kEmitNone) return bpd_argmax_dim_cuda(b.logits, b.picked, n_want, p.cfg.vocab, 1, s);
+        const unsigned slices = emit == kEmitAll ? (unsigned)((p.cfg.vocab + kEmitSlice - 1) / kEmitSlice) : 0u;
+        return launch_ordered(k_emit_rows, dim3(1 + slices, (unsigned)n_want), kEmitThreads, 0, s, (const float*)b.logits, b.picked,
+                              staged_logits(p.staging, n_want), (long long*)p.staging.base, p.cfg.vocab);
     }
 };
+
+template <int N>
+int send_inputs(const Buffers& b, const int32_t* ids, int T, int pos, const int32_t* want, int n_want, cudaStream_t s)
+{
+    StepInputs<N> in;
+    in.v[0] = pos;
+    memcpy(in.v + 1, ids, (size_t)T * 4);
+    if (n_want) memcpy(in.v + 1 + T, want, (size_t)n_want * 4);
+    k_step_inputs<N><<<1, 256, 0, s>>>(in, b.ids, b.pos, b.want, T, n_want);
+    return check_cuda(cudaGetLastError());
+}
 
 int check_layer(const Plan& p, int i)
 {
@@ -565,6 +667,75 @@ bool rows_suffice(const Plan& p, int pos, int T)
     return true;
 }
 
+int forward(Plan* p, const int32_t* token_ids, int n_tokens, int pos, void* state, const int32_t* want, int n_want, float* residuals, int use_graph,
+            cudaStream_t s, int emit)
+{
+    if (!p || !token_ids || n_tokens < 1 || pos < 0 || !state || n_want < 0 || (n_want && !want)) return latch(BPDQ_ERR_ARG);
+    if (n_tokens > 65535 || !rows_suffice(*p, pos, n_tokens)) return latch(BPDQ_ERR_RANGE);       // (tokens are a grid dimension)
+    bool all = n_want == n_tokens;
+    for (int i = 0; i < n_want; i++) {
+        if (want[i] < 0 || want[i] >= n_tokens) return latch(BPDQ_ERR_RANGE);
+        all = all && want[i] == i;
+    }
+    for (int i = 0; i < n_tokens; i++)
+        if (token_ids[i] < 0 || token_ids[i] >= p->cfg.vocab) return latch(BPDQ_ERR_RANGE);
+    const bool single = n_tokens == 1 && n_want <= 1;
+    Buffers& b = single ? p->one : p->many;
+    int rc = 0;
+    if (!single) rc = make_room(*p, b, n_tokens, pos + n_tokens, n_want, s);
+    else if (!b.base) rc = make_room(*p, b, 1, 1, 1, s);
+    if (rc) return rc;
+    p->last = &b;
+    Runner r{*p, b, n_tokens, pos + n_tokens, (uint8_t*)state, s, emit};
+    const bool recorded = single && use_graph && !residuals && n_want;
+    const auto it = recorded ? p->graphs.find({state, emit}) : p->graphs.end();
+    if (it != p->graphs.end()) {
+        const StepInputs<kFewInputs> in = {{pos, token_ids[0]}};
+        int one = 1, none = 0;
+        void* args[] = {(void*)&in, &b.ids, &b.pos, &b.want, &one, &none};
+        cudaKernelNodeParams k = {};
+        k.func = (void*)k_step_inputs<kFewInputs>;
+        k.gridDim = dim3(1);
+        k.blockDim = dim3(256);
+        k.kernelParams = args;
+        if ((rc = check_cuda(cudaGraphExecKernelNodeSetParams(it->second.exec, it->second.inputs, &k)))) return rc;
+        return check_cuda(cudaGraphLaunch(it->second.exec, s));
+    }
+    const int n_places = all ? 0 : n_want;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if ((rc = check_cuda(cudaStreamIsCapturing(s, &capturing)))) return rc;
+    if (1 + (long)n_tokens + n_places > kManyInputs || capturing != cudaStreamCaptureStatusNone) {
+        // (copies from pageable memory: staged before the calls return; in a caller's own recording they read the caller's memory at every replay)
+        if ((rc = check_cuda(cudaMemcpyAsync(b.ids, token_ids, (size_t)n_tokens * 4, cudaMemcpyHostToDevice, s)))) return rc;
+        if ((rc = check_cuda(cudaMemcpyAsync(b.pos, &pos, 4, cudaMemcpyHostToDevice, s)))) return rc;
+        if (n_places && (rc = check_cuda(cudaMemcpyAsync(b.want, want, (size_t)n_want * 4, cudaMemcpyHostToDevice, s)))) return rc;
+    } else if ((rc = 1 + n_tokens + n_places <= kFewInputs ? send_inputs<kFewInputs>(b, token_ids, n_tokens, pos, want, n_places, s)
+                                                           : send_inputs<kManyInputs>(b, token_ids, n_tokens, pos, want, n_places, s))) {
+        return rc;
+    }
+    if (!recorded) {
+        rc = r.run(residuals, n_want, all);
+        return rc ? latch(rc) : 0;
+    }
+    // the first one-token step of a slot runs launch by launch, so that every kernel's attributes are set outside a capture
+    if ((rc = r.run(nullptr, 1, true))) return latch(rc);
+    if ((rc = check_cuda(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)))) return rc;
+    int run_rc = send_inputs<kFewInputs>(b, token_ids, 1, pos, want, 0, s);
+    if (!run_rc) run_rc = r.run(nullptr, 1, true);
+    cudaGraph_t g = nullptr;
+    rc = check_cuda(cudaStreamEndCapture(s, &g));
+    Plan::Recorded made = {nullptr, g, nullptr};
+    size_t roots = 1;
+    if (!run_rc && !rc && g) rc = check_cuda(cudaGraphGetRootNodes(g, &made.inputs, &roots));
+    if (!run_rc && !rc && roots == 1) rc = check_cuda(cudaGraphInstantiate(&made.exec, g, 0));
+    if (run_rc || rc || !made.exec) {
+        if (g) cudaGraphDestroy(g);
+        return latch(run_rc ? run_rc : rc ? rc : BPDQ_ERR_CUDA);
+    }
+    p->graphs[{state, emit}] = made;
+    return 0;
+}
+
 }  // namespace
 
 }  // namespace bpdq
@@ -601,7 +772,8 @@ void bpdq_hybrid_destroy(void* plan)
     Plan* p = (Plan*)plan;
     if (!p) return;
     check_cuda(cudaDeviceSynchronize());
-    for (auto& g : p->graphs) check_cuda(cudaGraphExecDestroy(g.second));
+    for (auto& g : p->graphs) forget(g.second);
+    if (p->staging.base) check_cuda(cudaFreeHost(p->staging.base));
     for (Buffers* b : {&p->one, &p->many})
         if (b->base) check_cuda(cudaFree(b->base));
     delete p;
@@ -610,53 +782,31 @@ void bpdq_hybrid_destroy(void* plan)
 int bpdq_hybrid_forward(void* plan, const int32_t* token_ids, int n_tokens, int pos, void* state, const int32_t* want, int n_want,
                         float* residuals, int use_graph, void* stream)
 {
+    return forward((Plan*)plan, token_ids, n_tokens, pos, state, want, n_want, residuals, use_graph, (cudaStream_t)stream, kEmitNone);
+}
+
+int bpdq_hybrid_step(void* plan, const int32_t* token_ids, int n_tokens, int pos, void* state, const int32_t* want, int n_want, float* logits,
+                     long long* picked, int use_graph, void* stream)
+{
     Plan* p = (Plan*)plan;
     cudaStream_t s = (cudaStream_t)stream;
-    if (!p || !token_ids || n_tokens < 1 || pos < 0 || !state || n_want < 0 || (n_want && !want)) return latch(BPDQ_ERR_ARG);
-    if (n_tokens > 65535 || !rows_suffice(*p, pos, n_tokens)) return latch(BPDQ_ERR_RANGE);       // (tokens are a grid dimension)
-    bool all = n_want == n_tokens;
-    for (int i = 0; i < n_want; i++) {
-        if (want[i] < 0 || want[i] >= n_tokens) return latch(BPDQ_ERR_RANGE);
-        all = all && want[i] == i;
+    if (!p || (n_want > 0 && !picked)) return latch(BPDQ_ERR_ARG);
+    int emit = kEmitNone, rc;
+    if (n_want > 0 && n_want <= n_tokens && n_want <= 65535 && staged_bytes(n_want, p->cfg.vocab, logits != nullptr) <= kMaxStaging) {
+        if ((rc = make_staging(*p, staged_bytes(n_want, p->cfg.vocab, logits != nullptr)))) return latch(rc);
+        emit = logits ? kEmitAll : kEmitPicked;
     }
-    for (int i = 0; i < n_tokens; i++)
-        if (token_ids[i] < 0 || token_ids[i] >= p->cfg.vocab) return latch(BPDQ_ERR_RANGE);
-    const bool single = n_tokens == 1 && n_want <= 1;
-    Buffers& b = single ? p->one : p->many;
-    int rc = 0;
-    if (!single) rc = make_room(*p, b, n_tokens, pos + n_tokens, n_want, s);
-    else if (!b.base) rc = make_room(*p, b, 1, 1, 1, s);
-    if (rc) return rc;
-    // (copies from pageable memory: staged before the calls return)
-    if ((rc = check_cuda(cudaMemcpyAsync(b.ids, token_ids, (size_t)n_tokens * 4, cudaMemcpyHostToDevice, s)))) return rc;
-    if ((rc = check_cuda(cudaMemcpyAsync(b.pos, &pos, 4, cudaMemcpyHostToDevice, s)))) return rc;
-    if (n_want && !all && (rc = check_cuda(cudaMemcpyAsync(b.want, want, (size_t)n_want * 4, cudaMemcpyHostToDevice, s)))) return rc;
-    p->last = &b;
-    Runner r{*p, b, n_tokens, pos + n_tokens, (uint8_t*)state, s};
-    if (!single || !use_graph || residuals || n_want == 0) {
-        rc = r.run(residuals, n_want, all);
-        return rc ? latch(rc) : 0;
+    if ((rc = forward(p, token_ids, n_tokens, pos, state, want, n_want, nullptr, use_graph, s, emit))) return rc;
+    if (n_want > 0 && emit == kEmitNone) {
+        if (logits && (rc = check_cuda(cudaMemcpyAsync(logits, p->last->logits, (size_t)n_want * p->cfg.vocab * 4, cudaMemcpyDeviceToHost, s)))) return rc;
+        if ((rc = check_cuda(cudaMemcpyAsync(picked, p->last->picked, (size_t)n_want * 8, cudaMemcpyDeviceToHost, s)))) return rc;
     }
-    auto it = p->graphs.find(state);
-    if (it == p->graphs.end()) {
-        // the first one-token step of a slot runs launch by launch, so that every kernel's attributes are set outside a capture
-        if ((rc = r.run(nullptr, 1, true))) return latch(rc);
-        if ((rc = check_cuda(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)))) return rc;
-        const int run_rc = r.run(nullptr, 1, true);
-        cudaGraph_t g = nullptr;
-        rc = check_cuda(cudaStreamEndCapture(s, &g));
-        if (run_rc || rc || !g) {
-            if (g) cudaGraphDestroy(g);
-            return latch(run_rc ? run_rc : rc ? rc : BPDQ_ERR_CUDA);
-        }
-        cudaGraphExec_t e = nullptr;
-        rc = check_cuda(cudaGraphInstantiate(&e, g, 0));
-        cudaGraphDestroy(g);
-        if (rc) return rc;
-        p->graphs[state] = e;
-        return 0;
+    if ((rc = check_cuda(cudaStreamSynchronize(s)))) return rc;
+    if (emit != kEmitNone) {
+        memcpy(picked, p->staging.base, (size_t)n_want * 8);
+        if (logits) memcpy(logits, staged_logits(p->staging, n_want), (size_t)n_want * p->cfg.vocab * 4);
     }
-    return check_cuda(cudaGraphLaunch(it->second, s));
+    return 0;
 }
 
 float* bpdq_hybrid_logits(void* plan)

@@ -44,6 +44,9 @@ class Engine:
         tokens, want = np.asarray(tokens, np.int32), np.asarray(want, np.int64)
         if want.size and (want.min() < 0 or want.max() >= tokens.size):
             raise ValueError(f"wanted places {want.min()} .. {want.max()} of {tokens.size} tokens")
+        if 0 < tokens.size <= self.portion:
+            out, picked = self.model.step(seq, tokens, want, logits)      # one portion: its results are the whole call's
+            return (np.asarray(out, np.float32) if logits else None), np.asarray(picked, np.int64)
         out = np.empty((want.size, self.model.vocab), np.float32) if logits else None
         picked = np.empty(want.size, np.int64)
         for at in range(0, tokens.size, self.portion):

@@ -411,8 +411,7 @@ class DeviceHybrid:
     def state_parts(self):
         return self.parts
 
-    def launch(self, seq, tokens, want=(), residuals=None):
-        """Queues the tokens of `seq`; results stay on the device until the next call."""
+    def _inputs(self, seq, tokens, want):
         tokens = np.ascontiguousarray(tokens, np.int32)
         want = np.ascontiguousarray(want, np.int32)
         n = tokens.size
@@ -422,23 +421,26 @@ class DeviceHybrid:
             raise ValueError(f"the sequence would hold {seq.length + n} tokens, its slot has room for {seq.capacity}")
         if n > self.portion:
             raise ValueError(f"a step of {n} tokens; this model takes up to {self.portion}")
-        if tokens.min() < 0 or tokens.max() >= self.vocab:
+        low, high = (tokens.min(), tokens.max()) if n > 1 else (tokens.flat[0],) * 2
+        if low < 0 or high >= self.vocab:
             raise ValueError(f"token ids run from 0 to {self.vocab - 1}")
-        capi.check(self.lib.bpdq_hybrid_forward(self.plan, tokens.ctypes.data, n, seq.length, seq.base, want.ctypes.data, want.size, residuals,
+        return tokens, want
+
+    def launch(self, seq, tokens, want=(), residuals=None):
+        """Queues the tokens of `seq`; results stay on the device until the next call."""
+        tokens, want = self._inputs(seq, tokens, want)
+        capi.check(self.lib.bpdq_hybrid_forward(self.plan, tokens.ctypes.data, tokens.size, seq.length, seq.base, want.ctypes.data, want.size, residuals,
                                                 int(self.use_graph), self.stream), "bpdq_hybrid_forward")
-        seq.length += n
+        seq.length += tokens.size
 
     def step(self, seq, tokens, want=(), logits=True):
         """Runs the tokens; returns (logits [len(want), vocab] or None, greedy token ids [len(want)])."""
-        self.launch(seq, tokens, want)
-        n = len(want)
-        out = np.empty((n, self.vocab), np.float32) if logits else None
-        picked = np.empty(n, np.int64)
-        if n:
-            if logits:
-                capi.check(self.lib.bpdq_d2h_async(out.ctypes.data, self.lib.bpdq_hybrid_logits(self.plan), out.nbytes, self.stream))
-            capi.check(self.lib.bpdq_d2h_async(picked.ctypes.data, self.lib.bpdq_hybrid_picked(self.plan), picked.nbytes, self.stream))
-        capi.check(self.lib.bpdq_stream_sync(self.stream), "hybrid step")
+        tokens, want = self._inputs(seq, tokens, want)
+        out = np.empty((want.size, self.vocab), np.float32) if logits else None
+        picked = np.empty(want.size, np.int64)
+        capi.check(self.lib.bpdq_hybrid_step(self.plan, tokens.ctypes.data, tokens.size, seq.length, seq.base, want.ctypes.data, want.size,
+                                             out.ctypes.data if logits else None, picked.ctypes.data, int(self.use_graph), self.stream), "hybrid step")
+        seq.length += tokens.size
         return out, picked
 
     def residuals(self, seq, tokens):

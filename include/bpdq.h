@@ -571,6 +571,10 @@ void bpdq_hybrid_destroy(void* plan);
  * one-token steps as a CUDA graph per state address. */
 int bpdq_hybrid_forward(void* plan, const int32_t* token_ids, int n_tokens, int pos, void* state, const int32_t* want, int n_want,
                         float* residuals, int use_graph, void* stream);
+/* The same, then waits and brings the results to host memory: logits [n_want][vocab] (or NULL), picked [n_want].  Rows of up to 8 MB
+ * pass through pinned memory that the plan keeps. */
+int bpdq_hybrid_step(void* plan, const int32_t* token_ids, int n_tokens, int pos, void* state, const int32_t* want, int n_want, float* logits,
+                     long long* picked, int use_graph, void* stream);
 float* bpdq_hybrid_logits(void* plan);                /* device [n_want][vocab] */
 void* bpdq_hybrid_picked(void* plan);                 /* device int64 [n_want] */
 size_t bpdq_hybrid_scratch_bytes(void* plan);

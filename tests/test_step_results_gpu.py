@@ -1,0 +1,50 @@
+"""A step that brings its results to the host gives the bits that its buffers hold on the device, whatever way inputs and results take."""
+import numpy as np
+import pytest
+
+from bpd_substrate_b200.engine import Engine
+from tests import hybrid_models as hm
+from tests import test_hybrid_gpu as hybrid
+
+pytestmark = pytest.mark.gpu
+
+
+def on_device(m, seq, tokens, want):
+    """The same step, its results read from the device's buffers."""
+    m.launch(seq, tokens, want)
+    logits, picked = np.empty((len(want), m.vocab), np.float32), np.empty(len(want), np.int64)
+    assert m.lib.bpdq_stream_sync(m.stream) == 0
+    m.lib.bpdq_d2h(logits.ctypes.data, m.lib.bpdq_hybrid_logits(m.plan), logits.nbytes)
+    m.lib.bpdq_d2h(picked.ctypes.data, m.lib.bpdq_hybrid_picked(m.plan), picked.nbytes)
+    return logits, picked
+
+
+@pytest.mark.parametrize("vocab", [97, 4096 + 4, 2 * 4096 + 1])       # one slice of a row and several, rows that end inside 16 bytes
+def test_results(lib, vocab):
+    cfg = hm.config(vocab, 64, [hm.layer("retention", hm.retention(2, 16, 16, 16, [0.5, 0.98]), 33)])
+    m = hybrid.device(cfg, hm.weights(cfg, 5), lib, "bfloat16", capacity=8300)
+    e = Engine(m, slots=2)
+    a, b = e.slots.acquire(), e.slots.acquire()
+    toks = hm.tokens(cfg, 8300, 6)
+    # inputs as one launch's arguments (3 and 4 words, 4096) or copied (4097 words and more); choices alone and logits; rows beyond the
+    # pinned memory (300 of 8193 logits); recorded one-token steps, the pinned memory having moved in between
+    at = 0
+    for n, want in [(2, [1]), (1, [0]), (1, [0]), (1, [0]), (3, range(3)), (4094, [4093]), (1, [0]), (4090, [5, 0, 4089, 5, 77]), (1, [0]), (40, range(40)),
+                    (1, [0]), (1, [0]), (1, [0, 0]), (1, [])]:
+        part, want = toks[at:at + n], list(want)
+        ref = on_device(m, a, part, want)
+        choices_alone = n % 2 == 0
+        logits, picked = m.step(b, part, want, not choices_alone)
+        assert (logits is None) == choices_alone
+        if not choices_alone:
+            assert np.array_equal(logits.view(np.uint32), ref[0].view(np.uint32)), n
+        assert np.array_equal(picked, ref[1]) and np.array_equal(picked, np.argmax(ref[0], 1) if want else picked), n
+        at += n
+    for seq in (a, b):
+        e.slots.release(seq)
+    a, b = e.slots.acquire(), e.slots.acquire()
+    ref, (logits, picked) = on_device(m, a, toks[:300], list(range(300))), m.step(b, toks[:300], range(300))
+    assert np.array_equal(logits.view(np.uint32), ref[0].view(np.uint32)) and np.array_equal(picked, ref[1])
+    assert m.lib.bpdq_last_status() == 0
+    e.close()
+    m.close()
