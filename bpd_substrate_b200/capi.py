@@ -184,6 +184,7 @@ SIGNATURES = {
     "bpd_latent_attention_cuda": (i32, [vp, vp, vp, vp, vp, vp, i32, i32, i32, vp]),
     "bpd_delta_rule_cuda": (i32, [vp, vp, vp, i32, vp, vp, f32, f32, vp, vp, vp, vp, f32, i32, i32, i32, i32, i32, i32, i32, vp]),
     "bpd_grouped_attention_cuda": (i32, [vp, vp, i32, vp, i32, vp, vp, i32, i32, vp]),
+    "bpd_grouped_attention_context_cuda": (i32, [vp, vp, i32, vp, i32, vp, vp, i32, i32, i32, vp]),
     "bpd_stream_step_cuda": (i32, [vp, vp, vp, i32, vp, f32, i32, i32, i32, vp, vp, i32, vp]),
     "bpdq_hybrid_create": (vp, [vp, vp]),
     "bpdq_hybrid_destroy": (None, [vp]),

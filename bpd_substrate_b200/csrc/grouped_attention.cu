@@ -5,7 +5,8 @@
 //   k_grouped_split_mma  bf16, few queries (decoding): 16 rows per CTA, keys dealt to the warps of a cluster of CTAs; keys and
 //                        values go from HBM straight into mma.sync fragments (dimensions and columns are taken in the order in
 //                        which 16-byte loads bring them), the cluster joins its parts through distributed shared memory
-//   k_grouped_tile_mma   bf16, a prompt's portion: 64 rows per CTA, keys in double-buffered blocks of 64
+//   k_grouped_tile_mma   bf16, a prompt's portion: 64 rows per CTA, keys in double-buffered blocks of 64 (short contexts, caches whose rows are used
+//                        again, sizes that the kernel of prompt_attention.cu does not take; it has the others)
 //   k_grouped_rows       fp32 (and bf16 sizes beyond the others): a warp per row
 //
 // Scores and softmax are fp32; weights enter the product with the values as the sum of two bf16 numbers.
@@ -13,6 +14,7 @@
 #include "cluster_device.cuh"
 #include "launch.cuh"
 #include "mma_device.cuh"
+#include "prompt_attention.cuh"
 #include "../../include/bpdq.h"
 
 namespace bpdq {
@@ -568,7 +570,7 @@ static int launch_tile(const GroupedShape& p, const bf16* u, int ld_u, const bf1
     return launch_ordered(k_grouped_tile_mma<DV, kBounded>, grid, 128, tile_smem(p.dim_pad, DV), s, p, u, ld_u, cache, o, pos, T);
 }
 
-int grouped_attention(const GroupedShape& p, const void* u, int ld_u, const void* cache, void* o, const int* pos, int T, bool act_bf16,
+int grouped_attention(const GroupedShape& p, const void* u, int ld_u, const void* cache, void* o, const int* pos, int T, int context, bool act_bf16,
                       cudaStream_t s)
 {
     if (!act_bf16) return launch_rows<float>(p, u, ld_u, cache, o, pos, T, s);
@@ -579,6 +581,20 @@ int grouped_attention(const GroupedShape& p, const void* u, int ld_u, const void
         if (most <= 64) return launch_split<2, 1>(p, q, ld_u, c, out, pos, T, s);
         if (most <= 128) return launch_split<4, 2>(p, q, ld_u, c, out, pos, T, s);
         return launch_split<8, 4>(p, q, ld_u, c, out, pos, T, s);
+    }
+    // Larger tiles from about this context on, whatever the number of rows (us, tiles of 64 x 64, of 128 x 128; 16 heads on 4 of 128): 32 tokens of 32 keys
+    // 9.4, 10.3; 64 of 64 10.0, 10.3; 96 of 96 12.5, 10.6; 17 of 3017 146, 60.  4 heads on 2 of 64: 96 of 96 10.3, 10.3; 200 of 200 14.5, 9.9.
+    if (context >= 96 && context <= p.rows && (p.sink != 0) == (p.cap > 0.0f)) {      // every position in the row of its number
+        PromptAttention a = {};
+        a.T = T; a.context = context; a.pos = pos;
+        a.groups = p.groups; a.share = p.share();
+        a.dim = a.dim1 = p.dim_pad; a.value_dim = p.value_pad;
+        a.q = q; a.keys = c; a.values = c + (size_t)p.groups * p.dim_pad;
+        a.ld_q = ld_u; a.ld_keys = a.ld_values = p.row();
+        a.chunk = p.chunk;
+        a.scale = p.scale; a.cap = p.cap;
+        a.o = out;
+        if (prompt_attention_fits(a)) return prompt_attention(a, s);
     }
     if (tile_smem(p.dim_pad, p.value_pad <= 64 ? 64 : 128) <= 220 * 1024) {
         const bool bounded = p.sink && p.cap > 0.0f && p.cap <= kBoundedCap;
@@ -594,11 +610,11 @@ using namespace bpdq;
 
 extern "C" {
 
-int bpd_grouped_attention_cuda(const bpdq_grouped_shape* c, void* u, int ld_u, void* cache, int append, void* o, const int32_t* pos, int n_tokens,
-                               int act_bf16, void* stream)
+int bpd_grouped_attention_context_cuda(const bpdq_grouped_shape* c, void* u, int ld_u, void* cache, int append, void* o, const int32_t* pos, int n_tokens,
+                                       int context, int act_bf16, void* stream)
 {
     if (!c || n_tokens < 0 || c->heads < 1 || c->groups < 1 || c->heads % c->groups || c->dim < 1 || c->dim_pad < c->dim || c->value_pad < 1 ||
-        (c->dim_pad | c->value_pad) % 16 || c->chunk < 0 || c->rows < 1 || c->cap < 0.0f)
+        (c->dim_pad | c->value_pad) % 16 || c->chunk < 0 || c->rows < 1 || c->cap < 0.0f || context < 0)
         return latch(BPDQ_ERR_ARG);
     if (n_tokens == 0) return 0;
     if (!u || !cache || !o || !pos) return latch(BPDQ_ERR_ARG);
@@ -608,7 +624,12 @@ int bpd_grouped_attention_cuda(const bpdq_grouped_shape* c, void* u, int ld_u, v
     p.chunk = c->chunk; p.rows = c->rows; p.sink = c->sink;
     p.scale = c->scale; p.cap = c->cap; p.eps = c->eps;
     const int rc = grouped_prepare(p, u, ld_u, append ? cache : nullptr, pos, n_tokens, act_bf16 != 0, (cudaStream_t)stream);
-    return rc ? rc : grouped_attention(p, u, ld_u, cache, o, pos, n_tokens, act_bf16 != 0, (cudaStream_t)stream);
+    return rc ? rc : grouped_attention(p, u, ld_u, cache, o, pos, n_tokens, context, act_bf16 != 0, (cudaStream_t)stream);
+}
+int bpd_grouped_attention_cuda(const bpdq_grouped_shape* c, void* u, int ld_u, void* cache, int append, void* o, const int32_t* pos, int n_tokens,
+                               int act_bf16, void* stream)
+{
+    return bpd_grouped_attention_context_cuda(c, u, ld_u, cache, append, o, pos, n_tokens, 0, act_bf16, stream);
 }
 
 }  // extern "C"

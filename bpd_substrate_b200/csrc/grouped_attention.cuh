@@ -20,8 +20,9 @@ struct GroupedShape {
 // keys over their root mean square (per head, over dim), queries in place, keys and values to cache rows of *pos + t.
 int grouped_prepare(const GroupedShape& p, void* u, int ld_u, void* cache, const int* pos, int T, bool act_bf16, cudaStream_t s);
 
-// Normed queries of u against the cache, which holds positions up to *pos + T - 1; o [T][heads * value_pad].
-int grouped_attention(const GroupedShape& p, const void* u, int ld_u, const void* cache, void* o, const int* pos, int T, bool act_bf16,
+// Normed queries of u against the cache, which holds positions up to *pos + T - 1; o [T][heads * value_pad].  context = *pos + T where
+// the caller knows it, else 0.
+int grouped_attention(const GroupedShape& p, const void* u, int ld_u, const void* cache, void* o, const int* pos, int T, int context, bool act_bf16,
                       cudaStream_t s);
 
 }  // namespace bpdq

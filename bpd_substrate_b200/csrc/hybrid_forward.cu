@@ -513,7 +513,7 @@ struct Runner {
         int rc = linear_forward(open(sub, l.w_in, N, b.u, N, kLinAct), T, p.bf16_acts, s);
         if (rc) return rc;
         if ((rc = grouped_prepare(sh, b.u, N, own ? cache : nullptr, b.pos, T, p.bf16_acts, s))) return rc;
-        if ((rc = grouped_attention(sh, b.u, N, cache, b.o, b.pos, T, p.bf16_acts, s))) return rc;
+        if ((rc = grouped_attention(sh, b.u, N, cache, b.o, b.pos, T, context, p.bf16_acts, s))) return rc;
         return close(sub, l.w_o, l.heads * l.value_pad, b.o);
     }
 

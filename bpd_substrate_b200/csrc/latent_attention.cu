@@ -11,11 +11,13 @@
 //                          softmax fp32, weights enter the product as the sum of two bf16 numbers
 //   k_latent_attn_rows     fp32 (and bf16 sizes beyond the tile kernel's shared memory): a warp per row
 //   k_latent_values        joins the splits and applies W_uv
-//   k_expanded_attn_mma    bf16 prompts: 64 queries of a head per CTA against expanded keys and values
+//   k_expanded_attn_mma    bf16 prompts: 64 queries of a head per CTA against expanded keys and values, of the sizes that the kernel of
+//                          prompt_attention.cu does not take
 #include "latent_attention.cuh"
 #include "cluster_device.cuh"
 #include "launch.cuh"
 #include "mma_device.cuh"
+#include "prompt_attention.cuh"
 #include "../../include/bpdq.h"
 
 namespace bpdq {
@@ -888,6 +890,17 @@ int latent_attention(const LatentShape& p, void* q, const bf16* w_ukv, const voi
     int rc = linear_forward(l, context, true, s);
     if (rc) return rc;
     if ((rc = launch_ordered(k_rotate_queries, grid_1d((long)T * p.heads * p.rot_dims / 2), 256, 0, s, p, (bf16*)q, pos, T))) return rc;
+    PromptAttention a = {};
+    a.T = T; a.context = context; a.pos = pos;
+    a.groups = p.heads; a.share = 1;
+    a.dim = p.q_head(); a.dim1 = p.dim_pad; a.value_dim = p.value_pad;
+    a.q = (const bf16*)q;
+    a.keys = (const bf16*)b.expanded; a.values = a.keys + (size_t)p.heads * p.dim_pad;
+    a.rest = (const bf16*)cache + p.rank_pad;
+    a.ld_q = (long)p.heads * p.q_head(); a.ld_keys = a.ld_values = l.N; a.ld_rest = p.row();
+    a.scale = p.scale;
+    a.o = (bf16*)o;
+    if (prompt_attention_fits(a)) return prompt_attention(a, s);
     const dim3 tiles((T + kQueryTile - 1) / kQueryTile, p.heads, p.value_pad <= 64 ? 1 : (p.value_pad + 127) / 128);
     const bf16 *e = (const bf16*)b.expanded, *c = (const bf16*)cache;
     if (p.value_pad <= 64) {

@@ -14,6 +14,7 @@
 #include "decoder_device.cuh"
 #include "launch.cuh"
 #include "tcgen05_device.cuh"
+#include "tensor_map.cuh"
 #include "../../include/bpdq.h"
 
 namespace bpdq {
@@ -223,20 +224,6 @@ __host__ __device__ constexpr int tc5_stages(int bn)
     return fit < kTc5MaxStages ? fit : kTc5MaxStages;
 }
 constexpr int tc5_smem(int bn) { return 1024 + tc5_stages(bn) * tc5_stage_bytes(bn) + 8 * (2 * kTc5MaxStages + 4) + 16; }
-
-// K-major operand in the 128-byte swizzle: 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t swizzled_desc(uint32_t saddr)
-{
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-__device__ __forceinline__ void umma_bf16_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum)
-        : "memory");
-}
 
 template <int BN>
 __global__ void __launch_bounds__(Tc5Linear<BN>::kThreads, 1)
@@ -527,30 +514,6 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
 
 // ------------------------------------------------------------------ host side
 
-typedef CUresult (*TensorMapEncode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                    const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// bf16 matrix [rows][cols] with `ld` elements between rows, read in boxes of box_rows x 64 columns.
-static int bf16_map(CUtensorMap* map, const void* p, int rows, int cols, int ld, int box_rows)
-{
-    static TensorMapEncode encode = nullptr;
-    if (!encode) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q);
-        if (e != cudaSuccess || q != cudaDriverEntryPointSuccess || !fn) return latch(BPDQ_ERR_CUDA);
-        encode = (TensorMapEncode)fn;
-    }
-    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {64, (cuuint32_t)box_rows}, estr[2] = {1, 1};
-    CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? 0 : latch(BPDQ_ERR_CUDA - 900 - (int)r);
-}
-
 struct Tc5Tiles { int tokens, ranges; };      // of a tile; of K
 
 template <int BN>
@@ -559,8 +522,8 @@ static int launch_tc5(const Linear& l, int T, Tc5Tiles t, cudaStream_t s)
     using S = Tc5Linear<BN>;
     CUtensorMap wmap, xmap;
     int rc;
-    if ((rc = bf16_map(&wmap, l.W, l.N, l.K, l.K, kTc5Rows))) return rc;
-    if ((rc = bf16_map(&xmap, l.in, T, l.K, l.ld_in, t.tokens))) return rc;
+    if ((rc = bf16_map(&wmap, l.W, l.K, l.N, l.K, kTc5Rows))) return rc;
+    if ((rc = bf16_map(&xmap, l.in, l.K, T, l.ld_in, t.tokens))) return rc;
     if ((rc = allow_smem<k_linear_tc5<BN>>(227 * 1024))) return rc;
     const long tiles = (long)((l.N + kTc5Rows - 1) / kTc5Rows) * ((T + t.tokens - 1) / t.tokens);
     const unsigned grid = (unsigned)(t.ranges > 1 || tiles < sm_count() ? tiles : sm_count());

@@ -1,0 +1,35 @@
+"""Attention of prompts on tiles of 128 rows x 128 keys: the cases and bounds of the latent and grouped kernels at the edges of tiles."""
+import pytest
+
+from tests import test_hybrid_gpu as hybrid
+from tests import test_vuzelix_gpu as vuzelix
+
+pytestmark = pytest.mark.gpu
+
+
+# whole tiles and one row more, blocks that end inside the context, padded sizes, value slices of 64 and 128, two kinds of key pieces
+@pytest.mark.parametrize("T,pos,H,D,r,V,R", [(128, 0, 2, 64, 64, 64, 64), (129, 0, 1, 128, 64, 128, 96), (200, 65, 3, 128, 64, 128, 128), (131, 500, 2, 64, 64, 192, 64),
+                                             (255, 1, 1, 64, 128, 256, 64), (140, 3, 2, 60, 50, 120, 70), (384, 128, 1, 64, 64, 64, 64)])
+def test_latent(lib, T, pos, H, D, r, V, R):
+    hybrid.latent_case(lib, 1, T, pos, H, D, r, V, R, T + pos)
+
+
+class Known:
+    """The library, the host knowing the position of the portion that is checked."""
+
+    def __init__(self, lib, T, context):
+        self.lib, self.T, self.context = lib, T, context
+
+    def __getattr__(self, name):
+        return getattr(self.lib, name)
+
+    def bpd_grouped_attention_cuda(self, *a):
+        return self.lib.bpd_grouped_attention_context_cuda(*a[:8], self.context if a[7] == self.T else 0, *a[8:])
+
+
+# one row beyond what the split kernel takes, rows of 1, 2, 4 and 16 heads, chunks inside a block, across blocks and none, value slices
+@pytest.mark.parametrize("T,pos,H,G,D,V,chunk", [(65, 0, 1, 1, 64, 64, 0), (17, 100, 8, 2, 128, 128, 0), (128, 0, 2, 2, 64, 64, 0), (40, 90, 4, 1, 64, 192, 64),
+                                                 (130, 5, 2, 1, 128, 128, 37), (70, 260, 16, 1, 60, 60, 128), (257, 127, 1, 1, 64, 128, 200), (90, 300, 4, 2, 192, 64, 1)])
+@pytest.mark.parametrize("cap,sink", [(2.0, 1), (60.0, 1), (0.0, 0)])
+def test_grouped(lib, T, pos, H, G, D, V, chunk, cap, sink):
+    vuzelix.attention_case(Known(lib, T, pos + T), 1, T, pos, H, G, D, V, chunk, cap=cap, sink=sink)
