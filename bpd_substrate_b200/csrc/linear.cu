@@ -211,8 +211,11 @@ __global__ void __launch_bounds__(256) k_linear_tile(Linear l, int T)
 // BN: the most tokens of a tile; a launch takes bn of them, a multiple of 16 above BN / 2, and as many ring stages as fit then.
 template <int BN>
 struct Tc5Linear {
-    static constexpr int kEpiWarps = 8;                                // two per TMEM lane quarter, each half of the columns
-    static constexpr int kThreads = 32 * (2 + kEpiWarps);
+    // Epilogue warps: three or two per TMEM lane quarter, each a share of the columns.  What follows the sums of a launch's last tile runs under nothing:
+    // 8500 cycles of fp32 rows with eight warps and 256 tokens.  700 tokens, eight warps and one warp for all copies, now (us): 2048 x 2048 11.7, 10.5;
+    // 6400 x 2048 22.6, 20.9; 2048 x 10752 33.2, 31.4.  (Sixteen warps leave 96 registers, which spill: 11.5, 22.2, 32.4.)
+    static constexpr int kEpiWarps = BN > 64 ? 12 : 8;
+    static constexpr int kThreads = 32 * (3 + kEpiWarps);
     static constexpr int kTmemCols = 2 * BN;
 };
 constexpr int kTc5Rows = 128, kTc5Depth = 64;                          // weight rows per tile, K elements per ring stage
@@ -240,7 +243,7 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
-        for (int s = 0; s < stages; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < stages; s++) { mbar_init(&full[s], 2); mbar_init(&empty[s], 1); }
         for (int s = 0; s < 2; s++) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], S::kEpiWarps); }
         mbar_init_fence();
     }
@@ -362,47 +365,27 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
         return true;
     };
 
-    if (warp == 0) {
-        // ---------------- producer: the weights of the first ring round are requested before the launch ahead has finished
+    if (warp == 0 || warp == 2) {
+        // ---------------- copies: a warp for the weights, which do not wait for the launch ahead, one for the tokens.  (One thread for both took 470
+        // cycles between two K blocks, mostly its own chain of instructions, and bounded tiles of up to 200 tokens.)
         if (lane == 0) {
-            // two walks over the same (tile, K block)s, weights ahead of tokens by a ring round; counted, not divided out of a step's
-            // number: two 64-bit divisions per request held a K block of any width at 680 cycles
-            struct Walk { int tile, kb; };
-            Walk ww = {(int)blockIdx.x, 0}, wt = ww;
-            auto step = [&](Walk& w) {
-                if (++w.kb == kb_n) {
-                    w.kb = 0;
-                    w.tile += gridDim.x;
+            const bool tokens = warp == 2;
+            const uint32_t to0 = smem_addr(ring) + (tokens ? kTc5ABytes : 0), bytes = (uint32_t)(tokens ? bn * kTc5Depth * 2 : kTc5ABytes);
+            const uint32_t full0 = smem_addr(full), empty0 = smem_addr(empty);
+            const CUtensorMap* map = tokens ? &xmap : &wmap;
+            if (tokens) pdl_wait();
+            uint32_t s = 0, par = 1;        // (the first round's waits pass)
+            bool ok = true, ready = true;
+            for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
+                const int y = tokens ? (tile % t_tiles) * bn : (tile / t_tiles) * kTc5Rows;
+                int x = kb0 * kTc5Depth;
+                for (int kb = 0; kb < kb_n; kb++, x += kTc5Depth) {
+                    if (!ready && !mbar_wait_at(empty0 + 8 * s, par, err, 41)) { ok = false; break; }
+                    mbar_expect_tx_at(full0 + 8 * s, bytes);
+                    tma_rows_2d_at(to0 + s * stage_bytes, map, x, y, full0 + 8 * s);
+                    if (++s == (uint32_t)stages) { s = 0; par ^= 1u; }
+                    ready = mbar_test_at(empty0 + 8 * s, par);
                 }
-            };
-            int row = (ww.tile / t_tiles) * kTc5Rows, tok = (wt.tile % t_tiles) * bn;
-            auto weights = [&](int s) {
-                mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
-                tma_rows_2d(ring + (size_t)s * stage_bytes, &wmap, (kb0 + ww.kb) * kTc5Depth, row, &full[s]);
-                step(ww);
-                if (ww.kb == 0) row = (ww.tile / t_tiles) * kTc5Rows;
-            };
-            auto tokens = [&](int s) {
-                tma_rows_2d(ring + (size_t)s * stage_bytes + kTc5ABytes, &xmap, (kb0 + wt.kb) * kTc5Depth, tok, &full[s]);
-                step(wt);
-                if (wt.kb == 0) tok = (wt.tile % t_tiles) * bn;
-            };
-            int ahead = 0;
-            for (; ahead < stages && ww.tile < tiles; ahead++) weights(ahead);
-            pdl_wait();
-            for (int i = 0; i < ahead; i++) tokens(i);
-            int s = 0;
-            uint32_t par = 0;
-            bool ready = false;
-            while (ww.tile < tiles) {
-                if (!ready && !mbar_wait_bounded(&empty[s], par, err, 41)) break;
-                const int next = s + 1 == stages ? 0 : s + 1;
-                const uint32_t next_par = next ? par : par ^ 1u;
-                ready = mbar_test(&empty[next], next_par);
-                weights(s);
-                tokens(s);
-                s = next;
-                par = next_par;
             }
         }
     } else if (warp == 1) {
@@ -411,41 +394,39 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
         if (elect_one()) {
             // one thread walks the steps.  Whether the next stage is there is asked before this one's products are issued, so that the
             // answer's latency passes under them: 168 K blocks of 2048 rows took 49, 53, 70 us at 16, 80, 256 tokens a tile, now 34, 38, 68
-            int s = 0, local = 0;
-            uint32_t full_par = 0;
+            const uint32_t full0 = smem_addr(full), empty0 = smem_addr(empty), acc0 = smem_addr(acc_full);
+            const uint64_t a0 = swizzled_desc(smem_addr(ring)), b0 = swizzled_desc(smem_addr(ring) + kTc5ABytes);
+            const int steps_last = (l.K - (kb0 + kb_n - 1) * kTc5Depth) / 16;      // products of the last K block of a tile, if fewer than four
+            uint32_t s = 0, full_par = 0, local = 0;
             bool ok = true, ready = false;
             for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x, local++) {
-                const int a = local & 1;
-                if (local >= 2 && !mbar_wait_bounded(&acc_empty[a], (uint32_t)((local >> 1) - 1) & 1u, err, 42)) break;
-                const uint32_t d = tmem_base + (uint32_t)(a * BN);
+                const uint32_t a = local & 1;
+                if (local >= 2 && !mbar_wait_bounded(&acc_empty[a], ((local >> 1) - 1) & 1u, err, 42)) break;
+                const uint32_t d = tmem_base + a * BN;
                 for (int kb = 0; kb < kb_n; kb++) {
-                    if (!ready && !mbar_wait_bounded(&full[s], full_par, err, 43)) { ok = false; break; }
-                    const int next = s + 1 == stages ? 0 : s + 1;
-                    const uint32_t next_par = next ? full_par : full_par ^ 1u;
-                    ready = mbar_test(&full[next], next_par);
+                    if (!ready && !mbar_wait_at(full0 + 8 * s, full_par, err, 43)) { ok = false; break; }
+                    const uint32_t now = s, at = s * (uint32_t)(stage_bytes >> 4);
+                    if (++s == (uint32_t)stages) { s = 0; full_par ^= 1u; }
+                    ready = mbar_test_at(full0 + 8 * s, full_par);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t stage = smem_addr(ring + (size_t)s * stage_bytes);
-                    const uint64_t ad = swizzled_desc(stage), bd = swizzled_desc(stage + kTc5ABytes);
-                    const int left = (l.K - (kb0 + kb) * kTc5Depth) / 16;
+                    const uint64_t ad = a0 + at, bd = b0 + at;
                     umma_bf16_ss(d, ad, bd, idesc, kb ? 1u : 0u);
-                    if (left >= 4) {
+                    if (kb + 1 < kb_n || steps_last >= 4) {
 #pragma unroll
                         for (int k = 1; k < 4; k++) umma_bf16_ss(d, ad + 2 * k, bd + 2 * k, idesc, 1u);
                     } else {
-                        for (int k = 1; k < left; k++) umma_bf16_ss(d, ad + 2 * k, bd + 2 * k, idesc, 1u);
+                        for (int k = 1; k < steps_last; k++) umma_bf16_ss(d, ad + 2 * k, bd + 2 * k, idesc, 1u);
                     }
-                    umma_commit(&empty[s]);
-                    if (kb + 1 == kb_n) umma_commit(&acc_full[a]);
-                    s = next;
-                    full_par = next_par;
+                    umma_commit_at(empty0 + 8 * now);
                 }
+                if (ok) umma_commit_at(acc0 + 8 * a);
             }
         }
         __syncwarp();
     } else {
         // ---------------- epilogue
-        const int half = (warp - 2) >> 2;
-        const int split = (bn / 16 + 1) / 2 * 16, c_begin = half ? split : 0, c_end = half ? bn : split;
+        constexpr int kShares = S::kEpiWarps / 4;
+        const int share = (warp - 3) >> 2, steps = bn / 16, c_begin = share * steps / kShares * 16, c_end = (share + 1) * steps / kShares * 16;
         int local = 0;
         pdl_wait();
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, local++) {
@@ -487,9 +468,10 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
         __syncwarp();
         cluster_arrive();
         cluster_wait();
-        if (warp >= 2) {
-            const int turn = 32 * ranges;
-            finish(blockIdx.x, 16 * (2 * range + ((warp - 2) >> 2)), []() { return true; },
+        if (warp >= 3) {
+            constexpr int kShares = S::kEpiWarps / 4;
+            const int turn = 16 * kShares * ranges;
+            finish(blockIdx.x, 16 * (kShares * range + ((warp - 3) >> 2)), []() { return true; },
                    [&](int c0, int (&v)[16]) {
                        float t[16];
 #pragma unroll
