@@ -173,6 +173,7 @@ SIGNATURES = {
     "gpu_vecmat_q8_0": (None, [vp, vp, vp, i32, i32]),
     # hybrid decoder
     "bpd_linear_bf16_cuda": (i32, [vp, vp, vp, i32, i32, i32, i32, vp]),
+    "bpdq_linear_bf16_ctas": (i32, [i32, i32, i32]),
     "bpdq_linear_bf16_tiles": (i32, [i32, i32, i32, vp, vp]),
     "bpd_linear_map_cuda": (i32, [vp, vp, vp, i32, i32, i32, i32, vp, vp, f32, i32, vp]),
     "bpd_decayed_scan_cuda": (i32, [vp, i32, vp, i32, vp, i32, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp]),

@@ -8,7 +8,8 @@
 //                  launch ahead has finished (weights are constant); HBM bound
 //   k_linear_tc5   several tokens, bf16: tcgen05.mma kind::f16, 128 weight rows (TMEM lanes) x up to 256 tokens
 //                  (TMEM columns) per tile, persistent CTAs, operands by tiled TMA into a 128-byte-swizzled ring, two
-//                  accumulators so that a tile's epilogue runs under the next tile's products
+//                  accumulators so that a tile's epilogue runs under the next tile's products; large products on pairs of
+//                  CTAs (cta_group::2), 256 rows per tile, each CTA fetching its rows and half of the tokens
 //   k_linear_tile  several tokens, fp32: plain fp32 multiply-adds on tiles of 64 rows x 16 or 64 tokens
 #include "cluster_device.cuh"
 #include "decoder_device.cuh"
@@ -228,12 +229,14 @@ __host__ __device__ constexpr int tc5_stages(int bn)
 }
 constexpr int tc5_smem(int bn) { return 1024 + tc5_stages(bn) * tc5_stage_bytes(bn) + 8 * (2 * kTc5MaxStages + 4) + 16; }
 
-template <int BN>
+template <int BN, bool kPair>
 __global__ void __launch_bounds__(Tc5Linear<BN>::kThreads, 1)
 k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, Linear l, int T, int bn, int* err)
 {
     using S = Tc5Linear<BN>;
-    const int stages = tc5_stages(bn), stage_bytes = tc5_stage_bytes(bn);
+    constexpr int kCtas = kPair ? 2 : 1, kTileRows = kCtas * kTc5Rows;
+    const int own = bn / kCtas;                // tokens of a tile whose rows this CTA fetches
+    const int stages = tc5_stages(own), stage_bytes = tc5_stage_bytes(own);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* ring = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* full = reinterpret_cast<uint64_t*>(ring + (size_t)stages * stage_bytes);
@@ -244,21 +247,32 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
         for (int s = 0; s < stages; s++) { mbar_init(&full[s], 2); mbar_init(&empty[s], 1); }
-        for (int s = 0; s < 2; s++) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], S::kEpiWarps); }
+        for (int s = 0; s < 2; s++) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], kCtas * S::kEpiWarps); }
         mbar_init_fence();
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)), "r"(S::kTmemCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (kPair) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)), "r"(S::kTmemCols)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)), "r"(S::kTmemCols)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (kPair) {        // (the leader's barriers are there before anything is counted on them)
+        cluster_arrive();
+        cluster_wait();
+    }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     pdl_launch_dependents();
 
-    const int n_tiles = (l.N + kTc5Rows - 1) / kTc5Rows, t_tiles = (T + bn - 1) / bn;
+    const int rank = kPair ? (int)pair_rank() : 0, unit = (int)blockIdx.x / kCtas, units = (int)gridDim.x / kCtas;      // a unit has a tile at a time
+    const int n_tiles = (l.N + kTileRows - 1) / kTileRows, t_tiles = (T + bn - 1) / bn;
     // tokens vary fastest: the CTAs at work share few rows of weights, which go through HBM once
     const int tiles = n_tiles * t_tiles, kb_all = (l.K + kTc5Depth - 1) / kTc5Depth;
     // few tiles: the CTAs of a cluster take a range of K each and join their sums through shared memory (one tile per cluster then)
@@ -269,7 +283,7 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
     // of the row, next_of(c0) the step that this thread takes after c0 (bn and beyond: none); the first residual rows are fetched before ready().
     const int quarter = warp & 3, r = 32 * quarter + lane;
     auto finish = [&](int tile, int c_first, auto ready, auto sums, auto next_of) {
-        const int n = (tile / t_tiles) * kTc5Rows + r;
+        const int n = (tile / t_tiles) * kTileRows + rank * kTc5Rows + r;
         const int tb = (tile % t_tiles) * bn;
         const bool live = n < l.N;
         // residual rows are fetched a step of 16 tokens ahead, the first under the tile's products
@@ -370,19 +384,20 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
         // cycles between two K blocks, mostly its own chain of instructions, and bounded tiles of up to 200 tokens.)
         if (lane == 0) {
             const bool tokens = warp == 2;
-            const uint32_t to0 = smem_addr(ring) + (tokens ? kTc5ABytes : 0), bytes = (uint32_t)(tokens ? bn * kTc5Depth * 2 : kTc5ABytes);
-            const uint32_t full0 = smem_addr(full), empty0 = smem_addr(empty);
+            const uint32_t to0 = smem_addr(ring) + (tokens ? kTc5ABytes : 0), bytes = (uint32_t)(tokens ? own * kTc5Depth * 2 : kTc5ABytes);
+            const uint32_t full0 = smem_addr(full), empty0 = smem_addr(empty), lead0 = kPair ? leader_addr(full) : full0;
             const CUtensorMap* map = tokens ? &xmap : &wmap;
             if (tokens) pdl_wait();
             uint32_t s = 0, par = 1;        // (the first round's waits pass)
             bool ok = true, ready = true;
-            for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
-                const int y = tokens ? (tile % t_tiles) * bn : (tile / t_tiles) * kTc5Rows;
+            for (int tile = unit; ok && tile < tiles; tile += units) {
+                const int y = tokens ? (tile % t_tiles) * bn + rank * own : (tile / t_tiles) * kTileRows + rank * kTc5Rows;
                 int x = kb0 * kTc5Depth;
                 for (int kb = 0; kb < kb_n; kb++, x += kTc5Depth) {
                     if (!ready && !mbar_wait_at(empty0 + 8 * s, par, err, 41)) { ok = false; break; }
-                    mbar_expect_tx_at(full0 + 8 * s, bytes);
-                    tma_rows_2d_at(to0 + s * stage_bytes, map, x, y, full0 + 8 * s);
+                    if (!kPair || rank == 0) mbar_expect_tx_at(full0 + 8 * s, kCtas * bytes);
+                    if (kPair) tma_pair_rows_2d_at(to0 + s * stage_bytes, map, x, y, lead0 + 8 * s);
+                    else tma_rows_2d_at(to0 + s * stage_bytes, map, x, y, full0 + 8 * s);
                     if (++s == (uint32_t)stages) { s = 0; par ^= 1u; }
                     ready = mbar_test_at(empty0 + 8 * s, par);
                 }
@@ -390,8 +405,16 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer
-        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kTc5Rows >> 4) << 24);
-        if (elect_one()) {
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kTileRows >> 4) << 24);
+        auto mma = [&](uint32_t d, uint64_t ad, uint64_t bd, uint32_t accum) {
+            if (kPair) umma_pair_bf16_ss(d, ad, bd, idesc, accum);
+            else umma_bf16_ss(d, ad, bd, idesc, accum);
+        };
+        auto commit = [](uint32_t bar) {
+            if (kPair) umma_pair_commit_at(bar);
+            else umma_commit_at(bar);
+        };
+        if (rank == 0 && elect_one()) {
             // one thread walks the steps.  Whether the next stage is there is asked before this one's products are issued, so that the
             // answer's latency passes under them: 168 K blocks of 2048 rows took 49, 53, 70 us at 16, 80, 256 tokens a tile, now 34, 38, 68
             const uint32_t full0 = smem_addr(full), empty0 = smem_addr(empty), acc0 = smem_addr(acc_full);
@@ -399,9 +422,9 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
             const int steps_last = (l.K - (kb0 + kb_n - 1) * kTc5Depth) / 16;      // products of the last K block of a tile, if fewer than four
             uint32_t s = 0, full_par = 0, local = 0;
             bool ok = true, ready = false;
-            for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x, local++) {
-                const uint32_t a = local & 1;
-                if (local >= 2 && !mbar_wait_bounded(&acc_empty[a], ((local >> 1) - 1) & 1u, err, 42)) break;
+            for (int tile = unit; ok && tile < tiles; tile += units, local++) {
+                const uint32_t a = local & 1, acc_par = ((local >> 1) - 1) & 1u;
+                if (local >= 2 && !(kPair ? mbar_wait_cluster(&acc_empty[a], acc_par, err, 42) : mbar_wait_bounded(&acc_empty[a], acc_par, err, 42))) break;
                 const uint32_t d = tmem_base + a * BN;
                 for (int kb = 0; kb < kb_n; kb++) {
                     if (!ready && !mbar_wait_at(full0 + 8 * s, full_par, err, 43)) { ok = false; break; }
@@ -410,16 +433,16 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
                     ready = mbar_test_at(full0 + 8 * s, full_par);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t ad = a0 + at, bd = b0 + at;
-                    umma_bf16_ss(d, ad, bd, idesc, kb ? 1u : 0u);
+                    mma(d, ad, bd, kb ? 1u : 0u);
                     if (kb + 1 < kb_n || steps_last >= 4) {
 #pragma unroll
-                        for (int k = 1; k < 4; k++) umma_bf16_ss(d, ad + 2 * k, bd + 2 * k, idesc, 1u);
+                        for (int k = 1; k < 4; k++) mma(d, ad + 2 * k, bd + 2 * k, 1u);
                     } else {
-                        for (int k = 1; k < steps_last; k++) umma_bf16_ss(d, ad + 2 * k, bd + 2 * k, idesc, 1u);
+                        for (int k = 1; k < steps_last; k++) mma(d, ad + 2 * k, bd + 2 * k, 1u);
                     }
-                    umma_commit_at(empty0 + 8 * now);
+                    commit(empty0 + 8 * now);
                 }
-                if (ok) umma_commit_at(acc0 + 8 * a);
+                if (ok) commit(acc0 + 8 * a);
             }
         }
         __syncwarp();
@@ -429,7 +452,7 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
         const int share = (warp - 3) >> 2, steps = bn / 16, c_begin = share * steps / kShares * 16, c_end = (share + 1) * steps / kShares * 16;
         int local = 0;
         pdl_wait();
-        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, local++) {
+        for (int tile = unit; tile < tiles; tile += units, local++) {
             const int a = local & 1;
             const uint32_t ta = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(a * BN);
             auto ready = [&]() {
@@ -441,7 +464,7 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
                 tmem_ld(ta + c0, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             };
-            if (ranges > 1) {
+            if (!kPair && ranges > 1) {
                 if (!ready()) break;
                 for (int c0 = c_begin; c0 < c_end; c0 += 16) {
                     int v[16];
@@ -454,16 +477,27 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[a]);
+            if (lane == 0) {
+                if (kPair) mbar_arrive_leader(leader_addr(&acc_empty[a]));
+                else mbar_arrive(&acc_empty[a]);
+            }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 1) {
+    if (kPair) {        // nobody leaves while its operands or barriers are in use
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        if (warp == 1) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(S::kTmemCols) : "memory");
+        }
+    } else if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(S::kTmemCols) : "memory");
     }
-    if (ranges > 1) {
+    if (!kPair && ranges > 1) {
         // every CTA finishes some of the tile's steps of 16 tokens, its epilogue warps' halves taking turns; ranges are added in their order
         __syncwarp();
         cluster_arrive();
@@ -496,24 +530,27 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
 
 // ------------------------------------------------------------------ host side
 
-struct Tc5Tiles { int tokens, ranges; };      // of a tile; of K
+struct Tc5Tiles { int tokens, ranges, ctas; };      // of a tile; of K; CTAs that share a tile
 
-template <int BN>
+template <int BN, bool kPair>
 static int launch_tc5(const Linear& l, int T, Tc5Tiles t, cudaStream_t s)
 {
     using S = Tc5Linear<BN>;
     CUtensorMap wmap, xmap;
     int rc;
+    constexpr int kCtas = kPair ? 2 : 1;
+    const int own = t.tokens / kCtas;
     if ((rc = bf16_map(&wmap, l.W, l.K, l.N, l.K, kTc5Rows))) return rc;
-    if ((rc = bf16_map(&xmap, l.in, l.K, T, l.ld_in, t.tokens))) return rc;
-    if ((rc = allow_smem<k_linear_tc5<BN>>(227 * 1024))) return rc;
-    const long tiles = (long)((l.N + kTc5Rows - 1) / kTc5Rows) * ((T + t.tokens - 1) / t.tokens);
-    const unsigned grid = (unsigned)(t.ranges > 1 || tiles < sm_count() ? tiles : sm_count());
-    return launch_cluster(k_linear_tc5<BN>, dim3(grid, (unsigned)t.ranges), dim3(1, (unsigned)t.ranges, 1), S::kThreads, tc5_smem(t.tokens), s, wmap, xmap, l, T,
+    if ((rc = bf16_map(&xmap, l.in, l.K, T, l.ld_in, own))) return rc;
+    if ((rc = allow_smem<k_linear_tc5<BN, kPair>>(227 * 1024))) return rc;
+    const long tiles = (long)((l.N + kCtas * kTc5Rows - 1) / (kCtas * kTc5Rows)) * ((T + t.tokens - 1) / t.tokens);
+    const long units = sm_count() / kCtas;
+    const unsigned grid = (unsigned)(kCtas * (t.ranges > 1 || tiles < units ? tiles : units));
+    return launch_cluster(k_linear_tc5<BN, kPair>, dim3(grid, (unsigned)t.ranges), dim3(kCtas, (unsigned)t.ranges, 1), S::kThreads, tc5_smem(own), s, wmap, xmap, l, T,
                           t.tokens, device_error_flag());
 }
 
-// Tokens of a tile (a multiple of 16) and ranges of K with the least time in cycles: waves of CTAs over the SMs times a tile's K blocks, each
+// Tokens of a tile (a multiple of 16), ranges of K and CTAs of a tile with the least time in cycles: waves of CTAs over the SMs times a tile's K blocks, each
 // 310 + 1.3 per token (measured: 325 at 16 tokens, 650 at 256); K is cut, into ranges of at least four blocks, where all its tiles' clusters
 // run at once, and joining r ranges costs 3000 + 800 r + 25 per token.  2048 rows of 10752 (us, one range, several): 48 tokens 33.5, 14.2 at
 // six; 200 tokens 33.9, 19.0 at four; of 2048: 16 tokens 8.8, 7.3 at four; 200 tokens 9.2, 9.3.
@@ -521,16 +558,26 @@ static Tc5Tiles tc5_tiles(const Linear& l, int T)
 {
     const int n_tiles = (l.N + kTc5Rows - 1) / kTc5Rows, top = (T + 15) / 16 * 16 < 256 ? (T + 15) / 16 * 16 : 256;
     const int kb = (l.K + kTc5Depth - 1) / kTc5Depth, sms = sm_count();
-    const int* clusters = active_clusters<k_linear_tc5<256>>(Tc5Linear<256>::kThreads, 200 * 1024);      // (a CTA has an SM to itself)
-    Tc5Tiles best = {16, 1};
+    const int* clusters = active_clusters<k_linear_tc5<256, false>>(Tc5Linear<256>::kThreads, 200 * 1024);      // (a CTA has an SM to itself)
+    Tc5Tiles best = {16, 1, 1};
     double least = 0.0;
     for (int bn = 16; bn <= top; bn += 16) {
         const long tiles = (long)n_tiles * ((T + bn - 1) / bn);
         for (int ranges = 1; ranges <= 8 && (ranges == 1 || (clusters && tiles <= clusters[ranges] && kb / ranges >= 4)); ranges++) {
             const long waves = ranges > 1 ? 1 : (tiles + sms - 1) / sms;
             const double time = (double)waves * ((kb + ranges - 1) / ranges) * (310.0 + 1.3 * bn) + (ranges > 1 ? 3000.0 + 800.0 * ranges + 25.0 * bn : 0.0);
-            if ((bn == 16 && ranges == 1) || time <= least) { best = {bn, ranges}; least = time; }
+            if ((bn == 16 && ranges == 1) || time <= least) { best = {bn, ranges, 1}; least = time; }
         }
+    }
+    // A pair has 256 rows to a tile and fetches a third less per product; a K block takes 180 + 1.65 per token (168 of 2048 rows, 700 tokens, us: 128
+    // tokens a tile 39, 192 47, 256 58).  Setting it up costs more than one CTA, so only wide tiles and several waves.  Prompts through four layers
+    // of the hybrid decoder (us, single CTAs, pairs): 2048 tokens 1481, 1447; 900 835, 791; two layers of width 1024, 400 tokens, with pairs of any
+    // tile 248, 264.
+    const int pairs = sms / 2, row_pairs = (l.N + 2 * kTc5Rows - 1) / (2 * kTc5Rows);
+    for (int bn = 192; bn <= top; bn += 32) {
+        const long waves = ((long)row_pairs * ((T + bn - 1) / bn) + pairs - 1) / pairs;
+        const double time = (double)waves * kb * (180.0 + 1.65 * bn) + 2500.0;
+        if (waves >= 2 && time < least) { best = {bn, 1, 2}; least = time; }
     }
     return best;
 }
@@ -567,10 +614,11 @@ int linear_forward(const Linear& l, int T, bool act_bf16, cudaStream_t s)
         return launch_ordered(k_linear_tile<4>, dim3(n_tiles, (T + 63) / 64), 256, 0, s, l, T);
     }
     const Tc5Tiles t = tc5_tiles(l, T);
-    if (t.tokens > 128) return launch_tc5<256>(l, T, t, s);
-    if (t.tokens > 64) return launch_tc5<128>(l, T, t, s);
-    if (t.tokens > 32) return launch_tc5<64>(l, T, t, s);
-    return launch_tc5<32>(l, T, t, s);
+    if (t.ctas == 2) return t.tokens > 128 ? launch_tc5<256, true>(l, T, t, s) : launch_tc5<128, true>(l, T, t, s);
+    if (t.tokens > 128) return launch_tc5<256, false>(l, T, t, s);
+    if (t.tokens > 64) return launch_tc5<128, false>(l, T, t, s);
+    if (t.tokens > 32) return launch_tc5<64, false>(l, T, t, s);
+    return launch_tc5<32, false>(l, T, t, s);
 }
 
 }  // namespace bpdq
@@ -593,6 +641,14 @@ int bpd_linear_bf16_cuda(const uint16_t* W, const void* x, float* out, int n_tok
     l.out = out;
     l.ld_out = N;
     return linear_forward(l, n_tokens, act_bf16 != 0, (cudaStream_t)stream);
+}
+
+int bpdq_linear_bf16_ctas(int n_tokens, int N, int K)
+{
+    if (n_tokens < 2 || N < 1 || K < 16 || K % 16) return BPDQ_ERR_ARG;
+    Linear l = {};
+    l.N = N; l.K = K;
+    return tc5_tiles(l, n_tokens).ctas;
 }
 
 int bpdq_linear_bf16_tiles(int n_tokens, int N, int K, int* tokens, int* ranges)

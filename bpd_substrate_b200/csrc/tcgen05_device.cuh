@@ -196,4 +196,62 @@ __device__ __forceinline__ void tma_rows_3d(void* dst_smem, const CUtensorMap* m
         : "memory");
 }
 
+// ---- pairs of CTAs (clusters of two along x) that share a product: operands, accumulators and barriers of the even CTA, the leader, at the
+// same places in both
+__device__ __forceinline__ uint32_t pair_rank()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t leader_addr(const void* p)
+{
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(0));
+    return a;
+}
+__device__ __forceinline__ void umma_pair_bf16_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum)
+        : "memory");
+}
+// One arrival at the barrier of that place in both CTAs once the leader's MMAs so far are done.
+__device__ __forceinline__ void umma_pair_commit_at(uint32_t bar)
+{
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((unsigned short)3)
+                 : "memory");
+}
+// Into this CTA's shared memory, counted on the leader's barrier.
+__device__ __forceinline__ void tma_pair_rows_2d_at(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t leader_bar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+        "l"(map), "r"(x), "r"(y), "r"(leader_bar)
+        : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_leader(uint32_t leader_bar)
+{
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_bar) : "memory");
+}
+// A bounded wait for arrivals of the other CTA.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, int* err, int code)
+{
+    for (uint32_t i = 0; i < (1u << 22); i++) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_addr(bar)), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    if (err) atomicCAS(err, 0, code);
+    return false;
+}
+
 }  // namespace bpdq

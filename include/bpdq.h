@@ -467,6 +467,8 @@ int bpd_llama_forward_ws_cuda(const int32_t* token_ids, int n_tokens, const bpd_
 int bpd_linear_bf16_cuda(const uint16_t* W, const void* x, float* out, int n_tokens, int N, int K, int act_bf16, void* stream);
 /* how that cuts several tokens with bf16 activations: tokens of a tile, and ranges of K that the CTAs of a cluster take */
 int bpdq_linear_bf16_tiles(int n_tokens, int N, int K, int* tokens, int* ranges);
+/* the CTAs that share a tile: two for large products */
+int bpdq_linear_bf16_ctas(int n_tokens, int N, int K);
 /* the same product, each sum v of row n mapped: gelu(v), tanh form, in the activation type; or in fp32 cap tanh(v / cap),
  * rate[n] softplus(v + bias[n]), sigmoid(v) */
 enum { BPDQ_MAP_GELU = 0, BPDQ_MAP_CAP = 1, BPDQ_MAP_LOG_DECAY = 2, BPDQ_MAP_SIGMOID = 3 };
