@@ -69,6 +69,21 @@ bool scratch_fits(const Workspace* ws, int kind, size_t bytes, cudaStream_t s);
 int gemv_q8_0_fast(const uint8_t* W, const float* x, float* out, int N, int K, cudaStream_t s);
 int gemv_q8_0_fast_multi(int n, const uint8_t* const* Ws, float* const* outs, const int* Ns, const float* x, int K,
                          cudaStream_t s);
+// The same, the vector formed in the launch: x + r (null: x), kept in x_out (null: nowhere; another place than x), through the Llama's rms norm (norm_w null: x
+// as it is).  gated: two
+// matrices, out[0] = silu(W[0] v) * (W[1] v).  BPDQ_ERR_RANGE: not for this kernel (q8_0_llama_fits says so ahead).
+struct Q80Llama {
+    const float *x, *r, *norm_w;
+    float* x_out;
+    float eps;
+    int n, K;
+    const uint8_t* W[3];
+    float* out[3];
+    int N[3];
+    bool gated;
+};
+bool q8_0_llama_fits(const Q80Llama& l);
+int q8_0_llama(const Q80Llama& l, cudaStream_t s);
 // peer_exchange.cu: where a product's results are stored besides its own output (gathered buffers of all
 // ranks, byte shifts from the output address), and the flag slots of the per-step signal
 constexpr int kMaxPeerTargets = 8;

@@ -17,6 +17,7 @@
 //    FMAs of half_block_fma, then the rows are folded over the lanes by fold_rows.
 
 #include "gemv_q4k_device.cuh"
+#include "q8_0_tiles.cuh"
 
 namespace bpdq {
 
@@ -159,6 +160,7 @@ __global__ void __launch_bounds__(256) k_vector_records(const float* __restrict_
 // bulk copy of the tile it will need `slots` turns later, so a freed slot is on its way to being full again at
 // once and nobody has to notice that it became free.  (A producer warp polling the slots' "empty" barriers
 // reacted too slowly for tiles of a few KB: the weight stream then ran at 85 % of what HBM delivers.)
+// FMT: 0 Q4_K, 1 Q8_0, 2 Q8_0 with what a decoded token of the Llama adds (a vector formed in the launch, gates)
 template <int FMT, int LAYOUT, int MAXTHREADS, int ACC>
 __global__ void __launch_bounds__(MAXTHREADS, 1)
 k_gemv_batch_q4k_q8k(const BatchPlan p, int* __restrict__ err)
@@ -194,9 +196,11 @@ k_gemv_batch_q4k_q8k(const BatchPlan p, int* __restrict__ err)
         const BatchProblem& pb = p.prob[j];
         const int row0 = (lv - pb.tile_begin) * pb.rt;
         const uint32_t bytes = (uint32_t)min(pb.rt, pb.M - row0) * pb.row_bytes;
+        const bool gated = FMT == 2 && p.gated;
         if (lane == 0) {
-            mbar_expect_tx(&my_full[slot], bytes);
+            mbar_expect_tx(&my_full[slot], gated ? 2 * bytes : bytes);
             bulk_g2s(my_ring + (size_t)slot * p.slot_bytes, pb.W + (size_t)row0 * pb.row_bytes, bytes, &my_full[slot]);
+            if (gated) bulk_g2s(my_ring + (size_t)slot * p.slot_bytes + bytes, p.prob[1].W + (size_t)row0 * pb.row_bytes, bytes, &my_full[slot]);
         }
         lv += stride;
     };
@@ -221,6 +225,9 @@ k_gemv_batch_q4k_q8k(const BatchPlan p, int* __restrict__ err)
         BPDQ_TRACE(2);
         if (p.prologue == 1) {
             cta_rmsnorm_records(p.pro_a, p.pro_b, p.pro_eps, p.vec[0].nb, xq, reinterpret_cast<float*>(xbar + 1), warp, lane, p.nw);
+        } else if (FMT == 2 && p.prologue == 3) {
+            cta_add_rmsnorm_records_q80(p.pro_a, p.pro_r, p.pro_b, blockIdx.x == 0 ? p.pro_out : nullptr, p.pro_eps, p.vec[0].nb,
+                                        reinterpret_cast<float*>(smem + p.off_pro), xq, reinterpret_cast<double*>(xbar + 1), warp, lane, p.nw);
         } else if (p.prologue == 2) {
             cta_swiglu_records(p.pro_a, p.pro_b, p.vec[0].nb, xq, warp, lane, p.nw);
         } else {
@@ -261,6 +268,14 @@ k_gemv_batch_q4k_q8k(const BatchPlan p, int* __restrict__ err)
     int slot = 0;
     uint32_t parity = 0;
     bool first_tile = true;
+    // gate, up and row of a tile that this lane finishes (gated: the activation is in binary64, 32 rows at once)
+    float gate = 0.0f, up = 0.0f;
+    int gated_row = -1, waiting = 0;
+    auto finish_gated = [&]() {
+        if (gated_row >= 0) p.prob[0].out[gated_row] = swiglu_rounded(gate, up);
+        gated_row = -1;
+        waiting = 0;
+    };
     for (int v = first; v < p.n_tiles; v += stride) {
         if (!mbar_wait_bounded(&my_full[slot], parity, err, 2)) return;
         if (first_tile) { BPDQ_TRACE(5); first_tile = false; }
@@ -276,6 +291,14 @@ k_gemv_batch_q4k_q8k(const BatchPlan p, int* __restrict__ err)
             if (pb.rt == 4) batch_tile<4, LAYOUT, ACC>(tile_smem, xq + pb.xq_off, pb, row0, lane, peers);
             else if (pb.rt == 2) batch_tile<2, LAYOUT, ACC>(tile_smem, xq + pb.xq_off, pb, row0, lane, peers);
             else batch_tile<1, LAYOUT, ACC>(tile_smem, xq + pb.xq_off, pb, row0, lane, peers);
+        } else if (FMT == 2 && p.gated) {
+            const float sum = batch_tile_q80<2>(tile_smem, xq + pb.xq_off, pb, row0, lane, false), other = __shfl_xor_sync(0xFFFFFFFFu, sum, 16);
+            if (lane == waiting) {
+                gate = lane < 16 ? sum : other;
+                up = lane < 16 ? other : sum;
+                gated_row = row0;
+            }
+            if (++waiting == 32) finish_gated();
         } else {
             if (pb.rt == 4) batch_tile_q80<4>(tile_smem, xq + pb.xq_off, pb, row0, lane);
             else if (pb.rt == 2) batch_tile_q80<2>(tile_smem, xq + pb.xq_off, pb, row0, lane);
@@ -290,12 +313,13 @@ k_gemv_batch_q4k_q8k(const BatchPlan p, int* __restrict__ err)
             parity ^= 1u;
         }
     }
+    if (FMT == 2 && p.gated) finish_gated();
     BPDQ_TRACE(6);
 }
 
 // Builds the launch plan for descs[0..n); returns BPDQ_ERR_RANGE when the set does not fit one
 // launch (too many activations for shared memory, or rows longer than a ring slot).
-int make_batch_plan(const BatchDesc* d, int n, BatchPlan& p, int fmt, int ctas_per_sm)
+int make_batch_plan(const BatchDesc* d, int n, BatchPlan& p, int fmt, int ctas_per_sm, int pro_bytes, bool gated)
 {
     if (n < 1 || n > kMaxBatch) return BPDQ_ERR_RANGE;
     const Tuning& tu = tuning();
@@ -310,6 +334,9 @@ int make_batch_plan(const BatchDesc* d, int n, BatchPlan& p, int fmt, int ctas_p
     p.prologue = 0;
     p.pro_a = p.pro_b = nullptr;
     p.pro_eps = 0.0f;
+    p.pro_r = nullptr;
+    p.pro_out = nullptr;
+    p.gated = gated;
     int xq_bytes = 0;
     // Rows per tile: as many as fit tile_bytes (1, 2 or 4).  A launch with a lot of work gets a
     // slightly larger budget, 4 rows of K = 4096 (9216 bytes): the per-tile work of a consumer warp
@@ -332,9 +359,10 @@ int make_batch_plan(const BatchDesc* d, int n, BatchPlan& p, int fmt, int ctas_p
         pb.row_bytes = fmt == 0 ? pb.nb * BPDQ_Q4K_BYTES : pb.nb * 8 * BPDQ_Q80_BYTES;
         if (pb.row_bytes > slot_cap) return BPDQ_ERR_RANGE;
         pb.rt = 4 * pb.row_bytes <= tile_budget ? 4 : (2 * pb.row_bytes <= tile_budget ? 2 : 1);
+        if (gated) pb.rt = 1;
         if (pb.rt * pb.row_bytes > p.slot_bytes) p.slot_bytes = pb.rt * pb.row_bytes;
-        pb.tile_begin = p.n_tiles;
-        p.n_tiles += (pb.M + pb.rt - 1) / pb.rt;
+        pb.tile_begin = gated && j ? 0x7FFFFFFF : p.n_tiles;
+        if (!gated || !j) p.n_tiles += (pb.M + pb.rt - 1) / pb.rt;
         int k = 0;
         for (; k < p.n_vectors; k++)
             if (p.vec[k].x == d[j].x && p.vec[k].nb == pb.nb) break;
@@ -354,6 +382,7 @@ int make_batch_plan(const BatchDesc* d, int n, BatchPlan& p, int fmt, int ctas_p
     }
     for (int k = p.n_vectors; k < kMaxBatch; k++) p.vec[k] = p.vec[0];
     p.xq_bytes = xq_bytes;
+    if (gated) p.slot_bytes *= 2;
     p.slots = tu.stages < 2 ? 2 : tu.stages;
     p.nw = tu.warps < 1 ? 1 : (tu.warps > 16 ? 16 : tu.warps);
     for (;;) {
@@ -361,6 +390,7 @@ int make_batch_plan(const BatchDesc* d, int n, BatchPlan& p, int fmt, int ctas_p
         auto take = [&off](size_t bytes) { size_t at = off; off += (bytes + 127) / 128 * 128; return (int)at; };
         p.off_ring = take((size_t)p.nw * p.slots * p.slot_bytes);
         p.off_xq = take((size_t)xq_bytes);
+        p.off_pro = take((size_t)pro_bytes);
         p.off_bar = take((size_t)2 * p.nw * p.slots * 8 + 8 + 64);   // barriers, then nine floats of the rms_norm prologue
         p.smem = off;
         // ctas_per_sm = 2: a CTA takes less than half of the SM's shared memory (1 KB per CTA is the system's), so that
@@ -597,6 +627,30 @@ int gemv_q8_0_fast_multi(int n, const uint8_t* const* Ws, float* const* outs, co
     int rc = make_batch_plan(d, n, plan, 1);
     if (rc) return rc;
     return launch_batch<1, BPDQ_LAYOUT_BPD>(plan, s);
+}
+
+bool q8_0_llama_fits(const Q80Llama& l)
+{
+    if (l.n < 1 || l.n > kMaxBatch || l.K < 256 || l.K % 256 || (l.norm_w && l.K > 8192) || (l.gated && (l.n != 2 || l.N[0] != l.N[1]))) return false;
+    uintptr_t all = (uintptr_t)l.x | (uintptr_t)l.r | (uintptr_t)l.norm_w | (uintptr_t)l.x_out;
+    for (int j = 0; j < l.n; j++) all |= (uintptr_t)l.W[j];
+    return !(all & 15) && l.x;
+}
+int q8_0_llama(const Q80Llama& l, cudaStream_t s)
+{
+    if (!q8_0_llama_fits(l)) return BPDQ_ERR_RANGE;
+    BatchDesc d[kMaxBatch];
+    for (int j = 0; j < l.n; j++) d[j] = {l.W[j], l.x, l.out[j], l.N[j], l.K};
+    BatchPlan plan;
+    const int rc = make_batch_plan(d, l.n, plan, 1, 1, l.norm_w ? 4 * l.K : 0, l.gated);
+    if (rc) return rc;
+    plan.prologue = l.norm_w ? 3 : 0;
+    plan.pro_a = l.x;
+    plan.pro_r = l.r;
+    plan.pro_b = l.norm_w;
+    plan.pro_out = l.x_out;
+    plan.pro_eps = l.eps;
+    return launch_batch<2, BPDQ_LAYOUT_BPD>(plan, s);
 }
 
 // ---------------------------------------------------------------- scratch without an allocator

@@ -190,10 +190,17 @@ struct BatchPlan {
     int xq_bytes;
     // what the CTAs do to the launch's single input vector before they quantize it themselves (records
     // null): 0 nothing, 1 rms_norm(pro_a, weights pro_b, pro_eps), 2 silu(pro_a) * pro_b
+    // 3 (Q8_0 only): pro_a + pro_r (null: pro_a), kept in pro_out (null: nowhere), as the Llama's rms norm with weights pro_b leaves it; off_pro: its
+    // copy in shared memory
     int prologue;
     const float* pro_a;
     const float* pro_b;
     float pro_eps;
+    const float* pro_r;
+    float* pro_out;
+    int off_pro;
+    // Q8_0 only: problem 0 is a gate and problem 1 its up projection; a tile has the same rows of both and out[row] of problem 0 becomes silu(gate) * up
+    int gated;
     BatchProblem prob[kMaxBatch];
     BatchVector vec[kMaxBatch];
     // n > 0: every result is also stored at its output address + shift[t] (the gathered buffers of the ranks
@@ -257,11 +264,12 @@ __device__ __forceinline__ void write_records_q80(const float4& v0, const float4
     }
 }
 
+// Every lane ends with the sum of row lane / (32 / R); store: it goes to its place, of the rows that there are.
 template <int R>
-__device__ __forceinline__ void batch_tile_q80(const uint8_t* tile_smem, const uint8_t* xq, const BatchProblem& pb,
-                                               int row0, int lane)
+__device__ __forceinline__ float batch_tile_q80(const uint8_t* tile_smem, const uint8_t* xq, const BatchProblem& pb,
+                                                int row0, int lane, bool store = true)
 {
-    const int rows = min(R, pb.M - row0);
+    const int rows = store ? min(R, pb.M - row0) : R;
     const int n_pairs = 4 * pb.nb;
     float acc[R];
 #pragma unroll
@@ -302,7 +310,8 @@ __device__ __forceinline__ void batch_tile_q80(const uint8_t* tile_smem, const u
     const float total = fold_rows<R>(acc, lane);
     constexpr int kLanesPerRow = 32 / R;
     const int my_row = lane / kLanesPerRow;
-    if ((lane % kLanesPerRow) == 0 && my_row < rows) pb.out[row0 + my_row] = total;
+    if (store && (lane % kLanesPerRow) == 0 && my_row < rows) pb.out[row0 + my_row] = total;
+    return total;
 }
 
 template <int R, int LAYOUT, int ACC>
@@ -434,6 +443,46 @@ __device__ __forceinline__ void cta_rmsnorm_records(const float* __restrict__ a,
         emit(b, __ldcg(xb + lane), __ldcg(xb + 32 + lane), __ldg(wb + lane), __ldg(wb + 32 + lane));
     }
 }
+// The Llama's residual add and rms norm ahead of a Q8_0 product: the operations of k_add_rmsnorm_llama (llama_forward.cu) on the same values in the same
+// order, then the product's records.  256 threads' sums in binary64, thread t of columns t, t + 256, ..., are formed by the consumer warps in turn.
+__device__ __forceinline__ void cta_add_rmsnorm_records_q80(const float* x, const float* r, const float* __restrict__ w, float* x_out, float eps, int nb,
+                                                            float* v_smem, uint8_t* xq, double* s_sum, int warp, int lane, int nw)
+{
+    const int cols = nb * 256;
+    for (int b = warp; b < nb; b += nw) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int c = 256 * b + 128 * h + 4 * lane;
+            float4 v = __ldcg(reinterpret_cast<const float4*>(x + c));
+            if (r) {
+                const float4 a = __ldcg(reinterpret_cast<const float4*>(r + c));
+                v = make_float4(__fadd_rn(v.x, a.x), __fadd_rn(v.y, a.y), __fadd_rn(v.z, a.z), __fadd_rn(v.w, a.w));
+            }
+            *reinterpret_cast<float4*>(v_smem + c) = v;
+            if (x_out) *reinterpret_cast<float4*>(x_out + c) = v;
+        }
+    }
+    named_bar_sync(2, nw * 32);
+    for (int vw = warp; vw < 8; vw += nw) {
+        double t = 0.0;
+        for (int c = 32 * vw + lane; c < cols; c += 256) t += (double)v_smem[c] * (double)v_smem[c];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
+        if (lane == 0) s_sum[vw] = t;
+    }
+    named_bar_sync(2, nw * 32);
+    double tot = 0.0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) tot += s_sum[i];
+    const float mean = (float)(tot / (double)cols);
+    const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, eps)));
+    auto scaled = [&](int c) {
+        const float4 v = *reinterpret_cast<const float4*>(v_smem + c), g = __ldg(reinterpret_cast<const float4*>(w + c));
+        return make_float4(__fmul_rn(__fmul_rn(v.x, scale), g.x), __fmul_rn(__fmul_rn(v.y, scale), g.y), __fmul_rn(__fmul_rn(v.z, scale), g.z),
+                           __fmul_rn(__fmul_rn(v.w, scale), g.w));
+    };
+    for (int b = warp; b < nb; b += nw) write_records_q80(scaled(256 * b + 4 * lane), scaled(256 * b + 128 + 4 * lane), xq + (size_t)(4 * b) * kQ80PairStride, lane);
+}
 // silu(gate) * up with k_elementwise's arithmetic; three blocks' loads in flight per warp
 __device__ __forceinline__ void cta_swiglu_records(const float* __restrict__ gate, const float* __restrict__ up, int nb,
                                                    uint8_t* xq, int warp, int lane, int nw)
@@ -502,7 +551,7 @@ unsigned long long* trace_take();
 int gemm_q4k_q8k(const uint8_t* W, const void* x, float* out, int tokens, int M, int K, int layout, int xsrc,
                  int32_t* dbg, cudaStream_t s, Workspace* ws = nullptr);
 // gemv_batch.cu: plan and launch of the batched kernel (fmt 0: Q4_K weights, 1: Q8_0)
-int make_batch_plan(const BatchDesc* d, int n, BatchPlan& p, int fmt = 0, int ctas_per_sm = 1);
+int make_batch_plan(const BatchDesc* d, int n, BatchPlan& p, int fmt = 0, int ctas_per_sm = 1, int pro_bytes = 0, bool gated = false);
 int launch_batch_plan(const BatchPlan& p, int fmt, int layout, cudaStream_t s);
 
 // a small kernel (256 threads per CTA unless said otherwise) launched programmatically behind the launch before it

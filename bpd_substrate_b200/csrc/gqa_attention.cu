@@ -11,6 +11,7 @@
 #include "cluster_device.cuh"
 #include "launch.cuh"
 #include "mma_device.cuh"
+#include "rope_device.cuh"
 #include "../../include/bpdq.h"
 
 #include <cuda_fp16.h>
@@ -95,14 +96,17 @@ constexpr int kSplitThreads = 256, kSplitWarps = kSplitThreads / 32, kMaxCluster
 // A lane holds 16 bytes of a key row, so a load of the warp covers 32 lanes / (row / 16 bytes) keys; eight such loads are in
 // flight.  Scores go to shared memory; maximum, weights and their sum per CTA; values the same way as keys; the cluster then
 // weighs its CTAs' sums by exp(m_i - m).
-template <int F16, int D, int R>
-__global__ void __launch_bounds__(kSplitThreads) k_gqa_split(GqaShape p, const float* q, const void* kc, const void* vc, float* dst, int stretch)
+//
+// NEW: a decoded token's rotation and cache row, which were a launch of their own (4 us of a layer's 80 at 4000 keys), are part of it.  The angles take one
+// thread per pair; the CTA whose stretch holds the new row writes it and reads it back, for every cluster of a key head alike.
+template <int F16, int D, int R, bool NEW>
+__global__ void __launch_bounds__(kSplitThreads) k_gqa_split(GqaShape p, GqaNew in, const float* q, const void* kc, const void* vc, float* dst, int stretch)
 {
     constexpr int E = F16 ? 8 : 4;              // elements of a load
     constexpr int L = D / E, P = 32 / L;        // lanes per key, keys per load
     constexpr int NV = 8 * R, NR = NV / L > 0 ? NV / L : 1;
     pdl_launch_dependents();
-    pdl_wait();
+    if (!NEW) pdl_wait();
     extern __shared__ __align__(16) float sh[];
     float* s_out = sh;                          // [R][D] this CTA's sums
     float* s_part = s_out + R * D;              // [warps][R][D]
@@ -118,7 +122,50 @@ __global__ void __launch_bounds__(kSplitThreads) k_gqa_split(GqaShape p, const f
     const char* kbase = reinterpret_cast<const char*>(kc) + (size_t)first * row + ((size_t)kvh * D + (lane % L) * E) * (F16 ? 2 : 4);
     const char* vbase = reinterpret_cast<const char*>(vc) + (size_t)first * row + ((size_t)kvh * D + (lane % L) * E) * (F16 ? 2 : 4);
     auto head = [&](int r) { return kvh * rep + min(h0 + r, rep - 1); };      // a last group of fewer heads repeats one
-
+    __shared__ float2 s_turn[NEW ? D / 2 : 1];      // cosine and sine of a pair
+    uint4 kw[8];                                    // the warp's first keys
+    auto key_of = [&](int b, int j) { return min(b + j * P + lane / L, n - 1); };
+    auto fetch_keys = [&](int b) {
+#pragma unroll
+        for (int j = 0; j < 8; j++)         // cache rows may have been written by the launch before: not the read-only path
+            kw[j] = __ldcg(reinterpret_cast<const uint4*>(kbase + (size_t)key_of(b, j) * row));
+    };
+    if constexpr (NEW) {
+        // Position, angles and keys do not depend on the products of this token: a forward's first launch waits for everything ahead of it, and no launch
+        // of it but this one writes rows of this layer's cache, the new one.
+        const int pos = *in.pos;
+        if (warp * 8 * P < n) fetch_keys(warp * 8 * P);
+        if (tid % (D) < in.n_dims / 2 && tid < 2 * D) {      // cosines by the first D threads, sines by the next
+            float c, sn;
+            rope_angle(tid % D, pos, in.freq_factors, in.theta_scale, tid < D, c, sn);
+            if (tid < D) s_turn[tid].x = c;
+            else s_turn[tid - D].y = sn;
+        }
+        pdl_wait();
+        __syncthreads();
+        if (pos < 0 || pos >= in.max_seq_len) {
+            if (tid == 0 && rank == 0 && in.err) atomicCAS(in.err, 0, 20);
+        } else if (pos >= first && pos < first + n ? true : rank == 0 && pos >= sees) {
+            if (tid < D) {
+                const int i = tid % (D / 2);
+                const float2 x = *reinterpret_cast<const float2*>((tid < D / 2 ? in.k : in.v) + (size_t)kvh * D + 2 * i);
+                float y0 = x.x, y1 = x.y;
+                if (tid < D / 2 && i < in.n_dims / 2) rope_turn(x.x, x.y, s_turn[i].x, s_turn[i].y, y0, y1);
+                const size_t at = ((size_t)pos * p.kv_heads + kvh) * D + 2 * i;
+                void* cache = const_cast<void*>(tid < D / 2 ? kc : vc);
+                if (F16) {
+                    reinterpret_cast<__half*>(cache)[at] = __float2half_rn(y0);
+                    reinterpret_cast<__half*>(cache)[at + 1] = __float2half_rn(y1);
+                } else {
+                    *reinterpret_cast<float2*>(reinterpret_cast<float*>(cache) + at) = make_float2(y0, y1);
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                if (warp * 8 * P < n && first + key_of(warp * 8 * P, j) == pos) kw[j] = __ldcg(reinterpret_cast<const uint4*>(kbase + (size_t)(pos - first) * row));
+        }
+    }
     // scores
     {
         float qv[R][E];
@@ -127,19 +174,29 @@ __global__ void __launch_bounds__(kSplitThreads) k_gqa_split(GqaShape p, const f
             const float4* src = reinterpret_cast<const float4*>(q + ((size_t)qt * p.heads + head(r)) * D + (lane % L) * E);
 #pragma unroll
             for (int i = 0; i < E / 4; i++) *reinterpret_cast<float4*>(&qv[r][4 * i]) = src[i];
+            if constexpr (NEW) {
+#pragma unroll
+                for (int i = 0; i < E / 2; i++) {
+                    const int pair = (lane % L) * (E / 2) + i;
+                    const float2 turn = s_turn[min(pair, max(in.n_dims / 2 - 1, 0))];
+                    float y0, y1;
+                    rope_turn(qv[r][2 * i], qv[r][2 * i + 1], turn.x, turn.y, y0, y1);
+                    if (pair < in.n_dims / 2) {
+                        qv[r][2 * i] = y0;
+                        qv[r][2 * i + 1] = y1;
+                    }
+                }
+            }
         }
         const int at = first_of_lane<NV, L / 2>(lane);
         const bool writes = NV >= L || (lane % L) % (L / (NV < L ? NV : L)) == 0;
         for (int b = warp * 8 * P; b < n; b += kSplitWarps * 8 * P) {
-            uint4 w[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++)         // cache rows may have been written by the launch before: not the read-only path
-                w[j] = __ldcg(reinterpret_cast<const uint4*>(kbase + (size_t)min(b + j * P + lane / L, n - 1) * row));
+            if (!NEW || b != warp * 8 * P) fetch_keys(b);
             float s[NV];
 #pragma unroll
             for (int j = 0; j < 8; j++) {
                 float f[E];
-                unpack16<F16>(w[j], f);
+                unpack16<F16>(kw[j], f);
 #pragma unroll
                 for (int r = 0; r < R; r++) {
                     float t = 0.0f;
@@ -248,6 +305,49 @@ __global__ void __launch_bounds__(kSplitThreads) k_gqa_split(GqaShape p, const f
     cluster_arrive();
     cluster_wait();
     const int slice = (R * D + ranks - 1) / ranks;
+    if (ranks >= 8 && slice <= 32) {
+        // few results per CTA: a warp takes some of the CTAs, a lane a result (one thread for a result, 16 CTAs: 2.0 us of 17)
+        __shared__ float s_join[3][kSplitWarps][32];
+        const int i = rank * slice + lane;
+        const bool own = lane < slice && i < R * D;
+        float top = kLowest, sum = 0.0f, out = 0.0f;
+        constexpr int kEach = (kMaxCluster + kSplitWarps - 1) / kSplitWarps;
+        float pm[kEach], pl[kEach], po[kEach];
+#pragma unroll
+        for (int c = 0; c < kEach; c++) {
+            const int from = warp + c * kSplitWarps;
+            const bool there = own && from < ranks;
+            pm[c] = there ? load_peer(&s_m[i / D], from) : kLowest;
+            pl[c] = there ? load_peer(&s_l[i / D], from) : 0.0f;
+            po[c] = there ? load_peer(&s_out[i], from) : 0.0f;
+        }
+#pragma unroll
+        for (int c = 0; c < kEach; c++) top = fmaxf(top, pm[c]);
+#pragma unroll
+        for (int c = 0; c < kEach; c++)
+            if (warp + c * kSplitWarps < ranks) {
+                const float f = exp_below(pm[c] - top);
+                sum = fmaf(f, pl[c], sum);
+                out = fmaf(f, po[c], out);
+            }
+        s_join[0][warp][lane] = top;
+        s_join[1][warp][lane] = sum;
+        s_join[2][warp][lane] = out;
+        __syncthreads();
+        if (warp == 0 && own) {
+            const int used = min(ranks, kSplitWarps);
+            float all = kLowest;
+            for (int w = 0; w < used; w++) all = fmaxf(all, s_join[0][w][lane]);
+            sum = out = 0.0f;
+            for (int w = 0; w < used; w++) {
+                const float f = exp_below(s_join[0][w][lane] - all);
+                sum = fmaf(f, s_join[1][w][lane], sum);
+                out = fmaf(f, s_join[2][w][lane], out);
+            }
+            const int r = i / D;
+            if (h0 + r < rep) dst[((size_t)qt * p.heads + head(r)) * D + i % D] = out * (sum == 0.0f ? 0.0f : __fdiv_rn(1.0f, sum));
+        }
+    } else
     for (int i = rank * slice + tid; i < min(R * D, (rank + 1) * slice); i += kSplitThreads) {
         const int r = i / D;
         // all CTAs' loads in flight before the first is used (one after the other: 3 us of 12 with 16 CTAs)
@@ -540,11 +640,11 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_gqa_tile(GqaShape p, const 
 
 // ------------------------------------------------------------------ host side
 
-template <int F16, int D, int R>
-static int launch_split(const GqaShape& p, const float* q, const void* k, const void* v, float* dst, cudaStream_t s)
+template <int F16, int D, int R, bool NEW>
+static int launch_split(const GqaShape& p, const GqaNew& in, const float* q, const void* k, const void* v, float* dst, cudaStream_t s)
 {
     constexpr int kMaxSmem = 96 * 1024;
-    auto kern = k_gqa_split<F16, D, R>;
+    auto kern = k_gqa_split<F16, D, R, NEW>;
     static int ready[64] = {0};       // the largest cluster of the kernel on a device
     int dev = 0;
     cudaGetDevice(&dev);
@@ -582,16 +682,22 @@ static int launch_split(const GqaShape& p, const float* q, const void* k, const 
     const size_t smem = fixed + (size_t)stretch * R * sizeof(float);
     if (smem > (size_t)kMaxSmem) return 1;
     return launch_cluster(kern, dim3((unsigned)(p.kv_heads * groups), (unsigned)ranks, (unsigned)p.n_q), dim3(1, (unsigned)ranks, 1), kSplitThreads, smem, s,
-                          p, q, k, v, dst, stretch);
+                          p, in, q, k, v, dst, stretch);
 }
 
-template <int F16, int D>
-static int launch_split(const GqaShape& p, const float* q, const void* k, const void* v, float* dst, cudaStream_t s)
+template <bool NEW, int F16, int D>
+static int launch_split_of(const GqaShape& p, const GqaNew& in, const float* q, const void* k, const void* v, float* dst, cudaStream_t s)
 {
     const int rep = p.heads / p.kv_heads;
-    if (rep == 1) return launch_split<F16, D, 1>(p, q, k, v, dst, s);
-    if (rep == 2) return launch_split<F16, D, 2>(p, q, k, v, dst, s);
-    return launch_split<F16, D, 4>(p, q, k, v, dst, s);
+    if (rep == 1) return launch_split<F16, D, 1, NEW>(p, in, q, k, v, dst, s);
+    if (rep == 2) return launch_split<F16, D, 2, NEW>(p, in, q, k, v, dst, s);
+    return launch_split<F16, D, 4, NEW>(p, in, q, k, v, dst, s);
+}
+template <bool NEW>
+static int launch_split_of(const GqaShape& p, const GqaNew& in, const float* q, const void* k, const void* v, float* dst, cudaStream_t s)
+{
+    if (p.f16) return p.dim == 64 ? launch_split_of<NEW, 1, 64>(p, in, q, k, v, dst, s) : launch_split_of<NEW, 1, 128>(p, in, q, k, v, dst, s);
+    return p.dim == 64 ? launch_split_of<NEW, 0, 64>(p, in, q, k, v, dst, s) : launch_split_of<NEW, 0, 128>(p, in, q, k, v, dst, s);
 }
 
 template <int D>
@@ -635,8 +741,16 @@ int gqa_attention(const GqaShape& p, const float* q, const void* k, const void* 
     const int kernel = gqa_kernel(p);
     if (kernel == kGeneral) return 1;
     if (kernel == kTile) return p.dim == 64 ? launch_tile<64>(p, q, k, v, dst, s) : launch_tile<128>(p, q, k, v, dst, s);
-    if (p.f16) return p.dim == 64 ? launch_split<1, 64>(p, q, k, v, dst, s) : launch_split<1, 128>(p, q, k, v, dst, s);
-    return p.dim == 64 ? launch_split<0, 64>(p, q, k, v, dst, s) : launch_split<0, 128>(p, q, k, v, dst, s);
+    return launch_split_of<false>(p, GqaNew{}, q, k, v, dst, s);
+}
+
+bool gqa_takes_new(const GqaShape& p, const void* q, const void* k, const void* v, const void* dst)
+{
+    return p.n_q == 1 && !(((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)dst) & 15) && gqa_kernel(p) == kSplit;
+}
+int gqa_attention_new(const GqaShape& p, const GqaNew& in, const float* q, void* k, void* v, float* dst, cudaStream_t s)
+{
+    return launch_split_of<true>(p, in, q, k, v, dst, s);
 }
 
 }  // namespace bpdq

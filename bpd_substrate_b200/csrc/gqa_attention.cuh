@@ -10,6 +10,20 @@ struct GqaShape {
     int kv_offset;      // query t stands at kv_offset + t and sees keys 0 .. kv_offset + t, below n_kv
     int f16;            // caches are fp16 (else fp32)
 };
+// What one query's q/k/v products left: q is turned as it is read, the key turned and stored with the value in cache row *pos (beyond max_seq_len: nothing is
+// stored, code 20 is recorded), by the steps of k_rope_qk_store_kv (llama_forward.cu).
+struct GqaNew {
+    const float *k, *v;         // [kv_heads][dim]
+    const int32_t* pos;
+    const float* freq_factors;  // or null
+    int n_dims, max_seq_len;
+    float theta_scale;
+    int* err;
+};
+// Whether gqa_attention_new takes the shape.
+bool gqa_takes_new(const GqaShape& p, const void* q, const void* k, const void* v, const void* dst);
+// The same as gqa_attention behind those steps; q is not written.
+int gqa_attention_new(const GqaShape& p, const GqaNew& in, const float* q, void* k, void* v, float* dst, cudaStream_t s);
 // Runs the product on one of this file's kernels, or returns 1 if the shape or the pointers are not theirs.
 int gqa_attention(const GqaShape& p, const float* q, const void* k, const void* v, float* dst, cudaStream_t s);
 
