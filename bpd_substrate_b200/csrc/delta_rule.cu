@@ -12,9 +12,9 @@
 //                       the writes solve (1 + A) u = beta (v - (c k) S), so that
 //                         u = U - W S,  o = O + Q S,  S <- c_15 S + sum_j (g_{j+1} .. g_15 k_j) u_j^T
 //                       with (1 + A) W = beta c k,  (1 + A) U = beta v,  Q = c q - P W,  O = P U.  The first kernel works these out for
-//                       all chunks at once (fp32, a thread per key or value column; only products of decays, which cannot
-//                       overflow); the second walks the chunks with the transposed state in fp32 accumulators: a warp for
-//                       the state of 16 value columns and one for its read-out, fed by bulk copies of ready-made fragments.
+//                       all chunks at once (fp32, threads for keys and value columns; only products of decays, which cannot
+//                       overflow); the second walks the chunks with the transposed state in fp32 accumulators: two warps for
+//                       the state of 16 value columns and two for its read-out, fed by bulk copies of ready-made fragments.
 //                       What is fp32 enters mma.sync as the sum of two bf16 numbers, three products.
 #include "delta_rule.cuh"
 #include "cluster_device.cuh"
@@ -307,87 +307,105 @@ __device__ __forceinline__ float transposed_sum(float (&v)[32], int lane)
     return v[0];
 }
 
-// grid (heads, chunks), a thread per key (rounded up to whole warps); tokens t0 .. t1 - 1, those beyond count as zeros that
-// neither decay nor write.
+// grid (heads, chunks); tokens t0 .. t1 - 1, those beyond count as zeros that neither decay nor write.  A thread per key (rounded up to whole warps)
+// and as many again for the value columns.  Bound by latency: a CTA goes through a chain of some thousand instructions.  A and P are sums over
+// the keys: a warp takes whole columns of both, four keys per lane, from k, q and the decays in shared memory, so that a column
+// is added up across lanes once.  (With the sums of its own 32 keys of all columns in every warp, and the value columns after the keys in the
+// same threads: 16 heads of 128 x 128, 64 tokens, with the kernel below 22 us, now 20; 1500 tokens of a decoder with two such layers 1240, now 1227.)
 template <int kThreads, int kBlocks>
 __global__ void __launch_bounds__(kThreads, kBlocks) k_delta_prepare(DeltaRule a, uint8_t* frags, float* updates, int t0, int t1)
 {
-    extern __shared__ __align__(16) uint8_t sf[];     // the chunk's fragments
-    __shared__ float s_part[8][256], s_norm[8][32];
+    extern __shared__ __align__(16) uint8_t sf[];     // k, q, decays [token][key]; then the chunk's fragments
     __shared__ float4 sA[kChunk][4], sP[kChunk][4];
-    __shared__ float s_beta[kChunk];
+    __shared__ float s_norm[2 * kChunk], s_beta[kChunk];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
-    const int h = blockIdx.x, gr = h / (a.heads / a.groups), first = t0 + blockIdx.y * kChunk;
-    const int D = a.key_pad, V = a.value_pad, n = tid;
+    const int h = blockIdx.x, gr = h / (a.heads / a.groups), first = t0 + blockIdx.y * kChunk, left = t1 - first;
+    const int D = a.key_pad, V = a.value_pad, n = tid, values = blockDim.x >> 1;      // first thread of the value columns
     const bool key = n < D;
+    const bf16* pv = reinterpret_cast<const bf16*>(a.v) + (size_t)first * a.ld + (size_t)h * V;
     pdl_launch_dependents();
     pdl_wait();
-    float k[kChunk], q[kChunk], g[kChunk];
-    {
+    // the first half: k, q and decays of a key; the second: a value column
+    float x[kChunk];
+    if (tid < values) {
+        float k[kChunk], q[kChunk], g[kChunk];
         const bf16* pk = reinterpret_cast<const bf16*>(a.k) + (size_t)first * a.ld + gr * D + n;
         const bf16* pq = reinterpret_cast<const bf16*>(a.q) + (size_t)first * a.ld + gr * D + n;
         const float* pd = a.log_decay + ((size_t)first * a.heads + h) * D + n;
-        const int left = key ? t1 - first : 0, step = a.heads * D;
+        const int rows = key ? left : 0, step = a.heads * D;
 #pragma unroll
         for (int i = 0; i < kChunk; i++) {
-            k[i] = i < left ? act_load(pk + i * a.ld) : 0.0f;
-            q[i] = i < left ? act_load(pq + i * a.ld) : 0.0f;
-            g[i] = i < left ? pd[i * step] : 0.0f;
+            k[i] = i < rows ? act_load(pk + i * a.ld) : 0.0f;
+            q[i] = i < rows ? act_load(pq + i * a.ld) : 0.0f;
+            g[i] = i < rows ? pd[i * step] : 0.0f;
+        }
+        if (tid < kChunk) s_beta[tid] = first + tid < t1 ? a.beta[(size_t)(first + tid) * a.heads + h] : 0.0f;
+        float* to = reinterpret_cast<float*>(sf) + n;
+#pragma unroll
+        for (int i = 0; i < kChunk; i++)
+            if (key) {
+                to[i * D] = k[i];
+                to[(kChunk + i) * D] = q[i];
+                to[(2 * kChunk + i) * D] = expf(g[i]);
+            }
+    } else {
+        const int p = tid - values;
+#pragma unroll
+        for (int i = 0; i < kChunk; i++) x[i] = i < left && p < V ? act_load(pv + i * a.ld + p) : 0.0f;
+    }
+    __syncthreads();
+    // column m of P and A at distance d from the diagonal (A's diagonal: the key's square length); a long column and a short one to each warp
+    for (int pass = 0; pass * warps < kChunk; pass++) {
+        const int m = pass * warps + (pass & 1 ? warps - 1 - warp : warp);
+        if (m >= kChunk) continue;
+        float v[32], qq = 0.0f;
+#pragma unroll
+        for (int d = 0; d < 32; d++) v[d] = 0.0f;
+        for (int n4 = 4 * lane; n4 < D; n4 += 128) {
+            const float* col = reinterpret_cast<const float*>(sf) + m * D + n4;
+            float4 r = make_float4(0, 0, 0, 0);
+#pragma unroll
+            for (int d = 0; d < kChunk; d++) {
+                if (m + d >= kChunk) break;
+                const float4 kk = *reinterpret_cast<const float4*>(col + d * D), qv = *reinterpret_cast<const float4*>(col + (kChunk + d) * D);
+                if (d == 0) {
+                    r = kk;
+                    qq = fmaf(qv.x, qv.x, qq); qq = fmaf(qv.y, qv.y, qq); qq = fmaf(qv.z, qv.z, qq); qq = fmaf(qv.w, qv.w, qq);
+                } else {
+                    const float4 f = *reinterpret_cast<const float4*>(col + (2 * kChunk + d) * D);
+                    r = make_float4(r.x * f.x, r.y * f.y, r.z * f.z, r.w * f.w);
+                }
+                v[d] = fmaf(qv.x, r.x, v[d]); v[d] = fmaf(qv.y, r.y, v[d]); v[d] = fmaf(qv.z, r.z, v[d]); v[d] = fmaf(qv.w, r.w, v[d]);
+                float& w = v[kChunk + d];
+                w = fmaf(kk.x, r.x, w); w = fmaf(kk.y, r.y, w); w = fmaf(kk.z, r.z, w); w = fmaf(kk.w, r.w, w);
+            }
+        }
+        const float sum = transposed_sum(v, lane);
+        qq = warp_sum(qq);
+        const int i = m + (lane & (kChunk - 1));
+        if (i < kChunk) {
+            if (lane < kChunk) reinterpret_cast<float*>(sP)[i * kChunk + m] = sum;
+            else if (i > m) reinterpret_cast<float*>(sA)[i * kChunk + m] = sum;
+            else { s_norm[m] = sum; s_norm[kChunk + m] = qq; }
         }
     }
-    if (tid < kChunk) s_beta[tid] = first + tid < t1 ? a.beta[(size_t)(first + tid) * a.heads + h] : 0.0f;
-    float v[32];
-#pragma unroll
-    for (int i = 0; i < kChunk; i++) {
-        v[i] = k[i] * k[i];
-        v[kChunk + i] = q[i] * q[i];
-        g[i] = expf(g[i]);
-    }
-    s_norm[warp][lane] = transposed_sum(v, lane);
     __syncthreads();
-    {
-        float sum = 0.0f;
-        for (int w = 0; w < warps; w++) sum += s_norm[w][lane];
-        const float f = (lane < kChunk ? 1.0f : a.q_scale) / sqrtf(sum + a.unit_eps);
+    const float unit = (lane < kChunk ? 1.0f : a.q_scale) / sqrtf(s_norm[lane] + a.unit_eps);      // a lane per token: of its k, of its q
+    for (int c = tid; c < kChunk * kChunk; c += blockDim.x) {
+        const int i = c >> 4, j = c & (kChunk - 1);
+        const float ki = __shfl_sync(0xFFFFFFFFu, unit, i), kj = __shfl_sync(0xFFFFFFFFu, unit, j), qi = __shfl_sync(0xFFFFFFFFu, unit, kChunk + i);
+        if (j < i) reinterpret_cast<float*>(sA)[c] *= s_beta[i] * ki * kj;
+        if (j <= i) reinterpret_cast<float*>(sP)[c] *= qi * kj;
+    }
+    float k[kChunk], q[kChunk], g[kChunk];
+    if (tid < values) {
+        const float* from = reinterpret_cast<const float*>(sf) + (key ? n : 0);
 #pragma unroll
         for (int i = 0; i < kChunk; i++) {
-            k[i] *= __shfl_sync(0xFFFFFFFFu, f, i);
-            q[i] *= __shfl_sync(0xFFFFFFFFu, f, kChunk + i);
+            k[i] = from[i * D] * __shfl_sync(0xFFFFFFFFu, unit, i);
+            q[i] = from[(kChunk + i) * D] * __shfl_sync(0xFFFFFFFFu, unit, kChunk + i);
+            g[i] = from[(2 * kChunk + i) * D];
         }
-    }
-    // columns m and 15 - m of P and A together are 32 sums
-#pragma unroll
-    for (int m = 0; m < 8; m++) {
-        float r = k[m];
-#pragma unroll
-        for (int i = m; i < kChunk; i++) {
-            if (i > m) {
-                r *= g[i];
-                v[16 - m + i - m - 1] = k[i] * r;
-            }
-            v[i - m] = q[i] * r;
-        }
-        r = k[15 - m];
-#pragma unroll
-        for (int i = 15 - m; i < kChunk; i++) {
-            if (i > 15 - m) {
-                r *= g[i];
-                v[32 - m + i - (16 - m)] = k[i] * r;
-            }
-            v[31 - 2 * m + i - (15 - m)] = q[i] * r;
-        }
-        s_part[warp][32 * m + lane] = transposed_sum(v, lane);
-    }
-    __syncthreads();
-    for (int x = tid; x < 256; x += blockDim.x) {
-        float sum = 0.0f;
-        for (int w = 0; w < warps; w++) sum += s_part[w][x];
-        const int m = x >> 5, l = x & 31;
-        float *A = reinterpret_cast<float*>(sA), *P = reinterpret_cast<float*>(sP);
-        if (l < 16 - m) P[(m + l) * kChunk + m] = sum;
-        else if (l < 31 - 2 * m) { const int i = 2 * m + 1 + l - 16; A[i * kChunk + m] = sum * s_beta[i]; }
-        else if (l < 32 - m) P[(15 - m + l - (31 - 2 * m)) * kChunk + 15 - m] = sum;
-        else { const int i = 16 - m + l - (32 - m); A[i * kChunk + 15 - m] = sum * s_beta[i]; }
     }
     __syncthreads();
     // the first n entries of a row
@@ -396,8 +414,8 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_delta_prepare(DeltaRule a
         for (int j = 0; j < 4; j++)
             if (4 * j < n) *reinterpret_cast<float4*>(r + 4 * j) = m[i][j];
     };
-    const size_t unit = (size_t)blockIdx.y * a.heads + h;
-    if (key) {
+    const size_t cell = (size_t)blockIdx.y * a.heads + h;
+    if (key && tid < values) {
         uint32_t* fw = reinterpret_cast<uint32_t*>(sf);
         uint32_t* fq = fw + 16 * D;
         uint32_t* fk = fq + 16 * D;
@@ -421,17 +439,21 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_delta_prepare(DeltaRule a
 #pragma unroll
         for (int i = 0; i < kChunk; i++) {
             c *= g[i];
-            float x = s_beta[i] * k[i] * c, y = q[i] * c;
+            w[i] = s_beta[i] * k[i] * c;
+            z[i] = q[i] * c;
+        }
+#pragma unroll
+        for (int i = 0; i < kChunk; i++) {
+            asm volatile("" ::: "memory");      // (rows read far ahead would be kept in local memory)
             alignas(16) float ar[kChunk], pr[kChunk];
             load_row(sA, i, i, ar);
             load_row(sP, i, i + 1, pr);
 #pragma unroll
             for (int j = 0; j < i; j++) {
-                x = fmaf(-ar[j], w[j], x);
-                y = fmaf(-pr[j], w[j], y);
+                w[i] = fmaf(-ar[j], w[j], w[i]);
+                z[i] = fmaf(-pr[j], w[j], z[i]);
             }
-            w[i] = x;
-            z[i] = fmaf(-pr[i], x, y);
+            z[i] = fmaf(-pr[i], w[i], z[i]);
         }
         // keys n and n + 1 share a register: the even thread writes tokens 0 .. 7, the odd one 8 .. 15
         const unsigned live = D - (n & ~31) >= 32 ? 0xFFFFFFFFu : 0xFFFFu;
@@ -450,39 +472,41 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_delta_prepare(DeltaRule a
             fq[at + 16 * i] = hi;
             fq[at + 16 * i + 2] = lo;
         }
-    }
-    float* up = updates + unit * update_floats(V);
-    for (int p = tid; p < V; p += blockDim.x) {
-        const bf16* pv = reinterpret_cast<const bf16*>(a.v) + (size_t)first * a.ld + (size_t)h * V + p;
-        const int left = t1 - first;
-        float x[kChunk], u[kChunk], o[kChunk];
+    } else if (tid >= values) {
+        float* up = updates + cell * update_floats(V);
+        for (int p = tid - values; p < V; p += values) {
+            float u[kChunk], o[kChunk];
+            if (p != tid - values) {
 #pragma unroll
-        for (int i = 0; i < kChunk; i++) x[i] = i < left ? act_load(pv + i * a.ld) : 0.0f;
-#pragma unroll
-        for (int i = 0; i < kChunk; i++) {
-            float y = s_beta[i] * x[i], z = 0.0f;
-            alignas(16) float ar[kChunk], pr[kChunk];
-            load_row(sA, i, i, ar);
-            load_row(sP, i, i + 1, pr);
-#pragma unroll
-            for (int j = 0; j < i; j++) {
-                y = fmaf(-ar[j], u[j], y);
-                z = fmaf(pr[j], u[j], z);
+                for (int i = 0; i < kChunk; i++) x[i] = i < left ? act_load(pv + i * a.ld + p) : 0.0f;
             }
-            u[i] = y;
-            o[i] = fmaf(pr[i], y, z);
+#pragma unroll
+            for (int i = 0; i < kChunk; i++) {
+                asm volatile("" ::: "memory");      // (rows read far ahead would be kept in local memory)
+                float y = s_beta[i] * x[i], z = 0.0f;
+                alignas(16) float ar[kChunk], pr[kChunk];
+                load_row(sA, i, i, ar);
+                load_row(sP, i, i + 1, pr);
+#pragma unroll
+                for (int j = 0; j < i; j++) {
+                    y = fmaf(-ar[j], u[j], y);
+                    z = fmaf(pr[j], u[j], z);
+                }
+                u[i] = y;
+                o[i] = fmaf(pr[i], y, z);
+            }
+            float* dst = up + (size_t)(p >> 4) * 512 + (p & 7) * 32 + ((p >> 3) & 1) * 2;
+#pragma unroll
+            for (int t = 0; t < 4; t++)
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    *reinterpret_cast<float2*>(dst + t * 8 + e * 4) = make_float2(u[8 * e + 2 * t], u[8 * e + 2 * t + 1]);
+                    *reinterpret_cast<float2*>(dst + 256 + t * 8 + e * 4) = make_float2(o[8 * e + 2 * t], o[8 * e + 2 * t + 1]);
+                }
         }
-        float* dst = up + (size_t)(p >> 4) * 512 + (p & 7) * 32 + ((p >> 3) & 1) * 2;
-#pragma unroll
-        for (int t = 0; t < 4; t++)
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                *reinterpret_cast<float2*>(dst + t * 8 + e * 4) = make_float2(u[8 * e + 2 * t], u[8 * e + 2 * t + 1]);
-                *reinterpret_cast<float2*>(dst + 256 + t * 8 + e * 4) = make_float2(o[8 * e + 2 * t], o[8 * e + 2 * t + 1]);
-            }
     }
     __syncthreads();
-    uint4* dst = reinterpret_cast<uint4*>(frags + unit * fragment_bytes(D));
+    uint4* dst = reinterpret_cast<uint4*>(frags + cell * fragment_bytes(D));
     for (int i = tid; i < (int)(fragment_bytes(D) / 16); i += blockDim.x) dst[i] = reinterpret_cast<const uint4*>(sf)[i];
 }
 
@@ -492,36 +516,48 @@ __device__ __forceinline__ void store_shared(uint32_t at, const uint32_t (&v)[4]
     asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]));
 }
 
-template <int NMAX>
+// A whole warp's wait: `ready` is what a look ahead of time said.  After a wait that ran out (`alive` is false, the code is recorded) none waits.
+__device__ __forceinline__ void warp_wait(uint64_t* bar, uint32_t parity, bool ready, bool& alive, int* err, int code)
+{
+    if (__all_sync(0xFFFFFFFFu, ready)) return;
+    if (alive) alive = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(bar, parity, err, code));
+}
+
+template <int NMAX, int kBlocks>
 struct DeltaChunks {
-    static constexpr int kStages = NMAX == 256 ? 3 : 4;
+    static constexpr int kStages = NMAX == 256 ? (kBlocks == 1 ? 3 : 2) : 4;
     static constexpr size_t kState = (size_t)NMAX / 16 * 1024;      // fragments of 16 columns of the state, high and low parts
-    static size_t smem(int key_pad) { return kStages * fragment_bytes(key_pad) + 4 * kState; }
+    static size_t smem(int key_pad) { return kStages * (fragment_bytes(key_pad) + (size_t)kBlocks * kState); }
 };
 
-// grid (heads, value columns / 32): warps 0, 1 hold the state of 16 value columns each, warps 2, 3 read it out, warp 4 feeds.  kExact: the keys
-// are NMAX, so that no step of the products hangs on a branch.
-template <int NMAX, bool kExact>
-__global__ void __launch_bounds__(160, 1) k_delta_chunks(DeltaRule a, const uint8_t* frags, const float* updates, int t0, int t1, int chunks, int* err)
+// grid (heads, value columns / (16 kBlocks)).  Of each block of 16 value columns two warps hold the state, half of the keys each, and two read it
+// out, eight tokens each; the last warp feeds.  The chunks are one serial chain: 96 products of 10 cycles with and into a state of 128 keys, and what
+// lies between them.  So the keys are on two warps, which exchange their parts of u, and each chunk has one wait of
+// the state's warps on a barrier in memory, looked at ahead of time, and one meeting.  With a warp per block and three such waits (130 cycles each, even
+// of barriers long complete) a chunk took 0.93 us, now 0.6 (16 heads of 128 x 128).
+// kExact: the keys are NMAX, so that no step of the products hangs on a branch.
+template <int NMAX, bool kExact, int kBlocks>
+__global__ void __launch_bounds__(32 * (4 * kBlocks + 1), 1) k_delta_chunks(DeltaRule a, const uint8_t* frags, const float* updates, int t0, int t1, int chunks, int* err)
 {
-    using S = DeltaChunks<NMAX>;
-    constexpr int NT = NMAX / 8, KS = NMAX / 16;
+    using S = DeltaChunks<NMAX, kBlocks>;
+    constexpr int KS = NMAX / 16, KH = KS / 2, NT = NMAX / 16;      // K steps of a read-out and of a half, the half's tiles of 8 keys
     extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ uint64_t full[S::kStages], empty[S::kStages], state_full[2][2], state_empty[2][2];
+    __shared__ uint64_t full[S::kStages], empty[S::kStages], written[kBlocks][S::kStages];
+    __shared__ float4 s_part[kBlocks][2][2][2][32];                 // [block][buffer][half][..]: a half's part of u
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g4 = lane >> 2, t4 = lane & 3;
     const int h = blockIdx.x, D = kExact ? NMAX : a.key_pad, V = a.value_pad, ks_n = D / 16;
-    const int blocks = V / 16 - 2 * (int)blockIdx.y < 2 ? V / 16 - 2 * (int)blockIdx.y : 2;
+    const int left = V / 16 - kBlocks * (int)blockIdx.y, blocks = left < kBlocks ? left : kBlocks;
     const uint32_t bytes = (uint32_t)fragment_bytes(D);
     uint8_t* s_state = smem + S::kStages * (size_t)bytes;
     if (tid == 0) {
-        for (int i = 0; i < S::kStages; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], 2 * blocks); }
-        for (int i = 0; i < 4; i++) { mbar_init(&state_full[i >> 1][i & 1], 1); mbar_init(&state_empty[i >> 1][i & 1], 1); }
+        for (int i = 0; i < S::kStages; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], 4 * blocks); }
+        for (int i = 0; i < kBlocks * S::kStages; i++) mbar_init(&written[0][0] + i, 1);
         mbar_init_fence();
     }
     __syncthreads();
     pdl_launch_dependents();
     pdl_wait();
-    if (warp == 4) {
+    if (warp == 4 * kBlocks) {
         if (lane == 0) {
             int c = 0;
             for (; c < chunks; c++) {
@@ -535,47 +571,55 @@ __global__ void __launch_bounds__(160, 1) k_delta_chunks(DeltaRule a, const uint
         }
         return;
     }
-    const int pair = warp & 1, block = 2 * blockIdx.y + pair;
+    const bool reads = warp >= 2 * kBlocks;
+    const int pair = (warp >> 1) % kBlocks, half = warp & 1, block = kBlocks * blockIdx.y + pair;
     if (pair >= blocks) return;
-    uint8_t* mine = s_state + (size_t)pair * 2 * S::kState + lane * 16;
-    const float* up = updates + (size_t)h * update_floats(V) + (size_t)block * 512 + (warp >> 1) * 256 + lane * 8;
+    // a stage's state lies beside its fragments: whoever sees the next ones there knows that all warps have left both
+    uint8_t* mine = s_state + (size_t)pair * S::kStages * S::kState + lane * 16;
+    const float* up = updates + (size_t)h * update_floats(V) + (size_t)block * 512 + reads * 256 + lane * 8;
     const size_t next_up = (size_t)a.heads * update_floats(V);
-    float4 u0 = *reinterpret_cast<const float4*>(up), u1 = *reinterpret_cast<const float4*>(up + 4);
-    if (warp < 2) {
-        // ---------------- the state, transposed: rows are value columns, columns are keys
+    bool alive = true;
+    int s = 0;
+    uint32_t phase = 0;
+    if (!reads) {
+        // ---------------- the state, transposed: rows are value columns, columns are this half's keys
+        const int k0 = half * KH, n0 = half * (NMAX / 2);
         float st[NT][4];
         float* gs = a.state + (size_t)h * D * V + 16 * block + g4;
 #pragma unroll
         for (int j = 0; j < NT; j++)
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                const int n = 8 * j + 2 * t4 + (e & 1);
+                const int n = n0 + 8 * j + 2 * t4 + (e & 1);
                 st[j][e] = n < D ? gs[(size_t)n * V + 8 * (e >> 1)] : 0.0f;
             }
+        const float4 none = make_float4(0, 0, 0, 0);
+        float4 u0 = half ? none : *reinterpret_cast<const float4*>(up), u1 = half ? none : *reinterpret_cast<const float4*>(up + 4);
+        bool ready = false;
         for (int c = 0; c < chunks; c++) {
-            const int s = c % S::kStages, b = c & 1;
-            if (!mbar_wait_bounded(&full[s], (uint32_t)(c / S::kStages) & 1u, err, 62)) break;
-            if (c >= 2 && !mbar_wait_bounded(&state_empty[pair][b], (uint32_t)(c / 2 - 1) & 1u, err, 63)) break;
+            const int b = c & 1;
+            warp_wait(&full[s], phase, ready, alive, err, 62);
             const uint8_t* f = smem + s * (size_t)bytes;
-            const uint32_t to = smem_addr(mine + b * S::kState);
+            const uint32_t to = smem_addr(mine + s * S::kState);
             float x[2][4] = {{u0.x, u0.y, u0.z, u0.w}, {u1.x, u1.y, u1.z, u1.w}}, y[2][4] = {}, z[2][4] = {};
-            if (c + 1 < chunks) {
+            if (!half && c + 1 < chunks) {
                 up += next_up;
                 u0 = *reinterpret_cast<const float4*>(up);
                 u1 = *reinterpret_cast<const float4*>(up + 4);
             }
             const uint4* fw = reinterpret_cast<const uint4*>(f) + lane;
-            uint4 w0 = fw[0], w1 = fw[32];
+            const float* decay = reinterpret_cast<const float*>(f + (size_t)192 * D) + n0 + 2 * t4;
 #pragma unroll
-            for (int ks = 0; ks < KS; ks++) {
+            for (int i = 0; i < KH; i++) {
+                const int ks = k0 + i;
                 if (ks >= ks_n) break;
-                uint4 n0 = w0, n1 = w1;
-                if (ks + 1 < KS && ks + 1 < ks_n) { n0 = fw[(2 * ks + 2) * 32]; n1 = fw[(2 * ks + 3) * 32]; }
+                const uint4 w0 = fw[2 * ks * 32], w1 = fw[(2 * ks + 1) * 32];
+                const float2 d0 = *reinterpret_cast<const float2*>(decay + 16 * i), d1 = *reinterpret_cast<const float2*>(decay + 16 * i + 8);
                 uint32_t ah[4], al[4];
-                split_bf16(st[2 * ks][0], st[2 * ks][1], ah[0], al[0]);
-                split_bf16(st[2 * ks][2], st[2 * ks][3], ah[1], al[1]);
-                split_bf16(st[2 * ks + 1][0], st[2 * ks + 1][1], ah[2], al[2]);
-                split_bf16(st[2 * ks + 1][2], st[2 * ks + 1][3], ah[3], al[3]);
+                split_bf16(st[2 * i][0], st[2 * i][1], ah[0], al[0]);
+                split_bf16(st[2 * i][2], st[2 * i][3], ah[1], al[1]);
+                split_bf16(st[2 * i + 1][0], st[2 * i + 1][1], ah[2], al[2]);
+                split_bf16(st[2 * i + 1][2], st[2 * i + 1][3], ah[3], al[3]);
                 store_shared(to + ks * 1024, ah);
                 store_shared(to + ks * 1024 + 512, al);
                 mma_bf16(x[0], ah, w0.x, w0.y);
@@ -584,119 +628,120 @@ __global__ void __launch_bounds__(160, 1) k_delta_chunks(DeltaRule a, const uint
                 mma_bf16(y[1], ah, w1.z, w1.w);
                 mma_bf16(z[0], al, w0.x, w0.y);
                 mma_bf16(z[1], al, w1.x, w1.y);
-                w0 = n0;
-                w1 = n1;
+                st[2 * i][0] *= d0.x; st[2 * i][1] *= d0.y; st[2 * i][2] *= d0.x; st[2 * i][3] *= d0.y;
+                st[2 * i + 1][0] *= d1.x; st[2 * i + 1][1] *= d1.y; st[2 * i + 1][2] *= d1.x; st[2 * i + 1][3] *= d1.y;
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&state_full[pair][b]);
-            const uint8_t* fk = f + (size_t)128 * D;
-            const float* decay = reinterpret_cast<const float*>(f + (size_t)192 * D);
+            // u: this half's part to the other half, and its part from there
 #pragma unroll
-            for (int j = 0; j < NT; j++) {
-                if (8 * j >= D) break;
-                const float2 d = *reinterpret_cast<const float2*>(decay + 8 * j + 2 * t4);
-                st[j][0] *= d.x; st[j][1] *= d.y; st[j][2] *= d.x; st[j][3] *= d.y;
+            for (int e = 0; e < 2; e++) {
+#pragma unroll
+                for (int r = 0; r < 4; r++) x[e][r] += y[e][r] + z[e][r];
+                s_part[pair][b][half][e][lane] = make_float4(x[e][0], x[e][1], x[e][2], x[e][3]);
             }
+            named_bar_sync(1 + pair, 64);
+            if (half == 0 && lane == 0) mbar_arrive(&written[pair][s]);
+            const uint8_t* fk = f + (size_t)128 * D + (size_t)n0 * 64;
             uint32_t uh[4], ul[4];
 #pragma unroll
             for (int e = 0; e < 2; e++) {
-                split_bf16(x[e][0] + (y[e][0] + z[e][0]), x[e][1] + (y[e][1] + z[e][1]), uh[2 * e], ul[2 * e]);
-                split_bf16(x[e][2] + (y[e][2] + z[e][2]), x[e][3] + (y[e][3] + z[e][3]), uh[2 * e + 1], ul[2 * e + 1]);
+                const float4 v = s_part[pair][b][half ^ 1][e][lane];
+                split_bf16(x[e][0] + v.x, x[e][1] + v.y, uh[2 * e], ul[2 * e]);
+                split_bf16(x[e][2] + v.z, x[e][3] + v.w, uh[2 * e + 1], ul[2 * e + 1]);
             }
+            uint64_t* gone = &empty[s];
+            if (++s == S::kStages) { s = 0; phase ^= 1; }
+            ready = mbar_test(&full[s], phase);
+            constexpr int kAtOnce = NT < 8 ? NT : 8;
 #pragma unroll
-            for (int j = 0; j < NT; j += 8) {
-                if (8 * j >= D) break;
-                uint4 kf[8];
+            for (int j = 0; j < NT; j += kAtOnce) {
+                if (n0 + 8 * j >= D) break;
+                uint4 kf[kAtOnce];
 #pragma unroll
-                for (int i = 0; i < 8; i++) kf[i] = 8 * (j + i) < D ? *reinterpret_cast<const uint4*>(fk + ((j + i) * 32 + lane) * 16) : make_uint4(0, 0, 0, 0);
+                for (int i = 0; i < kAtOnce; i++)
+                    kf[i] = n0 + 8 * (j + i) < D ? *reinterpret_cast<const uint4*>(fk + ((j + i) * 32 + lane) * 16) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-                for (int i = 0; i < 8; i++) mma_bf16(st[j + i], uh, kf[i].x, kf[i].y);
+                for (int i = 0; i < kAtOnce; i++) mma_bf16(st[j + i], uh, kf[i].x, kf[i].y);
 #pragma unroll
-                for (int i = 0; i < 8; i++) mma_bf16(st[j + i], uh, kf[i].z, kf[i].w);
+                for (int i = 0; i < kAtOnce; i++) mma_bf16(st[j + i], uh, kf[i].z, kf[i].w);
 #pragma unroll
-                for (int i = 0; i < 8; i++) mma_bf16(st[j + i], ul, kf[i].x, kf[i].y);
+                for (int i = 0; i < kAtOnce; i++) mma_bf16(st[j + i], ul, kf[i].x, kf[i].y);
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[s]);
+            if (lane == 0) mbar_arrive(gone);
         }
 #pragma unroll
         for (int j = 0; j < NT; j++)
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                const int n = 8 * j + 2 * t4 + (e & 1);
+                const int n = n0 + 8 * j + 2 * t4 + (e & 1);
                 if (n < D) gs[(size_t)n * V + 8 * (e >> 1)] = st[j][e];
             }
     } else {
-        // ---------------- the read-out
+        // ---------------- the read-out of tokens 8 half .. 8 half + 7
         bf16* out = reinterpret_cast<bf16*>(a.o) + (size_t)h * V + 16 * block + (g4 & ~1);
+        up += 4 * half;
+        float4 u = *reinterpret_cast<const float4*>(up);
         for (int c = 0; c < chunks; c++) {
-            const int s = c % S::kStages, b = c & 1;
-            if (!mbar_wait_bounded(&full[s], (uint32_t)(c / S::kStages) & 1u, err, 64)) break;
-            if (!mbar_wait_bounded(&state_full[pair][b], (uint32_t)(c / 2) & 1u, err, 65)) break;
+            warp_wait(&written[pair][s], phase, false, alive, err, 65);      // (and so the fragments are there)
             const uint8_t* f = smem + s * (size_t)bytes + (size_t)64 * D;
-            float x[2][4] = {{u0.x, u0.y, u0.z, u0.w}, {u1.x, u1.y, u1.z, u1.w}}, y[2][4] = {}, z[2][4] = {};
-            if (c + 1 < chunks) {
-                up += next_up;
-                u0 = *reinterpret_cast<const float4*>(up);
-                u1 = *reinterpret_cast<const float4*>(up + 4);
-            }
-            const uint4* fq = reinterpret_cast<const uint4*>(f) + lane;
-            const uint4* from = reinterpret_cast<const uint4*>(mine + b * S::kState);
-            uint4 hi = from[0], lo = from[32], w0 = fq[0], w1 = fq[32];
+            float x[4] = {u.x, u.y, u.z, u.w}, y[4] = {}, z[4] = {};
+            if (c + 1 < chunks) u = *reinterpret_cast<const float4*>(up += next_up);
+            const uint4* fq = reinterpret_cast<const uint4*>(f) + 32 * half + lane;
+            const uint4* from = reinterpret_cast<const uint4*>(mine + s * S::kState);
 #pragma unroll
             for (int ks = 0; ks < KS; ks++) {
                 if (ks >= ks_n) break;
+                const uint4 hi = from[2 * ks * 32], lo = from[(2 * ks + 1) * 32], w = fq[2 * ks * 32];
                 const uint32_t ah[4] = {hi.x, hi.y, hi.z, hi.w}, al[4] = {lo.x, lo.y, lo.z, lo.w};
-                uint4 n0 = w0, n1 = w1;
-                if (ks + 1 < KS && ks + 1 < ks_n) {
-                    n0 = fq[(2 * ks + 2) * 32];
-                    n1 = fq[(2 * ks + 3) * 32];
-                    hi = from[(2 * ks + 2) * 32];
-                    lo = from[(2 * ks + 3) * 32];
-                }
-                mma_bf16(x[0], ah, w0.x, w0.y);
-                mma_bf16(x[1], ah, w1.x, w1.y);
-                mma_bf16(y[0], ah, w0.z, w0.w);
-                mma_bf16(y[1], ah, w1.z, w1.w);
-                mma_bf16(z[0], al, w0.x, w0.y);
-                mma_bf16(z[1], al, w1.x, w1.y);
-                w0 = n0;
-                w1 = n1;
+                mma_bf16(x, ah, w.x, w.y);
+                mma_bf16(y, ah, w.z, w.w);
+                mma_bf16(z, al, w.x, w.y);
             }
             __syncwarp();
-            if (lane == 0) { mbar_arrive(&state_empty[pair][b]); mbar_arrive(&empty[s]); }
+            if (lane == 0) mbar_arrive(&empty[s]);
+            if (++s == S::kStages) { s = 0; phase ^= 1; }
             // two neighbouring columns per store: lanes of even columns finish even tokens, those of odd ones odd tokens
             const bool odd = g4 & 1;
 #pragma unroll
-            for (int e = 0; e < 2; e++)
-#pragma unroll
-                for (int r = 0; r < 4; r += 2) {
-                    const float v0 = x[e][r] + (y[e][r] + z[e][r]), v1 = x[e][r + 1] + (y[e][r + 1] + z[e][r + 1]);
-                    const float other = __shfl_xor_sync(0xFFFFFFFFu, odd ? v0 : v1, 4);
-                    const int t = t0 + kChunk * c + 8 * e + 2 * t4 + odd;
-                    if (t < t1)
-                        *reinterpret_cast<uint32_t*>(out + (size_t)t * a.heads * V + 4 * r) = odd ? pack_bf16(other, v1) : pack_bf16(v0, other);
-                }
+            for (int r = 0; r < 4; r += 2) {
+                const float v0 = x[r] + (y[r] + z[r]), v1 = x[r + 1] + (y[r + 1] + z[r + 1]);
+                const float other = __shfl_xor_sync(0xFFFFFFFFu, odd ? v0 : v1, 4);
+                const int t = t0 + kChunk * c + 8 * half + 2 * t4 + odd;
+                if (t < t1)
+                    *reinterpret_cast<uint32_t*>(out + (size_t)t * a.heads * V + 4 * r) = odd ? pack_bf16(other, v1) : pack_bf16(v0, other);
+            }
         }
     }
+}
+
+template <int NMAX, bool kExact, int kBlocks>
+static int launch_walk(const DeltaRule& a, const uint8_t* frags, const float* updates, int t0, int t1, int chunks, cudaStream_t s)
+{
+    int rc = allow_smem<k_delta_chunks<NMAX, kExact, kBlocks>>((int)DeltaChunks<NMAX, kBlocks>::smem(NMAX));
+    if (rc) return rc;
+    return launch_ordered(k_delta_chunks<NMAX, kExact, kBlocks>, dim3(a.heads, (a.value_pad / 16 + kBlocks - 1) / kBlocks), 32 * (4 * kBlocks + 1),
+                          DeltaChunks<NMAX, kBlocks>::smem(a.key_pad), s, a, frags, updates, t0, t1, chunks, device_error_flag());
 }
 
 template <int NMAX, bool kExact>
 static int launch_chunks(const DeltaRule& a, int T, cudaStream_t s)
 {
-    int rc = allow_smem<k_delta_chunks<NMAX, kExact>>((int)DeltaChunks<NMAX>::smem(NMAX));
-    if (rc) return rc;
-    constexpr auto prepare = k_delta_prepare<NMAX == 256 ? 256 : 128, NMAX == 256 ? 1 : 3>;
+    int rc;
+    constexpr auto prepare = k_delta_prepare<NMAX == 256 ? 512 : 256, NMAX == 256 ? 1 : 2>;
     if ((rc = allow_smem<prepare>((int)fragment_bytes(256)))) return rc;
     for (int t0 = 0; t0 < T; t0 += kSegmentChunks * kChunk) {
         const int t1 = T - t0 < kSegmentChunks * kChunk ? T : t0 + kSegmentChunks * kChunk, chunks = (t1 - t0 + kChunk - 1) / kChunk;
         uint8_t* frags = (uint8_t*)a.scratch;
         float* updates = (float*)(frags + (size_t)chunks * a.heads * fragment_bytes(a.key_pad));
-        if ((rc = launch_ordered(prepare, dim3(a.heads, chunks), (a.key_pad + 31) / 32 * 32, fragment_bytes(a.key_pad), s, a, frags, updates, t0, t1)))
+        if ((rc = launch_ordered(prepare, dim3(a.heads, chunks), (a.key_pad + 31) / 32 * 64, fragment_bytes(a.key_pad), s, a, frags, updates, t0, t1)))
             return rc;
-        if ((rc = launch_ordered(k_delta_chunks<NMAX, kExact>, dim3(a.heads, (a.value_pad + 31) / 32), 160, DeltaChunks<NMAX>::smem(a.key_pad), s, a,
-                                 (const uint8_t*)frags, (const float*)updates, t0, t1, chunks, device_error_flag())))
-            return rc;
+        // One block of value columns per CTA while every CTA has an SM of its own: 16 heads of 128 x 128, 700 tokens 62 us, with two 66; 8 of
+        // 256 x 256, 95 and 128.  With more CTAs than SMs the fragments would only be read twice as often, and with few keys two blocks
+        // are the faster always (16 heads of 64 x 64: 56 us, with one 64; 8 of 64 x 128, 2000 tokens: 110, 131).
+        constexpr int kAlone = NMAX > 64 ? 1 : 2;
+        if (a.heads * (a.value_pad / 16) <= sm_count()) rc = launch_walk<NMAX, kExact, kAlone>(a, frags, updates, t0, t1, chunks, s);
+        else rc = launch_walk<NMAX, kExact, 2>(a, frags, updates, t0, t1, chunks, s);
+        if (rc) return rc;
     }
     return 0;
 }

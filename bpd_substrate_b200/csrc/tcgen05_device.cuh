@@ -20,20 +20,6 @@ __device__ __forceinline__ bool mbar_wait_sleepy(uint64_t* bar, uint32_t parity,
     return false;
 }
 
-// Whether a phase is complete, without waiting.
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_addr(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
 // The same operations on shared-memory addresses that a role's single thread has worked out ahead of its loop: what such a thread computes between two
 // requests or products is a chain of dependent instructions, and bounds the kernel where it is longer than the copies and products themselves.
 __device__ __forceinline__ bool mbar_test_at(uint32_t bar, uint32_t parity)
