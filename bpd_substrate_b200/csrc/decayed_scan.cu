@@ -544,7 +544,9 @@ int rotate_half_qk(void* q, void* k, int ld, int heads, int dim_pad, int rot_dim
 
 // ------------------------------------------------------------------ causal convolution
 
-constexpr int kConvTile = 32;      // tokens per thread
+// Tokens per thread: a tile reads taps - 1 tokens again, which lie in L2, and few tokens each give more loads in flight.  Four channels of eight
+// tokens: 6144 bf16 channels, 2048 tokens 14.0 us (two of 32: 15.4), 700 tokens 7.6 (11.7); eight channels of 16 tokens 16.1, 9.7.
+constexpr int kConvTile = 8;
 
 // Thread = (NC neighbouring channels, tile of tokens), the window in registers (up to four taps) or read again per token.
 template <typename A, int NC>
@@ -588,26 +590,24 @@ __global__ void __launch_bounds__(128) k_causal_conv(const A* in, int ld_in, A* 
             win[j] = Floats{};
             if (j - (4 - taps) >= 0) win[j] = input(t0 - 3 + j);
         }
-        for (int tb = t0; tb < t1; tb += 8) {
-            Floats x[8];
+        Floats x[kConvTile];
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
-                x[i] = Floats{};
-                if (tb + i < t1) x[i] = input(tb + i);
+        for (int i = 0; i < kConvTile; i++) {
+            x[i] = Floats{};
+            if (t0 + i < t1) x[i] = input(t0 + i);
+        }
+#pragma unroll
+        for (int i = 0; i < kConvTile; i++) {
+            Floats acc = bias;
+#pragma unroll
+            for (int k = 0; k < NC; k++) {
+                acc.v[k] = fmaf(wv[0].v[k], win[0].v[k], acc.v[k]);
+                acc.v[k] = fmaf(wv[1].v[k], win[1].v[k], acc.v[k]);
+                acc.v[k] = fmaf(wv[2].v[k], win[2].v[k], acc.v[k]);
+                acc.v[k] = fmaf(wv[3].v[k], x[i].v[k], acc.v[k]);
             }
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                Floats acc = bias;
-#pragma unroll
-                for (int k = 0; k < NC; k++) {
-                    acc.v[k] = fmaf(wv[0].v[k], win[0].v[k], acc.v[k]);
-                    acc.v[k] = fmaf(wv[1].v[k], win[1].v[k], acc.v[k]);
-                    acc.v[k] = fmaf(wv[2].v[k], win[2].v[k], acc.v[k]);
-                    acc.v[k] = fmaf(wv[3].v[k], x[i].v[k], acc.v[k]);
-                }
-                if (tb + i < t1) store(tb + i, acc);
-                win[0] = win[1]; win[1] = win[2]; win[2] = x[i];
-            }
+            if (t0 + i < t1) store(t0 + i, acc);
+            win[0] = win[1]; win[1] = win[2]; win[2] = x[i];
         }
     } else {
         pdl_wait();
@@ -641,10 +641,15 @@ template <typename A>
 static int launch_conv(const void* in, int ld_in, void* out, int channels, int taps, const float* w, const float* b, float* tail,
                        int T, cudaStream_t s)
 {
-    const bool pairs = channels % 2 == 0 && ld_in % 2 == 0 && !(((uintptr_t)in | (uintptr_t)out) % (2 * sizeof(A)));
-    const dim3 grid((channels / (pairs ? 2 : 1) + 127) / 128, (T + kConvTile - 1) / kConvTile);
-    int rc = pairs ? launch_ordered(k_causal_conv<A, 2>, grid, 128, 0, s, (const A*)in, ld_in, (A*)out, channels, taps, w, b, (const float*)tail, T)
-                   : launch_ordered(k_causal_conv<A, 1>, grid, 128, 0, s, (const A*)in, ld_in, (A*)out, channels, taps, w, b, (const float*)tail, T);
+    const uintptr_t acts = (uintptr_t)in | (uintptr_t)out, floats = (uintptr_t)w | (uintptr_t)b | (uintptr_t)tail;
+    const auto launch = [&](auto kernel, int nc) {
+        return launch_ordered(kernel, dim3((channels / nc + 127) / 128, (T + kConvTile - 1) / kConvTile), 128, 0, s, (const A*)in, ld_in, (A*)out, channels,
+                              taps, w, b, (const float*)tail, T);
+    };
+    int rc;
+    if (channels % 4 == 0 && ld_in % 4 == 0 && acts % (4 * sizeof(A)) == 0 && floats % 16 == 0) rc = launch(k_causal_conv<A, 4>, 4);
+    else if (channels % 2 == 0 && ld_in % 2 == 0 && acts % (2 * sizeof(A)) == 0) rc = launch(k_causal_conv<A, 2>, 2);
+    else rc = launch(k_causal_conv<A, 1>, 1);
     if (rc || taps < 2) return rc;
     return launch_ordered(k_conv_tail<A>, (channels + 127) / 128, 128, 0, s, (const A*)in, ld_in, channels, taps, tail, T);
 }
@@ -735,9 +740,10 @@ __global__ void __launch_bounds__(256) k_gated_norm(const A* o, int ld_o, const 
     }
 }
 
-// Unpadded heads, parts of whole groups of four: W warps per (part, token), four channels per lane and load, at most NJ
-// loads per lane.
-template <typename A, int W, int NJ>
+// Unpadded heads, parts of whole groups of C: W warps per (part, token), C channels per lane and load, at most NJ loads per lane.  Bound by memory
+// where a lane has no more loads than it needs, of 16 bytes: 2048 tokens of 8 parts of 512 channels, bf16 10.0 us and fp32 17 (with eight loads of four
+// channels, half of them empty: 17.9, 53), of one part of 4096 bf16 channels 10.2 (20.2).
+template <typename A, int W, int NJ, int C>
 __global__ void __launch_bounds__(256) k_gated_norm_vec(const A* o, int ld_o, const A* g, int ld_g, const float* __restrict__ w, A* y, int ld_y,
                                                         int part, int parts, int T, int form, float eps)
 {
@@ -747,23 +753,29 @@ __global__ void __launch_bounds__(256) k_gated_norm_vec(const A* o, int ld_o, co
     const long unit = (long)blockIdx.x * (8 / W) + warp / W;
     const int t = (int)(unit / parts), first = (int)(unit - (long)t * parts) * part;
     const bool live = t < T;
-    const int at = 4 * (lane + 32 * (warp % W)), step = 128 * W;
+    const int at = C * (lane + 32 * (warp % W)), step = 32 * C * W;
     pdl_wait();
-    float4 v[NJ], z[NJ];
+    float v[NJ][C], z[NJ][C];
 #pragma unroll
     for (int j = 0; j < NJ; j++) {
         const int i = at + step * j;
-        const bool in = live && i < part;
-        v[j] = in ? act_load4(o + (size_t)t * ld_o + first + i) : make_float4(0, 0, 0, 0);
-        z[j] = in ? act_load4(g + (size_t)t * ld_g + first + i) : make_float4(0, 0, 0, 0);
+        if (live && i < part) {
+            act_load_group(o + (size_t)t * ld_o + first + i, v[j]);
+            act_load_group(g + (size_t)t * ld_g + first + i, z[j]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < C; e++) v[j][e] = z[j][e] = 0.0f;
+        }
     }
     float sum = 0.0f;
 #pragma unroll
-    for (int j = 0; j < NJ; j++) {
-        z[j] = make_float4(gate_value<A>(form, z[j].x), gate_value<A>(form, z[j].y), gate_value<A>(form, z[j].z), gate_value<A>(form, z[j].w));
-        if (form == kGateThenNorm) v[j] = make_float4(v[j].x * z[j].x, v[j].y * z[j].y, v[j].z * z[j].z, v[j].w * z[j].w);
-        sum = fmaf(v[j].x, v[j].x, sum); sum = fmaf(v[j].y, v[j].y, sum); sum = fmaf(v[j].z, v[j].z, sum); sum = fmaf(v[j].w, v[j].w, sum);
-    }
+    for (int j = 0; j < NJ; j++)
+#pragma unroll
+        for (int e = 0; e < C; e++) {
+            z[j][e] = gate_value<A>(form, z[j][e]);
+            if (form == kGateThenNorm) v[j][e] *= z[j][e];
+            sum = fmaf(v[j][e], v[j][e], sum);
+        }
     sum = warp_sum(sum);
     if (W > 1) {
         if (lane == 0) s_part[warp] = sum;
@@ -777,14 +789,25 @@ __global__ void __launch_bounds__(256) k_gated_norm_vec(const A* o, int ld_o, co
     for (int j = 0; j < NJ; j++) {
         const int i = at + step * j;
         if (live && i < part) {
-            float4 f = z[j];
-            if (form != kNormThenGate) {
-                f = *reinterpret_cast<const float4*>(w + first + i);
-                if (form == kNormWeightGate) f = make_float4(f.x * z[j].x, f.y * z[j].y, f.z * z[j].z, f.w * z[j].w);
+            float f[C], r[C];
+            if (form != kNormThenGate) act_load_group(w + first + i, f);
+#pragma unroll
+            for (int e = 0; e < C; e++) {
+                const float m = form == kNormThenGate ? z[j][e] : form == kNormWeightGate ? f[e] * z[j][e] : f[e];
+                r[e] = v[j][e] * scale * m;
             }
-            act_store4(y + (size_t)t * ld_y + first + i, make_float4(v[j].x * scale * f.x, v[j].y * scale * f.y, v[j].z * scale * f.z, v[j].w * scale * f.w));
+            act_store_group(y + (size_t)t * ld_y + first + i, r);
         }
     }
+}
+
+template <typename A, int W, int NJ, int C>
+static int launch_gated_vec(const A* o, int ld_o, const A* g, int ld_g, const float* w, A* y, int ld_y, int part, int parts, int form, float eps, int T,
+                            cudaStream_t s)
+{
+    const long units = (long)T * parts;
+    return launch_ordered(k_gated_norm_vec<A, W, NJ, C>, (unsigned)((units + 8 / W - 1) / (8 / W)), 256, 0, s, o, ld_o, g, ld_g, w, y, ld_y, part, parts, T,
+                          form, eps);
 }
 
 template <typename A>
@@ -793,18 +816,18 @@ static int launch_gated_norm(const A* o, int ld_o, const A* g, int ld_g, const f
 {
     const int part = heads * value_dim / parts;
     const bool vec = value_dim == value_pad && part % 4 == 0 && ld_o % 4 == 0 && ld_g % 4 == 0 && ld_y % 4 == 0;
-    const long units = (long)T * parts;
-    const unsigned packed = (unsigned)((units + 7) / 8), single = (unsigned)units;
-    // a single token has few parts: spread one over the CTA's warps
-    const bool few = units <= 64;
-    if (vec && !few && part <= 256)
-        return launch_ordered(k_gated_norm_vec<A, 1, 2>, packed, 256, 0, s, o, ld_o, g, ld_g, w, y, ld_y, part, parts, T, form, eps);
-    if (vec && !few && part <= 1024)
-        return launch_ordered(k_gated_norm_vec<A, 1, 8>, packed, 256, 0, s, o, ld_o, g, ld_g, w, y, ld_y, part, parts, T, form, eps);
-    if (vec && part <= 2048)
-        return launch_ordered(k_gated_norm_vec<A, 8, 2>, single, 256, 0, s, o, ld_o, g, ld_g, w, y, ld_y, part, parts, T, form, eps);
-    if (vec && part <= 8192)
-        return launch_ordered(k_gated_norm_vec<A, 8, 8>, single, 256, 0, s, o, ld_o, g, ld_g, w, y, ld_y, part, parts, T, form, eps);
+    constexpr int kWide = 16 / sizeof(A);           // channels of 16 bytes
+    // a single token has few parts: spread one over the CTA's warps, with small loads so that all of them have some
+    if (vec && (long)T * parts > 64 && part % kWide == 0 && ld_o % kWide == 0 && ld_g % kWide == 0 && ld_y % kWide == 0 &&
+        !(((uintptr_t)o | (uintptr_t)g | (uintptr_t)y | (uintptr_t)w) & 15)) {
+        if (part <= 32 * kWide) return launch_gated_vec<A, 1, 1, kWide>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
+        if (part <= 64 * kWide) return launch_gated_vec<A, 1, 2, kWide>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
+        if (part <= 128 * kWide) return launch_gated_vec<A, 2, 2, kWide>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
+        if (part <= 512 * kWide) return launch_gated_vec<A, 8, 2, kWide>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
+    }
+    if (vec && part <= 1024) return launch_gated_vec<A, 8, 1, 4>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
+    if (vec && part <= 2048) return launch_gated_vec<A, 8, 2, 4>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
+    if (vec && part <= 8192) return launch_gated_vec<A, 8, 8, 4>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
     int threads = (part / 4 + 31) / 32 * 32;
     threads = threads < 32 ? 32 : threads > 256 ? 256 : threads;
     return launch_ordered(k_gated_norm<A>, dim3(parts, T), threads, 0, s, o, ld_o, g, ld_g, w, y, ld_y, heads, value_dim, value_pad, part, form, eps);

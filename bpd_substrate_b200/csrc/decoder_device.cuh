@@ -108,6 +108,36 @@ __device__ __forceinline__ void act_store4(bf16* p, float4 v)
     *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
 
+// Neighbouring activations, four (16 or 8 bytes) or eight bf16 ones (16 bytes) at a time.
+template <typename A> __device__ __forceinline__ void act_load_group(const A* p, float (&v)[4])
+{
+    const float4 f = act_load4(p);
+    v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+}
+__device__ __forceinline__ void act_load_group(const bf16* p, float (&v)[8])
+{
+    const uint4 u = *reinterpret_cast<const uint4*>(p);
+    const uint32_t r[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        v[2 * i] = __uint_as_float(r[i] << 16);
+        v[2 * i + 1] = __uint_as_float(r[i] & 0xFFFF0000u);
+    }
+}
+__device__ __forceinline__ void act_load_group(const float* p, float (&v)[8])
+{
+    act_load_group(p, *reinterpret_cast<float(*)[4]>(&v[0]));
+    act_load_group(p + 4, *reinterpret_cast<float(*)[4]>(&v[4]));
+}
+template <typename A> __device__ __forceinline__ void act_store_group(A* p, const float (&v)[4]) { act_store4(p, make_float4(v[0], v[1], v[2], v[3])); }
+__device__ __forceinline__ void act_store_group(bf16* p, const float (&v)[8])
+{
+    union { __nv_bfloat162 h[4]; uint4 u; } r;
+#pragma unroll
+    for (int i = 0; i < 4; i++) r.h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    *reinterpret_cast<uint4*>(p) = r.u;
+}
+
 __device__ __forceinline__ float ex2(float x)
 {
     float y;
