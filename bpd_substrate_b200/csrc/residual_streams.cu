@@ -7,9 +7,11 @@
 
 namespace bpdq {
 
-// Thread = four columns, NJ times; NS: the most streams.
+// Thread = four columns, NJ times; NS: the most streams.  Bound by memory, mostly L2, and by how evenly the tokens' CTAs fill the chip: small CTAs whose
+// threads have the loads of two groups of columns in flight (width 2048, four streams: 700 tokens 7.5 us, 1500 tokens 12.1; with one group per
+// thread and twice the threads 8.0, 13.6).
 template <typename A, int NS, int NJ>
-__global__ void __launch_bounds__(1024) k_stream_step(const __grid_constant__ StreamStep p, int* err)
+__global__ void __launch_bounds__(NJ == 2 ? 256 : 1024, NJ == 2 ? 3 : 1) k_stream_step(const __grid_constant__ StreamStep p, int* err)
 {
     __shared__ float s_sum[32];
     pdl_launch_dependents();
@@ -95,6 +97,7 @@ int stream_step(const StreamStep& p, int T, bool act_bf16, cudaStream_t s)
     if (T < 1 || p.m.n < 1 || p.m.n > kMaxStreams || p.width < 1 || p.width_pad < p.width || p.width_pad % 4 || !p.x || (p.h && !p.norm_w) ||
         (p.table ? !p.tokens : !p.y))
         return latch(BPDQ_ERR_ARG);
+    if (p.width_pad > 1024 && p.width_pad <= 2048) return act_bf16 ? launch_stream_step<bf16, 2>(p, T, s) : launch_stream_step<float, 2>(p, T, s);
     if (p.width_pad <= 4096) return act_bf16 ? launch_stream_step<bf16, 1>(p, T, s) : launch_stream_step<float, 1>(p, T, s);
     return act_bf16 ? launch_stream_step<bf16, 4>(p, T, s) : launch_stream_step<float, 4>(p, T, s);
 }
