@@ -524,8 +524,8 @@ typedef struct {
  * cache rows of *pos + t; queries (in place) and keys are divided by their root mean square first.  o [tokens][heads][value_pad] */
 int bpd_grouped_attention_cuda(const bpdq_grouped_shape* shape, void* u, int ld_u, void* cache, int append, void* o, const int32_t* pos, int n_tokens,
                                int act_bf16, void* stream);
-/* The same where the host knows the position: context = *pos + n_tokens (0: unknown).  bf16 prompts whose positions have not wrapped round the
- * cache (context <= rows) then run on larger tiles. */
+/* The same where the host knows the position: context = *pos + n_tokens (0: unknown).  bf16 prompts of two tokens and more whose positions have not
+ * wrapped round the cache (context <= rows) then run on larger tiles, whose launches hold for this context only. */
 int bpd_grouped_attention_context_cuda(const bpdq_grouped_shape* shape, void* u, int ld_u, void* cache, int append, void* o, const int32_t* pos,
                                        int n_tokens, int context, int act_bf16, void* stream);
 /* Residual streams x [tokens][streams][width_pad] joined by hyper-connections: x_t = sum_s mix[s][t] x_s + out[t] y, all from the

@@ -1,8 +1,13 @@
 """Attention of prompts on tiles of 128 rows x 128 keys: the cases and bounds of the latent and grouped kernels at the edges of tiles."""
+import numpy as np
 import pytest
 
+from bpd_substrate_b200.engine import Engine
+from bpd_substrate_b200.vuzelix import VuzelixSpec
+from tests import hybrid_models as hm
 from tests import test_hybrid_gpu as hybrid
 from tests import test_vuzelix_gpu as vuzelix
+from tests import vuzelix_models as vm
 
 pytestmark = pytest.mark.gpu
 
@@ -33,3 +38,26 @@ class Known:
 @pytest.mark.parametrize("cap,sink", [(2.0, 1), (60.0, 1), (0.0, 0)])
 def test_grouped(lib, T, pos, H, G, D, V, chunk, cap, sink):
     vuzelix.attention_case(Known(lib, T, pos + T), 1, T, pos, H, G, D, V, chunk, cap=cap, sink=sink)
+
+
+class ShortPortions(VuzelixSpec):
+    portion = 128           # a cache of chunk + 128 rows
+
+
+# a token's rows beyond the split kernel's: 128 heads on a key head, values of 320; recorded at 100 keys (the larger tiles' contexts begin at 96), and
+# replayed beyond a block of keys, a chunk and the cache's rows
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,chunk", [(128, 1, 64, 64, 0), (2, 1, 128, 320, 0), (128, 1, 64, 64, 90), (2, 1, 128, 320, 90)])
+def test_recorded_tokens(lib, heads, kv_heads, dim, vdim, chunk):
+    """One-token steps that are replayed give the bits of those that are launched."""
+    cfg = vm.config(97, 64, 2, [vm.layer("attention", vm.attention(heads, kv_heads, dim, vdim, chunk, 0.3, 15.0))])
+    w, toks = vm.weights(cfg, 8), hm.tokens(cfg, 270, 9)
+    results = []
+    for use_graph in (True, False):
+        m = vuzelix.device(cfg, w, lib, "bfloat16", capacity=300, spec_class=ShortPortions, use_graph=use_graph)
+        e = Engine(m)
+        e.feed("a", toks[:99])
+        results.append(np.stack([e.feed("a", toks[t:t + 1], [0])[0][0] for t in range(99, 270)]))
+        e.close()
+        m.close()
+    assert lib.bpdq_last_status() == 0
+    assert np.isfinite(results[0]).all() and np.array_equal(*results)
