@@ -614,7 +614,7 @@ int send_inputs(const Buffers& b, const int32_t* ids, int T, int pos, const int3
 {
     StepInputs<N> in;
     in.v[0] = pos;
-    memcpy(in.v + 1, ids, (size_t)T * 4);
+    if (T) memcpy(in.v + 1, ids, (size_t)T * 4);
     if (n_want) memcpy(in.v + 1 + T, want, (size_t)n_want * 4);
     k_step_inputs<N><<<1, 256, 0, s>>>(in, b.ids, b.pos, b.want, T, n_want);
     return check_cuda(cudaGetLastError());
@@ -705,9 +705,10 @@ int forward(Plan* p, const int32_t* token_ids, int n_tokens, int pos, void* stat
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if ((rc = check_cuda(cudaStreamIsCapturing(s, &capturing)))) return rc;
     if (1 + (long)n_tokens + n_places > kManyInputs || capturing != cudaStreamCaptureStatusNone) {
-        // (copies from pageable memory: staged before the calls return; in a caller's own recording they read the caller's memory at every replay)
+        // (copies from pageable memory: staged before the calls return; in a caller's own recording they read the caller's tokens and places at every
+        // replay.  The position is an argument of this call, whose memory is gone by then: it is recorded by value)
+        if ((rc = send_inputs<kFewInputs>(b, nullptr, 0, pos, nullptr, 0, s))) return rc;
         if ((rc = check_cuda(cudaMemcpyAsync(b.ids, token_ids, (size_t)n_tokens * 4, cudaMemcpyHostToDevice, s)))) return rc;
-        if ((rc = check_cuda(cudaMemcpyAsync(b.pos, &pos, 4, cudaMemcpyHostToDevice, s)))) return rc;
         if (n_places && (rc = check_cuda(cudaMemcpyAsync(b.want, want, (size_t)n_want * 4, cudaMemcpyHostToDevice, s)))) return rc;
     } else if ((rc = 1 + n_tokens + n_places <= kFewInputs ? send_inputs<kFewInputs>(b, token_ids, n_tokens, pos, want, n_places, s)
                                                            : send_inputs<kManyInputs>(b, token_ids, n_tokens, pos, want, n_places, s))) {

@@ -574,7 +574,8 @@ void bpdq_hybrid_destroy(void* plan);
 /* Runs n_tokens (up to 65535; once a sequence outgrows a layer's cache_rows, up to cache_rows - chunk + 1) tokens (host ids) of one
  * sequence that already holds `pos` tokens; `state` is the sequence's device memory.  Logits and their argmax are computed at the
  * n_want places of `want` (host, 0 .. n_tokens - 1) and stay in the plan's buffers until its next call.  residuals: device [n_layers][n_tokens][width] or NULL.  use_graph: replay
- * one-token steps as a CUDA graph per state address. */
+ * one-token steps as a CUDA graph per state address.  In a recording of the caller's own (use_graph 0, after a call of these sizes; valid until a
+ * larger call moves the plan's buffers) every replay reads tokens and places from the caller's memory again; the position is the recorded one. */
 int bpdq_hybrid_forward(void* plan, const int32_t* token_ids, int n_tokens, int pos, void* state, const int32_t* want, int n_want,
                         float* residuals, int use_graph, void* stream);
 /* The same, then waits and brings the results to host memory: logits [n_want][vocab] (or NULL), picked [n_want].  Rows of up to 8 MB

@@ -48,3 +48,44 @@ def test_results(lib, vocab):
     assert m.lib.bpdq_last_status() == 0
     e.close()
     m.close()
+
+
+def churn(depth=40):
+    """Leaves other numbers where earlier calls had their frames."""
+    a = np.full(64, 12345, np.int32)
+    return int(a[depth]) + (churn(depth - 1) if depth else 0)
+
+
+@pytest.mark.parametrize("places", [[2], [0, 1, 2]])
+def test_recorded_by_the_caller(lib, places):
+    """A step inside the caller's own recording: replays read the caller's tokens and stand at the recorded position, long after the call has returned."""
+    cfg = hm.config(97, 64, [hm.layer("latent_attention", hm.latent(2, 16, 8, 16, 24, 20, 0.3), 33)] * 2)
+    s = lib.bpdq_stream_create()
+    m = hybrid.device(cfg, hm.weights(cfg, 5), lib, "bfloat16", capacity=128, stream=s)
+    e = Engine(m, slots=2)
+    a, b = e.slots.acquire(), e.slots.acquire()
+    toks = hm.tokens(cfg, 46, 7)
+    for seq in (a, b):
+        m.step(seq, toks[:40])
+    mine, want = np.array(toks[43:46], np.int32), np.array(places, np.int32)
+    assert lib.bpdq_graph_begin(s) == 0
+    rc = lib.bpdq_hybrid_forward(m.plan, mine.ctypes.data, 3, 40, a.base, want.ctypes.data, want.size, None, 0, s)
+    graph = lib.bpdq_graph_end(s)
+    assert rc == 0 and graph
+    mine[:] = toks[40:43]
+    churn()
+    assert lib.bpdq_graph_launch(graph, s) == 0
+    assert lib.bpdq_stream_sync(s) == 0
+    logits, picked = np.empty((want.size, 97), np.float32), np.empty(want.size, np.int64)
+    lib.bpdq_d2h(logits.ctypes.data, lib.bpdq_hybrid_logits(m.plan), logits.nbytes)
+    lib.bpdq_d2h(picked.ctypes.data, lib.bpdq_hybrid_picked(m.plan), picked.nbytes)
+    lib.bpdq_graph_destroy(graph)
+    ref = m.step(b, toks[40:43], places)
+    assert np.array_equal(logits.view(np.uint32), ref[0].view(np.uint32)) and np.array_equal(picked, ref[1])
+    # (the cache rows it wrote are those of positions 40 to 42: the next tokens agree too)
+    a.length += 3
+    assert np.array_equal(m.step(a, toks[43:46], [2])[0], m.step(b, toks[43:46], [2])[0])
+    assert lib.bpdq_last_status() == 0
+    e.close()
+    m.close()
+    lib.bpdq_stream_destroy(s)
