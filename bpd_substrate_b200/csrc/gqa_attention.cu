@@ -9,6 +9,7 @@
 // Both read a key head's rows once for all query heads that share it and hold scores, weights and sums in fp32.
 #include "gqa_attention.cuh"
 #include "cluster_device.cuh"
+#include "gqa_split.h"
 #include "launch.cuh"
 #include "mma_device.cuh"
 #include "rope_device.cuh"
@@ -86,7 +87,6 @@ __device__ __forceinline__ void unpack16(const uint4& w, float (&f)[F16 ? 8 : 4]
     }
 }
 
-constexpr int kSplitThreads = 256, kSplitWarps = kSplitThreads / 32, kMaxCluster = 16;
 
 // What bounds it: the read of the cache rows (4001 keys of 8 heads of 128: 16.4 MB, 2.5 us), and below about 1000 keys the launch.
 // One CTA per (token, head) took 202 us there, most of it in the sums that one thread added in order; 12 us now (65 keys: 9.2,
@@ -643,21 +643,20 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_gqa_tile(GqaShape p, const 
 template <int F16, int D, int R, bool NEW>
 static int launch_split(const GqaShape& p, const GqaNew& in, const float* q, const void* k, const void* v, float* dst, cudaStream_t s)
 {
-    constexpr int kMaxSmem = 96 * 1024;
     auto kern = k_gqa_split<F16, D, R, NEW>;
     static int ready[64] = {0};       // the largest cluster of the kernel on a device
     int dev = 0;
     cudaGetDevice(&dev);
     int largest = dev >= 0 && dev < 64 ? ready[dev] : 0;
     if (!largest) {
-        int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
+        int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSplitMaxSmem));
         if (rc) return rc;
         rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         if (rc) return rc;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(1, kMaxCluster);
         cfg.blockDim = dim3(kSplitThreads);
-        cfg.dynamicSmemBytes = kMaxSmem;
+        cfg.dynamicSmemBytes = kSplitMaxSmem;
         cudaLaunchAttribute at;
         at.id = cudaLaunchAttributeClusterDimension;
         at.val.clusterDim.x = at.val.clusterDim.z = 1;
@@ -672,17 +671,11 @@ static int launch_split(const GqaShape& p, const GqaNew& in, const float* q, con
     }
     const int rep = p.heads / p.kv_heads, groups = (rep + R - 1) / R;
     const int sees = p.kv_offset + p.n_q < p.n_kv ? p.kv_offset + p.n_q : p.n_kv;
-    // as many CTAs per cluster as bring a CTA to every SM, while each keeps 64 keys; more where the scores would not fit
-    constexpr size_t fixed = (size_t)(kSplitWarps + 1) * R * D * sizeof(float);
-    int ranks = 1;
-    while (ranks < largest && (long)p.kv_heads * groups * p.n_q * ranks < sm_count() && sees > 64 * ranks) ranks *= 2;
-    auto stretch_of = [&](int n) { return (sees + n - 1) / n; };
-    while (ranks < largest && fixed + (size_t)stretch_of(ranks) * R * sizeof(float) > (size_t)kMaxSmem) ranks *= 2;
-    const int stretch = stretch_of(ranks);
-    const size_t smem = fixed + (size_t)stretch * R * sizeof(float);
-    if (smem > (size_t)kMaxSmem) return 1;
-    return launch_cluster(kern, dim3((unsigned)(p.kv_heads * groups), (unsigned)ranks, (unsigned)p.n_q), dim3(1, (unsigned)ranks, 1), kSplitThreads, smem, s,
-                          p, in, q, k, v, dst, stretch);
+    const GqaSplit split = gqa_split((long)p.kv_heads * groups * p.n_q, sees, R, D, largest, sm_count());
+    if (!split.fits) return 1;
+    const unsigned ranks = (unsigned)split.ranks;
+    return launch_cluster(kern, dim3((unsigned)(p.kv_heads * groups), ranks, (unsigned)p.n_q), dim3(1, ranks, 1), kSplitThreads, split.smem, s, p, in, q, k, v,
+                          dst, split.stretch);
 }
 
 template <bool NEW, int F16, int D>
@@ -744,12 +737,9 @@ int gqa_attention(const GqaShape& p, const float* q, const void* k, const void* 
     return launch_split_of<false>(p, GqaNew{}, q, k, v, dst, s);
 }
 
-bool gqa_takes_new(const GqaShape& p, const void* q, const void* k, const void* v, const void* dst)
-{
-    return p.n_q == 1 && !(((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)dst) & 15) && gqa_kernel(p) == kSplit;
-}
 int gqa_attention_new(const GqaShape& p, const GqaNew& in, const float* q, void* k, void* v, float* dst, cudaStream_t s)
 {
+    if (p.n_q != 1 || (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)dst) & 15) || gqa_kernel(p) != kSplit) return 1;
     return launch_split_of<true>(p, in, q, k, v, dst, s);
 }
 

@@ -20,9 +20,7 @@ struct GqaNew {
     float theta_scale;
     int* err;
 };
-// Whether gqa_attention_new takes the shape.
-bool gqa_takes_new(const GqaShape& p, const void* q, const void* k, const void* v, const void* dst);
-// The same as gqa_attention behind those steps; q is not written.
+// The same as gqa_attention behind those steps, for one query; q is not written.  1, and nothing is launched, where the split kernel does not take it.
 int gqa_attention_new(const GqaShape& p, const GqaNew& in, const float* q, void* k, void* v, float* dst, cudaStream_t s);
 // Runs the product on one of this file's kernels, or returns 1 if the shape or the pointers are not theirs.
 int gqa_attention(const GqaShape& p, const float* q, const void* k, const void* v, float* dst, cudaStream_t s);

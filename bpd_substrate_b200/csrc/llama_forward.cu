@@ -627,14 +627,12 @@ static int decode_forward(const bpd_llama_weights* weights, const bpd_llama_conf
         qkv.N[0] = E; qkv.N[1] = qkv.N[2] = row;
         if ((rc = q8_0_llama(qkv, s))) return rc;
         const GqaShape shape = {1, cfg->max_seq_len, H, HKV, D, 1.0f / sqrtf((float)D), kv_pos, cfg->kv_cache_f16};
-        if (gqa_takes_new(shape, b.s1, kc, vc, b.s2)) {
-            const GqaNew in = {b.s3, b.s3 + row, pos_ids, weights->rope_freqs, cfg->rope_dim, cfg->max_seq_len,
-                               powf(cfg->rope_base, -2.0f / (float)cfg->rope_dim), device_error_flag()};
-            rc = gqa_attention_new(shape, in, b.s1, kc, vc, b.s2, s);
-        } else if (!(rc = launch_rope_qk_store_kv(b.s1, b.s3, b.s3 + row, kc, vc, pos_ids, weights->rope_freqs, 1, H, HKV, D, cfg->rope_dim, cfg->rope_base,
-                                                  cfg->kv_cache_f16, cfg->max_seq_len, s))) {
+        const GqaNew in = {b.s3, b.s3 + row, pos_ids, weights->rope_freqs, cfg->rope_dim, cfg->max_seq_len,
+                           powf(cfg->rope_base, -2.0f / (float)cfg->rope_dim), device_error_flag()};
+        rc = gqa_attention_new(shape, in, b.s1, kc, vc, b.s2, s);
+        if (rc == 1 && !(rc = launch_rope_qk_store_kv(b.s1, b.s3, b.s3 + row, kc, vc, pos_ids, weights->rope_freqs, 1, H, HKV, D, cfg->rope_dim, cfg->rope_base,
+                                                      cfg->kv_cache_f16, cfg->max_seq_len, s)))
             rc = launch_attn(b.s1, kc, vc, b.s2, 1, cfg->max_seq_len, H, HKV, D, shape.scale, kv_pos, cfg->kv_cache_f16, s);
-        }
         if (rc || (rc = plain_product(lw->w_o, b.s2, b.s3, E, E, s))) return rc;
         r = b.s3;
         Q80Llama ff = normed_product(b.x, r, lw->ffn_norm_w, nullptr, cfg);
