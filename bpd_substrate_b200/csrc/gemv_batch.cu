@@ -629,19 +629,14 @@ int gemv_q8_0_fast_multi(int n, const uint8_t* const* Ws, float* const* outs, co
     return launch_batch<1, BPDQ_LAYOUT_BPD>(plan, s);
 }
 
-bool q8_0_llama_fits(const Q80Llama& l)
+static int plan_q8_0_llama(const Q80Llama& l, BatchPlan& plan)
 {
-    if (l.n < 1 || l.n > kMaxBatch || l.K < 256 || l.K % 256 || (l.norm_w && l.K > 8192) || (l.gated && (l.n != 2 || l.N[0] != l.N[1]))) return false;
+    if (l.n < 1 || l.n > kMaxBatch || l.K < 256 || l.K % 256 || (l.norm_w && l.K > 8192) || (l.gated && (l.n != 2 || l.N[0] != l.N[1]))) return BPDQ_ERR_RANGE;
     uintptr_t all = (uintptr_t)l.x | (uintptr_t)l.r | (uintptr_t)l.norm_w | (uintptr_t)l.x_out;
     for (int j = 0; j < l.n; j++) all |= (uintptr_t)l.W[j];
-    return !(all & 15) && l.x;
-}
-int q8_0_llama(const Q80Llama& l, cudaStream_t s)
-{
-    if (!q8_0_llama_fits(l)) return BPDQ_ERR_RANGE;
+    if ((all & 15) || !l.x) return BPDQ_ERR_RANGE;
     BatchDesc d[kMaxBatch];
     for (int j = 0; j < l.n; j++) d[j] = {l.W[j], l.x, l.out[j], l.N[j], l.K};
-    BatchPlan plan;
     const int rc = make_batch_plan(d, l.n, plan, 1, 1, l.norm_w ? 4 * l.K : 0, l.gated);
     if (rc) return rc;
     plan.prologue = l.norm_w ? 3 : 0;
@@ -650,7 +645,18 @@ int q8_0_llama(const Q80Llama& l, cudaStream_t s)
     plan.pro_b = l.norm_w;
     plan.pro_out = l.x_out;
     plan.pro_eps = l.eps;
-    return launch_batch<2, BPDQ_LAYOUT_BPD>(plan, s);
+    return 0;
+}
+bool q8_0_llama_fits(const Q80Llama& l)
+{
+    BatchPlan plan;
+    return plan_q8_0_llama(l, plan) == 0;
+}
+int q8_0_llama(const Q80Llama& l, cudaStream_t s)
+{
+    BatchPlan plan;
+    const int rc = plan_q8_0_llama(l, plan);
+    return rc ? rc : launch_batch<2, BPDQ_LAYOUT_BPD>(plan, s);
 }
 
 // ---------------------------------------------------------------- scratch without an allocator

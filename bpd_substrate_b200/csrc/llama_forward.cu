@@ -587,6 +587,36 @@ static int plain_product(const uint8_t* W, const float* x, float* out, int N, in
     return rc == BPDQ_ERR_RANGE ? bpd_qmatmul_q8_0_cuda(W, x, out, 1, N, K, s) : rc;
 }
 
+static Q80Llama qkv_product(const float* x, const float* r, float* x_out, const bpd_llama_layer_weights* lw, const bpd_llama_config* cfg, float* q, float* k,
+                            float* v)
+{
+    Q80Llama l = normed_product(x, r, lw->attn_norm_w, x_out, cfg);
+    l.n = 3;
+    l.W[0] = lw->w_q; l.W[1] = lw->w_k; l.W[2] = lw->w_v;
+    l.out[0] = q; l.out[1] = k; l.out[2] = v;
+    l.N[0] = cfg->embed_dim; l.N[1] = l.N[2] = cfg->n_kv_heads * cfg->head_dim;
+    return l;
+}
+static Q80Llama gated_product(const float* x, const float* r, float* x_out, const bpd_llama_layer_weights* lw, const bpd_llama_config* cfg, float* out)
+{
+    Q80Llama l = normed_product(x, r, lw->ffn_norm_w, x_out, cfg);
+    l.n = 2;
+    l.W[0] = lw->w_gate; l.W[1] = lw->w_up;
+    l.out[0] = l.out[1] = out;
+    l.N[0] = l.N[1] = cfg->ffn_dim;
+    l.gated = true;
+    return l;
+}
+static Q80Llama head_product(const float* x, const float* r, const bpd_llama_weights* w, const bpd_llama_config* cfg, float* logits)
+{
+    Q80Llama l = normed_product(x, r, w->output_norm_w, nullptr, cfg);
+    l.n = 1;
+    l.W[0] = w->output_w;
+    l.out[0] = logits;
+    l.N[0] = cfg->vocab_size;
+    return l;
+}
+
 // Whether the products of a token have the sizes and alignments for it.
 static bool decodes_fused(const bpd_llama_weights* w, const bpd_llama_config* cfg)
 {
@@ -602,7 +632,14 @@ static bool decodes_fused(const bpd_llama_weights* w, const bpd_llama_config* cf
             given = given && p;
         }
     }
-    return given && !(all & 15);
+    if (!given || (all & 15)) return false;
+    // a launch that also holds the vector in shared memory must have room for it beside the tiles that bpdq_set_tuning asks for; sizes are those of every layer
+    alignas(16) float any[4];
+    const Q80Llama kinds[] = {qkv_product(any, nullptr, nullptr, w->layers, cfg, any, any, any), gated_product(any, nullptr, nullptr, w->layers, cfg, any),
+                              head_product(any, nullptr, w, cfg, any)};
+    for (const Q80Llama& l : kinds)
+        if (!q8_0_llama_fits(l)) return false;
+    return true;
 }
 
 static int decode_forward(const bpd_llama_weights* weights, const bpd_llama_config* cfg, const int32_t* pos_ids, int kv_pos, void* k_cache, void* v_cache,
@@ -611,21 +648,16 @@ static int decode_forward(const bpd_llama_weights* weights, const bpd_llama_conf
     const int E = cfg->embed_dim, H = cfg->n_heads, HKV = cfg->n_kv_heads, D = cfg->head_dim, F = cfg->ffn_dim, row = HKV * D;
     const size_t kv_layer = (size_t)cfg->max_seq_len * row * (cfg->kv_cache_f16 ? 2 : 4);
     const float* r = nullptr;       // what the last product left to be added
-    auto add_of = [&](Q80Llama& l) {
-        l.x_out = r ? b.other : nullptr;
+    auto sum_to = [&]() { return r ? b.other : nullptr; };
+    auto summed = [&]() {
         if (r) { float* t = b.x; b.x = b.other; b.other = t; }
     };
     int rc;
     for (int layer = 0; layer < cfg->n_layers; layer++) {
         const bpd_llama_layer_weights* lw = &weights->layers[layer];
         void *kc = (uint8_t*)k_cache + layer * kv_layer, *vc = (uint8_t*)v_cache + layer * kv_layer;
-        Q80Llama qkv = normed_product(b.x, r, lw->attn_norm_w, nullptr, cfg);
-        add_of(qkv);
-        qkv.n = 3;
-        qkv.W[0] = lw->w_q; qkv.W[1] = lw->w_k; qkv.W[2] = lw->w_v;
-        qkv.out[0] = b.s1; qkv.out[1] = b.s3; qkv.out[2] = b.s3 + row;
-        qkv.N[0] = E; qkv.N[1] = qkv.N[2] = row;
-        if ((rc = q8_0_llama(qkv, s))) return rc;
+        if ((rc = q8_0_llama(qkv_product(b.x, r, sum_to(), lw, cfg, b.s1, b.s3, b.s3 + row), s))) return rc;
+        summed();
         const GqaShape shape = {1, cfg->max_seq_len, H, HKV, D, 1.0f / sqrtf((float)D), kv_pos, cfg->kv_cache_f16};
         const GqaNew in = {b.s3, b.s3 + row, pos_ids, weights->rope_freqs, cfg->rope_dim, cfg->max_seq_len,
                            powf(cfg->rope_base, -2.0f / (float)cfg->rope_dim), device_error_flag()};
@@ -635,23 +667,12 @@ static int decode_forward(const bpd_llama_weights* weights, const bpd_llama_conf
             rc = launch_attn(b.s1, kc, vc, b.s2, 1, cfg->max_seq_len, H, HKV, D, shape.scale, kv_pos, cfg->kv_cache_f16, s);
         if (rc || (rc = plain_product(lw->w_o, b.s2, b.s3, E, E, s))) return rc;
         r = b.s3;
-        Q80Llama ff = normed_product(b.x, r, lw->ffn_norm_w, nullptr, cfg);
-        add_of(ff);
-        ff.n = 2;
-        ff.W[0] = lw->w_gate; ff.W[1] = lw->w_up;
-        ff.out[0] = ff.out[1] = b.s1;
-        ff.N[0] = ff.N[1] = F;
-        ff.gated = true;
-        if ((rc = q8_0_llama(ff, s))) return rc;
+        if ((rc = q8_0_llama(gated_product(b.x, r, sum_to(), lw, cfg, b.s1), s))) return rc;
+        summed();
         if ((rc = plain_product(lw->w_down, b.s1, b.s2, E, F, s))) return rc;
         r = b.s2;
     }
-    Q80Llama head = normed_product(b.x, r, weights->output_norm_w, nullptr, cfg);
-    head.n = 1;
-    head.W[0] = weights->output_w;
-    head.out[0] = logits;
-    head.N[0] = cfg->vocab_size;
-    return q8_0_llama(head, s);
+    return q8_0_llama(head_product(b.x, r, weights, cfg, logits), s);
 }
 
 }  // namespace bpdq

@@ -51,3 +51,13 @@ def test_token(lib, heads, kv_heads, dim, ff, f16, rope_dim, context, pos):
     for a, b in zip(*results):
         assert np.array_equal(a, b)
     dev.close()
+
+
+def test_tiles_that_leave_no_room_for_the_vector(lib):
+    """Weight tiles as large as bpdq_set_tuning lets them be: a launch of several steps also holds its vector in shared memory, where 6144 numbers then do not
+    fit beside them."""
+    lib.bpdq_set_tuning(27000, 2, 0, 16, -1)
+    try:
+        test_token(lib, 48, 8, 128, 256, 1, 128, 70, 70)
+    finally:
+        lib.bpdq_set_tuning(8192, 2, 0, 16, -1)     # the library's defaults
