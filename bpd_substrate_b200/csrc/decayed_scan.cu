@@ -544,38 +544,43 @@ int rotate_half_qk(void* q, void* k, int ld, int heads, int dim_pad, int rot_dim
 
 // ------------------------------------------------------------------ causal convolution
 
-// Tokens per thread: a tile reads taps - 1 tokens again, which lie in L2, and few tokens each give more loads in flight.  Four channels of eight
-// tokens: 6144 bf16 channels, 2048 tokens 14.0 us (two of 32: 15.4), 700 tokens 7.6 (11.7); eight channels of 16 tokens 16.1, 9.7.
-constexpr int kConvTile = 8;
+constexpr unsigned kConvAtOnce = 8;      // tokens whose loads are in flight together
 
-// Thread = (NC neighbouring channels, tile of tokens), the window in registers (up to four taps) or read again per token.
+// Thread = (NC neighbouring channels, tile of tokens), the window in registers (up to four taps) or read again per token.  c_blocks: blocks of
+// channels, which vary fastest over the grid (of one dimension: tiles are more than the others take).  Bound by instructions: pointers that move by whole
+// rows, and blocks of tokens that need no checks, are a third of the time of 8192 tokens.
 template <typename A, int NC>
 __global__ void __launch_bounds__(128) k_causal_conv(const A* in, int ld_in, A* out, int channels, int taps,
-                                                     const float* __restrict__ w, const float* __restrict__ b, const float* tail, int T)
+                                                     const float* __restrict__ w, const float* __restrict__ b, const float* tail, int T, unsigned c_blocks, int tile)
 {
     struct alignas(NC * sizeof(A)) Group { A v[NC]; };
     struct alignas(NC * 4) Floats { float v[NC]; };
     pdl_launch_dependents();
-    const int c = NC * (blockIdx.x * 128 + threadIdx.x);
-    if (c >= channels) return;
-    const int t0 = blockIdx.y * kConvTile, t1 = t0 + kConvTile < T ? t0 + kConvTile : T;
+    const unsigned part = blockIdx.x / c_blocks;
+    const unsigned c = NC * ((blockIdx.x - part * c_blocks) * 128 + threadIdx.x);
+    if (c >= (unsigned)channels) return;
+    const unsigned t0 = part * (unsigned)tile, n = (unsigned)T - t0 < (unsigned)tile ? (unsigned)T - t0 : (unsigned)tile;
+    const size_t ls = (size_t)ld_in, lo = (size_t)channels;
+    const A* src = in + t0 * ls + c;
+    A* dst = out + t0 * lo + c;
     auto floats = [&](const float* p) -> Floats { return *reinterpret_cast<const Floats*>(p + c); };
     Floats bias = {};
     if (b) bias = floats(b);
-    auto input = [&](int t) -> Floats {      // t >= -(taps - 1)
-        if (t < 0) return floats(tail + (size_t)(t + taps - 1) * channels);
-        const Group g = *reinterpret_cast<const Group*>(in + (size_t)t * ld_in + c);
+    auto load = [&](const A* p) -> Floats {
+        const Group g = *reinterpret_cast<const Group*>(p);
         Floats f;
 #pragma unroll
         for (int i = 0; i < NC; i++) f.v[i] = act_load(&g.v[i]);
         return f;
     };
-    auto store = [&](int t, const Floats& f) {
+    auto store = [&](A* p, const Floats& f) {
         Group g;
 #pragma unroll
         for (int i = 0; i < NC; i++) g.v[i] = act_from<A>(silu_act<A>(f.v[i]));
-        *reinterpret_cast<Group*>(out + (size_t)t * channels + c) = g;
+        *reinterpret_cast<Group*>(p) = g;
     };
+    // `back` tokens before the tile, at most taps - 1: the window of the tokens before, where there are none
+    auto before = [&](unsigned back) -> Floats { return back > t0 ? floats(tail + (t0 + taps - 1 - back) * lo) : load(src - back * ls); };
     if (taps <= 4) {
         Floats wv[4], win[3];
 #pragma unroll
@@ -588,37 +593,57 @@ __global__ void __launch_bounds__(128) k_causal_conv(const A* in, int ld_in, A* 
 #pragma unroll
         for (int j = 0; j < 3; j++) {
             win[j] = Floats{};
-            if (j - (4 - taps) >= 0) win[j] = input(t0 - 3 + j);
+            if (j - (4 - taps) >= 0) win[j] = before(3 - j);
         }
-        Floats x[kConvTile];
-#pragma unroll
-        for (int i = 0; i < kConvTile; i++) {
-            x[i] = Floats{};
-            if (t0 + i < t1) x[i] = input(t0 + i);
-        }
-#pragma unroll
-        for (int i = 0; i < kConvTile; i++) {
+        auto step = [&](const Floats& x) {
             Floats acc = bias;
 #pragma unroll
             for (int k = 0; k < NC; k++) {
                 acc.v[k] = fmaf(wv[0].v[k], win[0].v[k], acc.v[k]);
                 acc.v[k] = fmaf(wv[1].v[k], win[1].v[k], acc.v[k]);
                 acc.v[k] = fmaf(wv[2].v[k], win[2].v[k], acc.v[k]);
-                acc.v[k] = fmaf(wv[3].v[k], x[i].v[k], acc.v[k]);
+                acc.v[k] = fmaf(wv[3].v[k], x.v[k], acc.v[k]);
             }
-            if (t0 + i < t1) store(t0 + i, acc);
-            win[0] = win[1]; win[1] = win[2]; win[2] = x[i];
+            win[0] = win[1]; win[1] = win[2]; win[2] = x;
+            return acc;
+        };
+        unsigned left = n;
+        for (; left >= kConvAtOnce; left -= kConvAtOnce, src += kConvAtOnce * ls, dst += kConvAtOnce * lo) {
+            Floats x[kConvAtOnce];
+#pragma unroll
+            for (int i = 0; i < kConvAtOnce; i++) x[i] = load(src + i * ls);
+#pragma unroll
+            for (int i = 0; i < kConvAtOnce; i++) store(dst + i * lo, step(x[i]));
+        }
+        if (left) {
+            Floats x[kConvAtOnce - 1];
+#pragma unroll
+            for (int i = 0; i < kConvAtOnce - 1; i++) {
+                x[i] = Floats{};
+                if (i < left) x[i] = load(src + i * ls);
+            }
+#pragma unroll
+            for (int i = 0; i < kConvAtOnce - 1; i++) {
+                const Floats y = step(x[i]);
+                if (i < left) store(dst + i * lo, y);
+            }
         }
     } else {
         pdl_wait();
-        for (int t = t0; t < t1; t++) {
+        const unsigned window = taps - 1;
+        for (unsigned t = t0; t < t0 + n; t++, dst += lo) {
             Floats acc = bias;
-            for (int j = 0; j < taps; j++) {
-                const Floats x = input(t - taps + 1 + j), wj = floats(w + (size_t)j * channels);
+            auto add = [&](const Floats& f, const Floats& x) {
 #pragma unroll
-                for (int k = 0; k < NC; k++) acc.v[k] = fmaf(wj.v[k], x.v[k], acc.v[k]);
-            }
-            store(t, acc);
+                for (int k = 0; k < NC; k++) acc.v[k] = fmaf(f.v[k], x.v[k], acc.v[k]);
+            };
+            const unsigned none = t < window ? window - t : 0;      // taps on tokens before the first
+            for (unsigned j = 0; j < none; j++) add(floats(w + j * lo), floats(tail + (t + j) * lo));
+            const A* p = in + (t + none - window) * ls + c;
+            const float* f = w + none * lo;
+#pragma unroll 4
+            for (unsigned j = none; j <= window; j++, p += ls, f += lo) add(floats(f), load(p));
+            store(dst, acc);
         }
     }
 }
@@ -637,17 +662,34 @@ __global__ void __launch_bounds__(128) k_conv_tail(const A* in, int ld_in, int c
     }
 }
 
+// Tokens of a tile.  A tile reads taps - 1 tokens again and its weights once, so long ones cost less work and short ones fill the chip: eight up to 16 CTAs
+// per SM, 16 up to 40 of them, 24 beyond, and always eight where every token reads its whole window again.  us at 8, 16, 24, 32 tokens: 6144 bf16
+// channels, 700 tokens 6.9, 7.6, 8.3, 8.5; 2048 12.9, 12.1, 12.9, 15.6; 4096 30.2, 24.5, 23.2, 24.7; fp32, 2048 tokens 24.5, 24.3, 24.7, 27.7; channel by channel
+// 6145 of bf16, 700 tokens 9.0, 7.8, 7.8, 8.8; 4096 41.5, 31.3, 27.4, 26.4.  (Six taps, 6144 bf16 channels, 2048 tokens: 29 at eight; 35 and, at 32, 55 with a check of
+// every load.)
+static int conv_tile(unsigned c_blocks, int taps, int T)
+{
+    const long ctas = (long)c_blocks * ((T + 7) / 8);
+    if (taps > 4 || ctas <= 16l * sm_count()) return 8;
+    return ctas <= 40l * sm_count() ? 16 : 24;
+}
+
 template <typename A>
 static int launch_conv(const void* in, int ld_in, void* out, int channels, int taps, const float* w, const float* b, float* tail,
                        int T, cudaStream_t s)
 {
     const uintptr_t acts = (uintptr_t)in | (uintptr_t)out, floats = (uintptr_t)w | (uintptr_t)b | (uintptr_t)tail;
     const auto launch = [&](auto kernel, int nc) {
-        return launch_ordered(kernel, dim3((channels / nc + 127) / 128, (T + kConvTile - 1) / kConvTile), 128, 0, s, (const A*)in, ld_in, (A*)out, channels,
-                              taps, w, b, (const float*)tail, T);
+        const unsigned c_blocks = (unsigned)((channels / nc + 127) / 128);
+        const int tile = conv_tile(c_blocks, taps, T);
+        const long ctas = (long)c_blocks * ((T + tile - 1) / tile);
+        if (ctas > 0x7FFFFFFF) return latch(BPDQ_ERR_RANGE);
+        return launch_ordered(kernel, (unsigned)ctas, 128, 0, s, (const A*)in, ld_in, (A*)out, channels, taps, w, b, (const float*)tail, T, c_blocks, tile);
     };
     int rc;
-    if (channels % 4 == 0 && ld_in % 4 == 0 && acts % (4 * sizeof(A)) == 0 && floats % 16 == 0) rc = launch(k_causal_conv<A, 4>, 4);
+    // loads of 8 bytes (of 16, 2048 tokens of 6144 fp32 channels 24.0 us, 20.5 so); more channels at a time where windows are read again and again
+    constexpr int kMost = sizeof(A) == 2 ? 4 : 2;
+    if ((kMost == 4 || taps > 4) && channels % 4 == 0 && ld_in % 4 == 0 && acts % (4 * sizeof(A)) == 0 && floats % 16 == 0) rc = launch(k_causal_conv<A, 4>, 4);
     else if (channels % 2 == 0 && ld_in % 2 == 0 && acts % (2 * sizeof(A)) == 0) rc = launch(k_causal_conv<A, 2>, 2);
     else rc = launch(k_causal_conv<A, 1>, 1);
     if (rc || taps < 2) return rc;

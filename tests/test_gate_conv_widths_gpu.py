@@ -69,3 +69,11 @@ def test_causal_conv(lib, dtype, T, channels, taps, offset):
     close(y, a * sigmoid(a), dtype)
     if taps > 1:
         assert torch.equal(tail.double(), seen[T:])
+
+
+# tiles of 16 and 24 tokens with whole and ragged last ones, every load width; more tiles than a grid's second dimension takes; windows longer than a tile
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T,channels,taps,offset", [(19001, 512, 4, 0), (19007, 130, 3, 0), (19016, 101, 2, 0), (48000, 64, 4, 0), (50011, 34, 4, 0), (50017, 33, 4, 0),
+                                                    (524296, 8, 4, 0), (524289, 3, 2, 0), (30, 12, 19, 0), (3, 8, 12, 0)])
+def test_causal_conv_tiles(lib, dtype, T, channels, taps, offset):
+    test_causal_conv(lib, dtype, T, channels, taps, offset)
