@@ -783,8 +783,7 @@ __global__ void __launch_bounds__(256) k_gated_norm(const A* o, int ld_o, const 
 }
 
 // Unpadded heads, parts of whole groups of C: W warps per (part, token), C channels per lane and load, at most NJ loads per lane.  Bound by memory
-// where a lane has no more loads than it needs, of 16 bytes: 2048 tokens of 8 parts of 512 channels, bf16 10.0 us and fp32 17 (with eight loads of four
-// channels, half of them empty: 17.9, 53), of one part of 4096 bf16 channels 10.2 (20.2).
+// where a lane has no more loads than it needs and no more warps than have some.
 template <typename A, int W, int NJ, int C>
 __global__ void __launch_bounds__(256) k_gated_norm_vec(const A* o, int ld_o, const A* g, int ld_g, const float* __restrict__ w, A* y, int ld_y,
                                                         int part, int parts, int T, int form, float eps)
@@ -796,6 +795,15 @@ __global__ void __launch_bounds__(256) k_gated_norm_vec(const A* o, int ld_o, co
     const int t = (int)(unit / parts), first = (int)(unit - (long)t * parts) * part;
     const bool live = t < T;
     const int at = C * (lane + 32 * (warp % W)), step = 32 * C * W;
+    // the weights ahead of the wait where few CTAs fit anyway (parts of 8192: bf16 10.2 us for 12.0, fp32 23 for 26; elsewhere they cost occupancy: bf16 in loads
+    // of four, parts of 4100, 22 us, 28 so)
+    constexpr bool kEarly = NJ * C >= 32 && (C == 8 || sizeof(A) == 4);
+    float early[kEarly ? NJ : 1][C];
+    if constexpr (kEarly) {
+#pragma unroll
+        for (int j = 0; j < NJ; j++)
+            if (form != kNormThenGate && live && at + step * j < part) act_load_group(w + first + at + step * j, early[j]);
+    }
     pdl_wait();
     float v[NJ][C], z[NJ][C];
 #pragma unroll
@@ -832,7 +840,12 @@ __global__ void __launch_bounds__(256) k_gated_norm_vec(const A* o, int ld_o, co
         const int i = at + step * j;
         if (live && i < part) {
             float f[C], r[C];
-            if (form != kNormThenGate) act_load_group(w + first + i, f);
+            if constexpr (kEarly) {
+#pragma unroll
+                for (int e = 0; e < C; e++) f[e] = early[j][e];
+            } else if (form != kNormThenGate) {
+                act_load_group(w + first + i, f);
+            }
 #pragma unroll
             for (int e = 0; e < C; e++) {
                 const float m = form == kNormThenGate ? z[j][e] : form == kNormWeightGate ? f[e] * z[j][e] : f[e];
@@ -858,17 +871,27 @@ static int launch_gated_norm(const A* o, int ld_o, const A* g, int ld_g, const f
 {
     const int part = heads * value_dim / parts;
     const bool vec = value_dim == value_pad && part % 4 == 0 && ld_o % 4 == 0 && ld_g % 4 == 0 && ld_y % 4 == 0;
-    constexpr int kWide = 16 / sizeof(A);           // channels of 16 bytes
-    // a single token has few parts: spread one over the CTA's warps, with small loads so that all of them have some
-    if (vec && (long)T * parts > 64 && part % kWide == 0 && ld_o % kWide == 0 && ld_g % kWide == 0 && ld_y % kWide == 0 &&
-        !(((uintptr_t)o | (uintptr_t)g | (uintptr_t)y | (uintptr_t)w) & 15)) {
-        if (part <= 32 * kWide) return launch_gated_vec<A, 1, 1, kWide>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
-        if (part <= 64 * kWide) return launch_gated_vec<A, 1, 2, kWide>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
-        if (part <= 128 * kWide) return launch_gated_vec<A, 2, 2, kWide>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
-        if (part <= 512 * kWide) return launch_gated_vec<A, 8, 2, kWide>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
+    // A single token has few parts: spread one over the CTA's warps, with loads of few channels so that all of them have some.
+    if (vec && (long)T * parts <= 64) {
+        if (part <= 1024) return launch_gated_vec<A, 8, 1, 4>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
+        if (part <= 2048) return launch_gated_vec<A, 8, 2, 4>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
     }
-    if (vec && part <= 1024) return launch_gated_vec<A, 8, 1, 4>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
+    // Else up to four loads of four channels per lane, in as many warps as that takes; two bf16 rows of eight channels in half as many loads where a warp would
+    // have two, and where four would not do.  us at 2048 x 4096 values, bf16: parts of 100 17 (eight warps a part 97), 256 9.8 (11.1 in loads of four), 512 9.7,
+    // 1024 9.5, 2048 9.5 (eight warps and loads of eight, half of them empty, 15.5), 4096 9.5, 8192 10.2 (18.4 in loads of four); fp32: 100 23, 1024 17.0 (eight
+    // warps 26), 4096 17 (eight loads a lane 38).
+    const bool wide = sizeof(A) == 2 && !((part | ld_o | ld_g | ld_y) & 7) && !(((uintptr_t)o | (uintptr_t)g | (uintptr_t)y | (uintptr_t)w) & 15);
+    if constexpr (sizeof(A) == 2) {
+        if (vec && wide && part > 128 && part <= 256) return launch_gated_vec<A, 1, 1, 8>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
+        if (vec && wide && part > 4096 && part <= 8192) return launch_gated_vec<A, 8, 4, 8>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
+        if (vec && part > 1024 && part <= 2048) return launch_gated_vec<A, 4, 4, 4>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
+    }
+    if (vec && part <= 128) return launch_gated_vec<A, 1, 1, 4>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
+    if (vec && part <= 256) return launch_gated_vec<A, 1, 2, 4>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
+    if (vec && part <= 512) return launch_gated_vec<A, 1, 4, 4>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
+    if (vec && part <= 1024) return launch_gated_vec<A, 2, 4, 4>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
     if (vec && part <= 2048) return launch_gated_vec<A, 8, 2, 4>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
+    if (vec && part <= 4096) return launch_gated_vec<A, 8, 4, 4>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
     if (vec && part <= 8192) return launch_gated_vec<A, 8, 8, 4>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);
     int threads = (part / 4 + 31) / 32 * 32;
     threads = threads < 32 ? 32 : threads > 256 ? 256 : threads;

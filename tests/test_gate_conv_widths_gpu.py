@@ -77,3 +77,13 @@ def test_causal_conv(lib, dtype, T, channels, taps, offset):
                                                     (524296, 8, 4, 0), (524289, 3, 2, 0), (30, 12, 19, 0), (3, 8, 12, 0)])
 def test_causal_conv_tiles(lib, dtype, T, channels, taps, offset):
     test_causal_conv(lib, dtype, T, channels, taps, offset)
+
+
+# parts at the edges of every number of warps and loads, in channels that only loads of four take and on pointers that only they take
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T,parts,part,offset", [(70, 1, 4, 0), (33, 2, 100, 0), (33, 2, 128, 4), (33, 2, 132, 0), (33, 2, 136, 0), (33, 2, 252, 0), (65, 1, 256, 4), (65, 1, 260, 0),
+                                                 (65, 1, 508, 0), (65, 1, 1020, 0), (65, 1, 1028, 0), (65, 1, 2044, 0), (65, 1, 2048, 4), (65, 1, 2052, 0), (65, 1, 4092, 0),
+                                                 (65, 1, 4100, 0), (65, 1, 8188, 0), (65, 1, 8192, 4), (1, 8, 2048, 0), (2, 1, 2052, 0), (64, 1, 8192, 0)])
+def test_gated_norm_narrow_loads(lib, dtype, T, parts, part, offset):
+    for form in (0, 1, 2):
+        test_gated_norm(lib, dtype, T, parts, part, offset, form)
