@@ -7,11 +7,10 @@
 
 namespace bpdq {
 
-// Thread = four columns, NJ times; NS: the most streams.  Bound by memory, mostly L2, and by how evenly the tokens' CTAs fill the chip: small CTAs whose
-// threads have the loads of two groups of columns in flight (width 2048, four streams: 700 tokens 7.5 us, 1500 tokens 12.1; with one group per
-// thread and twice the threads 8.0, 13.6).
+// Thread = four columns, NJ times; NS: the most streams.  Bound by memory, mostly L2, and by how evenly the tokens' CTAs fill the chip.  (No least number of
+// CTAs where a thread has one group: asked for one, the compiler takes 36 and 64 registers instead of 32 and 61, 3 to 8 % of one, two and eight streams.)
 template <typename A, int NS, int NJ>
-__global__ void __launch_bounds__(NJ == 2 ? 256 : 1024, NJ == 2 ? 3 : 1) k_stream_step(const __grid_constant__ StreamStep p, int* err)
+__global__ void __launch_bounds__(NJ == 2 ? 256 : 1024, NJ == 2 ? 3 : 0) k_stream_step(const __grid_constant__ StreamStep p, int* err)
 {
     __shared__ float s_sum[32];
     pdl_launch_dependents();
@@ -87,9 +86,10 @@ static int launch_stream_step(const StreamStep& p, int T, cudaStream_t s)
 {
     int threads = (p.width_pad / 4 + 32 * NJ - 1) / (32 * NJ) * 32;
     if (threads > 1024) return latch(BPDQ_ERR_RANGE);
-    if (p.m.n <= 2) return launch_ordered(k_stream_step<A, 2, NJ>, T, threads, 0, s, p, device_error_flag());
-    if (p.m.n <= 4) return launch_ordered(k_stream_step<A, 4, NJ>, T, threads, 0, s, p, device_error_flag());
-    return launch_ordered(k_stream_step<A, kMaxStreams, NJ>, T, threads, 0, s, p, device_error_flag());
+    if constexpr (NJ == 2) return launch_ordered(k_stream_step<A, 4, NJ>, T, threads, 0, s, p, device_error_flag());
+    else if (p.m.n <= 2) return launch_ordered(k_stream_step<A, 2, NJ>, T, threads, 0, s, p, device_error_flag());
+    else if (p.m.n <= 4) return launch_ordered(k_stream_step<A, 4, NJ>, T, threads, 0, s, p, device_error_flag());
+    else return launch_ordered(k_stream_step<A, kMaxStreams, NJ>, T, threads, 0, s, p, device_error_flag());
 }
 
 int stream_step(const StreamStep& p, int T, bool act_bf16, cudaStream_t s)
@@ -97,7 +97,11 @@ int stream_step(const StreamStep& p, int T, bool act_bf16, cudaStream_t s)
     if (T < 1 || p.m.n < 1 || p.m.n > kMaxStreams || p.width < 1 || p.width_pad < p.width || p.width_pad % 4 || !p.x || (p.h && !p.norm_w) ||
         (p.table ? !p.tokens : !p.y))
         return latch(BPDQ_ERR_ARG);
-    if (p.width_pad > 1024 && p.width_pad <= 2048) return act_bf16 ? launch_stream_step<bf16, 2>(p, T, s) : launch_stream_step<float, 2>(p, T, s);
+    // Half the threads, each with the loads of two groups of columns in flight, for three and four streams of 1537 to 2048 columns and 500 to 2000 tokens: 2 to
+    // 10 % less there (four streams of 2048, us, one group, two: 300 tokens 5.5, 5.9; 700 8.3, 8.1; 1500 14.9, 13.7; 2400 32.3, 33.1).  On the other sides
+    // of these lines they are level or cost time: 8 streams of 1280, 300 tokens 5.8, 8.0; two streams of 1792, 3000 tokens 17.9, 19.2.
+    if (p.m.n >= 3 && p.m.n <= 4 && p.width_pad > 1536 && p.width_pad <= 2048 && T >= 500 && T <= 2000)
+        return act_bf16 ? launch_stream_step<bf16, 2>(p, T, s) : launch_stream_step<float, 2>(p, T, s);
     if (p.width_pad <= 4096) return act_bf16 ? launch_stream_step<bf16, 1>(p, T, s) : launch_stream_step<float, 1>(p, T, s);
     return act_bf16 ? launch_stream_step<bf16, 4>(p, T, s) : launch_stream_step<float, 4>(p, T, s);
 }
