@@ -584,9 +584,10 @@ int grouped_attention(const GroupedShape& p, const void* u, int ld_u, const void
     }
     // Larger tiles from about this context on, whatever the number of rows (us, tiles of 64 x 64, of 128 x 128; 16 heads on 4 of 128): 32 tokens of 32 keys
     // 9.4, 10.3; 64 of 64 10.0, 10.3; 96 of 96 12.5, 10.6; 17 of 3017 146, 60.  4 heads on 2 of 64: 96 of 96 10.3, 10.3; 200 of 200 14.5, 9.9.
+    // A chunk of up to 64 positions is one block there and a padded one here (100 tokens after 4000 in chunks of 64: 9.2, 10.2; of 80 13.5, 10.3; of 128 14.4, 10.3).
     // Never one token: its launches may be recorded and replayed at later positions, of which only the one in device memory is known; the maps of these
     // tiles end at `context`.
-    if (T > 1 && context >= 96 && context <= p.rows && (p.sink != 0) == (p.cap > 0.0f)) {      // every position in the row of its number
+    if (T > 1 && context >= 96 && (p.chunk == 0 || p.chunk > kKeyBlock) && context <= p.rows && (p.sink != 0) == (p.cap > 0.0f)) {      // every position in the row of its number
         PromptAttention a = {};
         a.T = T; a.context = context; a.pos = pos;
         a.groups = p.groups; a.share = p.share();

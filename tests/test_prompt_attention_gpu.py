@@ -40,6 +40,13 @@ def test_grouped(lib, T, pos, H, G, D, V, chunk, cap, sink):
     vuzelix.attention_case(Known(lib, T, pos + T), 1, T, pos, H, G, D, V, chunk, cap=cap, sink=sink)
 
 
+# chunks just longer than those that stay on the smaller tiles, and about as long as a block
+@pytest.mark.parametrize("T,pos,H,G,D,V,chunk", [(130, 5, 2, 1, 128, 128, 65), (40, 90, 4, 1, 64, 192, 80), (90, 300, 4, 2, 192, 64, 100), (300, 11, 4, 2, 64, 64, 127), (70, 260, 16, 1, 60, 60, 129)])
+@pytest.mark.parametrize("cap,sink", [(14.0, 1), (0.0, 0)])
+def test_grouped_short_chunks(lib, T, pos, H, G, D, V, chunk, cap, sink):
+    test_grouped(lib, T, pos, H, G, D, V, chunk, cap, sink)
+
+
 class ShortPortions(VuzelixSpec):
     portion = 128           # a cache of chunk + 128 rows
 
