@@ -551,9 +551,12 @@ static int launch_tc5(const Linear& l, int T, Tc5Tiles t, cudaStream_t s)
 }
 
 // Tokens of a tile (a multiple of 16), ranges of K and CTAs of a tile with the least time in cycles: waves of CTAs over the SMs times a tile's K blocks, each
-// 310 + 1.3 per token (measured: 325 at 16 tokens, 650 at 256); K is cut, into ranges of at least four blocks, where all its tiles' clusters
-// run at once, and joining r ranges costs 3000 + 800 r + 25 per token.  2048 rows of 10752 (us, one range, several): 48 tokens 33.5, 14.2 at
-// six; 200 tokens 33.9, 19.0 at four; of 2048: 16 tokens 8.8, 7.3 at four; 200 tokens 9.2, 9.3.
+// 310 + 1.3 per token; K is cut, into ranges of at least four blocks, where all its tiles' clusters run at once, and joining r ranges costs
+// 3000 + 800 r + 25 per token.  168 K blocks of 2048 rows take 28.2 us at 16 tokens a tile, 29.7 at 128, 36.5 at 160, 53.4 at 256 (320, 340, 415, 605 cycles a
+// block: the estimate, which was fitted to one copying thread and eight epilogue warps, is high around 128 tokens).  Over 37 shapes of 5 to 4096 tokens
+// its tiles are within 4 % of the best ones, but for 128 tokens of 4096 x 4096 (12.3 us, 11.2 possible) and 400 of 1024 x 4096 (11.7, 11.0).
+// 2048 rows of 10752 (us, one range, several): 48 tokens 28.7, 11.5 at six; 200 tokens 29.2, 16.8 at four; of 2048: 16 tokens 8.2, 6.9 at four; 200 tokens
+// 8.5, 8.7 at two.
 static Tc5Tiles tc5_tiles(const Linear& l, int T)
 {
     const int n_tiles = (l.N + kTc5Rows - 1) / kTc5Rows, top = (T + 15) / 16 * 16 < 256 ? (T + 15) / 16 * 16 : 256;
@@ -570,9 +573,8 @@ static Tc5Tiles tc5_tiles(const Linear& l, int T)
         }
     }
     // A pair has 256 rows to a tile and fetches a third less per product; a K block takes 180 + 1.65 per token (168 of 2048 rows, 700 tokens, us: 128
-    // tokens a tile 39, 192 47, 256 58).  Setting it up costs more than one CTA, so only wide tiles and several waves.  Prompts through four layers
-    // of the hybrid decoder (us, single CTAs, pairs): 2048 tokens 1481, 1447; 900 835, 791; two layers of width 1024, 400 tokens, with pairs of any
-    // tile 248, 264.
+    // tokens a tile 36, 192 43, 256 56).  Setting it up costs more than one CTA, so only wide tiles and several waves: us, best single CTAs, pairs:
+    // 2048 tokens of 10752 x 2048 82.8, 79.8; of 21504 x 2048 165, 157; 1024 of 14336 x 4096 115, 105; 2048 of 2048 x 2048 15.7, 17.8.
     const int pairs = sms / 2, row_pairs = (l.N + 2 * kTc5Rows - 1) / (2 * kTc5Rows);
     for (int bn = 192; bn <= top; bn += 32) {
         const long waves = ((long)row_pairs * ((T + bn - 1) / bn) + pairs - 1) / pairs;
@@ -614,7 +616,7 @@ int linear_forward(const Linear& l, int T, bool act_bf16, cudaStream_t s)
         return launch_ordered(k_linear_tile<4>, dim3(n_tiles, (T + 63) / 64), 256, 0, s, l, T);
     }
     const Tc5Tiles t = tc5_tiles(l, T);
-    if (t.ctas == 2) return t.tokens > 128 ? launch_tc5<256, true>(l, T, t, s) : launch_tc5<128, true>(l, T, t, s);
+    if (t.ctas == 2) return launch_tc5<256, true>(l, T, t, s);
     if (t.tokens > 128) return launch_tc5<256, false>(l, T, t, s);
     if (t.tokens > 64) return launch_tc5<128, false>(l, T, t, s);
     if (t.tokens > 32) return launch_tc5<64, false>(l, T, t, s);
