@@ -310,14 +310,15 @@ __device__ __forceinline__ float transposed_sum(float (&v)[32], int lane)
 // grid (heads, chunks); tokens t0 .. t1 - 1, those beyond count as zeros that neither decay nor write.  A thread per key (rounded up to whole warps)
 // and as many again for the value columns.  Bound by latency: a CTA goes through a chain of some thousand instructions.  A and P are sums over
 // the keys: a warp takes whole columns of both, four keys per lane, from k, q and the decays in shared memory, so that a column
-// is added up across lanes once.  (With the sums of its own 32 keys of all columns in every warp, and the value columns after the keys in the
-// same threads: 16 heads of 128 x 128, 64 tokens, with the kernel below 22 us, now 20; 1500 tokens of a decoder with two such layers 1240, now 1227.)
+// is added up across lanes once.  16 heads of 128 x 128, 64 tokens, with the kernel below: 15.6 us; with the sums of its own 32 keys of all columns in every
+// warp and the value columns after the keys in the same threads 15.9; with lengths that scale the finished sums 15.1, but NaN where a square length
+// leaves fp32.
 template <int kThreads, int kBlocks>
 __global__ void __launch_bounds__(kThreads, kBlocks) k_delta_prepare(DeltaRule a, uint8_t* frags, float* updates, int t0, int t1)
 {
     extern __shared__ __align__(16) uint8_t sf[];     // k, q, decays [token][key]; then the chunk's fragments
     __shared__ float4 sA[kChunk][4], sP[kChunk][4];
-    __shared__ float s_norm[2 * kChunk], s_beta[kChunk];
+    __shared__ float s_norm[kThreads / 64][2 * kChunk], s_beta[kChunk];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
     const int h = blockIdx.x, gr = h / (a.heads / a.groups), first = t0 + blockIdx.y * kChunk, left = t1 - first;
     const int D = a.key_pad, V = a.value_pad, n = tid, values = blockDim.x >> 1;      // first thread of the value columns
@@ -340,25 +341,42 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_delta_prepare(DeltaRule a
             g[i] = i < rows ? pd[i * step] : 0.0f;
         }
         if (tid < kChunk) s_beta[tid] = first + tid < t1 ? a.beta[(size_t)(first + tid) * a.heads + h] : 0.0f;
+        // unit lengths ahead of every product: whatever a square length is, products of two unit vectors are at most 1 (an infinite one leaves zeros)
+        float v[32];
+#pragma unroll
+        for (int i = 0; i < kChunk; i++) {
+            v[i] = k[i] * k[i];
+            v[kChunk + i] = q[i] * q[i];
+        }
+        s_norm[warp][lane] = transposed_sum(v, lane);
         float* to = reinterpret_cast<float*>(sf) + n;
 #pragma unroll
         for (int i = 0; i < kChunk; i++)
+            if (key) to[(2 * kChunk + i) * D] = expf(g[i]);
+        named_bar_sync(1, values);
+        float sum = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kThreads / 64; w++) sum += 32 * w < values ? s_norm[w][lane] : 0.0f;
+        const float unit = (lane < kChunk ? 1.0f : a.q_scale) / sqrtf(sum + a.unit_eps);      // a lane per token: of its k, of its q
+#pragma unroll
+        for (int i = 0; i < kChunk; i++) {
+            const float ku = k[i] * __shfl_sync(0xFFFFFFFFu, unit, i), qu = q[i] * __shfl_sync(0xFFFFFFFFu, unit, kChunk + i);
             if (key) {
-                to[i * D] = k[i];
-                to[(kChunk + i) * D] = q[i];
-                to[(2 * kChunk + i) * D] = expf(g[i]);
+                to[i * D] = ku;
+                to[(kChunk + i) * D] = qu;
             }
+        }
     } else {
         const int p = tid - values;
 #pragma unroll
         for (int i = 0; i < kChunk; i++) x[i] = i < left && p < V ? act_load(pv + i * a.ld + p) : 0.0f;
     }
     __syncthreads();
-    // column m of P and A at distance d from the diagonal (A's diagonal: the key's square length); a long column and a short one to each warp
+    // column m of P and A at distance d from the diagonal (A has none on it); a long column and a short one to each warp
     for (int pass = 0; pass * warps < kChunk; pass++) {
         const int m = pass * warps + (pass & 1 ? warps - 1 - warp : warp);
         if (m >= kChunk) continue;
-        float v[32], qq = 0.0f;
+        float v[32];
 #pragma unroll
         for (int d = 0; d < 32; d++) v[d] = 0.0f;
         for (int n4 = 4 * lane; n4 < D; n4 += 128) {
@@ -370,40 +388,30 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_delta_prepare(DeltaRule a
                 const float4 kk = *reinterpret_cast<const float4*>(col + d * D), qv = *reinterpret_cast<const float4*>(col + (kChunk + d) * D);
                 if (d == 0) {
                     r = kk;
-                    qq = fmaf(qv.x, qv.x, qq); qq = fmaf(qv.y, qv.y, qq); qq = fmaf(qv.z, qv.z, qq); qq = fmaf(qv.w, qv.w, qq);
                 } else {
                     const float4 f = *reinterpret_cast<const float4*>(col + (2 * kChunk + d) * D);
                     r = make_float4(r.x * f.x, r.y * f.y, r.z * f.z, r.w * f.w);
                 }
                 v[d] = fmaf(qv.x, r.x, v[d]); v[d] = fmaf(qv.y, r.y, v[d]); v[d] = fmaf(qv.z, r.z, v[d]); v[d] = fmaf(qv.w, r.w, v[d]);
+                if (d == 0) continue;
                 float& w = v[kChunk + d];
                 w = fmaf(kk.x, r.x, w); w = fmaf(kk.y, r.y, w); w = fmaf(kk.z, r.z, w); w = fmaf(kk.w, r.w, w);
             }
         }
         const float sum = transposed_sum(v, lane);
-        qq = warp_sum(qq);
         const int i = m + (lane & (kChunk - 1));
         if (i < kChunk) {
             if (lane < kChunk) reinterpret_cast<float*>(sP)[i * kChunk + m] = sum;
-            else if (i > m) reinterpret_cast<float*>(sA)[i * kChunk + m] = sum;
-            else { s_norm[m] = sum; s_norm[kChunk + m] = qq; }
+            else if (i > m) reinterpret_cast<float*>(sA)[i * kChunk + m] = sum * s_beta[i];
         }
-    }
-    __syncthreads();
-    const float unit = (lane < kChunk ? 1.0f : a.q_scale) / sqrtf(s_norm[lane] + a.unit_eps);      // a lane per token: of its k, of its q
-    for (int c = tid; c < kChunk * kChunk; c += blockDim.x) {
-        const int i = c >> 4, j = c & (kChunk - 1);
-        const float ki = __shfl_sync(0xFFFFFFFFu, unit, i), kj = __shfl_sync(0xFFFFFFFFu, unit, j), qi = __shfl_sync(0xFFFFFFFFu, unit, kChunk + i);
-        if (j < i) reinterpret_cast<float*>(sA)[c] *= s_beta[i] * ki * kj;
-        if (j <= i) reinterpret_cast<float*>(sP)[c] *= qi * kj;
     }
     float k[kChunk], q[kChunk], g[kChunk];
     if (tid < values) {
         const float* from = reinterpret_cast<const float*>(sf) + (key ? n : 0);
 #pragma unroll
         for (int i = 0; i < kChunk; i++) {
-            k[i] = from[i * D] * __shfl_sync(0xFFFFFFFFu, unit, i);
-            q[i] = from[(kChunk + i) * D] * __shfl_sync(0xFFFFFFFFu, unit, kChunk + i);
+            k[i] = from[i * D];
+            q[i] = from[(kChunk + i) * D];
             g[i] = from[(2 * kChunk + i) * D];
         }
     }
