@@ -191,6 +191,8 @@ SIGNATURES = {
     "bpdq_hybrid_destroy": (None, [vp]),
     "bpdq_hybrid_forward": (i32, [vp, vp, i32, i32, vp, vp, i32, vp, i32, vp]),
     "bpdq_hybrid_step": (i32, [vp, vp, i32, i32, vp, vp, i32, vp, vp, i32, vp]),
+    "bpdq_hybrid_forget": (None, [vp, vp, sz]),
+    "bpdq_hybrid_recordings": (i32, [vp]),
     "bpdq_hybrid_logits": (vp, [vp]),
     "bpdq_hybrid_picked": (vp, [vp]),
     "bpdq_hybrid_scratch_bytes": (sz, [vp]),

@@ -25,7 +25,6 @@
 #include <cstring>
 #include <map>
 #include <new>
-#include <utility>
 #include <vector>
 
 namespace bpdq {
@@ -76,7 +75,8 @@ __global__ void __launch_bounds__(256) k_step_inputs(const __grid_constant__ Ste
 }
 constexpr int kFewInputs = 4, kManyInputs = 4096;       // (16 KB of arguments; 32 KB are the limit)
 
-// grid (1 + slices, rows): the first CTA of a row finds its largest logit (the lowest index of equal ones), the others bring the row to the host.
+// grid (1 + slices, rows): the first CTA of a row finds its largest logit (the lowest index of equal ones; host_picked null: for the device alone), the others
+// bring the row to the host.
 constexpr int kEmitThreads = 1024, kEmitSlice = 4 * kEmitThreads;
 __global__ void __launch_bounds__(kEmitThreads) k_emit_rows(const float* logits, long long* picked, float* host_logits, long long* host_picked, int vocab)
 {
@@ -85,7 +85,10 @@ __global__ void __launch_bounds__(kEmitThreads) k_emit_rows(const float* logits,
     const float* row = logits + (size_t)blockIdx.y * vocab;
     if (blockIdx.x == 0) {
         const int best = argmax_of_row(row, vocab);
-        if (threadIdx.x == 0) picked[blockIdx.y] = host_picked[blockIdx.y] = best;
+        if (threadIdx.x == 0) {
+            picked[blockIdx.y] = best;
+            if (host_picked) host_picked[blockIdx.y] = best;
+        }
         return;
     }
     const int at = (blockIdx.x - 1) * kEmitSlice + 4 * threadIdx.x;
@@ -125,12 +128,17 @@ struct Plan {
     Buffers* last = nullptr;                        // holds the results of the last call
     struct Recorded {
         cudaGraphExec_t exec;
-        cudaGraph_t graph;                          // (what `inputs` belongs to)
-        cudaGraphNode_t inputs;                     // its k_step_inputs
+        cudaGraph_t graph;                          // (what the nodes belong to)
+        cudaGraphNode_t inputs, results;            // its k_step_inputs and k_emit_rows
+        int emit;                                   // where the results go at present ..
+        const void* staged;                         // .. and the staging memory that has them
+        unsigned long long idle;                    // 0, or when its state went: the next state at the address takes it over
     };
-    std::map<std::pair<void*, int>, Recorded> graphs;        // by state base and where the results go
+    unsigned long long idlings = 0;
+    std::map<void*, Recorded> graphs;               // by state base
     Staging staging;
 };
+constexpr int kIdleRecordings = 8;      // of states that have gone: an engine that follows another often gets its memory
 // Where the results of a step go besides the device: nowhere, or through `staging` (logits too, or the choices alone).
 enum { kEmitNone, kEmitPicked, kEmitAll };
 
@@ -254,17 +262,12 @@ void forget(const Plan::Recorded& r)
     check_cuda(cudaGraphDestroy(r.graph));
 }
 
-// (a step that stages has waited for its results, so nothing writes here between steps; recorded steps know the address)
+// (a step that stages has waited for its results, so nothing writes here between steps; recorded steps are told where it is)
 int make_staging(Plan& p, size_t need)
 {
     if (need <= p.staging.bytes) return 0;
     int rc;
     if (p.staging.base) {
-        for (auto it = p.graphs.begin(); it != p.graphs.end();) {
-            if (it->first.second == kEmitNone) { ++it; continue; }
-            forget(it->second);
-            it = p.graphs.erase(it);
-        }
         rc = check_cuda(cudaFreeHost(p.staging.base));
         p.staging = Staging{};
         if (rc) return rc;
@@ -275,6 +278,24 @@ int make_staging(Plan& p, size_t need)
     p.staging.bytes = need;
     return 0;
 }
+
+// A launch of k_emit_rows: arguments that live as long as this does.
+struct Emission {
+    const float* logits;
+    long long* picked;
+    float* host_logits;
+    long long* host_picked;
+    int vocab;
+    dim3 grid;
+    void* args[5] = {&logits, &picked, &host_logits, &host_picked, &vocab};
+
+    Emission(const Plan& p, const Buffers& b, int n_want, int emit)
+        : logits(b.logits), picked(b.picked), host_logits(emit == kEmitAll ? staged_logits(p.staging, n_want) : nullptr),
+          host_picked(emit == kEmitNone ? nullptr : (long long*)p.staging.base), vocab(p.cfg.vocab),
+          grid(1 + (emit == kEmitAll ? (unsigned)((p.cfg.vocab + kEmitSlice - 1) / kEmitSlice) : 0u), (unsigned)n_want)
+    {
+    }
+};
 
 // Makes room for a call.  Buffers are laid out anew for every call's sizes (what depends on the number of tokens, like
 // the number of key splits, is then as that call needs it) and the memory only grows.
@@ -306,6 +327,7 @@ struct Runner {
     uint8_t* state;
     cudaStream_t s;
     int emit;
+    bool recording;
 
     void* at(void* base, size_t elements) const { return (uint8_t*)base + elements * (p.bf16_acts ? 2 : 4); }
 
@@ -602,10 +624,9 @@ struct Runner {
             head.cap = p.cfg.logit_cap;
             if ((rc = linear_forward(head, vec ? 1 : n_want, p.bf16_acts, s))) return rc;
         }
-        if (emit == kEmitNone) return bpd_argmax_dim_cuda(b.logits, b.picked, n_want, p.cfg.vocab, 1, s);
-        const unsigned slices = emit == kEmitAll ? (unsigned)((p.cfg.vocab + kEmitSlice - 1) / kEmitSlice) : 0u;
-        return launch_ordered(k_emit_rows, dim3(1 + slices, (unsigned)n_want), kEmitThreads, 0, s, (const float*)b.logits, b.picked,
-                              staged_logits(p.staging, n_want), (long long*)p.staging.base, p.cfg.vocab);
+        if (emit == kEmitNone && !recording) return bpd_argmax_dim_cuda(b.logits, b.picked, n_want, p.cfg.vocab, 1, s);
+        const Emission e(p, b, n_want, emit);
+        return launch_ordered(k_emit_rows, e.grid, kEmitThreads, 0, s, e.logits, e.picked, e.host_logits, e.host_picked, e.vocab);
     }
 };
 
@@ -686,10 +707,23 @@ int forward(Plan* p, const int32_t* token_ids, int n_tokens, int pos, void* stat
     else if (!b.base) rc = make_room(*p, b, 1, 1, 1, s);
     if (rc) return rc;
     p->last = &b;
-    Runner r{*p, b, n_tokens, pos + n_tokens, (uint8_t*)state, s, emit};
+    Runner r{*p, b, n_tokens, pos + n_tokens, (uint8_t*)state, s, emit, false};
     const bool recorded = single && use_graph && !residuals && n_want;
-    const auto it = recorded ? p->graphs.find({state, emit}) : p->graphs.end();
+    const auto it = recorded ? p->graphs.find(state) : p->graphs.end();
     if (it != p->graphs.end()) {
+        Plan::Recorded& made = it->second;
+        made.idle = 0;
+        if (made.emit != emit || made.staged != p->staging.base) {
+            Emission e(*p, b, 1, emit);
+            cudaKernelNodeParams k = {};
+            k.func = (void*)k_emit_rows;
+            k.gridDim = e.grid;
+            k.blockDim = dim3(kEmitThreads);
+            k.kernelParams = e.args;
+            if ((rc = check_cuda(cudaGraphExecKernelNodeSetParams(made.exec, made.results, &k)))) return rc;
+            made.emit = emit;
+            made.staged = p->staging.base;
+        }
         const StepInputs<kFewInputs> in = {{pos, token_ids[0]}};
         int one = 1, none = 0;
         void* args[] = {(void*)&in, &b.ids, &b.pos, &b.want, &one, &none};
@@ -698,8 +732,8 @@ int forward(Plan* p, const int32_t* token_ids, int n_tokens, int pos, void* stat
         k.gridDim = dim3(1);
         k.blockDim = dim3(256);
         k.kernelParams = args;
-        if ((rc = check_cuda(cudaGraphExecKernelNodeSetParams(it->second.exec, it->second.inputs, &k)))) return rc;
-        return check_cuda(cudaGraphLaunch(it->second.exec, s));
+        if ((rc = check_cuda(cudaGraphExecKernelNodeSetParams(made.exec, made.inputs, &k)))) return rc;
+        return check_cuda(cudaGraphLaunch(made.exec, s));
     }
     const int n_places = all ? 0 : n_want;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
@@ -722,18 +756,27 @@ int forward(Plan* p, const int32_t* token_ids, int n_tokens, int pos, void* stat
     if ((rc = r.run(nullptr, 1, true))) return latch(rc);
     if ((rc = check_cuda(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)))) return rc;
     int run_rc = send_inputs<kFewInputs>(b, token_ids, 1, pos, want, 0, s);
+    r.recording = true;
     if (!run_rc) run_rc = r.run(nullptr, 1, true);
-    cudaGraph_t g = nullptr;
-    rc = check_cuda(cudaStreamEndCapture(s, &g));
-    Plan::Recorded made = {nullptr, g, nullptr};
+    Plan::Recorded made = {nullptr, nullptr, nullptr, nullptr, emit, p->staging.base, 0};
+    // the launch that the next one would wait for is the last, k_emit_rows
+    cudaStreamCaptureStatus state_of;
+    const cudaGraphNode_t* ends = nullptr;
+    const cudaGraphEdgeData* edges = nullptr;
+    size_t n_ends = 0;
+    if (!run_rc && !(run_rc = check_cuda(cudaStreamGetCaptureInfo_v3(s, &state_of, nullptr, nullptr, &ends, &edges, &n_ends)))) {
+        if (n_ends == 1) made.results = ends[0];
+        else run_rc = BPDQ_ERR_CUDA;
+    }
+    rc = check_cuda(cudaStreamEndCapture(s, &made.graph));
     size_t roots = 1;
-    if (!run_rc && !rc && g) rc = check_cuda(cudaGraphGetRootNodes(g, &made.inputs, &roots));
-    if (!run_rc && !rc && roots == 1) rc = check_cuda(cudaGraphInstantiate(&made.exec, g, 0));
+    if (!run_rc && !rc && made.graph) rc = check_cuda(cudaGraphGetRootNodes(made.graph, &made.inputs, &roots));
+    if (!run_rc && !rc && roots == 1) rc = check_cuda(cudaGraphInstantiate(&made.exec, made.graph, 0));
     if (run_rc || rc || !made.exec) {
-        if (g) cudaGraphDestroy(g);
+        if (made.graph) cudaGraphDestroy(made.graph);
         return latch(run_rc ? run_rc : rc ? rc : BPDQ_ERR_CUDA);
     }
-    p->graphs[{state, emit}] = made;
+    p->graphs[state] = made;
     return 0;
 }
 
@@ -809,6 +852,27 @@ int bpdq_hybrid_step(void* plan, const int32_t* token_ids, int n_tokens, int pos
     }
     return 0;
 }
+
+void bpdq_hybrid_forget(void* plan, const void* state, size_t bytes)
+{
+    Plan* p = (Plan*)plan;
+    if (!p) return;
+    for (auto& g : p->graphs)
+        if ((uintptr_t)g.first - (uintptr_t)state < bytes && !g.second.idle) g.second.idle = ++p->idlings;
+    for (;;) {
+        auto oldest = p->graphs.end();
+        int idle = 0;
+        for (auto it = p->graphs.begin(); it != p->graphs.end(); ++it) {
+            if (!it->second.idle) continue;
+            idle++;
+            if (oldest == p->graphs.end() || it->second.idle < oldest->second.idle) oldest = it;
+        }
+        if (idle <= kIdleRecordings) return;
+        forget(oldest->second);
+        p->graphs.erase(oldest);
+    }
+}
+int bpdq_hybrid_recordings(void* plan) { return plan ? (int)((Plan*)plan)->graphs.size() : 0; }
 
 float* bpdq_hybrid_logits(void* plan)
 {

@@ -1,8 +1,8 @@
 """Generation: sequences of a model in slots, prompts in portions, one token per step after that.
 
 A model brings ``state_parts()``, ``capacity``, ``vocab``, ``stream``, ``lib`` and
-``step(seq, tokens, want, logits)``, and ``portion`` if a step takes no more tokens than that; the engine is
-the same for every family.  A step runs one sequence:
+``step(seq, tokens, want, logits)``, ``portion`` if a step takes no more tokens than that, and ``forget(base, nbytes)`` if it keeps
+anything by a state's address; the engine is the same for every family.  A step runs one sequence:
 the next portion of its prompt or its last token.  Live requests take turns.
 """
 from collections import deque
@@ -105,4 +105,7 @@ class Engine:
         return [r.output for r in self.run([Request(list(p), max_new_tokens, frozenset(stop)) for p in prompts])]
 
     def close(self):
-        self.slots.close()
+        block, nbytes = self.slots.block, self.slots.nbytes
+        self.slots.close()              # (which waits for what the device has been given)
+        if block and hasattr(self.model, "forget"):
+            self.model.forget(block, nbytes)

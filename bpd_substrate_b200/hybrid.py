@@ -411,6 +411,11 @@ class DeviceHybrid:
     def state_parts(self):
         return self.parts
 
+    def forget(self, base, nbytes):
+        """The states that were in this memory are gone, and no step on them is under way: few of their recordings are kept."""
+        if self.plan:           # (a model may be closed before its engine)
+            self.lib.bpdq_hybrid_forget(self.plan, base, nbytes)
+
     def _inputs(self, seq, tokens, want):
         tokens = np.ascontiguousarray(tokens, np.int32)
         want = np.ascontiguousarray(want, np.int32)
@@ -459,6 +464,7 @@ class DeviceHybrid:
     def close(self):
         self.lib.bpdq_stream_sync(self.stream)
         self.lib.bpdq_hybrid_destroy(self.plan)
+        self.plan = None
         for p in self._allocs:
             self.lib.bpdq_free(p)
         self._allocs = []

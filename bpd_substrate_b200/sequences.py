@@ -59,9 +59,10 @@ class SequenceSlots:
         self.parts = list(parts)
         self.layout = lay_out(self.parts, capacity)
         self.zero_bytes = sum(p.size(capacity) for p in self.parts if p.zero)
-        self.block = lib.bpdq_alloc(self.layout.slot_bytes * slots)
+        self.nbytes = self.layout.slot_bytes * slots
+        self.block = lib.bpdq_alloc(self.nbytes)
         if not self.block:
-            raise MemoryError(f"device allocation of {self.layout.slot_bytes * slots} bytes for {slots} sequences failed")
+            raise MemoryError(f"device allocation of {self.nbytes} bytes for {slots} sequences failed")
         self.free = list(range(slots))
 
     def acquire(self):

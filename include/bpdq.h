@@ -582,6 +582,10 @@ int bpdq_hybrid_forward(void* plan, const int32_t* token_ids, int n_tokens, int 
  * pass through pinned memory that the plan keeps. */
 int bpdq_hybrid_step(void* plan, const int32_t* token_ids, int n_tokens, int pos, void* state, const int32_t* want, int n_want, float* logits,
                      long long* picked, int use_graph, void* stream);
+/* One-token steps are recorded once per state address, whatever results are asked for.  bpdq_hybrid_forget: the states in [state, state + bytes) have gone, and
+ * none of their steps is under way; of such addresses' recordings the plan keeps the last eight, for the states that may follow there. */
+void bpdq_hybrid_forget(void* plan, const void* state, size_t bytes);
+int bpdq_hybrid_recordings(void* plan);
 float* bpdq_hybrid_logits(void* plan);                /* device [n_want][vocab] */
 void* bpdq_hybrid_picked(void* plan);                 /* device int64 [n_want] */
 size_t bpdq_hybrid_scratch_bytes(void* plan);

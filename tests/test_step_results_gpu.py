@@ -89,3 +89,45 @@ def test_recorded_by_the_caller(lib, places):
     e.close()
     m.close()
     lib.bpdq_stream_destroy(s)
+
+
+def test_one_recording_per_slot(lib):
+    """Whatever is asked of a slot's one-token steps, and wherever the pinned memory lies, one recording gives the bits of launched steps; few outlive the
+    engine's slots."""
+    cfg = hm.config(5000, 64, [hm.layer("retention", hm.retention(2, 16, 16, 16, [0.5, 0.98]), 33), hm.layer("latent_attention", hm.latent(2, 16, 8, 16, 24, 20, 0.3))])
+    w, toks = hm.weights(cfg, 5), hm.tokens(cfg, 40, 6)
+    m, plain = (hybrid.device(cfg, w, lib, "bfloat16", capacity=64, use_graph=g) for g in (True, False))
+    e, f = Engine(m, slots=2), Engine(plain, slots=2)
+    held = [(e.slots.acquire(), f.slots.acquire()) for _ in range(2)]
+    for t in range(24):
+        a, b = held[t % 5 % 2]
+        ref = plain.step(b, toks[t:t + 1], [0])
+        if t % 3 == 0:
+            got = on_device(m, a, toks[t:t + 1], [0])
+        else:
+            got = m.step(a, toks[t:t + 1], [0], t % 3 == 1)
+        assert np.array_equal(got[1], ref[1]) and (got[0] is None or np.array_equal(got[0].view(np.uint32), ref[0].view(np.uint32))), t
+        if t == 10:         # the pinned memory grows under both recordings
+            for s in held:
+                assert np.array_equal(*(x.step(q, toks[24:40], range(16))[0] for x, q in zip((m, plain), s)))
+        assert lib.bpdq_hybrid_recordings(m.plan) <= 2
+    assert lib.bpdq_hybrid_recordings(m.plan) == 2 and lib.bpdq_hybrid_recordings(plain.plan) == 0
+    e.close()
+    # recordings of slots that have gone: a few wait for the next engine, as many engines as there are
+    many = [Engine(m, slots=7) for _ in range(3)]
+    for i, other in enumerate(many):
+        for k in range(7):
+            other.feed(k, toks[:1], [0])
+    assert lib.bpdq_hybrid_recordings(m.plan) <= 21 + 2
+    for other in many:
+        other.close()
+    assert lib.bpdq_hybrid_recordings(m.plan) == 8
+    f.slots.release(held[0][1])
+    again = Engine(m, slots=7)          # (at one of their addresses, or not)
+    for x, y in zip([again.feed("x", toks[t:t + 1], [0]) for t in range(4)], [f.feed("x", toks[t:t + 1], [0]) for t in range(4)]):
+        assert np.array_equal(x[0], y[0]) and np.array_equal(x[1], y[1])
+    again.close()
+    assert lib.bpdq_hybrid_recordings(m.plan) == 8 and lib.bpdq_last_status() == 0
+    m.close()
+    plain.close()
+    f.close()               # (after its model)
