@@ -20,6 +20,7 @@
 #include "latent_attention.cuh"
 #include "launch.cuh"
 #include "residual_streams.cuh"
+#include "staging.h"
 #include "../../include/bpdq.h"
 
 #include <cstring>
@@ -102,12 +103,8 @@ __global__ void __launch_bounds__(kEmitThreads) k_emit_rows(const float* logits,
 
 namespace {
 
-// Pinned memory that a step's results pass through, at most kMaxStaging bytes per plan.
+// Pinned memory that a step's results pass through, at most so many bytes per plan.
 constexpr size_t kMaxStaging = 8u << 20;
-struct Staging {
-    uint8_t* base = nullptr;
-    size_t bytes = 0;
-};
 
 struct Buffers {
     uint8_t* base = nullptr;
@@ -262,21 +259,19 @@ void forget(const Plan::Recorded& r)
     check_cuda(cudaGraphDestroy(r.graph));
 }
 
-// (a step that stages has waited for its results, so nothing writes here between steps; recorded steps are told where it is)
-int make_staging(Plan& p, size_t need)
+// Whether there is pinned memory for that much.  (A step that stages has waited for its results, so nothing writes here between steps; recorded steps are told
+// where it is.)
+bool make_staging(Plan& p, size_t need)
 {
-    if (need <= p.staging.bytes) return 0;
-    int rc;
-    if (p.staging.base) {
-        rc = check_cuda(cudaFreeHost(p.staging.base));
-        p.staging = Staging{};
-        if (rc) return rc;
-    }
-    void* m = nullptr;
-    if ((rc = check_cuda(cudaHostAlloc(&m, need, cudaHostAllocDefault)))) return rc;
-    p.staging.base = (uint8_t*)m;
-    p.staging.bytes = need;
-    return 0;
+    return p.staging.reserve(
+        need,
+        [](size_t n) {
+            void* m = nullptr;
+            if (cudaHostAlloc(&m, n, cudaHostAllocDefault) == cudaSuccess) return m;
+            (void)cudaGetLastError();       // (the step has another way)
+            return (void*)nullptr;
+        },
+        [](void* m) { check_cuda(cudaFreeHost(m)); });
 }
 
 // A launch of k_emit_rows: arguments that live as long as this does.
@@ -836,10 +831,8 @@ int bpdq_hybrid_step(void* plan, const int32_t* token_ids, int n_tokens, int pos
     cudaStream_t s = (cudaStream_t)stream;
     if (!p || (n_want > 0 && !picked)) return latch(BPDQ_ERR_ARG);
     int emit = kEmitNone, rc;
-    if (n_want > 0 && n_want <= n_tokens && n_want <= 65535 && staged_bytes(n_want, p->cfg.vocab, logits != nullptr) <= kMaxStaging) {
-        if ((rc = make_staging(*p, staged_bytes(n_want, p->cfg.vocab, logits != nullptr)))) return latch(rc);
-        emit = logits ? kEmitAll : kEmitPicked;
-    }
+    const size_t staged = n_want > 0 ? staged_bytes(n_want, p->cfg.vocab, logits != nullptr) : 0;
+    if (n_want > 0 && n_want <= n_tokens && n_want <= 65535 && staged <= kMaxStaging && make_staging(*p, staged)) emit = logits ? kEmitAll : kEmitPicked;
     if ((rc = forward(p, token_ids, n_tokens, pos, state, want, n_want, nullptr, use_graph, s, emit))) return rc;
     if (n_want > 0 && emit == kEmitNone) {
         if (logits && (rc = check_cuda(cudaMemcpyAsync(logits, p->last->logits, (size_t)n_want * p->cfg.vocab * 4, cudaMemcpyDeviceToHost, s)))) return rc;
