@@ -306,7 +306,8 @@ __global__ void __launch_bounds__(kSplitThreads) k_gqa_split(GqaShape p, GqaNew 
     cluster_wait();
     const int slice = (R * D + ranks - 1) / ranks;
     if (ranks >= 8 && slice <= 32) {
-        // few results per CTA: a warp takes some of the CTAs, a lane a result (one thread for a result, 16 CTAs: 2.0 us of 17)
+        // few results per CTA: a warp takes some of the CTAs, a lane a result (one thread for a result, 16 CTAs: 2.0 us of 17).  Sums per warp, then over the
+        // warps: last bits differ from one thread's
         __shared__ float s_join[3][kSplitWarps][32];
         const int i = rank * slice + lane;
         const bool own = lane < slice && i < R * D;

@@ -128,3 +128,19 @@ def test_short_prompts_of_unshared_fp32_heads(lib, T, off):
     q, k, v = inputs(T, off + T, 16, 16, 64, np.float32, T)
     got, want = attend(lib, q, k, v, off, np.float32(0.125), off + T), expected(q, k, v, off, 0.125, off + T)
     assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+
+
+# clusters of 8 and 16 CTAs: results joined by all warps (up to 32 per CTA) and by a thread each
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,off,H,HKV,D", [(1, 300, 4, 4, 64), (1, 511, 8, 4, 128), (1, 400, 8, 2, 64), (2, 300, 6, 2, 64), (1, 300, 8, 2, 128), (1, 513, 4, 4, 64), (1, 1500, 3, 1, 128), (1, 4000, 32, 8, 128),
+                                           (3, 600, 4, 2, 64)])
+@pytest.mark.parametrize("kind", [np.float16, np.float32])
+def test_joined_parts(lib, T, off, H, HKV, D, kind):
+    """Parts of a cluster whose maxima lie far apart, in one CTA's stretch, in every CTA's, and nowhere."""
+    q, k, v = inputs(T, off + T, H, HKV, D, kind, off)
+    scale = np.float32(D ** -0.5)
+    q[:, 0] = 0.0                                  # all keys alike
+    q[:, 1] *= 30.0                                # one key, somewhere
+    k[off // 3] = 4 * k[off // 3]                  # and one that many look at
+    got, want = attend(lib, q, k, v, off, scale, off + T), expected(q, k, v, off, float(scale), off + T)
+    assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()

@@ -1,5 +1,5 @@
 """One token of the Q8_0 Llama: the launches that hold several steps give the bits of the step-by-step forward, which a workspace without room for a second
-residual gets."""
+residual gets.  (Both share the attention's sums, which are compared with 64 bits where the attention is tested alone.)"""
 import ctypes as C
 
 import numpy as np

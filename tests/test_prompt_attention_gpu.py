@@ -47,6 +47,20 @@ def test_grouped_short_chunks(lib, T, pos, H, G, D, V, chunk, cap, sink):
     test_grouped(lib, T, pos, H, G, D, V, chunk, cap, sink)
 
 
+# values of several slices, rows of 64 and 128 heads of few tokens, one token (which stays where the position is read from the device)
+@pytest.mark.parametrize("T,pos,H,G,D,V", [(33, 150, 2, 1, 128, 320), (33, 100, 2, 1, 64, 512), (2, 150, 2, 1, 128, 320), (1, 150, 2, 1, 128, 320), (2, 130, 128, 1, 64, 64), (1, 130, 128, 1, 64, 64),
+                                           (2, 130, 64, 1, 128, 128), (1, 130, 64, 1, 128, 128)])
+@pytest.mark.parametrize("cap,sink", [(14.0, 1), (0.0, 0)])
+def test_grouped_many_columns_and_heads(lib, T, pos, H, G, D, V, cap, sink):
+    test_grouped(lib, T, pos, H, G, D, V, 0, cap, sink)
+
+
+# a portion that fills the cache's last row, and one that begins again at its first
+@pytest.mark.parametrize("T,pos,rows", [(100, 100, 200), (100, 100, 199), (100, 101, 200), (70, 260, 330), (70, 260, 300)])
+def test_grouped_at_the_end_of_the_rows(lib, T, pos, rows):
+    vuzelix.attention_case(Known(lib, T, pos + T), 1, T, pos, 4, 2, 64, 64, 80, rows)
+
+
 class ShortPortions(VuzelixSpec):
     portion = 128           # a cache of chunk + 128 rows
 
