@@ -20,7 +20,6 @@
 #include "latent_attention.cuh"
 #include "launch.cuh"
 #include "residual_streams.cuh"
-#include "staging.h"
 #include "../../include/bpdq.h"
 
 #include <cstring>
@@ -103,8 +102,14 @@ __global__ void __launch_bounds__(kEmitThreads) k_emit_rows(const float* logits,
 
 namespace {
 
-// Pinned memory that a step's results pass through, at most so many bytes per plan.
-constexpr size_t kMaxStaging = 8u << 20;
+// Pinned memory that a step's results pass through, made with the plan: room for one row of logits at least, if that is not too much, and for so many bytes.
+// Larger results are copied to the caller's memory (us per step of 32 tokens, rows of 32000 logits, staged and copied: 1 row 350, 390; 8 rows 415, 440; 16 rows
+// 525, 505).  It does not grow: new pinned memory takes milliseconds.
+constexpr size_t kStaging = 1u << 20, kMaxStaging = 8u << 20;
+struct Staging {
+    uint8_t* base = nullptr;
+    size_t bytes = 0;
+};
 
 struct Buffers {
     uint8_t* base = nullptr;
@@ -127,8 +132,7 @@ struct Plan {
         cudaGraphExec_t exec;
         cudaGraph_t graph;                          // (what the nodes belong to)
         cudaGraphNode_t inputs, results;            // its k_step_inputs and k_emit_rows
-        int emit;                                   // where the results go at present ..
-        const void* staged;                         // .. and the staging memory that has them
+        int emit;                                   // where the results go at present
         unsigned long long idle;                    // 0, or when its state went: the next state at the address takes it over
     };
     unsigned long long idlings = 0;
@@ -257,21 +261,6 @@ void forget(const Plan::Recorded& r)
 {
     check_cuda(cudaGraphExecDestroy(r.exec));
     check_cuda(cudaGraphDestroy(r.graph));
-}
-
-// Whether there is pinned memory for that much.  (A step that stages has waited for its results, so nothing writes here between steps; recorded steps are told
-// where it is.)
-bool make_staging(Plan& p, size_t need)
-{
-    return p.staging.reserve(
-        need,
-        [](size_t n) {
-            void* m = nullptr;
-            if (cudaHostAlloc(&m, n, cudaHostAllocDefault) == cudaSuccess) return m;
-            (void)cudaGetLastError();       // (the step has another way)
-            return (void*)nullptr;
-        },
-        [](void* m) { check_cuda(cudaFreeHost(m)); });
 }
 
 // A launch of k_emit_rows: arguments that live as long as this does.
@@ -708,7 +697,7 @@ int forward(Plan* p, const int32_t* token_ids, int n_tokens, int pos, void* stat
     if (it != p->graphs.end()) {
         Plan::Recorded& made = it->second;
         made.idle = 0;
-        if (made.emit != emit || made.staged != p->staging.base) {
+        if (made.emit != emit) {
             Emission e(*p, b, 1, emit);
             cudaKernelNodeParams k = {};
             k.func = (void*)k_emit_rows;
@@ -717,7 +706,6 @@ int forward(Plan* p, const int32_t* token_ids, int n_tokens, int pos, void* stat
             k.kernelParams = e.args;
             if ((rc = check_cuda(cudaGraphExecKernelNodeSetParams(made.exec, made.results, &k)))) return rc;
             made.emit = emit;
-            made.staged = p->staging.base;
         }
         const StepInputs<kFewInputs> in = {{pos, token_ids[0]}};
         int one = 1, none = 0;
@@ -753,7 +741,7 @@ int forward(Plan* p, const int32_t* token_ids, int n_tokens, int pos, void* stat
     int run_rc = send_inputs<kFewInputs>(b, token_ids, 1, pos, want, 0, s);
     r.recording = true;
     if (!run_rc) run_rc = r.run(nullptr, 1, true);
-    Plan::Recorded made = {nullptr, nullptr, nullptr, nullptr, emit, p->staging.base, 0};
+    Plan::Recorded made = {nullptr, nullptr, nullptr, nullptr, emit, 0};
     // the launch that the next one would wait for is the last, k_emit_rows
     cudaStreamCaptureStatus state_of;
     const cudaGraphNode_t* ends = nullptr;
@@ -803,6 +791,11 @@ void* bpdq_hybrid_create(const bpdq_hybrid_config* cfg, const bpdq_hybrid_layer*
             return nullptr;
         }
     }
+    // (where there is none to be had, all results are copied)
+    const size_t row = staged_bytes(1, cfg->vocab, true), bytes = row > kStaging && row <= kMaxStaging ? row : kStaging;
+    void* m = nullptr;
+    if (cudaHostAlloc(&m, bytes, cudaHostAllocDefault) == cudaSuccess) p->staging = {(uint8_t*)m, bytes};
+    else (void)cudaGetLastError();
     return p;
 }
 
@@ -832,7 +825,7 @@ int bpdq_hybrid_step(void* plan, const int32_t* token_ids, int n_tokens, int pos
     if (!p || (n_want > 0 && !picked)) return latch(BPDQ_ERR_ARG);
     int emit = kEmitNone, rc;
     const size_t staged = n_want > 0 ? staged_bytes(n_want, p->cfg.vocab, logits != nullptr) : 0;
-    if (n_want > 0 && n_want <= n_tokens && n_want <= 65535 && staged <= kMaxStaging && make_staging(*p, staged)) emit = logits ? kEmitAll : kEmitPicked;
+    if (n_want > 0 && n_want <= n_tokens && n_want <= 65535 && staged <= p->staging.bytes) emit = logits ? kEmitAll : kEmitPicked;
     if ((rc = forward(p, token_ids, n_tokens, pos, state, want, n_want, nullptr, use_graph, s, emit))) return rc;
     if (n_want > 0 && emit == kEmitNone) {
         if (logits && (rc = check_cuda(cudaMemcpyAsync(logits, p->last->logits, (size_t)n_want * p->cfg.vocab * 4, cudaMemcpyDeviceToHost, s)))) return rc;

@@ -578,8 +578,8 @@ void bpdq_hybrid_destroy(void* plan);
  * larger call moves the plan's buffers) every replay reads tokens and places from the caller's memory again; the position is the recorded one. */
 int bpdq_hybrid_forward(void* plan, const int32_t* token_ids, int n_tokens, int pos, void* state, const int32_t* want, int n_want,
                         float* residuals, int use_graph, void* stream);
-/* The same, then waits and brings the results to host memory: logits [n_want][vocab] (or NULL), picked [n_want].  Rows of up to 8 MB
- * pass through pinned memory that the plan keeps (larger ones, and all where there is none to be had, are copied). */
+/* The same, then waits and brings the results to host memory: logits [n_want][vocab] (or NULL), picked [n_want].  Results of up
+ * to 1 MB, and one row, pass through pinned memory that the plan keeps (larger ones, and all where there is none to be had, are copied). */
 int bpdq_hybrid_step(void* plan, const int32_t* token_ids, int n_tokens, int pos, void* state, const int32_t* want, int n_want, float* logits,
                      long long* picked, int use_graph, void* stream);
 /* One-token steps are recorded once per state address, whatever results are asked for.  bpdq_hybrid_forget: the states in [state, state + bytes) have gone, and

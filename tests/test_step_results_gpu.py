@@ -27,7 +27,7 @@ def test_results(lib, vocab):
     a, b = e.slots.acquire(), e.slots.acquire()
     toks = hm.tokens(cfg, 8300, 6)
     # inputs as one launch's arguments (3 and 4 words, 4096) or copied (4097 words and more); choices alone and logits; rows beyond the
-    # pinned memory (300 of 8193 logits); recorded one-token steps, the pinned memory having moved in between
+    # pinned memory (40 and 300 of 8193 logits); recorded one-token steps in between
     at = 0
     for n, want in [(2, [1]), (1, [0]), (1, [0]), (1, [0]), (3, range(3)), (4094, [4093]), (1, [0]), (4090, [5, 0, 4089, 5, 77]), (1, [0]), (40, range(40)),
                     (1, [0]), (1, [0]), (1, [0, 0]), (1, [])]:
@@ -92,7 +92,7 @@ def test_recorded_by_the_caller(lib, places):
 
 
 def test_one_recording_per_slot(lib):
-    """Whatever is asked of a slot's one-token steps, and wherever the pinned memory lies, one recording gives the bits of launched steps; few outlive the
+    """Whatever is asked of a slot's one-token steps, one recording gives the bits of launched steps; few outlive the
     engine's slots."""
     cfg = hm.config(5000, 64, [hm.layer("retention", hm.retention(2, 16, 16, 16, [0.5, 0.98]), 33), hm.layer("latent_attention", hm.latent(2, 16, 8, 16, 24, 20, 0.3))])
     w, toks = hm.weights(cfg, 5), hm.tokens(cfg, 40, 6)
@@ -107,7 +107,7 @@ def test_one_recording_per_slot(lib):
         else:
             got = m.step(a, toks[t:t + 1], [0], t % 3 == 1)
         assert np.array_equal(got[1], ref[1]) and (got[0] is None or np.array_equal(got[0].view(np.uint32), ref[0].view(np.uint32))), t
-        if t == 10:         # the pinned memory grows under both recordings
+        if t == 10:
             for s in held:
                 assert np.array_equal(*(x.step(q, toks[24:40], range(16))[0] for x, q in zip((m, plain), s)))
         assert lib.bpdq_hybrid_recordings(m.plan) <= 2
