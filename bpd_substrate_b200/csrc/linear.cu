@@ -381,25 +381,25 @@ k_linear_tc5(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
 
     if (warp == 0 || warp == 2) {
         // ---------------- copies: a warp for the weights, which do not wait for the launch ahead, one for the tokens.  (One thread for both took 470
-        // cycles between two K blocks, mostly its own chain of instructions, and bounded tiles of up to 200 tokens.)
+        // cycles between two K blocks, mostly its own chain of instructions, and bounded tiles of up to 200 tokens.  A look at the next barrier ahead of time, by
+        // which the issuing thread gains, is one answer more to wait for here: 32 tokens of 1024 x 1024 5.65 us, 5.28 without; 200 of 2048 x 2048 8.15, 7.82.)
         if (lane == 0) {
             const bool tokens = warp == 2;
             const uint32_t to0 = smem_addr(ring) + (tokens ? kTc5ABytes : 0), bytes = (uint32_t)(tokens ? own * kTc5Depth * 2 : kTc5ABytes);
             const uint32_t full0 = smem_addr(full), empty0 = smem_addr(empty), lead0 = kPair ? leader_addr(full) : full0;
             const CUtensorMap* map = tokens ? &xmap : &wmap;
             if (tokens) pdl_wait();
-            uint32_t s = 0, par = 1;        // (the first round's waits pass)
-            bool ok = true, ready = true;
+            uint32_t s = 0, par = 1;
+            bool ok = true, first = true;       // (the ring's first round waits for nothing)
             for (int tile = unit; ok && tile < tiles; tile += units) {
                 const int y = tokens ? (tile % t_tiles) * bn + rank * own : (tile / t_tiles) * kTileRows + rank * kTc5Rows;
                 int x = kb0 * kTc5Depth;
                 for (int kb = 0; kb < kb_n; kb++, x += kTc5Depth) {
-                    if (!ready && !mbar_wait_at(empty0 + 8 * s, par, err, 41)) { ok = false; break; }
+                    if (!first && !mbar_wait_at(empty0 + 8 * s, par, err, 41)) { ok = false; break; }
                     if (!kPair || rank == 0) mbar_expect_tx_at(full0 + 8 * s, kCtas * bytes);
                     if (kPair) tma_pair_rows_2d_at(to0 + s * stage_bytes, map, x, y, lead0 + 8 * s);
                     else tma_rows_2d_at(to0 + s * stage_bytes, map, x, y, full0 + 8 * s);
-                    if (++s == (uint32_t)stages) { s = 0; par ^= 1u; }
-                    ready = mbar_test_at(empty0 + 8 * s, par);
+                    if (++s == (uint32_t)stages) { s = 0; par ^= 1u; first = false; }
                 }
             }
         }
@@ -552,11 +552,11 @@ static int launch_tc5(const Linear& l, int T, Tc5Tiles t, cudaStream_t s)
 
 // Tokens of a tile (a multiple of 16), ranges of K and CTAs of a tile with the least time in cycles: waves of CTAs over the SMs times a tile's K blocks, each
 // 310 + 1.3 per token; K is cut, into ranges of at least four blocks, where all its tiles' clusters run at once, and joining r ranges costs
-// 3000 + 800 r + 25 per token.  168 K blocks of 2048 rows take 28.2 us at 16 tokens a tile, 29.7 at 128, 36.5 at 160, 53.4 at 256 (320, 340, 415, 605 cycles a
+// 3000 + 800 r + 25 per token.  168 K blocks of 2048 rows take 29.2 us at 16 tokens a tile, 30.9 at 128, 34.6 at 160, 53.6 at 256 (335, 355, 395, 615 cycles a
 // block: the estimate, which was fitted to one copying thread and eight epilogue warps, is high around 128 tokens).  Over 37 shapes of 5 to 4096 tokens
-// its tiles are within 4 % of the best ones, but for 128 tokens of 4096 x 4096 (12.3 us, 11.2 possible) and 400 of 1024 x 4096 (11.7, 11.0).
-// 2048 rows of 10752 (us, one range, several): 48 tokens 28.7, 11.5 at six; 200 tokens 29.2, 16.8 at four; of 2048: 16 tokens 8.2, 6.9 at four; 200 tokens
-// 8.5, 8.7 at two.
+// its tiles are within 5 % of the best ones, but for 128 tokens of 4096 x 4096 (12.2 us, 11.1 possible) and 400 of 1024 x 4096 (11.6, 10.8).
+// 2048 rows of 10752 (us, one range, several): 48 tokens 29.6, 11.3 at six; 200 tokens 30.1, 16.6 at four; of 2048: 16 tokens 7.9, 6.7 at four; 200 tokens
+// 8.2, 8.6 at two.
 static Tc5Tiles tc5_tiles(const Linear& l, int T)
 {
     const int n_tiles = (l.N + kTc5Rows - 1) / kTc5Rows, top = (T + 15) / 16 * 16 < 256 ? (T + 15) / 16 * 16 : 256;
@@ -574,7 +574,7 @@ static Tc5Tiles tc5_tiles(const Linear& l, int T)
     }
     // A pair has 256 rows to a tile and fetches a third less per product; a K block takes 180 + 1.65 per token (168 of 2048 rows, 700 tokens, us: 128
     // tokens a tile 36, 192 43, 256 56).  Setting it up costs more than one CTA, so only wide tiles and several waves: us, best single CTAs, pairs:
-    // 2048 tokens of 10752 x 2048 82.8, 79.8; of 21504 x 2048 165, 157; 1024 of 14336 x 4096 115, 105; 2048 of 2048 x 2048 15.7, 17.8.
+    // 2048 tokens of 10752 x 2048 81.2, 78.8; of 21504 x 2048 172, 161; 1024 of 14336 x 4096 111, 99; 2048 of 2048 x 2048 16.0, 17.9.
     const int pairs = sms / 2, row_pairs = (l.N + 2 * kTc5Rows - 1) / (2 * kTc5Rows);
     for (int bn = 192; bn <= top; bn += 32) {
         const long waves = ((long)row_pairs * ((T + bn - 1) / bn) + pairs - 1) / pairs;
