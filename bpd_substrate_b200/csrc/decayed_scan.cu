@@ -690,7 +690,7 @@ static int launch_conv(const void* in, int ld_in, void* out, int channels, int t
     // loads of 8 bytes (of 16, 2048 tokens of 6144 fp32 channels 24.0 us, 20.5 so); more channels at a time where windows are read again and again
     constexpr int kMost = sizeof(A) == 2 ? 4 : 2;
     if ((kMost == 4 || taps > 4) && channels % 4 == 0 && ld_in % 4 == 0 && acts % (4 * sizeof(A)) == 0 && floats % 16 == 0) rc = launch(k_causal_conv<A, 4>, 4);
-    else if (channels % 2 == 0 && ld_in % 2 == 0 && acts % (2 * sizeof(A)) == 0) rc = launch(k_causal_conv<A, 2>, 2);
+    else if (channels % 2 == 0 && ld_in % 2 == 0 && acts % (2 * sizeof(A)) == 0 && floats % 8 == 0) rc = launch(k_causal_conv<A, 2>, 2);
     else rc = launch(k_causal_conv<A, 1>, 1);
     if (rc || taps < 2) return rc;
     return launch_ordered(k_conv_tail<A>, (channels + 127) / 128, 128, 0, s, (const A*)in, ld_in, channels, taps, tail, T);
@@ -870,7 +870,8 @@ static int launch_gated_norm(const A* o, int ld_o, const A* g, int ld_g, const f
                              int parts, int form, float eps, int T, cudaStream_t s)
 {
     const int part = heads * value_dim / parts;
-    const bool vec = value_dim == value_pad && part % 4 == 0 && ld_o % 4 == 0 && ld_g % 4 == 0 && ld_y % 4 == 0;
+    const bool vec = value_dim == value_pad && part % 4 == 0 && ld_o % 4 == 0 && ld_g % 4 == 0 && ld_y % 4 == 0 &&
+                     !(((uintptr_t)o | (uintptr_t)g | (uintptr_t)y) % (4 * sizeof(A))) && (form == kNormThenGate || !((uintptr_t)w & 15));
     // A single token has few parts: spread one over the CTA's warps, with loads of few channels so that all of them have some.
     if (vec && (long)T * parts <= 64) {
         if (part <= 1024) return launch_gated_vec<A, 8, 1, 4>(o, ld_o, g, ld_g, w, y, ld_y, part, parts, form, eps, T, s);

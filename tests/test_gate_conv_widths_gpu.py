@@ -87,3 +87,29 @@ def test_causal_conv_tiles(lib, dtype, T, channels, taps, offset):
 def test_gated_norm_narrow_loads(lib, dtype, T, parts, part, offset):
     for form in (0, 1, 2):
         test_gated_norm(lib, dtype, T, parts, part, offset, form)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T,part,offset", [(70, 256, 1), (70, 512, 2), (3, 1024, 1), (65, 4096, 3)])
+def test_gated_norm_anywhere(lib, dtype, T, part, offset):
+    """Rows that begin where no load of several channels may."""
+    for form in (0, 1, 2):
+        test_gated_norm(lib, dtype, T, 1, part, offset, form)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T,channels,taps,offset", [(23, 512, 4, 1), (9, 514, 4, 2), (23, 512, 6, 1), (40, 130, 3, 3)])
+def test_causal_conv_floats_anywhere(lib, dtype, T, channels, taps, offset):
+    """Weights, biases and window at any float."""
+    rng = np.random.default_rng(T + channels)
+    x = acts(rng, T, channels, dtype, 0)
+    w, b, tail = (acts(rng, 1, n, torch.float32, offset).view(-1, channels) for n in (taps * channels, channels, (taps - 1) * channels))
+    old, y = tail.clone(), torch.full((T, channels), float("nan"), dtype=dtype, device="cuda")
+    torch.cuda.synchronize()
+    assert lib.bpd_causal_conv_silu_cuda(x.data_ptr(), channels, y.data_ptr(), T, channels, taps, w.data_ptr(), b.data_ptr(), tail.data_ptr(),
+                                         int(dtype == torch.bfloat16), None) == 0
+    torch.cuda.synchronize()
+    seen = torch.cat([old.double(), x.double()])
+    a = b.double() + sum(w[j].double() * seen[j:j + T] for j in range(taps))
+    close(y, a * sigmoid(a), dtype)
+    assert torch.equal(tail.double(), seen[T:])
